@@ -297,7 +297,7 @@ class KernelSet:
         return dim * vdim + -(-vdim // 32) * (-(-(dim + 1) // 4) * 4)
 
     def delta_scan(self, x, out, batch, state, *, heads, kv_heads, dim, vdim, columns, a_log, dt_bias, q_scale,
-                   unit_eps=1e-6, state_offset=0, split_rows=None):
+                   unit_eps=1e-6, state_offset=0, split_rows=None, chunked=None):
         """The gated delta rule, token by token, for every segment of the step from the matrix its request's slot holds
         (zeros: the start of a sequence); the slot receives the matrix after the segment's last token.  x float32 [M, *]
         holds, from the columns `columns` = (q, k, v, b, a) on, q and k [kv_heads * dim], v [heads * vdim] and two
@@ -306,7 +306,8 @@ class KernelSet:
         k <- k / sqrt(|k|^2 + unit_eps), q <- q / sqrt(|q|^2 + unit_eps) * q_scale, beta = sigmoid(b),
         g = exp(-exp(a_log[h]) * softplus(a + dt_bias[h])); S <- g S; u = beta (v - S^T k); S <- S + k u^T; out = S^T q.
         All float32.  `split_rows`: more lanes share a value column's key rows (the same sums in another order; for steps
-        with long segments); None leaves the choice to the kernel set."""
+        with long segments); `chunked`: long segments go 32 tokens at a time (the same sums in another order).  None leaves
+        the choice to the kernel set."""
         raise NotImplementedError
 
     @staticmethod

@@ -300,6 +300,13 @@ class CudaKernels(KernelSet):
         # Scout shapes, one token 2.90 ms with (110 KiB, 2 per multiprocessor) against 3.01 with (74 KiB, 3), eight
         # tokens 7.10 against 7.02, sixty-four alike; one block per multiprocessor with 110 or 200 KiB: 3.2 and 3.1 ms
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
+        # Recurrences over prompts: segments of at least so many tokens go in chunks of 32 on the tensor cores, the others token by
+        # token.  Delta rule, 16 heads of 128 x 128, us in chunks / token by token: one prompt of 32 tokens 21 / 24, 64:
+        # 23 / 42, 512: 52 / 291, 2,048: 170 / 1,147; sixteen prompts of 16: 59 / 52, of 32: 61 / 95.
+        self.chunk_min_tokens = 32
+        # how much working memory a call may take for that (a step of 8,192 tokens of 32 heads of 128 x 128 takes 0.45 GB); a call that
+        # would need more goes token by token
+        self.chunk_scratch_limit = 1 << 30
         # arrival counters of the splits (zero between calls), one set per stream, since calls that share a set must not
         # overlap.  The sets are made ahead: one made while a CUDA graph is captured would lie in the graphs' memory
         # pool, where a graph captured before keeps its temporaries.
@@ -1180,8 +1187,15 @@ class CudaKernels(KernelSet):
         self._count("recurrent", 2 if chunked else 1)
         _check(st, "mlstm_scan")
 
+    def _chunk_scratch(self, library, query, *sizes):
+        """Working memory of a walk in chunks, or None: sizes that it does not take, or more memory than the limit."""
+        f = getattr(self._lib(library), query)
+        f.restype = C.c_longlong
+        need = f(*(int(n) for n in sizes))
+        return torch.empty(need, dtype=torch.uint8, device=self.device) if 0 < need <= self.chunk_scratch_limit else None
+
     def delta_scan(self, x, out, batch, state, *, heads, kv_heads, dim, vdim, columns, a_log, dt_bias, q_scale,
-                   unit_eps=1e-6, state_offset=0, split_rows=None):
+                   unit_eps=1e-6, state_offset=0, split_rows=None, chunked=None):
         self._t(x, torch.float32, "x"); self._t(out, torch.float32, "out"); self._t(state, torch.float32, "state")
         self._t(a_log, torch.float32, "a_log"); self._t(dt_bias, torch.float32, "dt_bias")
         M = x.shape[0]
@@ -1200,12 +1214,25 @@ class CudaKernels(KernelSet):
                         cu_seqlens=batch.cu_seqlens.data_ptr(), slots=batch.slots.data_ptr(),
                         n_segments=batch.cu_seqlens.numel() - 1, heads=int(heads), kv_heads=int(kv_heads), dim=int(dim),
                         vdim=int(vdim), q_scale=float(q_scale), unit_eps=float(unit_eps), gates=gates.data_ptr(), n_tokens=M)
+        n_seg = batch.cu_seqlens.numel() - 1
+        if chunked is None:
+            # Prompts and their portions go 32 tokens at a time.  The float32 set keeps the walk token by token for every step,
+            # so that its results do not depend on how a prompt was cut, to the last bit.
+            chunked = split_rows is None and self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_min_tokens
+        if chunked:
+            n_chunks = (M + 31) // 32 + n_seg
+            scratch = self._chunk_scratch("delta", "spite_delta_chunk_bytes", dim, vdim, heads, kv_heads, M, n_chunks, n_seg)
+            if scratch is not None:
+                st = self._lib("delta").spite_delta_scan_chunked(C.byref(p), C.c_void_p(scratch.data_ptr()), n_chunks, self.chunk_min_tokens,
+                                                                 self._stream())
+                self._count("delta", 3)
+                _check(st, "delta_scan")
+                return
         if split_rows is None:
             # A warp on eight value columns (whole sectors of the state per row) serves every step.  More lanes a column
             # and fewer columns a block was measured and is no faster: the walk's time is the length of its chain per token
             # (a barrier, the sums, the shuffles), not the multiply-adds (2,048 tokens of 16 heads of 128 x 128: 1.73 ms
-            # against 2.05 ms; eight such prompts 3.48 against 3.98 ms).  One form for every step also keeps the float32
-            # set's results independent of how a prompt was cut, to the last bit.
+            # against 2.05 ms; eight such prompts 3.48 against 3.98 ms).
             split_rows = False
         st = self._lib("delta").spite_delta_scan(C.byref(p), C.c_int(int(bool(split_rows))), self._stream())
         self._count("delta", 2)
