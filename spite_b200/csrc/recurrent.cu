@@ -14,7 +14,7 @@
 // them (RPL rows a lane), so the sums over the key rows are warp shuffles and no block-wide barrier stands in the
 // token loop.  The next token's inputs are loaded while the current one is worked on.  A decoded token costs one
 // read and one write of the state (a lane moves 8 consecutive floats of a key row: whole 32-byte sectors).
-#include "common.cuh"
+#include "chunk.cuh"
 
 struct MlstmParams {
     const float* proj;          // [tokens, stride]: the projection's float32 output
@@ -43,7 +43,7 @@ constexpr int COLS_PER_BLOCK = 32;
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
 template <int RPL>
-__global__ void __launch_bounds__(128) mlstm_scan_kernel(const MlstmParams p) {
+__global__ void __launch_bounds__(128) mlstm_scan_kernel(const MlstmParams p, const chunk::Leftovers left) {
     pdl_wait();
     pdl_launch_dependents();
     const int seg = blockIdx.z, head = blockIdx.y;
@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(128) mlstm_scan_kernel(const MlstmParams p) {
     const int t0 = p.cu_seqlens[seg], t1 = p.cu_seqlens[seg + 1];
     const int dim = p.dim, vdim = p.vdim;
     if (t0 >= t1) return;
+    // (the walk in chunks leaves whole blocks of 32 columns)
+    if (chunk::left_over(left, p.cu_seqlens, seg, head, p.heads, blockIdx.x * COLS_PER_BLOCK, COLS_PER_BLOCK) == chunk::NOTHING) return;
     const int slot = p.slots[seg];
     // A captured step pads its rows with copies of its first row: a copy would update the first row's state a second
     // time.  It leaves zeros instead (its results are never read).
@@ -577,9 +579,186 @@ int launch_mlstm_chunk(const MlstmParams& p, float* scratch, int scratch_chunks,
     return spite_launch_status();
 }
 
-}  // namespace
+// ---- the same in chunks of 32 tokens on the tensor cores (chunk.cuh), for up to 256 key rows.  What a chunk needs that does not depend on
+// the state, one block a (chunk, head): q and k as split tiles; a_s, F_t and the running maximum M_t of a_s within the chunk (m0
+// joins in the walk: max(m0, M_t)); the scores exp(a_s - M_t) q_t . k_s (s <= t) as a split tile, and their sums over s; the weights
+// exp(a_s - M_last) and sum_s of them times k_s, which n takes.
+template <int DP> struct MemoryChunkSmem {
+    __half qk[4][chunk::CT * DP];
+    float P[chunk::CT][36], kn[8][DP], w[chunk::CT];
+    double a[chunk::CT], M[chunk::CT];
+    unsigned largest[3], bad;                             // of q, k and the scores
+};
 
-static int mlstm_scan_launch(const MlstmParams* p, float* scratch, int scratch_chunks, void* stream) {
+template <int DP>
+__global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, const chunk::Made out) {
+    using namespace chunk;
+    constexpr int CL = chunk::CT;
+    using Rec = Record<MATRIX_MEMORY, DP>;
+    extern __shared__ __align__(16) unsigned char smem_bytes[];
+    auto& sm = *reinterpret_cast<MemoryChunkSmem<DP>*>(smem_bytes);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, head = blockIdx.y;
+    pdl_wait();
+    pdl_launch_dependents();
+    int seg, first;
+    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
+    if (first == p.cu_seqlens[seg]) clear_marks(out.columns, out.column_groups, seg, head, p.heads, tid, 256);
+    if (p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens) return;
+    const int len = min(CL, p.cu_seqlens[seg + 1] - first), dim = p.dim;
+    const float* rows = p.proj + (size_t)first * p.stride;
+    const size_t at_head = (size_t)blockIdx.x * p.heads + head;
+    float* rec = out.records + at_head * Rec::FLOATS;
+    if (tid < 3) sm.largest[tid] = 0;
+    if (tid == 3) sm.bad = 0;
+
+    // a warp has the tokens warp, warp + 8, ..., a lane the elements lane, lane + 32, ...
+    constexpr int E = DP / 32;
+    float kv[4][E], qv[4][E];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = warp + 8 * i;
+        const float* row = rows + (size_t)t * p.stride + head * dim;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int d = lane + 32 * e;
+            const bool on = t < len && d < dim;
+            kv[i][e] = on ? row[p.k_col + d] : 0.f;
+            qv[i][e] = on ? row[p.q_col + d] : 0.f;
+        }
+    }
+    bool bad = false;
+    if (warp == 0) {
+        const bool on = lane < len;
+        const float bi = p.i_bias ? p.i_bias[head] : 0.f, bf = p.f_bias ? p.f_bias[head] : 0.f;
+        const float cap = p.gate_cap, inv_cap = 1.0f / p.gate_cap;
+        float ig = 0.f, fg = 0.f;
+        if (on) {
+            ig = cap * tanhf((rows[(size_t)lane * p.stride + p.i_col + head] + bi) * inv_cap);
+            fg = log_sigmoid(cap * tanhf((rows[(size_t)lane * p.stride + p.f_col + head] + bf) * inv_cap));
+            bad = !(fabsf(ig) < 3e38f) || !(fabsf(fg) < 3e38f);
+        }
+        const double F = prefix_sum((double)fg, lane), a = on ? (double)ig - F : -1.0e300;
+        const double M = prefix_max(a, lane), M_last = __shfl_sync(0xffffffffu, M, len - 1);
+        const float w = on ? expf((float)(a - M_last)) : 0.f;
+        sm.a[lane] = a; sm.M[lane] = M; sm.w[lane] = w;
+        double* md = reinterpret_cast<double*>(rec);
+        md[lane] = M; md[CL + lane] = F;
+        rec[Rec::W + lane] = w;
+    }
+    unsigned lq = 0, lk = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) { lq = max(lq, abs_bits(qv[i][e])); lk = max(lk, abs_bits(kv[i][e])); }
+    lq = __reduce_max_sync(0xffffffffu, lq);
+    lk = __reduce_max_sync(0xffffffffu, lk);
+    __syncthreads();
+    if (lane == 0) { atomicMax(&sm.largest[0], lq); atomicMax(&sm.largest[1], lk); }
+    __syncthreads();
+    const Scale sq = scale_of(sm.largest[0]), sk = scale_of(sm.largest[1]);
+    bad |= max(sm.largest[0], sm.largest[1]) >= 0x7f800000u;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = warp + 8 * i, at = tile_at<DP>(t, lane + 32 * e);
+            split1(qv[i][e] * sq.up, sm.qk[0][at], sm.qk[1][at]);
+            split1(kv[i][e] * sk.up, sm.qk[2][at], sm.qk[3][at]);
+            sum = fmaf(sm.w[t], kv[i][e], sum);
+        }
+        sm.kn[warp][lane + 32 * e] = sum;
+    }
+    __syncthreads();
+    // ---- q_t . k_s: a warp has sixteen tokens t and eight tokens s
+    {
+        const int m = warp & 1, n = warp >> 1;
+        float main[4] = {}, cross[4] = {};
+        if (n < 2 || m == 1) {
+#pragma unroll 4
+            for (int k = 0; k < DP / 16; k += 2) {
+                unsigned bh[4], bl[4], ah[4], al[4];
+                ldsm(bh, sm.qk[2] + tile_at<DP>(8 * n + (lane & 7), 16 * k + 8 * (lane >> 3)));
+                ldsm(bl, sm.qk[3] + tile_at<DP>(8 * n + (lane & 7), 16 * k + 8 * (lane >> 3)));
+                ldsm_left<DP>(ah, sm.qk[0], 16 * m, 16 * k, lane);
+                ldsm_left<DP>(al, sm.qk[1], 16 * m, 16 * k, lane);
+                mma3(main, cross, ah, al, bh[0], bh[1], bl[0], bl[1]);
+                ldsm_left<DP>(ah, sm.qk[0], 16 * m, 16 * k + 16, lane);
+                ldsm_left<DP>(al, sm.qk[1], 16 * m, 16 * k + 16, lane);
+                mma3(main, cross, ah, al, bh[2], bh[3], bl[2], bl[3]);
+            }
+        }
+        unsigned largest = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 16 * m + g + 8 * (i >> 1), s = 8 * n + 2 * t4 + (i & 1);
+            const float x = s <= t ? (main[i] + cross[i]) * sq.down * sk.down * expf((float)(sm.a[s] - sm.M[t])) : 0.f;
+            sm.P[t][s] = x;
+            largest = max(largest, abs_bits(x));
+        }
+        largest = __reduce_max_sync(0xffffffffu, largest);
+        if (lane == 0) atomicMax(&sm.largest[2], largest);
+        if (bad) sm.bad = 1;
+    }
+    __syncthreads();
+    {   // a thread has a token and four tokens s
+        const int t = tid >> 3, s = 4 * (tid & 7);
+        const Scale sp = scale_of(sm.largest[2]);
+        const float4 x = *(const float4*)&sm.P[t][s];
+        float sum = (x.x + x.y) + (x.z + x.w);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        if ((tid & 7) == 0) rec[Rec::SUMS + t] = sum;
+        uint2 h, l;
+        split2(x.x * sp.up, x.y * sp.up, h.x, l.x);
+        split2(x.z * sp.up, x.w * sp.up, h.y, l.y);
+        __half* scores = out.scores + at_head * (2 * CL * CL) + score_at(t, s);
+        *(uint2*)scores = h;
+        *(uint2*)(scores + CL * CL) = l;
+        if (tid < 8)
+            rec[Rec::SCALARS + tid] = tid == Q_DOWN ? sq.down : tid == K_DOWN ? sk.down : tid == P_DOWN ? sp.down
+                                    : tid == BAD ? (sm.bad || sm.largest[2] >= 0x7f800000u ? 1.f : 0.f) : 0.f;
+    }
+    for (int d = tid; d < DP; d += 256) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += sm.kn[i][d];
+        rec[Rec::KEYS + d] = sum;
+    }
+    uint4* dst = reinterpret_cast<uint4*>(out.qk + at_head * (4 * CL * DP));
+    const uint4* src = reinterpret_cast<const uint4*>(sm.qk[0]);
+#pragma unroll 4
+    for (int e = tid; e < 4 * CL * DP / 8; e += 256) dst[e] = src[e];
+}
+
+template <int DP> constexpr int memory_record() { return chunk::Record<chunk::MATRIX_MEMORY, DP>::FLOATS; }
+inline int memory_dp(int dim) { return dim <= 64 ? 64 : dim <= 128 ? 128 : 256; }
+inline chunk::Layout memory_layout(int dim, int vdim, int heads, int n_chunks, int n_segments) {
+    const int dp = memory_dp(dim);
+    return chunk::layout_of(dp, dp == 64 ? memory_record<64>() : dp == 128 ? memory_record<128>() : memory_record<256>(), heads, heads, vdim,
+                            n_chunks, n_segments, false, 0);
+}
+
+template <int DP, int KPW>
+int launch_memory_chunks(const MlstmParams& p, const chunk::Made& out, int n_chunks, cudaStream_t st) {
+    auto prep = memory_chunk_kernel<DP>;
+    if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MemoryChunkSmem<DP>)) != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    SPITE_LAUNCH(prep, dim3(n_chunks, p.heads), 256, sizeof(MemoryChunkSmem<DP>), st, p, out);
+    if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    chunk::Walk w = chunk::walk_of(out);
+    w.v = p.proj + p.v_col; w.v_stride = p.stride;
+    w.out = p.out; w.out_stride = (long long)p.heads * p.vdim;
+    w.state = p.state; w.slot_stride = (long long)p.heads * p.head_stride; w.head_stride = p.head_stride;
+    w.key_stride = p.vdim; w.col_stride = 1;
+    w.n_offset = (long long)p.dim * p.vdim; w.n_stride = (p.dim + 1 + 3) & ~3;
+    w.cu_seqlens = p.cu_seqlens; w.slots = p.slots;
+    w.n_segments = p.n_segments; w.heads = p.heads; w.qk_heads = p.heads; w.dim = p.dim; w.vdim = p.vdim;
+    w.out_scale = p.q_scale;
+    return chunk::launch_walk<KPW, DP / KPW, 2, chunk::MATRIX_MEMORY>(w, st);
+}
+
+int check_mlstm(const MlstmParams* p) {
     if (!p || !p->proj || !p->out || !p->state || !p->cu_seqlens || !p->slots) return SPITE_BAD_ARG;
     if (p->n_segments < 0 || p->heads < 1 || p->dim < 1 || p->vdim < 1 || !(p->gate_cap > 0.f) || !(p->q_scale == p->q_scale))
         return SPITE_BAD_ARG;
@@ -588,24 +767,35 @@ static int mlstm_scan_launch(const MlstmParams* p, float* scratch, int scratch_c
     if (p->stride < need) return SPITE_BAD_ARG;
     if (p->dim > 512) return SPITE_UNSUPPORTED;
     if (p->heads > 65535 || p->n_segments > 65535) return SPITE_UNSUPPORTED;
-    if (p->n_segments == 0) return SPITE_OK;
     const long long col_blocks = (p->vdim + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK;
-    if (p->head_stride < (long long)p->dim * p->vdim + col_blocks * ((p->dim + 1 + 3) & ~3)) return SPITE_BAD_ARG;
+    if (p->n_segments && p->head_stride < (long long)p->dim * p->vdim + col_blocks * ((p->dim + 1 + 3) & ~3)) return SPITE_BAD_ARG;
+    return SPITE_OK;
+}
+
+int launch_mlstm_scan(const MlstmParams* p, const chunk::Leftovers& left, cudaStream_t st) {
     dim3 grid((p->vdim + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK, p->heads, p->n_segments);
-    cudaStream_t st = (cudaStream_t)stream;
-    if (p->chunked) {
-        if (!scratch || scratch_chunks < 1 || (((uintptr_t)scratch) & 15)) return SPITE_BAD_ARG;
-        if (p->dim <= 64) return launch_mlstm_chunk<1>(*p, scratch, scratch_chunks, grid, st);
-        if (p->dim <= 128) return launch_mlstm_chunk<2>(*p, scratch, scratch_chunks, grid, st);
-        if (p->dim <= 256) return launch_mlstm_chunk<4>(*p, scratch, scratch_chunks, grid, st);
-        return launch_mlstm_chunk<8>(*p, scratch, scratch_chunks, grid, st);
-    }
-    if (p->dim <= 32) SPITE_LAUNCH(mlstm_scan_kernel<1>, grid, 128, 0, st, *p);
-    else if (p->dim <= 64) SPITE_LAUNCH(mlstm_scan_kernel<2>, grid, 128, 0, st, *p);
-    else if (p->dim <= 128) SPITE_LAUNCH(mlstm_scan_kernel<4>, grid, 128, 0, st, *p);
-    else if (p->dim <= 256) SPITE_LAUNCH(mlstm_scan_kernel<8>, grid, 128, 0, st, *p);
-    else SPITE_LAUNCH(mlstm_scan_kernel<16>, grid, 128, 0, st, *p);
+    if (p->dim <= 32) SPITE_LAUNCH(mlstm_scan_kernel<1>, grid, 128, 0, st, *p, left);
+    else if (p->dim <= 64) SPITE_LAUNCH(mlstm_scan_kernel<2>, grid, 128, 0, st, *p, left);
+    else if (p->dim <= 128) SPITE_LAUNCH(mlstm_scan_kernel<4>, grid, 128, 0, st, *p, left);
+    else if (p->dim <= 256) SPITE_LAUNCH(mlstm_scan_kernel<8>, grid, 128, 0, st, *p, left);
+    else SPITE_LAUNCH(mlstm_scan_kernel<16>, grid, 128, 0, st, *p, left);
     return spite_launch_status();
+}
+
+}  // namespace
+
+static int mlstm_scan_launch(const MlstmParams* p, float* scratch, int scratch_chunks, void* stream) {
+    const int chk = check_mlstm(p);
+    if (chk != SPITE_OK) return chk;
+    if (p->n_segments == 0) return SPITE_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!p->chunked) return launch_mlstm_scan(p, chunk::Leftovers{}, st);
+    if (!scratch || scratch_chunks < 1 || (((uintptr_t)scratch) & 15)) return SPITE_BAD_ARG;
+    dim3 grid((p->vdim + COLS_PER_BLOCK - 1) / COLS_PER_BLOCK, p->heads, p->n_segments);
+    if (p->dim <= 64) return launch_mlstm_chunk<1>(*p, scratch, scratch_chunks, grid, st);
+    if (p->dim <= 128) return launch_mlstm_chunk<2>(*p, scratch, scratch_chunks, grid, st);
+    if (p->dim <= 256) return launch_mlstm_chunk<4>(*p, scratch, scratch_chunks, grid, st);
+    return launch_mlstm_chunk<8>(*p, scratch, scratch_chunks, grid, st);
 }
 
 SPITE_API int spite_mlstm_scan(const MlstmParams* p, void* stream) {
@@ -617,4 +807,28 @@ SPITE_API int spite_mlstm_scan(const MlstmParams* p, void* stream) {
 // chunks, the sum over the segments of ceil(tokens / 32).  Takes p->chunked as it is given.
 SPITE_API int spite_mlstm_scan_chunked(const MlstmParams* p, float* scratch, int scratch_chunks, void* stream) {
     return mlstm_scan_launch(p, scratch, scratch_chunks, stream);
+}
+
+// Bytes of working memory that `spite_mlstm_scan_tiles` needs for a step of `n_chunks` chunks of 32 tokens; -2: sizes that it does not take.
+SPITE_API long long spite_mlstm_tiles_bytes(int dim, int vdim, int heads, int n_chunks, int n_segments) {
+    if (dim < 1 || vdim < 1 || heads < 1 || n_chunks < 0 || n_segments < 0) return SPITE_BAD_ARG;
+    if (dim > 256) return SPITE_UNSUPPORTED;
+    return memory_layout(dim, vdim, heads, n_chunks, n_segments).bytes;
+}
+
+// Segments of at least `min_tokens` tokens in chunks of 32 on the tensor cores, the others token by token.
+SPITE_API int spite_mlstm_scan_tiles(const MlstmParams* p, void* scratch, int n_chunks, int min_tokens, void* stream) {
+    const int chk = check_mlstm(p);
+    if (chk != SPITE_OK) return chk;
+    if (!scratch || ((uintptr_t)scratch & 15) || n_chunks < 1 || min_tokens < 1) return SPITE_BAD_ARG;
+    if (p->dim > 256) return SPITE_UNSUPPORTED;
+    if (p->n_segments == 0) return SPITE_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int dp = memory_dp(p->dim);
+    const chunk::Layout l = memory_layout(p->dim, p->vdim, p->heads, n_chunks, p->n_segments);
+    const chunk::Made out = chunk::made_at(scratch, l, min_tokens);
+    const int rc = dp == 64 ? launch_memory_chunks<64, 32>(*p, out, n_chunks, st) : dp == 128 ? launch_memory_chunks<128, 32>(*p, out, n_chunks, st)
+                                                                                            : launch_memory_chunks<256, 64>(*p, out, n_chunks, st);
+    if (rc != SPITE_OK) return rc;
+    return launch_mlstm_scan(p, chunk::leftovers_of(out, l, p->heads, chunk::Record<chunk::MATRIX_MEMORY, 64>::SCALARS), st);
 }

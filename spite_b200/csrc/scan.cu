@@ -21,7 +21,12 @@
 //
 // The slot holds S transposed: value column j's keys are contiguous, [vdim, dim4] with dim4 = dim rounded up to a multiple
 // of four (the padding stays zero), so that a lane's rows are whole 16-byte groups and a warp's loads whole lines.
-#include "common.cuh"
+//
+// Prompts and their portions go 32 tokens at a time on the tensor cores (chunk.cuh), for up to 128 keys.  With b_t the sum of a chunk's
+// log decays up to token t: the scores P[t, s] = (q_t . k_s) e^(b_t - b_s) dt_s (s <= t) where one number a head decays, and
+// sum_i q_ti k_si e^(b_ti - b_si) where every key channel does; the operands Q, K of the second kind carry e^(b_t) and e^(b_last - b_s).
+// No exponent is ever positive.  The kernels below make these for all chunks and heads of a step at once.
+#include "chunk.cuh"
 
 struct ScanParams {
     const float* q; const float* k; const float* v;       // first element of token 0's q, k [kv_heads * dim], v [heads * vdim]
@@ -38,6 +43,8 @@ struct ScanParams {
 };
 
 namespace {
+
+using namespace chunk;
 
 typedef unsigned long long f2;                            // two packed floats
 
@@ -58,17 +65,6 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
     return r;
 }
 
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 constexpr int RING = 4;
 
 constexpr int MAX_WARPS = 4;                              // walking warps a block
@@ -77,7 +73,7 @@ constexpr int MAX_WARPS = 4;                              // walking warps a blo
 enum Walk { PER_HEAD = 0, PER_CHANNEL_BONUS = 1, PER_CHANNEL = 2 };
 
 template <int LR, int RPV, int CC, int TB, int WALK>
-struct Shape {
+struct WalkShape {
     static constexpr bool CH = WALK != PER_HEAD;          // a decay per key channel
     static constexpr bool SCALARS = WALK != PER_CHANNEL;  // a token brings scalars
     static constexpr int DP = LR * RPV * 4;               // key rows a warp covers
@@ -124,9 +120,9 @@ struct Bringer {
             float* d = stage + dst[s];
             if (n == TB) {
 #pragma unroll
-                for (int tt = 0; tt < TB; ++tt) { cp_async16(d + tt * SH::TOKEN, src[s]); src[s] += stride[s]; }
+                for (int tt = 0; tt < TB; ++tt) { copy16(d + tt * SH::TOKEN, src[s]); src[s] += stride[s]; }
             } else {
-                for (int tt = 0; tt < n; ++tt) { cp_async16(d + tt * SH::TOKEN, src[s]); src[s] += stride[s]; }
+                for (int tt = 0; tt < n; ++tt) { copy16(d + tt * SH::TOKEN, src[s]); src[s] += stride[s]; }
             }
         }
     }
@@ -143,19 +139,19 @@ __device__ __forceinline__ void bring_elements(const ScanParams& p, const float*
         float* d = stage + tt * SH::TOKEN;
         const long long t = tb + tt;
         for (int e = lane; e < dim; e += 32) {
-            cp_async4(d + e, qp + t * p.q_stride + e);
-            cp_async4(d + SH::DP + e, kp + t * p.k_stride + e);
-            if constexpr (CH) cp_async4(d + 2 * SH::DP + e, wp + t * p.w_stride + e);
+            copy4(d + e, qp + t * p.q_stride + e);
+            copy4(d + SH::DP + e, kp + t * p.k_stride + e);
+            if constexpr (CH) copy4(d + 2 * SH::DP + e, wp + t * p.w_stride + e);
         }
-        for (int e = lane; e < n_cols; e += 32) cp_async4(d + V + e, vp + t * p.v_stride + e);
-        if (SH::SCALARS && lane < 2) cp_async4(d + SH::TOKEN - 4 + lane, sp + t * (4 * p.heads) + lane);
+        for (int e = lane; e < n_cols; e += 32) copy4(d + V + e, vp + t * p.v_stride + e);
+        if (SH::SCALARS && lane < 2) copy4(d + SH::TOKEN - 4 + lane, sp + t * (4 * p.heads) + lane);
     }
 }
 
 // grid (ceil(vdim / (WC * warps)), heads, segments), block 32 * (warps + 1)
 template <int LR, int RPV, int CC, int TB, int WALK>
-__global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanParams p, const int wide) {
-    using SH = Shape<LR, RPV, CC, TB, WALK>;
+__global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanParams p, const int wide, const Leftovers left) {
+    using SH = WalkShape<LR, RPV, CC, TB, WALK>;
     constexpr bool CH = SH::CH;
     constexpr int DP = SH::DP, WC = SH::WC, NP = RPV * 2, TOKEN = SH::TOKEN, V = SH::ROWS * DP;
     extern __shared__ __align__(16) float ring[];
@@ -174,6 +170,8 @@ __global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanPa
     pdl_wait();
     const int t0 = p.cu_seqlens[seg], t1 = p.cu_seqlens[seg + 1];
     if (t0 >= t1) return;
+    const int what = left_over(left, p.cu_seqlens, seg, head, p.heads, c0, BC);
+    if (what == NOTHING) return;
     const int slot = p.slots[seg];
     if (seg > 0 && slot == p.slots[0]) {                  // a captured step's padding row (a copy of the first row): the state
         for (int e = threadIdx.x; e < (t1 - t0) * BC; e += blockDim.x)      // moves on once; the copy's results are never read
@@ -192,15 +190,15 @@ __global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanPa
         const float* sp = SH::SCALARS ? p.scalars + 4 * head : nullptr;
         const auto pump = [&](auto&& bring) {             // bring(batch): starts its copies
 #pragma unroll 1
-            for (int b = 0; b < RING - 1; ++b) { bring(b); cp_commit(); }
+            for (int b = 0; b < RING - 1; ++b) { bring(b); copy_commit(); }
 #pragma unroll 1
             for (int b = 0; b < n_batches; ++b) {
-                cp_wait<RING - 2>();
+                copy_wait<RING - 2>();
                 block_barrier(blockDim.x);                // batch b has landed, and every warp is done with batch b - 1
                 bring(b + RING - 1);                      // (into the stage that batch b - 1 had)
-                cp_commit();
+                copy_commit();
             }
-            cp_wait<0>();
+            copy_wait<0>();
         };
         if (wide) {
             Bringer<SH, TB> br(p, qp, kp, wp, vp, sp, n_cols, t0, lane);
@@ -219,6 +217,7 @@ __global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanPa
     const int r = lane % LR, cl = lane / LR;
     float* st = p.state + (size_t)slot * p.slot_stride + (size_t)head * vdim * dim4;
     const int j0 = warp * WC + cl * CC;                   // within the block's columns
+    const bool mine = j0 < n_cols && left_column(left, what, seg, head, p.heads, c0 + j0);     // (a lane's columns are in one group of 16)
     f2 S[NP][CC];
 #pragma unroll
     for (int c = 0; c < CC; ++c)
@@ -279,18 +278,18 @@ __global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanPa
     float* out = p.out + (size_t)t0 * p.out_stride + (size_t)head * vdim + c0 + j0;
     int stage = 0;
 #pragma unroll 1
-    for (int left = t1 - t0; left > 0; left -= TB) {
+    for (int rest = t1 - t0; rest > 0; rest -= TB) {
         block_barrier(blockDim.x);
         const float* in = ring + stage * (TB * TOKEN);
         stage = stage + 1 == RING ? 0 : stage + 1;
         float o[TB * CC];
-        if (left >= TB) {
+        if (rest >= TB) {
 #pragma unroll
             for (int tt = 0; tt < TB; ++tt) token(in + tt * TOKEN, o + tt * CC);
         } else {
 #pragma unroll
             for (int tt = 0; tt < TB; ++tt) {
-                if (tt < left) token(in + tt * TOKEN, o + tt * CC);
+                if (tt < rest) token(in + tt * TOKEN, o + tt * CC);
                 else
 #pragma unroll
                     for (int c = 0; c < CC; ++c) o[tt * CC + c] = 0.f;
@@ -309,7 +308,7 @@ __global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanPa
 #pragma unroll
         for (int i = 0; i < SH::KEEP; ++i) {
             const int num = r * SH::KEEP + i, tt = num / CC, c = num % CC;
-            if (tt < left && j0 + c < n_cols) {
+            if (tt < rest && mine && j0 + c < n_cols) {
                 const float* tok = in + tt * TOKEN;
                 out[(long long)tt * p.out_stride + c] =
                     WALK == PER_CHANNEL ? p.out_scale * o[i] : fmaf(CH ? tok[TOKEN - 4] : skip, tok[V + j0 + c], o[i]);
@@ -322,7 +321,7 @@ __global__ void __launch_bounds__(32 * (MAX_WARPS + 1)) scan_kernel(const ScanPa
 #pragma unroll
         for (int i = 0; i < RPV; ++i) {
             const int row = 4 * (r + LR * i);
-            if (row < dim4 && j0 + c < n_cols) {
+            if (row < dim4 && mine && j0 + c < n_cols) {
                 float4 f;
                 unpack2(S[2 * i][c], f.x, f.y); unpack2(S[2 * i + 1][c], f.z, f.w);
                 *(float4*)(st + (size_t)(c0 + j0 + c) * dim4 + row) = f;
@@ -414,8 +413,8 @@ __global__ void __launch_bounds__(128) channel_decays_kernel(const float* __rest
 }
 
 template <int LR, int RPV, int CC, int TB, int WALK>
-int launch_scan(const ScanParams& p, int wide, cudaStream_t st) {
-    using SH = Shape<LR, RPV, CC, TB, WALK>;
+int launch_scan(const ScanParams& p, int wide, const Leftovers& left, cudaStream_t st) {
+    using SH = WalkShape<LR, RPV, CC, TB, WALK>;
     // four walking warps a block, fewer where a step has so few (segment, head) pairs that more and smaller blocks spread better
     int warps = MAX_WARPS;
     while (warps > 1 && ((long long)((p.vdim + SH::WC * warps - 1) / (SH::WC * warps)) * p.heads * p.n_segments < 148 ||
@@ -427,22 +426,418 @@ int launch_scan(const ScanParams& p, int wide, cudaStream_t st) {
     dim3 grid((p.vdim + SH::WC * warps - 1) / (SH::WC * warps), p.heads, p.n_segments);
     // A step of single tokens is launched as a programmatic dependent; a longer walk in the ordinary way: started early, its
     // blocks would take the multiprocessors that the kernel before frees first, several to one, for the whole walk.
-    if (p.n_tokens == p.n_segments) SPITE_LAUNCH(kernel, grid, 32 * (warps + 1), bytes, st, p, wide);
-    else kernel<<<grid, 32 * (warps + 1), bytes, st>>>(p, wide);
+    if (p.n_tokens == p.n_segments) SPITE_LAUNCH(kernel, grid, 32 * (warps + 1), bytes, st, p, wide, left);
+    else kernel<<<grid, 32 * (warps + 1), bytes, st>>>(p, wide, left);
     return spite_launch_status();
 }
 
 template <int WALK>
-int choose_scan(const ScanParams& p, cudaStream_t st) {
+int choose_scan(const ScanParams& p, cudaStream_t st, const Leftovers& left = {}) {
     constexpr bool CH = WALK != PER_HEAD;
     const auto al = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
     const int wide = p.dim % 4 == 0 && p.vdim % 4 == 0 && p.q_stride % 4 == 0 && p.k_stride % 4 == 0 && p.v_stride % 4 == 0 &&
                      al(p.q) && al(p.k) && al(p.v) && (WALK == PER_CHANNEL || al(p.scalars)) && (!CH || (p.w_stride % 4 == 0 && al(p.w)));
-    if (p.dim <= 32) return launch_scan<8, 1, 2, 8, WALK>(p, wide, st);
-    if (p.dim <= 64) return launch_scan<8, 2, 2, 8, WALK>(p, wide, st);
-    if (p.dim <= 128) return launch_scan<8, 4, 2, 8, WALK>(p, wide, st);
-    if (p.dim <= 256) return launch_scan<16, 4, 2, 8, WALK>(p, wide, st);
-    return launch_scan<32, 4, 4, 8, WALK>(p, wide, st);
+    if (p.dim <= 32) return launch_scan<8, 1, 2, 8, WALK>(p, wide, left, st);
+    if (p.dim <= 64) return launch_scan<8, 2, 2, 8, WALK>(p, wide, left, st);
+    if (p.dim <= 128) return launch_scan<8, 4, 2, 8, WALK>(p, wide, left, st);
+    if (p.dim <= 256) return launch_scan<16, 4, 2, 8, WALK>(p, wide, left, st);
+    return launch_scan<32, 4, 4, 8, WALK>(p, wide, left, st);
+}
+
+// ---- what the walk in chunks needs that does not depend on the state
+// q and k of a chunk (a warp has the tokens warp, warp + 8, ..., a lane the elements lane, lane + 32, ...; 256 threads) into split tiles;
+// q_t . k_s into `scores`.  Returns the tiles' scales, and whether a number is not finite.  `largest`: two zeroed words.
+template <int DP>
+__device__ __forceinline__ bool split_tiles(const float* q, long long q_stride, const float* k, long long k_stride, int len, int dim, __half* tiles,
+                                            float (*scores)[36], unsigned* largest, Scale& sq, Scale& sk) {
+    constexpr int E = DP / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    float qv[4][E], kv[4][E];
+    unsigned lq = 0, lk = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int t = warp + 8 * i, d = lane + 32 * e;
+            const bool on = t < len && d < dim;
+            qv[i][e] = on ? q[t * q_stride + d] : 0.f;
+            kv[i][e] = on ? k[t * k_stride + d] : 0.f;
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) { lq = max(lq, abs_bits(qv[i][e])); lk = max(lk, abs_bits(kv[i][e])); }
+    lq = __reduce_max_sync(0xffffffffu, lq);
+    lk = __reduce_max_sync(0xffffffffu, lk);
+    if (lane == 0) { atomicMax(&largest[0], lq); atomicMax(&largest[1], lk); }
+    __syncthreads();
+    sq = scale_of(largest[0]);
+    sk = scale_of(largest[1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int at = tile_at<DP>(warp + 8 * i, lane + 32 * e);
+            split1(qv[i][e] * sq.up, tiles[at], tiles[CT * DP + at]);
+            split1(kv[i][e] * sk.up, tiles[2 * CT * DP + at], tiles[3 * CT * DP + at]);
+        }
+    __syncthreads();
+    const int m = warp & 1, n = warp >> 1;                // sixteen tokens t and eight tokens s a warp
+    float main[4] = {}, cross[4] = {};
+    if (n < 2 || m == 1) {
+#pragma unroll 4
+        for (int k16 = 0; k16 < DP / 16; k16 += 2) {
+            unsigned bh[4], bl[4], ah[4], al[4];
+            ldsm(bh, tiles + 2 * CT * DP + tile_at<DP>(8 * n + (lane & 7), 16 * k16 + 8 * (lane >> 3)));
+            ldsm(bl, tiles + 3 * CT * DP + tile_at<DP>(8 * n + (lane & 7), 16 * k16 + 8 * (lane >> 3)));
+            ldsm_left<DP>(ah, tiles, 16 * m, 16 * k16, lane);
+            ldsm_left<DP>(al, tiles + CT * DP, 16 * m, 16 * k16, lane);
+            mma3(main, cross, ah, al, bh[0], bh[1], bl[0], bl[1]);
+            ldsm_left<DP>(ah, tiles, 16 * m, 16 * k16 + 16, lane);
+            ldsm_left<DP>(al, tiles + CT * DP, 16 * m, 16 * k16 + 16, lane);
+            mma3(main, cross, ah, al, bh[2], bh[3], bl[2], bl[3]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+        *(float2*)&scores[16 * m + g + 8 * r][8 * n + 2 * t4] = make_float2((main[2 * r] + cross[2 * r]) * sq.down * sk.down,
+                                                                             (main[2 * r + 1] + cross[2 * r + 1]) * sq.down * sk.down);
+    return max(largest[0], largest[1]) >= 0x7f800000u;
+}
+template <int DP> __device__ __forceinline__ void store_tiles(__half* to, const __half* tiles) {
+    uint4* dst = reinterpret_cast<uint4*>(to);
+    const uint4* src = reinterpret_cast<const uint4*>(tiles);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < 4 * CT * DP / 8; e += blockDim.x) dst[e] = src[e];
+}
+
+// One decay a head.  A block has a chunk of one q/k head and up to SSM_HEADS of the heads that share it, a warp one of them at a time.
+constexpr int SSM_HEADS = 16;
+template <int DP> struct StateSpaceChunkSmem {
+    __half tiles[4 * CT * DP];
+    float scores[CT][36];
+    double b[8][CT];
+    float dt[8][CT];
+    unsigned largest[2];
+};
+template <int DP>
+__global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams p, const float* __restrict__ a, long long a_stride,
+                                                                const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                                                                float* __restrict__ scalars, const Made out, int slices) {
+    using Rec = Record<HEAD_DECAY, DP>;
+    extern __shared__ __align__(16) unsigned char smem_bytes[];
+    auto& sm = *reinterpret_cast<StateSpaceChunkSmem<DP>*>(smem_bytes);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int group = p.heads / p.kv_heads, kvh = blockIdx.y / slices, slice = blockIdx.y % slices;
+    const int h0 = kvh * group + slice * SSM_HEADS, h1 = min(h0 + SSM_HEADS, (kvh + 1) * group);
+    pdl_wait();
+    pdl_launch_dependents();
+    int seg, first;
+    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
+    const int len = min(CT, p.cu_seqlens[seg + 1] - first);
+    const bool brief = p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens;     // walked token by token: the tokens' scalars alone
+    if (first == p.cu_seqlens[seg])
+        for (int h = h0 + warp; h < h1; h += 8) clear_marks(out.columns, out.column_groups, seg, h, p.heads, lane, 32);
+    Scale sq, sk;
+    bool bad = false;
+    if (!brief) {
+        if (tid < 2) sm.largest[tid] = 0;
+        __syncthreads();
+        bad = split_tiles<DP>(p.q + (size_t)first * p.q_stride + (size_t)kvh * p.dim, p.q_stride, p.k + (size_t)first * p.k_stride + (size_t)kvh * p.dim,
+                              p.k_stride, len, p.dim, sm.tiles, sm.scores, sm.largest, sq, sk);
+        if (slice == 0) store_tiles<DP>(out.qk + ((size_t)blockIdx.x * p.kv_heads + kvh) * (4 * CT * DP), sm.tiles);
+        __syncthreads();
+    }
+    for (int h = h0 + warp; h < h1; h += 8) {             // a lane a token
+        float dt = 0.f, log_decay = 0.f;
+        bool lost = false;
+        if (lane < len) {
+            const float z = a[(long long)(first + lane) * a_stride + h] + dt_bias[h];
+            dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
+            log_decay = -expf(a_log[h]) * dt;
+            lost = !(dt < 3e38f) || !(log_decay <= 0.f);
+            *(float4*)(scalars + 4 * ((size_t)(first + lane) * p.heads + h)) = make_float4(expf(log_decay), dt, 0.f, 0.f);
+        }
+        if (brief) continue;
+        const double b = prefix_sum((double)bounded_log(log_decay), lane), last = __shfl_sync(0xffffffffu, b, len - 1);
+        __syncwarp();
+        sm.b[warp][lane] = b;
+        sm.dt[warp][lane] = dt;
+        __syncwarp();
+        const int s = 2 * (lane & 15);
+        const double b0 = sm.b[warp][s], b1 = sm.b[warp][s + 1];
+        const float d0 = sm.dt[warp][s], d1 = sm.dt[warp][s + 1];
+        float2 x[CT / 2];
+        unsigned largest = 0;
+#pragma unroll
+        for (int i = 0; i < CT / 2; ++i) {
+            const int t = 2 * i + (lane >> 4);
+            const double bt = sm.b[warp][t];
+            const float2 gs = *(const float2*)&sm.scores[t][s];
+            x[i].x = s <= t ? gs.x * expf((float)(bt - b0)) * d0 : 0.f;
+            x[i].y = s + 1 <= t ? gs.y * expf((float)(bt - b1)) * d1 : 0.f;
+            largest = max(largest, max(abs_bits(x[i].x), abs_bits(x[i].y)));
+        }
+        largest = __reduce_max_sync(0xffffffffu, largest);
+        const Scale sp = scale_of(largest);
+        const size_t at_head = (size_t)blockIdx.x * p.heads + h;
+        __half* scores = out.scores + at_head * (2 * CT * CT);
+#pragma unroll
+        for (int i = 0; i < CT / 2; ++i) {
+            unsigned hi, lo;
+            split2(x[i].x * sp.up, x[i].y * sp.up, hi, lo);
+            const int at = score_at(2 * i + (lane >> 4), s);
+            *(unsigned*)(scores + at) = hi;
+            *(unsigned*)(scores + CT * CT + at) = lo;
+        }
+        lost = __any_sync(0xffffffffu, lost || bad || largest >= 0x7f800000u);
+        float* rec = out.records + at_head * Rec::FLOATS;
+        rec[Rec::G + lane] = expf((float)b);
+        rec[Rec::W + lane] = dt * expf((float)(last - b));          // (beyond the chunk's tokens dt is zero)
+        if (lane < 8)
+            rec[Rec::SCALARS + lane] = lane == Q_DOWN ? sq.down : lane == K_DOWN ? sk.down : lane == P_DOWN ? sp.down
+                                     : lane == DECAY ? expf((float)last) : lane == BAD ? (lost ? 1.f : 0.f) : 0.f;
+    }
+}
+
+// A decay per key channel: one block a (chunk, head), 256 threads.  Scores of two tokens in the same half of the chunk are summed with
+// the products of the decays between them; those of the later half with the earlier are one product of operands that are brought to
+// the decays at the border.  BONUS (the decaying memory): a token's read-out sees the state before its own write, plus the bonus.
+template <int DP> struct KeyDecayChunkSmem {
+    __half tiles[4 * CT * DP], off[2 * CT * DP];          // `off`: rows 0 .. 15 k of the first half, 16 .. 31 q of the second, brought to the border
+    float q[CT][DP + 4], k[CT][DP + 4], w[CT][DP + 4];
+    float P[CT][36];
+    double part[256 / DP][DP];                            // sums of log decays of a thread's tokens
+    unsigned largest[5];                                  // of q and k in `tiles`, k and q in `off`, the scores
+    int bad;
+};
+template <int DP, bool BONUS>
+__global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p, const Made out) {
+    using Rec = Record<KEY_DECAY, DP>;
+    constexpr int PARTS = 256 / DP, TN = CT / PARTS;      // a thread has a channel of TN tokens
+    extern __shared__ __align__(16) unsigned char smem_bytes[];
+    auto& sm = *reinterpret_cast<KeyDecayChunkSmem<DP>*>(smem_bytes);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, dim = p.dim;
+    pdl_wait();
+    pdl_launch_dependents();
+    int seg, first;
+    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
+    if (first == p.cu_seqlens[seg]) clear_marks(out.columns, out.column_groups, seg, head, p.heads, tid, 256);
+    if (p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens) return;
+    const int len = min(CT, p.cu_seqlens[seg + 1] - first);
+    if (tid < 5) sm.largest[tid] = 0;
+    if (tid == 5) sm.bad = 0;
+    const size_t at_head = (size_t)blockIdx.x * p.heads + head;
+    const int ch = tid % DP, part = tid / DP;
+    float qv[TN], kv[TN];
+    double cum[TN];                                       // sum of the log decays up to the token, within the thread's tokens at first
+    bool bad = false;
+    {
+        const float* q = p.q + (size_t)first * p.q_stride + (size_t)head * dim + ch;
+        const float* k = p.k + (size_t)first * p.k_stride + (size_t)head * dim + ch;
+        const float* w = p.w + (size_t)first * p.w_stride + (size_t)head * dim + ch;
+        float wv[TN];
+#pragma unroll
+        for (int i = 0; i < TN; ++i) {
+            const int t = part * TN + i;
+            const bool on = t < len && ch < dim;
+            qv[i] = on ? q[(size_t)t * p.q_stride] : 0.f;
+            kv[i] = on ? k[(size_t)t * p.k_stride] : 0.f;
+            wv[i] = on ? w[(size_t)t * p.w_stride] : 1.f;
+        }
+        double sum = 0.0;
+#pragma unroll
+        for (int i = 0; i < TN; ++i) {
+            const int t = part * TN + i;
+            sm.q[t][ch] = qv[i]; sm.k[t][ch] = kv[i]; sm.w[t][ch] = wv[i];
+            bad |= !(wv[i] >= 0.f && wv[i] <= 1.f);
+            sum += (double)bounded_log(logf(wv[i]));
+            cum[i] = sum;
+        }
+        sm.part[part][ch] = sum;
+    }
+    for (int e = tid; e < CT * CT; e += 256) sm.P[e / CT][e % CT] = 0.f;
+    __syncthreads();
+    {
+        double before = 0.0, border = 0.0, last = 0.0;
+#pragma unroll
+        for (int i = 0; i < PARTS; ++i) {
+            const double s = sm.part[i][ch];
+            if (i < part) before += s;
+            if (i < PARTS / 2) border += s;
+            last += s;
+        }
+        float qs[TN], ks[TN], os[TN];
+        unsigned lq = 0, lk = 0, lo = 0;
+#pragma unroll
+        for (int i = 0; i < TN; ++i) {
+            const double c = before + cum[i];             // (a token of the memory is read before its own decay)
+            const double cq = BONUS ? before + (i ? cum[i ? i - 1 : 0] : 0.0) : c;
+            qs[i] = qv[i] * expf((float)cq);
+            ks[i] = kv[i] * expf((float)(last - c));
+            os[i] = part < PARTS / 2 ? kv[i] * expf((float)(border - c)) : qv[i] * expf((float)(cq - border));
+            lq = max(lq, abs_bits(qs[i])); lk = max(lk, abs_bits(ks[i])); lo = max(lo, abs_bits(os[i]));
+            bad |= max(abs_bits(qv[i]), abs_bits(kv[i])) >= 0x7f800000u;
+        }
+        lq = __reduce_max_sync(0xffffffffu, lq);
+        lk = __reduce_max_sync(0xffffffffu, lk);
+        lo = __reduce_max_sync(0xffffffffu, lo);
+        if (lane == 0) {
+            atomicMax(&sm.largest[0], lq); atomicMax(&sm.largest[1], lk);
+            atomicMax(&sm.largest[part < PARTS / 2 ? 2 : 3], lo);
+        }
+        if (bad) sm.bad = 1;
+        __syncthreads();
+        const Scale sq = scale_of(sm.largest[0]), sk = scale_of(sm.largest[1]), so = scale_of(sm.largest[part < PARTS / 2 ? 2 : 3]);
+#pragma unroll
+        for (int i = 0; i < TN; ++i) {
+            const int at = tile_at<DP>(part * TN + i, ch);
+            split1(qs[i] * sq.up, sm.tiles[at], sm.tiles[CT * DP + at]);
+            split1(ks[i] * sk.up, sm.tiles[2 * CT * DP + at], sm.tiles[3 * CT * DP + at]);
+            split1(os[i] * so.up, sm.off[at], sm.off[CT * DP + at]);
+        }
+        float* rec = out.records + at_head * Rec::FLOATS;
+        if (part == 0) rec[Rec::KEYS + ch] = ch < dim ? expf((float)last) : 0.f;
+        if (tid < CT) { rec[Rec::G + tid] = 1.f; rec[Rec::W + tid] = 1.f; }
+    }
+    // ---- scores within a half of the chunk: a warp has four tokens s, its lanes the channels
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const int s = warp + 8 * i, end = (s & 16) + 16;
+        constexpr int C2 = DP / 64;                       // pairs of channels a lane
+        float2 kf[C2];
+        float o[16];
+#pragma unroll
+        for (int c = 0; c < C2; ++c) kf[c] = *(const float2*)&sm.k[s][2 * lane + 64 * c];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {                    // token s + j
+            o[j] = 0.f;
+            if (s + j < end) {
+#pragma unroll
+                for (int c = 0; c < C2; ++c) {
+                    const float2 w = *(const float2*)&sm.w[s + j][2 * lane + 64 * c], q = *(const float2*)&sm.q[s + j][2 * lane + 64 * c];
+                    if (!BONUS && j) { kf[c].x *= w.x; kf[c].y *= w.y; }
+                    if (!BONUS || j) { o[j] = fmaf(q.x, kf[c].x, o[j]); o[j] = fmaf(q.y, kf[c].y, o[j]); }
+                    if (BONUS && j) { kf[c].x *= w.x; kf[c].y *= w.y; }
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 8; h >= 1; h >>= 1) {
+            const bool up = (lane & h) != 0;
+#pragma unroll
+            for (int j = 0; j < h; ++j) {
+                const float give = up ? o[j] : o[j + h], keep = up ? o[j + h] : o[j];
+                o[j] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+            }
+        }
+        float x = o[0] + __shfl_xor_sync(0xffffffffu, o[0], 16);
+        const int t = s + lane;
+        if (lane < 16 && t < end) {
+            if (BONUS && lane == 0) x = t < len ? p.scalars[4 * ((size_t)(first + t) * p.heads + head)] : 0.f;
+            sm.P[t][s] = x;
+        }
+    }
+    __syncthreads();
+    // ---- scores of the second half with the first: two warps, eight tokens s each
+    if (warp < 2) {
+        const Scale s0 = scale_of(sm.largest[2]), s1 = scale_of(sm.largest[3]);
+        float main[4] = {}, cross[4] = {};
+#pragma unroll
+        for (int k = 0; k < DP / 16; k += 2) {
+            unsigned bh[4], bl[4], ah[4], al[4];
+            ldsm(bh, sm.off + tile_at<DP>(8 * warp + (lane & 7), 16 * k + 8 * (lane >> 3)));
+            ldsm(bl, sm.off + CT * DP + tile_at<DP>(8 * warp + (lane & 7), 16 * k + 8 * (lane >> 3)));
+            ldsm_left<DP>(ah, sm.off, 16, 16 * k, lane);
+            ldsm_left<DP>(al, sm.off + CT * DP, 16, 16 * k, lane);
+            mma3(main, cross, ah, al, bh[0], bh[1], bl[0], bl[1]);
+            ldsm_left<DP>(ah, sm.off, 16, 16 * k + 16, lane);
+            ldsm_left<DP>(al, sm.off + CT * DP, 16, 16 * k + 16, lane);
+            mma3(main, cross, ah, al, bh[2], bh[3], bl[2], bl[3]);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            *(float2*)&sm.P[16 + (lane >> 2) + 8 * r][8 * warp + 2 * (lane & 3)] =
+                make_float2((main[2 * r] + cross[2 * r]) * s0.down * s1.down, (main[2 * r + 1] + cross[2 * r + 1]) * s0.down * s1.down);
+    }
+    store_tiles<DP>(out.qk + at_head * (4 * CT * DP), sm.tiles);
+    __syncthreads();
+    const int t = tid >> 3, s = 4 * (tid & 7);
+    const float4 x = *(const float4*)&sm.P[t][s];
+    const unsigned largest = __reduce_max_sync(0xffffffffu, max(max(abs_bits(x.x), abs_bits(x.y)), max(abs_bits(x.z), abs_bits(x.w))));
+    if (lane == 0) atomicMax(&sm.largest[4], largest);
+    __syncthreads();
+    const Scale sp = scale_of(sm.largest[4]);
+    uint2 h, l;
+    split2(x.x * sp.up, x.y * sp.up, h.x, l.x);
+    split2(x.z * sp.up, x.w * sp.up, h.y, l.y);
+    __half* scores = out.scores + at_head * (2 * CT * CT) + score_at(t, s);
+    *(uint2*)scores = h;
+    *(uint2*)(scores + CT * CT) = l;
+    if (tid < 8)
+        out.records[at_head * Rec::FLOATS + Rec::SCALARS + tid] =
+            tid == Q_DOWN ? scale_of(sm.largest[0]).down : tid == K_DOWN ? scale_of(sm.largest[1]).down : tid == P_DOWN ? sp.down
+          : tid == BAD ? (sm.bad || sm.largest[4] >= 0x7f800000u ? 1.f : 0.f) : 0.f;
+}
+
+inline Layout scan_layout(bool per_channel, int dim, int vdim, int heads, int kv_heads, int n_chunks, int n_segments) {
+    const int dp = dim <= 64 ? 64 : 128;
+    const int record = !per_channel ? Record<HEAD_DECAY, 64>::FLOATS : dp == 64 ? Record<KEY_DECAY, 64>::FLOATS : Record<KEY_DECAY, 128>::FLOATS;
+    return layout_of(dp, record, heads, kv_heads, vdim, n_chunks, n_segments, false, 0);
+}
+inline chunk::Walk scan_walk(const ScanParams& p, const Made& out) {
+    chunk::Walk w = walk_of(out);
+    const int dim4 = (p.dim + 3) & ~3;
+    w.v = p.v; w.v_stride = p.v_stride;
+    w.out = p.out; w.out_stride = p.out_stride;
+    w.state = p.state; w.slot_stride = p.slot_stride; w.head_stride = (long long)p.vdim * dim4;
+    w.key_stride = 1; w.col_stride = dim4;
+    w.cu_seqlens = p.cu_seqlens; w.slots = p.slots;
+    w.n_segments = p.n_segments; w.heads = p.heads; w.qk_heads = p.kv_heads; w.dim = p.dim; w.vdim = p.vdim;
+    return w;
+}
+inline bool one_wave(const ScanParams& p, int cols) { return (long long)((p.vdim + cols - 1) / cols) * p.heads * p.n_segments <= 148; }
+
+template <int DP>
+int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_stride, const float* a_log, const float* dt_bias, const Made& out,
+                              int n_chunks, cudaStream_t st) {
+    auto prep = state_space_chunk_kernel<DP>;
+    constexpr int bytes = (int)sizeof(StateSpaceChunkSmem<DP>);
+    if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    const int slices = (p.heads / p.kv_heads + SSM_HEADS - 1) / SSM_HEADS;
+    SPITE_LAUNCH(prep, dim3(n_chunks, p.kv_heads * slices), 256, bytes, st, p, a, a_stride, a_log, dt_bias, (float*)p.scalars, out, slices);
+    if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    chunk::Walk w = scan_walk(p, out);
+    w.skip = p.skip;
+    // 32 columns a block while that leaves every multiprocessor one block at most, else 64
+    if (one_wave(p, 32)) return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, st);
+    return launch_walk<DP / 2, 2, 4, HEAD_DECAY>(w, st);
+}
+template <int DP, bool BONUS>
+int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, cudaStream_t st) {
+    auto prep = key_decay_chunk_kernel<DP, BONUS>;
+    constexpr int bytes = (int)sizeof(KeyDecayChunkSmem<DP>);
+    if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    SPITE_LAUNCH(prep, dim3(n_chunks, p.heads), 256, bytes, st, p, out);
+    if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    chunk::Walk w = scan_walk(p, out);
+    w.out_scale = BONUS ? 1.f : p.out_scale;
+    if (one_wave(p, 32)) return launch_walk<32, DP / 32, 2, KEY_DECAY>(w, st);
+    return launch_walk<32, DP / 32, DP == 64 ? 4 : 2, KEY_DECAY>(w, st);
+}
+template <bool BONUS, int WALK>
+int key_decay_in_chunks(const ScanParams& p, void* scratch, int n_chunks, int min_tokens, cudaStream_t st) {
+    const Layout l = scan_layout(true, p.dim, p.vdim, p.heads, p.heads, n_chunks, p.n_segments);
+    const Made out = made_at(scratch, l, min_tokens);
+    const int rc = p.dim <= 64 ? launch_key_decay_chunks<64, BONUS>(p, out, n_chunks, st) : launch_key_decay_chunks<128, BONUS>(p, out, n_chunks, st);
+    if (rc != SPITE_OK) return rc;
+    return choose_scan<WALK>(p, st, leftovers_of(out, l, p.heads, Record<KEY_DECAY, 64>::SCALARS));
+}
+
+// the working memory of a call in chunks: refused before anything is launched
+int check_chunks(const ScanParams& p, const void* scratch, int n_chunks, int min_tokens) {
+    if (!scratch || ((uintptr_t)scratch & 15) || n_chunks < 1 || min_tokens < 1) return SPITE_BAD_ARG;
+    return p.dim > 128 ? SPITE_UNSUPPORTED : SPITE_OK;
 }
 
 int check_scan(const ScanParams* p) {
@@ -459,12 +854,38 @@ int check_scan(const ScanParams* p) {
 
 }  // namespace
 
+// Bytes of working memory that the three walks in chunks need for a step of `n_chunks` chunks of 32 tokens; -2: sizes they do not take.
+SPITE_API long long spite_scan_chunk_bytes(int per_channel, int dim, int vdim, int heads, int kv_heads, int n_chunks, int n_segments) {
+    if (dim < 1 || vdim < 1 || heads < 1 || kv_heads < 1 || n_chunks < 0 || n_segments < 0) return SPITE_BAD_ARG;
+    if (dim > 128) return SPITE_UNSUPPORTED;
+    return scan_layout(per_channel != 0, dim, vdim, heads, kv_heads, n_chunks, n_segments).bytes;
+}
+
 // `a` [tokens, heads] with rows of a_stride: the projection's step columns; p->scalars is filled here
-SPITE_API int spite_state_space_scan(const ScanParams* p, const float* a, long long a_stride, const float* a_log,
-                                     const float* dt_bias, void* stream) {
+static int check_state_space(const ScanParams* p, const float* a, long long a_stride, const float* a_log, const float* dt_bias) {
     const int chk = check_scan(p);
     if (chk != SPITE_OK) return chk;
-    if (!a || !a_log || !dt_bias || !p->scalars || p->w || a_stride < p->heads) return SPITE_BAD_ARG;
+    return !a || !a_log || !dt_bias || !p->scalars || p->w || a_stride < p->heads ? SPITE_BAD_ARG : SPITE_OK;
+}
+// Segments of at least `min_tokens` tokens in chunks of 32, the others token by token.
+SPITE_API int spite_state_space_scan_chunked(const ScanParams* p, const float* a, long long a_stride, const float* a_log, const float* dt_bias,
+                                             void* scratch, int n_chunks, int min_tokens, void* stream) {
+    int chk = check_state_space(p, a, a_stride, a_log, dt_bias);
+    if (chk == SPITE_OK) chk = check_chunks(*p, scratch, n_chunks, min_tokens);
+    if (chk != SPITE_OK) return chk;
+    if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    const Layout l = scan_layout(false, p->dim, p->vdim, p->heads, p->kv_heads, n_chunks, p->n_segments);
+    const Made out = made_at(scratch, l, min_tokens);
+    const int rc = p->dim <= 64 ? launch_state_space_chunks<64>(*p, a, a_stride, a_log, dt_bias, out, n_chunks, st)
+                                : launch_state_space_chunks<128>(*p, a, a_stride, a_log, dt_bias, out, n_chunks, st);
+    if (rc != SPITE_OK) return rc;
+    return choose_scan<PER_HEAD>(*p, st, leftovers_of(out, l, p->heads, Record<HEAD_DECAY, 64>::SCALARS));
+}
+SPITE_API int spite_state_space_scan(const ScanParams* p, const float* a, long long a_stride, const float* a_log,
+                                     const float* dt_bias, void* stream) {
+    const int chk = check_state_space(p, a, a_stride, a_log, dt_bias);
+    if (chk != SPITE_OK) return chk;
     if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const long long n = (long long)p->n_tokens * p->heads;
@@ -474,8 +895,9 @@ SPITE_API int spite_state_space_scan(const ScanParams* p, const float* a, long l
 }
 
 // p->w holds the decay's pre-activations on entry and the decays afterwards; `u` and `w0` [heads * dim]
-SPITE_API int spite_decay_scan(const ScanParams* p, const float* w0, const float* u, void* stream) {
-    const int chk = check_scan(p);
+static int decay_scan(const ScanParams* p, const float* w0, const float* u, bool chunks, void* scratch, int n_chunks, int min_tokens, void* stream) {
+    int chk = check_scan(p);
+    if (chk == SPITE_OK && chunks) chk = check_chunks(*p, scratch, n_chunks, min_tokens);
     if (chk != SPITE_OK) return chk;
     if (!w0 || !u || !p->scalars || !p->w || p->w_stride < (long long)p->heads * p->dim || p->kv_heads != p->heads || p->skip) return SPITE_BAD_ARG;
     if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
@@ -485,14 +907,22 @@ SPITE_API int spite_decay_scan(const ScanParams* p, const float* w0, const float
     SPITE_LAUNCH(memory_gates_kernel, (int)((rows + 3) / 4), 128, 0, st, (float*)p->w, p->w_stride, w0, p->q, p->q_stride, p->k,
                  p->k_stride, u, (float*)p->scalars, rows, p->heads, p->dim);
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    if (chunks) return key_decay_in_chunks<true, PER_CHANNEL_BONUS>(*p, scratch, n_chunks, min_tokens, st);
     return choose_scan<PER_CHANNEL_BONUS>(*p, st);
+}
+SPITE_API int spite_decay_scan(const ScanParams* p, const float* w0, const float* u, void* stream) {
+    return decay_scan(p, w0, u, false, nullptr, 0, 0, stream);
+}
+SPITE_API int spite_decay_scan_chunked(const ScanParams* p, const float* w0, const float* u, void* scratch, int n_chunks, int min_tokens, void* stream) {
+    return decay_scan(p, w0, u, true, scratch, n_chunks, min_tokens, stream);
 }
 
 // p->w [tokens, heads * dim] receives the decays, from the short vectors `a` [tokens, rank] (rows of a_stride), `a2` [rank,
 // heads * dim] and `b` [heads * dim]
-SPITE_API int spite_gated_linear_scan(const ScanParams* p, const float* a, long long a_stride, const float* a2, const float* b,
-                                      int rank, float tau, void* stream) {
-    const int chk = check_scan(p);
+static int gated_linear_scan(const ScanParams* p, const float* a, long long a_stride, const float* a2, const float* b, int rank, float tau,
+                             bool chunks, void* scratch, int n_chunks, int min_tokens, void* stream) {
+    int chk = check_scan(p);
+    if (chk == SPITE_OK && chunks) chk = check_chunks(*p, scratch, n_chunks, min_tokens);
     if (chk != SPITE_OK) return chk;
     if (!a || !a2 || !b || rank < 1 || a_stride < rank || !(tau > 0.f) || !(p->out_scale == p->out_scale)) return SPITE_BAD_ARG;
     if (!p->w || p->w_stride < (long long)p->heads * p->dim || p->kv_heads != p->heads || p->skip) return SPITE_BAD_ARG;
@@ -505,5 +935,14 @@ SPITE_API int spite_gated_linear_scan(const ScanParams* p, const float* a, long 
     auto decays = few ? channel_decays_kernel<1> : channel_decays_kernel<8>;
     SPITE_LAUNCH(decays, grid, 128, 0, st, a, a_stride, a2, b, (float*)p->w, p->w_stride, p->n_tokens, n, rank, 1.f / tau);
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
+    if (chunks) return key_decay_in_chunks<false, PER_CHANNEL>(*p, scratch, n_chunks, min_tokens, st);
     return choose_scan<PER_CHANNEL>(*p, st);
+}
+SPITE_API int spite_gated_linear_scan(const ScanParams* p, const float* a, long long a_stride, const float* a2, const float* b,
+                                      int rank, float tau, void* stream) {
+    return gated_linear_scan(p, a, a_stride, a2, b, rank, tau, false, nullptr, 0, 0, stream);
+}
+SPITE_API int spite_gated_linear_scan_chunked(const ScanParams* p, const float* a, long long a_stride, const float* a2, const float* b, int rank,
+                                              float tau, void* scratch, int n_chunks, int min_tokens, void* stream) {
+    return gated_linear_scan(p, a, a_stride, a2, b, rank, tau, true, scratch, n_chunks, min_tokens, stream);
 }

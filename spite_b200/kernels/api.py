@@ -316,22 +316,23 @@ class KernelSet:
         return vdim * (-(-dim // 4) * 4)
 
     def state_space_scan(self, q, k, v, step, out, batch, state, *, heads, kv_heads, dim, vdim, a_log, dt_bias, skip,
-                         state_offset=0):
+                         state_offset=0, chunked=None):
         """A state space with one decay per head and token (Mamba-2), for every segment of the step from the matrices its
         request's slot holds (zeros: the start of a sequence); the slot receives the matrices after the segment's last
         token.  Per head h: dt = softplus(step + dt_bias[h]); S <- exp(-exp(a_log[h]) dt) S + dt k v^T; out = S^T q + skip[h] v.
         q, k, v, step are pairs (float32 tensor [M, *], first column) of widths kv_heads * dim (twice), heads * vdim and heads;
         head h reads q and k of head h // (heads / kv_heads); out float32 [M, heads * vdim]; state float32 [slots, *], head h's
-        S at state[slot, state_offset + h * scan_state_size(dim, vdim)], transposed ([vdim, keys]).  All float32."""
+        S at state[slot, state_offset + h * scan_state_size(dim, vdim)], transposed ([vdim, keys]).  All float32.  `chunked`: long
+        segments go 32 tokens at a time (the same sums in another order); None leaves the choice to the kernel set."""
         raise NotImplementedError
 
-    def decay_scan(self, r, k, v, w, out, batch, state, *, heads, dim, vdim, w0, u, state_offset=0):
+    def decay_scan(self, r, k, v, w, out, batch, state, *, heads, dim, vdim, w0, u, state_offset=0, chunked=None):
         """A memory that decays per key channel (RWKV), walked and kept as above: out = S^T r + (sum_i r_i u_i k_i) v, then
         S <- diag(exp(-exp(w + w0))) S + k v^T.  w float32 [M, heads * dim] holds the decay's pre-activations and is
         overwritten with the decays; w0, u float32 [heads * dim]."""
         raise NotImplementedError
 
-    def gated_linear_scan(self, q, k, v, a, w, out, batch, state, *, heads, dim, vdim, a2, a2_bias, tau, q_scale, state_offset=0):
+    def gated_linear_scan(self, q, k, v, a, w, out, batch, state, *, heads, dim, vdim, a2, a2_bias, tau, q_scale, state_offset=0, chunked=None):
         """Gated linear attention, walked and kept as above: S <- diag(w) S + k v^T, then out = q_scale S^T q, with the decays
         w = sigmoid(a A_2 + a2_bias)^(1 / tau) per head and key channel made first.  q, k, v and a (the short vectors of
         a2.shape[0] elements) are pairs (float32 tensor, first column); a2 float32 [rank, heads * dim] (input-major), a2_bias

@@ -304,6 +304,7 @@ class CudaKernels(KernelSet):
         # token.  Delta rule, 16 heads of 128 x 128, us in chunks / token by token: one prompt of 32 tokens 21 / 24, 64:
         # 23 / 42, 512: 52 / 291, 2,048: 170 / 1,147; sixteen prompts of 16: 59 / 52, of 32: 61 / 95.
         self.chunk_min_tokens = 32
+        self.memory_min_tokens = 8             # ... the matrix memory's
         # how much working memory a call may take for that (a step of 8,192 tokens of 32 heads of 128 x 128 takes 0.45 GB); a call that
         # would need more goes token by token
         self.chunk_scratch_limit = 1 << 30
@@ -1170,16 +1171,24 @@ class CudaKernels(KernelSet):
         if chunked is None:
             # Prompts and their portions go 32 tokens at a time.  The float32 set keeps the walk token by token for
             # every step, so that its results do not depend on how a prompt was cut, to the last bit.
-            chunked = self.dtype != torch.float32 and batch.max_seg_len >= 8
+            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.memory_min_tokens
         p = MlstmParams(proj=proj.data_ptr(), stride=proj.shape[1], q_col=q_col, k_col=k_col, v_col=v_col, i_col=i_col,
                         f_col=f_col, i_bias=i_bias.data_ptr(), f_bias=f_bias.data_ptr(), out=out.data_ptr(),
                         state=state.data_ptr(), head_stride=state.shape[2], cu_seqlens=batch.cu_seqlens.data_ptr(),
                         slots=batch.slots.data_ptr(), n_segments=n_seg, heads=int(heads), dim=int(dim), vdim=int(vdim),
                         gate_cap=float(gate_cap), q_scale=float(q_scale), chunked=int(bool(chunked)))
         if chunked:
+            n_chunks = (M + 31) // 32 + n_seg
+            scratch = self._chunk_scratch("recurrent", "spite_mlstm_tiles_bytes", dim, vdim, heads, n_chunks, n_seg)
+            if scratch is not None:
+                st = self._lib("recurrent").spite_mlstm_scan_tiles(C.byref(p), C.c_void_p(scratch.data_ptr()), n_chunks,
+                                                                   self.memory_min_tokens, self._stream())
+                self._count("recurrent", 3)
+                _check(st, "mlstm_scan")
+                return
+            # (more than 256 key rows: the chunks' products on the float32 units)
             # working memory for what the chunks need ahead of the state (scores, sums of the gates): a record for every
             # chunk and head; the segments' chunks are at most tokens / 32 + segments
-            n_chunks = (M + 31) // 32 + n_seg
             scratch = torch.empty((n_chunks, heads, 1152), dtype=torch.float32, device=proj.device)
             st = self._lib("recurrent").spite_mlstm_scan_chunked(C.byref(p), C.c_void_p(scratch.data_ptr()), C.c_int(n_chunks), self._stream())
         else:
@@ -1259,8 +1268,27 @@ class CudaKernels(KernelSet):
                        dim=int(dim), vdim=int(vdim))
         return p, scalars
 
+    def _run_scan(self, entry, p, batch, kv_heads, per_channel, chunked, *rest):
+        """One of the three walks: in chunks where that is asked for or pays and the sizes allow it, else token by token."""
+        lib = self._lib("scan")
+        if chunked is None:
+            # (the float32 set keeps the walk token by token, so that its results do not depend on how a prompt was cut)
+            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_min_tokens
+        if chunked:
+            n_chunks = (p.n_tokens + 31) // 32 + p.n_segments
+            scratch = self._chunk_scratch("scan", "spite_scan_chunk_bytes", per_channel, p.dim, p.vdim, p.heads, kv_heads, n_chunks, p.n_segments)
+            if scratch is not None:
+                st = getattr(lib, entry + "_chunked")(C.byref(p), *rest, C.c_void_p(scratch.data_ptr()), n_chunks, self.chunk_min_tokens,
+                                                      self._stream())
+                self._count("scan", 4 if per_channel else 3)
+                _check(st, entry)
+                return
+        st = getattr(lib, entry)(C.byref(p), *rest, self._stream())
+        self._count("scan", 2)
+        _check(st, entry)
+
     def state_space_scan(self, q, k, v, step, out, batch, state, *, heads, kv_heads, dim, vdim, a_log, dt_bias, skip,
-                         state_offset=0):
+                         state_offset=0, chunked=None):
         p, scalars = self._scan("state_space_scan", q, k, v, out, batch, state, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim,
                                 state_offset=state_offset)
         for name, t in (("a_log", a_log), ("dt_bias", dt_bias), ("skip", skip)):
@@ -1270,12 +1298,10 @@ class CudaKernels(KernelSet):
         self._t(t, torch.float32, "step")
         a = self._columns(t, column, heads, out.shape[0], "state_space_scan: step")
         p.skip = skip.data_ptr()
-        st = self._lib("scan").spite_state_space_scan(C.byref(p), C.c_void_p(a), C.c_longlong(t.shape[1]),
-                                                      C.c_void_p(a_log.data_ptr()), C.c_void_p(dt_bias.data_ptr()), self._stream())
-        self._count("scan", 2)
-        _check(st, "state_space_scan")
+        self._run_scan("spite_state_space_scan", p, batch, kv_heads, False, chunked, C.c_void_p(a), C.c_longlong(t.shape[1]),
+                       C.c_void_p(a_log.data_ptr()), C.c_void_p(dt_bias.data_ptr()))
 
-    def decay_scan(self, r, k, v, w, out, batch, state, *, heads, dim, vdim, w0, u, state_offset=0):
+    def decay_scan(self, r, k, v, w, out, batch, state, *, heads, dim, vdim, w0, u, state_offset=0, chunked=None):
         p, scalars = self._scan("decay_scan", r, k, v, out, batch, state, heads=heads, kv_heads=heads, dim=dim, vdim=vdim,
                                 state_offset=state_offset)
         self._t(w, torch.float32, "w")
@@ -1285,11 +1311,9 @@ class CudaKernels(KernelSet):
             if self._t(t, torch.float32, name).numel() != heads * dim:
                 raise KernelError(f"decay_scan: {name} has one element per head and key channel")
         p.w, p.w_stride = w.data_ptr(), w.shape[1]
-        st = self._lib("scan").spite_decay_scan(C.byref(p), C.c_void_p(w0.data_ptr()), C.c_void_p(u.data_ptr()), self._stream())
-        self._count("scan", 2)
-        _check(st, "decay_scan")
+        self._run_scan("spite_decay_scan", p, batch, heads, True, chunked, C.c_void_p(w0.data_ptr()), C.c_void_p(u.data_ptr()))
 
-    def gated_linear_scan(self, q, k, v, a, w, out, batch, state, *, heads, dim, vdim, a2, a2_bias, tau, q_scale, state_offset=0):
+    def gated_linear_scan(self, q, k, v, a, w, out, batch, state, *, heads, dim, vdim, a2, a2_bias, tau, q_scale, state_offset=0, chunked=None):
         p, _ = self._scan("gated_linear_scan", q, k, v, out, batch, state, heads=heads, kv_heads=heads, dim=dim, vdim=vdim,
                           state_offset=state_offset, scalars=False)
         self._t(w, torch.float32, "w"); self._t(a2, torch.float32, "a2")
@@ -1300,10 +1324,8 @@ class CudaKernels(KernelSet):
         self._t(t, torch.float32, "a")
         at = self._columns(t, column, rank, out.shape[0], "gated_linear_scan: a")
         p.w, p.w_stride, p.out_scale = w.data_ptr(), n, float(q_scale)
-        st = self._lib("scan").spite_gated_linear_scan(C.byref(p), C.c_void_p(at), C.c_longlong(t.shape[1]), C.c_void_p(a2.data_ptr()),
-                                                       C.c_void_p(a2_bias.data_ptr()), int(rank), C.c_float(tau), self._stream())
-        self._count("scan", 2)
-        _check(st, "gated_linear_scan")
+        self._run_scan("spite_gated_linear_scan", p, batch, heads, True, chunked, C.c_void_p(at), C.c_longlong(t.shape[1]),
+                       C.c_void_p(a2.data_ptr()), C.c_void_p(a2_bias.data_ptr()), int(rank), C.c_float(tau))
 
     # ------------------------------------------------------------------ mixture of experts
     def moe_identity(self, x, routing, first_identity, out, *, accumulate=True):

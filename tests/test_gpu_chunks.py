@@ -132,3 +132,233 @@ def test_delta_entry_points_refuse_malformed_calls():
     assert call(n_segments=0) == 0
     torch.cuda.synchronize()
     assert not t.any()
+
+
+# ---------------------------------------------------------------------------- the walks of scan.cu
+def scan_reference(kind, q, k, v, w, extra, S):
+    """One segment in float64, q, k [T, heads, dim], v [T, heads, vdim], S [heads, vdim, dim]."""
+    out = torch.zeros_like(v)
+    for t in range(q.shape[0]):
+        kv = v[t][:, :, None] * k[t][:, None, :]
+        if kind == "memory":
+            out[t] = torch.einsum("hvk,hk->hv", S, q[t]) + (q[t] * extra * k[t]).sum(-1)[:, None] * v[t]
+        S = w[t] * S + kv
+        if kind != "memory":
+            out[t] = torch.einsum("hvk,hk->hv", S, q[t])
+    return out, S
+
+
+# (heads, kv heads (state space), dim, vdim, segments as token counts of two steps)
+SCANS = [
+    (2, 1, 64, 64, [(64, 1), (33, 31), (1, 95)]),
+    (3, 1, 20, 12, [(32, 17), (15, 16), (129, 2)]),
+    (20, 1, 128, 70, [(31, 65), (16, 1)]),
+    (2, 2, 100, 5, [(250, 97)]),
+    (34, 2, 128, 64, [(40, 33), (70, 1), (18, 20)]),
+]
+
+
+@pytest.mark.parametrize("case", range(len(SCANS)))
+@pytest.mark.parametrize("gates", ["mild", "harsh"])
+@pytest.mark.parametrize("kind", ["state_space", "memory", "linear_attention"])
+def test_scans_in_chunks(kind, gates, case):
+    heads, kvh, dim, vdim, segs = SCANS[case]
+    kvh = kvh if kind == "state_space" else heads
+    ks = kernels(torch.bfloat16)
+    ks.chunk_min_tokens = 16
+    g = torch.Generator().manual_seed(50 + case)
+    rnd = lambda *s: torch.randn(s, generator=g).to(DEV)
+    size = heads * ks.scan_state_size(dim, vdim)
+    dim4 = -(-dim // 4) * 4
+    slots = torch.randperm(len(segs) + 2, generator=g)[:len(segs)].tolist()
+    state = rnd(len(segs) + 2, 8 + size)
+    state[slots] = 0.0
+    harsh = 1.0 if gates == "mild" else 5.0
+    carried = [torch.zeros((heads, vdim, dim), dtype=torch.float64, device=DEV) for _ in segs]
+    a_log, dt, skip, w0, u = rnd(heads) * harsh - 1.0, rnd(heads), rnd(heads), rnd(heads * dim) * harsh - 2.0, rnd(heads * dim)
+    a2, a2_bias = rnd(6, heads * dim), rnd(heads * dim) * harsh
+    for step in range(2):
+        counts = [s[step] for s in segs]
+        batch, M = step_batch(counts, slots, step == 0)
+        q, k, v = rnd(M, kvh * dim + 4), rnd(M, kvh * dim + 4) * 1e-2, rnd(M, heads * vdim + 4) * (1e3 if case % 2 else 1.0)
+        a = rnd(M, heads + 3) if kind == "state_space" else rnd(M, 8)
+        out = torch.empty((M, heads * vdim), dtype=torch.float32, device=DEV)
+        more = dict(heads=heads, dim=dim, vdim=vdim, state_offset=8, chunked=True)
+        qd, kd, vd = ((t.double()[:, 4 * i:4 * i + n].view(M, -1, s)) for t, i, n, s in
+                      ((q, 1, kvh * dim, dim), (k, 0, kvh * dim, dim), (v, 1, heads * vdim, vdim)))
+        qd, kd = qd.repeat_interleave(heads // kvh, 1), kd.repeat_interleave(heads // kvh, 1)
+        extra = None
+        if kind == "state_space":
+            ks.state_space_scan((q, 4), (k, 0), (v, 4), (a, 2), out, batch, state, kv_heads=kvh, a_log=a_log, dt_bias=dt, skip=skip, **more)
+            step_size = torch.nn.functional.softplus(a.double()[:, 2:2 + heads] + dt.double())
+            w = torch.exp(-torch.exp(a_log.double()) * step_size)[:, :, None, None]
+            kd = kd * step_size[:, :, None]
+        elif kind == "memory":
+            z = rnd(M, heads * dim)
+            w = torch.exp(-torch.exp(z.double() + w0.double())).view(M, heads, 1, dim)
+            ks.decay_scan((q, 4), (k, 0), (v, 4), z, out, batch, state, w0=w0, u=u, **more)
+            extra = u.double().view(heads, dim)
+        else:
+            decays = torch.empty((M, heads * dim), device=DEV)
+            ks.gated_linear_scan((q, 4), (k, 0), (v, 4), (a, 1), decays, out, batch, state, a2=a2, a2_bias=a2_bias, tau=4.0, q_scale=0.3, **more)
+            w = torch.sigmoid(a.double()[:, 1:7] @ a2.double() + a2_bias.double()).pow(0.25).view(M, heads, 1, dim)
+            qd = qd * 0.3
+        off = 0
+        for s, n in enumerate(counts):
+            part = slice(off, off + n)
+            ref, carried[s] = scan_reference(kind, qd[part], kd[part], vd[part], w[part], extra, carried[s])
+            if kind == "state_space":
+                ref = ref + skip.double()[:, None] * vd[part]
+            near(out[part].view(n, heads, vdim), ref, f"step {step}, segment {s}")
+            got = state[slots[s], 8:8 + size].view(heads, vdim, dim4)
+            near(got[:, :, :dim], carried[s], f"step {step}, state of segment {s}")
+            assert not got[:, :, dim:].any()
+            off += n
+
+
+@pytest.mark.parametrize("kind", ["state_space", "memory"])
+def test_scans_with_an_infinity_are_walked_token_by_token(kind):
+    heads, dim, vdim, counts = 2, 64, 32, [70, 40]
+    ks = kernels(torch.bfloat16)
+    g = torch.Generator().manual_seed(6)
+    rnd = lambda *s: torch.randn(s, generator=g).to(DEV)
+    batch, M = step_batch(counts, [0, 1], True)
+    q, k, v, a = rnd(M, heads * dim), rnd(M, heads * dim), rnd(M, heads * vdim), rnd(M, heads)
+    v[50, 20] = float("inf")                                              # head 0, second group of 16 columns, first segment
+    z, par, chan = rnd(M, heads * dim), rnd(heads), rnd(heads * dim)
+    outs, states = [], []
+    for chunked in (True, False):
+        state = torch.zeros((2, heads * dim * vdim), device=DEV)
+        out = torch.empty((M, heads * vdim), device=DEV)
+        if kind == "state_space":
+            ks.state_space_scan((q, 0), (k, 0), (v, 0), (a, 0), out, batch, state, heads=heads, kv_heads=heads, dim=dim, vdim=vdim, a_log=par,
+                                dt_bias=par, skip=par, chunked=chunked)
+        else:
+            ks.decay_scan((q, 0), (k, 0), (v, 0), z.clone(), out, batch, state, heads=heads, dim=dim, vdim=vdim, w0=chan, u=chan, chunked=chunked)
+        outs.append(out)
+        states.append(state)
+    torch.testing.assert_close(outs[0][:70, 16:32], outs[1][:70, 16:32], rtol=TOL, atol=0, equal_nan=True)
+    assert not torch.isfinite(outs[0][50:70, 20]).any()
+    near(outs[0][:50], outs[1][:50].double(), "before the infinity")
+    near(outs[0][:, vdim:], outs[1][:, vdim:].double(), "the other head")
+    near(outs[0][:, :16], outs[1][:, :16].double(), "the other columns")
+    torch.testing.assert_close(states[0], states[1], rtol=1e-3, atol=1e-3, equal_nan=True)
+
+
+# ---------------------------------------------------------------------------- the matrix memory
+MEMORY = [
+    (1, 256, 64, [(64, 1), (33, 31), (1, 95)]),
+    (3, 20, 12, [(32, 17), (15, 16), (129, 2)]),
+    (2, 128, 70, [(31, 65), (16, 1)]),
+    (2, 200, 33, [(250, 97)]),
+    (8, 64, 96, [(40, 33), (70, 1), (18, 9)]),
+]
+
+
+@pytest.mark.parametrize("case", range(len(MEMORY)))
+@pytest.mark.parametrize("cap", [5.0, 30.0])
+def test_matrix_memory_in_chunks(cap, case):
+    heads, dim, vdim, segs = MEMORY[case]
+    ks = kernels(torch.bfloat16)
+    g = torch.Generator().manual_seed(90 + case)
+    rnd = lambda *s: torch.randn(s, generator=g).to(DEV)
+    size = ks.mlstm_state_size(dim, vdim)
+    slots = torch.randperm(len(segs) + 2, generator=g)[:len(segs)].tolist()
+    state = rnd(len(segs) + 2, heads, size)
+    state[slots] = 0.0
+    bi, bf = rnd(heads), rnd(heads) + 3.0
+    cols = (1, 1 + heads * dim, 3 + 2 * heads * dim, 3 + 2 * heads * dim + heads * vdim, 4 + 2 * heads * dim + heads * (vdim + 1))
+    carried = [[torch.zeros(s, dtype=torch.float64, device=DEV) for s in ((heads, dim, vdim), (heads, dim), (heads,))] for _ in segs]
+    for step in range(2):
+        counts = [s[step] for s in segs]
+        batch, M = step_batch(counts, slots, step == 0)
+        x = rnd(M, cols[4] + heads + 1)
+        x[:, cols[3]:] *= cap
+        x[:, cols[2]:cols[3]] *= 1e3 if case % 2 else 1e-2
+        out = torch.empty((M, heads * vdim), dtype=torch.float32, device=DEV)
+        ks.mlstm_scan(x, out, batch, state, heads=heads, dim=dim, vdim=vdim, gate_cap=cap, q_scale=dim ** -0.5, columns=cols, i_bias=bi,
+                      f_bias=bf, chunked=True)
+        xd, off = x.double(), 0
+        q, k = xd[:, cols[0]:cols[0] + heads * dim].view(M, heads, dim) * dim ** -0.5, xd[:, cols[1]:cols[1] + heads * dim].view(M, heads, dim)
+        v = xd[:, cols[2]:cols[2] + heads * vdim].view(M, heads, vdim)
+        gi = cap * torch.tanh((xd[:, cols[3]:cols[3] + heads] + bi.double()) / cap)
+        gf = torch.nn.functional.logsigmoid(cap * torch.tanh((xd[:, cols[4]:cols[4] + heads] + bf.double()) / cap))
+        for s, n in enumerate(counts):
+            S, nn, m = carried[s]
+            ref = torch.zeros((n, heads, vdim), dtype=torch.float64, device=DEV)
+            for t in range(off, off + n):
+                new = torch.maximum(gf[t] + m, gi[t])
+                keep, take = torch.exp(gf[t] + m - new)[:, None], torch.exp(gi[t] - new)[:, None] * k[t]
+                m = new
+                S, nn = keep[:, :, None] * S + take[:, :, None] * v[t][:, None, :], keep * nn + take
+                den = torch.maximum((nn * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+                ref[t - off] = torch.einsum("hkv,hk->hv", S, q[t]) / den[:, None]
+            carried[s] = [S, nn, m]
+            got = out[off:off + n].view(n, heads, vdim)
+            # (a denominator near its floor of exp(-m) is a small difference of large sums: the tokens' own scale)
+            near(got, ref, f"step {step}, segment {s}", 1e-4)
+            st = state[slots[s]]
+            near(st[:, :dim * vdim].view(heads, dim, vdim), S, f"step {step}, state of segment {s}")
+            for c in range(-(-vdim // 32)):
+                copy = st[:, dim * vdim + c * (-(-(dim + 1) // 4) * 4):][:, :dim + 1]
+                near(copy[:, :dim], nn, "n")
+                near(copy[:, dim], m, "m")
+            off += n
+
+
+def test_matrix_memory_with_an_infinity_is_walked_token_by_token():
+    heads, dim, vdim, counts = 2, 64, 64, [70, 40]
+    ks = kernels(torch.bfloat16)
+    g = torch.Generator().manual_seed(7)
+    batch, M = step_batch(counts, [0, 1], True)
+    cols = (0, heads * dim, 2 * heads * dim, 2 * heads * dim + heads * vdim, 2 * heads * dim + heads * vdim + heads)
+    x = torch.randn((M, cols[4] + heads), generator=g).to(DEV)
+    x[50, cols[2] + 40] = float("inf")
+    outs, states = [], []
+    for chunked in (True, False):
+        state = torch.zeros((2, heads, ks.mlstm_state_size(dim, vdim)), device=DEV)
+        out = torch.empty((M, heads * vdim), device=DEV)
+        ks.mlstm_scan(x, out, batch, state, heads=heads, dim=dim, vdim=vdim, gate_cap=5.0, q_scale=0.1, columns=cols,
+                      i_bias=torch.zeros(heads, device=DEV), f_bias=torch.zeros(heads, device=DEV), chunked=chunked)
+        outs.append(out)
+        states.append(state)
+    torch.testing.assert_close(outs[0][:70, 32:64], outs[1][:70, 32:64], rtol=TOL, atol=0, equal_nan=True)
+    near(outs[0][:50], outs[1][:50].double(), "before the infinity", 1e-4)
+    near(outs[0][:, vdim:], outs[1][:, vdim:].double(), "the other head", 1e-4)
+    near(outs[0][:, :32], outs[1][:, :32].double(), "the other block of columns", 1e-4)
+    torch.testing.assert_close(states[0], states[1], rtol=1e-3, atol=1e-3, equal_nan=True)
+
+
+def test_scan_and_memory_entry_points_refuse_malformed_calls():
+    from spite_b200.kernels import build
+    from spite_b200.kernels.cuda import MlstmParams, ScanParams
+    scan, rec = build.load("scan"), build.load("recurrent")
+    for f in (scan.spite_scan_chunk_bytes, rec.spite_mlstm_tiles_bytes):
+        f.restype = C.c_longlong
+    assert scan.spite_scan_chunk_bytes(0, 129, 8, 1, 1, 1, 1) == -2 and scan.spite_scan_chunk_bytes(1, 8, 0, 1, 1, 1, 1) == -1
+    assert rec.spite_mlstm_tiles_bytes(257, 8, 1, 1, 1) == -2 and rec.spite_mlstm_tiles_bytes(8, 8, 0, 1, 1) == -1
+    t = torch.zeros(1 << 16, device=DEV)
+    at, stride = t.data_ptr(), C.c_longlong(16)
+    vp = C.c_void_p
+    a = dict.fromkeys(("q", "k", "v", "scalars", "out", "state", "cu_seqlens", "slots"), at)
+    a.update(q_stride=16, k_stride=16, v_stride=16, out_stride=16, slot_stride=256, n_segments=1, n_tokens=4, heads=1, kv_heads=1, dim=16, vdim=16,
+             out_scale=1.0)
+
+    def walks(scratch=at, chunks=1, least=1, **k):
+        p, w = ScanParams(**dict(a, **k)), ScanParams(**dict(a, w=at, w_stride=k.get("dim", 16), **k))
+        tail = (vp(scratch), chunks, least, None)
+        return [scan.spite_state_space_scan_chunked(C.byref(p), vp(at), stride, vp(at), vp(at), *tail),
+                scan.spite_decay_scan_chunked(C.byref(w), vp(at), vp(at), *tail),
+                scan.spite_gated_linear_scan_chunked(C.byref(w), vp(at), stride, vp(at), vp(at), 4, C.c_float(2.0), *tail)]
+    for bad in (dict(scratch=None), dict(scratch=at + 4), dict(chunks=0), dict(least=0), dict(heads=0), dict(vdim=0)):
+        assert walks(**bad) == [-1] * 3, bad
+    assert walks(dim=160, q_stride=160, k_stride=160, slot_stride=1 << 14) == [-2] * 3
+    assert walks(n_segments=0) == [0] * 3 and walks(n_tokens=0) == [0] * 3
+    m = dict.fromkeys(("proj", "out", "state", "cu_seqlens", "slots"), at)
+    m.update(stride=200, q_col=0, k_col=16, v_col=32, i_col=48, f_col=49, head_stride=400, n_segments=1, heads=1, dim=16, vdim=16, gate_cap=1.0,
+             q_scale=1.0)
+    tiles = lambda scratch=at, chunks=1, least=1, **k: rec.spite_mlstm_scan_tiles(C.byref(MlstmParams(**dict(m, **k))), vp(scratch), chunks, least, None)
+    assert tiles(scratch=None) == tiles(scratch=at + 4) == tiles(chunks=0) == tiles(least=0) == tiles(heads=0) == tiles(gate_cap=0.0) == -1
+    assert tiles(dim=300, stride=1000, head_stride=1 << 14) == -2 and tiles(n_segments=0) == 0
+    torch.cuda.synchronize()
+    assert not t.any()
