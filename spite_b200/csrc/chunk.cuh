@@ -16,15 +16,18 @@
 //
 // Work.  A block owns 16 CW value columns of one (segment, head), a warp KPW keys by 16 of those columns.  It keeps the state
 // transposed, as mma accumulators (rows: columns of S, columns: keys): split, they are the left operand of (Q S0)^T = S0^T Q^T without
-// leaving the registers.  The warps of different keys meet in shared memory once a chunk.  Operand tiles and values come by asynchronous
-// copies a chunk or two ahead.
+// leaving the registers.  The warps of different keys meet in shared memory once a chunk.  Operand tiles come by bulk copies a chunk or two
+// ahead (16-byte asynchronous copies by all threads took a third of a chunk's time to issue: 1,900 of 6,900 clocks for 70 KB), the
+// values by 16-byte copies.
 #pragma once
-#include "common.cuh"
+#include "tcgen05.cuh"
 #include <cuda_fp16.h>
 
 namespace chunk {
 
 constexpr int CT = 32;                                    // tokens of a chunk
+
+__device__ int walk_error = 0;                            // the library's word for a wait that ran out, where it is given no other
 
 enum Mode { HEAD_DECAY = 0, MATRIX_MEMORY = 1, DELTA = 2, KEY_DECAY = 3 };
 
@@ -47,8 +50,47 @@ __device__ __forceinline__ void split1(float a, __half& high, __half& low) {
     low = __float2half_rn(a - __half2float(high));
 }
 
+// two floats in one register pair, for the two-at-a-time multiply-adds of sm_100
+typedef unsigned long long pair;
+__device__ __forceinline__ pair pair_of(float lo, float hi) {
+    pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 floats_of(pair v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ pair mul2(pair a, pair b) {
+    pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair fma2(pair a, pair b, pair c) {
+    pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// the split of two numbers times `up`
+__device__ __forceinline__ void split2(pair x, pair up, unsigned& high, unsigned& low) {
+    x = mul2(x, up);
+    const float2 f = floats_of(x);
+    const __half2 h = __floats2half2_rn(f.x, f.y);
+    const float2 hf = __half22float2(h), r = floats_of(fma2(pair_of(hf.x, hf.y), pair_of(-1.f, -1.f), x));
+    const __half2 l = __floats2half2_rn(r.x, r.y);
+    high = *reinterpret_cast<const unsigned*>(&h);
+    low = *reinterpret_cast<const unsigned*>(&l);
+}
+// the largest magnitude of three; a NaN stays one (its bits are above infinity's)
+__device__ __forceinline__ float max_abs(float a, float b, float c) {
+    float r;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 __device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void ldsm(unsigned (&r)[4], const __half* p) {
@@ -59,7 +101,17 @@ __device__ __forceinline__ void ldsm_t(unsigned (&r)[4], const __half* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
 }
-// c += (ah + al)(bh + bl) without al bl: `main` takes the first, `cross` the other two
+// c += (ah + al)(bh + bl) without al bl, the three terms in sums of their own; and the sum of those, elements 2 i and 2 i + 1
+__device__ __forceinline__ void mma3(float (&c)[3][4], const unsigned (&ah)[4], const unsigned (&al)[4], unsigned bh0, unsigned bh1, unsigned bl0,
+                                     unsigned bl1) {
+    mma(c[0], al, bh0, bh1);
+    mma(c[1], ah, bl0, bl1);
+    mma(c[2], ah, bh0, bh1);
+}
+__device__ __forceinline__ float2 sum3(const float (&c)[3][4], int i) {
+    return make_float2(c[2][2 * i] + (c[0][2 * i] + c[1][2 * i]), c[2][2 * i + 1] + (c[0][2 * i + 1] + c[1][2 * i + 1]));
+}
+// ... in two sums: `main` takes the first, `cross` the other two
 __device__ __forceinline__ void mma3(float (&main)[4], float (&cross)[4], const unsigned (&ah)[4], const unsigned (&al)[4],
                                      unsigned bh0, unsigned bh1, unsigned bl0, unsigned bl1) {
     mma(cross, al, bh0, bh1);
@@ -242,24 +294,31 @@ template <int KPW, int KW, int CW, int MODE> struct Shape {
     // two sets of partial sums: in turn (a chunk's are read while the next one's are written), or a delta rule's two products
     static constexpr int SUM_FLOATS = KW * COLS * TP;
     static constexpr int SUMS = 2 * SUM_FLOATS * 4;
-    static constexpr int EXTRA = MODE == DELTA ? 2 * COLS * TP * 4 : MODE == MATRIX_MEMORY ? (2 * DP + 2 * CT) * 4 : 0;
+    // a delta rule: u, and what the read-outs start from; the memory: n, the parts of q . n of the tokens, and the tokens' factors, two of each
+    static constexpr int FACTORS = 3 * CT + 4;
+    static constexpr int EXTRA = MODE == DELTA ? 2 * COLS * TP * 4 : MODE == MATRIX_MEMORY ? 2 * (DP + KW * CT + FACTORS) * 4 : 0;
     static constexpr int bytes(int stages) { return stages * STAGE + SUMS + EXTRA; }
 };
 
 // grid (ceil(vdim / COLS), heads, segments)
 template <int KPW, int KW, int CW, int MODE>
-__global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) {
+__global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, const tc::WaitControl waits) {
     using SH = Shape<KPW, KW, CW, MODE>;
     using Rec = typename SH::Rec;
     constexpr int DP = SH::DP, COLS = SH::COLS, THREADS = SH::THREADS, VP = SH::VP, TP = SH::TP, NK = KPW / 8, KS = KPW / 16;
     constexpr int NT = KW >= 4 ? 1 : 4 / KW;              // groups of eight tokens whose read-outs a warp finishes
+    constexpr bool WEIGHTED = MODE == DELTA || MODE == HEAD_DECAY;       // the values that join the state have a factor per token
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned largest_of[2][3];                 // largest magnitudes at the start of chunk c: of the state, of the memory's n; c % 3
+    __shared__ __align__(8) unsigned long long full[3];   // a stage's tiles have landed
+    __shared__ int abort_flag;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
     const int kw = warp % KW, cw = warp / KW;             // the warp's keys and columns
     const int seg = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * COLS;
     float* sums = reinterpret_cast<float*>(smem + (size_t)p.stages * SH::STAGE);
     float* extra = sums + SH::SUMS / 4;
-    bool lost = false;                                    // a number that is not finite
+    bool lost = false;                                    // a number that is not finite, or a wait that ran out
+    int* const error_word = waits.error_word ? waits.error_word : &walk_error;
     pdl_wait();
     const int t0 = p.cu_seqlens[seg], t1 = p.cu_seqlens[seg + 1];
     if (t1 - t0 < p.min_tokens) return;
@@ -270,6 +329,12 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
         return;
     }
     const int n_cols = min(COLS, p.vdim - col0), n_chunks = (t1 - t0 + CT - 1) / CT, chunk0 = chunks_before(p.cu_seqlens, seg);
+    if (tid < 3) { largest_of[0][tid] = 0; largest_of[1][tid] = 0; }
+    if (tid == 0) {
+        for (int i = 0; i < 3; ++i) tc::mbar_init(tc::smem_u32(&full[i]), 1);
+        abort_flag = 0;
+        tc::mbar_init_fence();
+    }
     {
         bool bad = false;
         for (int c = tid; c < n_chunks; c += THREADS)
@@ -280,24 +345,20 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
     const float* v_rows = p.v + (size_t)head * p.vdim + col0;
     const bool wide = (p.v_stride & 3) == 0 && (p.vdim & 3) == 0 && (((uintptr_t)v_rows) & 15) == 0;
 
-    const auto fetch = [&](int c) {                       // the chunk's operands into its stage
+    constexpr int REC_AT = SH::QK_BYTES + SH::W_BYTES + SH::P_BYTES;
+    const auto fetch = [&](int c, int stage) {            // chunk c's operands into a stage
         if (c < n_chunks) {
-            unsigned char* st = smem + (size_t)(c % p.stages) * SH::STAGE;
-            const size_t at = (size_t)(chunk0 + c) * p.heads + head;
-            const unsigned char* qk = (const unsigned char*)p.qk + ((size_t)(chunk0 + c) * p.qk_heads + qk_head) * SH::QK_BYTES;
-#pragma unroll 4
-            for (int e = tid * 16; e < SH::QK_BYTES; e += THREADS * 16) copy16(st + e, qk + e);
-            if constexpr (MODE == DELTA) {
-                const unsigned char* w = (const unsigned char*)p.w + at * SH::W_BYTES;
-#pragma unroll 4
-                for (int e = tid * 16; e < SH::W_BYTES; e += THREADS * 16) copy16(st + SH::QK_BYTES + e, w + e);
+            unsigned char* st = smem + (size_t)stage * SH::STAGE;
+            if (tid == THREADS - 32) {
+                const size_t at = (size_t)(chunk0 + c) * p.heads + head;
+                const unsigned bar = tc::smem_u32(&full[stage]), to = tc::smem_u32(st);
+                tc::mbar_expect_tx(bar, REC_AT + SH::REC_BYTES + (c == 0 ? waits.extra_tx : 0));
+                tc::bulk_load(to, (const unsigned char*)p.qk + ((size_t)(chunk0 + c) * p.qk_heads + qk_head) * SH::QK_BYTES, SH::QK_BYTES, bar);
+                if constexpr (MODE == DELTA) tc::bulk_load(to + SH::QK_BYTES, (const unsigned char*)p.w + at * SH::W_BYTES, SH::W_BYTES, bar);
+                tc::bulk_load(to + SH::QK_BYTES + SH::W_BYTES, (const unsigned char*)p.scores + at * SH::P_BYTES, SH::P_BYTES, bar);
+                tc::bulk_load(to + REC_AT, p.records + at * Rec::FLOATS, SH::REC_BYTES, bar);
             }
-            unsigned char* rest = st + SH::QK_BYTES + SH::W_BYTES;
-            const unsigned char* sc = (const unsigned char*)p.scores + at * SH::P_BYTES;
-            const unsigned char* rec = (const unsigned char*)(p.records + at * Rec::FLOATS);
-            for (int e = tid * 16; e < SH::P_BYTES; e += THREADS * 16) copy16(rest + e, sc + e);
-            for (int e = tid * 16; e < SH::REC_BYTES; e += THREADS * 16) copy16(rest + SH::P_BYTES + e, rec + e);
-            float* vs = reinterpret_cast<float*>(rest + SH::P_BYTES + SH::REC_BYTES);
+            float* vs = reinterpret_cast<float*>(st + REC_AT + SH::REC_BYTES);
             const int tb = t0 + c * CT, len = min(CT, t1 - tb);
             if (wide) {
                 for (int e = tid; e < CT * (COLS / 4); e += THREADS) {
@@ -315,8 +376,14 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
         }
         copy_commit();
     };
-    fetch(0);
-    if (p.stages > 2) fetch(1);
+    // chunk c has landed, as far as this thread waits for it (another barrier makes it so for the block)
+    const auto wait_for = [&](int c, int stage, unsigned parity) {
+        if (p.stages > 2) copy_wait<1>(); else copy_wait<0>();
+        if (c < n_chunks)
+            lost |= !tc::mbar_wait(tc::smem_u32(&full[stage]), parity, &abort_flag, error_word, 2, waits.limit_cycles);
+    };
+    fetch(0, 0);
+    if (p.stages > 2) fetch(1, 1);
 
     // the state's columns 16 cw + g (and + 8), keys KPW kw + 8 n + 2 t4 (and + 1)
     float* st = p.state + (size_t)slot * p.slot_stride + (size_t)head * p.head_stride;
@@ -326,6 +393,13 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
         key = KPW * kw + 8 * n + 2 * t4 + (i & 1);
         return col < n_cols && key < p.dim;
     };
+    const auto mark_largest = [&](unsigned& slot_of) {    // of the warp's part of the state
+        float m = 0.f;
+#pragma unroll
+        for (int n = 0; n < NK; ++n) m = max_abs(m, max_abs(S[n][0], S[n][1], S[n][2]), S[n][3]);
+        const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if (lane == 0) atomicMax(&slot_of, bits);
+    };
 #pragma unroll
     for (int n = 0; n < NK; ++n)
 #pragma unroll
@@ -333,102 +407,111 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
             int col, key;
             S[n][i] = state_at(n, i, col, key) ? st[(size_t)key * p.key_stride + (size_t)(col0 + col) * p.col_stride] : 0.f;
         }
+    mark_largest(largest_of[0][0]);
     const float skip = p.skip ? p.skip[head] : 0.f;
-    float m_run = 0.f;
-    float* n_s = extra;                                   // MATRIX_MEMORY: n, two copies in turn, then q . n of the chunk's tokens
+    float m_run = 0.f;                                    // MATRIX_MEMORY: the running maximum (warp 0)
+    float* n_s = extra;                                   // n, then the warps' parts of q . n of the chunk's tokens
+    float* nq_s = extra + 2 * DP;
+    float* factors = extra + 2 * (DP + KW * CT);          // of chunk c: g, h, the denominator's floor [CT] each, decay, the weights' factor
     float* st_n = st + p.n_offset + (size_t)(blockIdx.x * (COLS / 32)) * p.n_stride;
+    // The memory's factors per token (a lane has token `lane`): g on Q S0, h on P V.  Warp 0 makes them a chunk ahead.
+    const auto make_factors = [&](const float* rec, int len, float* to) {
+        const double* md = reinterpret_cast<const double*>(rec);
+        const double m_local = md[lane], F = md[CT + lane];
+        const double m_last = md[len - 1], F_last = md[CT + len - 1];
+        const double M = fmax((double)m_run, m_local);
+        to[lane] = expf((float)((double)m_run - M));
+        to[CT + lane] = expf((float)(m_local - M));
+        to[2 * CT + lane] = expf(-(float)(F + M));
+        // the maximum goes on as a float, and the state is scaled to that rounded value
+        const float m_next = (float)(F_last + fmax((double)m_run, m_last));
+        const double M_state = (double)m_next - F_last;
+        if (lane == 0) {
+            to[3 * CT] = expf((float)((double)m_run - M_state));
+            to[3 * CT + 1] = expf((float)(m_last - M_state));
+        }
+        m_run = m_next;
+    };
     if constexpr (MODE == MATRIX_MEMORY) {
         static_assert(COLS % 32 == 0, "a copy of n serves 32 columns");
-        m_run = st_n[p.dim];
-        for (int d = tid; d < DP; d += THREADS) n_s[d] = d < p.dim ? st_n[d] : 0.f;
+        if (warp == 0) m_run = st_n[p.dim];
+        for (int d = tid; d < DP; d += THREADS) {
+            n_s[d] = d < p.dim ? st_n[d] : 0.f;
+            atomicMax(&largest_of[1][0], abs_bits(n_s[d]));
+        }
     }
-    if (p.stages > 2) copy_wait<1>(); else copy_wait<0>();
+    wait_for(0, 0, 0);
     __syncthreads();
+    if constexpr (MODE == MATRIX_MEMORY) {
+        if (warp == 0) make_factors(reinterpret_cast<const float*>(smem + REC_AT), min(CT, t1 - t0), factors);
+        __syncthreads();
+    }
+    // where a lane reads the operand tiles (halves from a tile's start), whatever the chunk
+    int at_q[KS];
+#pragma unroll
+    for (int k = 0; k < KS; ++k) at_q[k] = tile_at<DP>(8 * (lane >> 4) + (lane & 7), KPW * kw + 16 * k + 8 * ((lane >> 3) & 1));
 
+    int stage = 0;                                        // of chunk c
+    unsigned parity = 0, slot3 = 0;                       // of the stage's barrier for chunk c; c % 3
+    int c = 0;
 #pragma unroll 1
-    for (int c = 0; c < n_chunks; ++c) {
-        fetch(c + p.stages - 1);                          // (into the stage of the chunk before, which every warp has left)
-        unsigned char* stg = smem + (size_t)(c % p.stages) * SH::STAGE;
+    for (; c < n_chunks; ++c) {
+        // (into the stage of the chunk before, which every warp has left)
+        fetch(c + p.stages - 1, stage == 0 ? p.stages - 1 : stage - 1);
+        unsigned char* stg = smem + (size_t)stage * SH::STAGE;
+        if (++stage == p.stages) { stage = 0; parity ^= 1; }          // (of the next chunk from here on)
         const __half* q_s = reinterpret_cast<const __half*>(stg);
         const __half* k_s = q_s + 2 * CT * DP;
         const __half* w_s = k_s + 2 * CT * DP;
         const __half* p_s = reinterpret_cast<const __half*>(stg + SH::QK_BYTES + SH::W_BYTES);
-        const float* rec = reinterpret_cast<const float*>(stg + SH::QK_BYTES + SH::W_BYTES + SH::P_BYTES);
-        const float* v_s = reinterpret_cast<const float*>(stg + SH::QK_BYTES + SH::W_BYTES + SH::P_BYTES + SH::REC_BYTES);
+        const float* rec = reinterpret_cast<const float*>(stg + REC_AT);
+        const float* v_s = reinterpret_cast<const float*>(stg + REC_AT + SH::REC_BYTES);
         const int tb = t0 + c * CT, len = min(CT, t1 - tb);
         float* sum = sums + (MODE == DELTA ? 0 : (c & 1) * SH::SUM_FLOATS);
+        const float* fac = factors + (c & 1) * SH::FACTORS;
+        const unsigned state_largest = largest_of[0][slot3], slot_now = slot3, slot_next = slot3 == 2 ? 0 : slot3 + 1;
+        lost |= state_largest >= 0x7f800000u;
+        if (tid < 2) largest_of[tid][slot_next == 2 ? 0 : slot_next + 1] = 0;
+        const Scale ss = scale_of(state_largest);
 
-        // factors per token (a lane has token `lane`): g on Q S0, h on P V, w on V in the state's renewal
-        float gt, ht = 1.f, wt, decay, den = 1.f, w_more = 1.f;
-        if constexpr (MODE == MATRIX_MEMORY) {
-            const double* md = reinterpret_cast<const double*>(rec);
-            const double m_local = md[lane], F = md[CT + lane];
-            const double m_last = md[len - 1], F_last = md[CT + len - 1];
-            const double M = fmax((double)m_run, m_local);
-            gt = expf((float)((double)m_run - M));
-            ht = expf((float)(m_local - M));
-            // the maximum goes on as a float, and the state is scaled to that rounded value
-            const float m_next = (float)(F_last + fmax((double)m_run, m_last));
-            const double M_state = (double)m_next - F_last;
-            w_more = expf((float)(m_last - M_state));
-            wt = rec[Rec::W + lane] * w_more;
-            decay = expf((float)((double)m_run - M_state));
-            den = expf(-(float)(F + M));
-            m_run = m_next;
-        } else {
-            gt = rec[Rec::G + lane];
-            wt = rec[Rec::W + lane];
-            decay = rec[Rec::SCALARS + DECAY];
-        }
-        const float q_down = rec[Rec::SCALARS + Q_DOWN], k_down = rec[Rec::SCALARS + K_DOWN], p_down = rec[Rec::SCALARS + P_DOWN];
-
-        // ---- (Q S0)^T, and (W S0)^T, over the warp's keys
+        // ---- (Q S0)^T, and (W S0)^T, over the warp's keys: still scaled
         {
-            unsigned largest = 0;
-#pragma unroll
-            for (int n = 0; n < NK; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) largest = max(largest, abs_bits(S[n][i]));
-            largest = __reduce_max_sync(0xffffffffu, largest);
-            lost |= largest >= 0x7f800000u;
-            const Scale s = scale_of(largest);
+            const pair up = pair_of(ss.up, ss.up);
             unsigned ah[KS][4], al[KS][4];
 #pragma unroll
             for (int k = 0; k < KS; ++k)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    split2(S[2 * k + (i >> 1)][2 * (i & 1)] * s.up, S[2 * k + (i >> 1)][2 * (i & 1) + 1] * s.up, ah[k][i], al[k][i]);
-            const auto product = [&](const __half* tile, float down, float* to) {
+                    split2(pair_of(S[2 * k + (i >> 1)][2 * (i & 1)], S[2 * k + (i >> 1)][2 * (i & 1) + 1]), up, ah[k][i], al[k][i]);
+            const auto product = [&](const __half* tile, float* to) {
                 to += (kw * COLS + 16 * cw + g) * TP + 2 * t4;
+                float acc[4][3][4] = {};                  // groups of eight tokens; the terms apart, so that no sum waits for another
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {    // sixteen tokens at a time
-                    float main[2][4] = {}, cross[2][4] = {};
+                for (int k = 0; k < KS; ++k)
 #pragma unroll
-                    for (int k = 0; k < KS; ++k) {
-                        const int row = 16 * half + 8 * (lane >> 4) + (lane & 7), col = KPW * kw + 16 * k + 8 * ((lane >> 3) & 1);
+                    for (int half = 0; half < 2; ++half) {
                         unsigned bh[4], bl[4];
-                        ldsm(bh, tile + tile_at<DP>(row, col));
-                        ldsm(bl, tile + CT * DP + tile_at<DP>(row, col));
-                        mma3(main[0], cross[0], ah[k], al[k], bh[0], bh[1], bl[0], bl[1]);
-                        mma3(main[1], cross[1], ah[k], al[k], bh[2], bh[3], bl[2], bl[3]);
+                        ldsm(bh, tile + at_q[k] + half * 16 * DP);
+                        ldsm(bl, tile + CT * DP + at_q[k] + half * 16 * DP);
+                        mma3(acc[2 * half], ah[k], al[k], bh[0], bh[1], bl[0], bl[1]);
+                        mma3(acc[2 * half + 1], ah[k], al[k], bh[2], bh[3], bl[2], bl[3]);
                     }
 #pragma unroll
-                    for (int n = 0; n < 2; ++n)
+                for (int n = 0; n < 4; ++n)
 #pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            *(float2*)(to + 8 * i * TP + 16 * half + 8 * n) =
-                                make_float2((main[n][2 * i] + cross[n][2 * i]) * down, (main[n][2 * i + 1] + cross[n][2 * i + 1]) * down);
-                }
+                    for (int i = 0; i < 2; ++i) *(float2*)(to + 8 * i * TP + 8 * n) = sum3(acc[n], i);
             };
-            product(q_s, s.down * q_down, sum);
-            if constexpr (MODE == DELTA) product(w_s, s.down * rec[Rec::SCALARS + W_DOWN], sum + SH::SUM_FLOATS);
+            product(q_s, sum);
+            if constexpr (MODE == DELTA) product(w_s, sum + SH::SUM_FLOATS);
         }
+        const float q_down = ss.down * rec[Rec::SCALARS + Q_DOWN];
         // ---- the chunk's values as left operands (columns g, g + 8; tokens 16 k + 2 t4, + 1, + 8, + 9)
-        float va[2][4][2];                                // [sixteen tokens][register][its two tokens]
+        float2 va[2][4];                                  // [sixteen tokens][register]
         if constexpr (MODE == DELTA) {                    // V <- U0 - g (W S0); what the read-outs start from beside it
             __syncthreads();
             float* u_s = extra;
             float* z_s = extra + COLS * TP;
+            const float w_down = ss.down * rec[Rec::SCALARS + W_DOWN];
             for (int e = tid; e < COLS * (CT / 4); e += THREADS) {
                 const int j = e % COLS, t = 4 * (e / COLS);
                 float4 y = make_float4(0.f, 0.f, 0.f, 0.f), z = y;
@@ -439,171 +522,233 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
                     y.x += b.x; y.y += b.y; y.z += b.z; y.w += b.w;
                 }
                 const float4 gg = *(const float4*)(rec + Rec::G + t);
-                *(float4*)(u_s + j * TP + t) = make_float4(fmaf(-gg.x, y.x, v_s[t * VP + j]), fmaf(-gg.y, y.y, v_s[(t + 1) * VP + j]),
-                                                           fmaf(-gg.z, y.z, v_s[(t + 2) * VP + j]), fmaf(-gg.w, y.w, v_s[(t + 3) * VP + j]));
-                *(float4*)(z_s + j * TP + t) = make_float4(gg.x * z.x, gg.y * z.y, gg.z * z.z, gg.w * z.w);
+                *(float4*)(u_s + j * TP + t) =
+                    make_float4(fmaf(-gg.x, y.x * w_down, v_s[t * VP + j]), fmaf(-gg.y, y.y * w_down, v_s[(t + 1) * VP + j]),
+                                fmaf(-gg.z, y.z * w_down, v_s[(t + 2) * VP + j]), fmaf(-gg.w, y.w * w_down, v_s[(t + 3) * VP + j]));
+                *(float4*)(z_s + j * TP + t) = make_float4(gg.x * (z.x * q_down), gg.y * (z.y * q_down), gg.z * (z.z * q_down), gg.w * (z.w * q_down));
             }
             __syncthreads();
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 x = *(const float2*)(u_s + (16 * cw + g + 8 * (i & 1)) * TP + 16 * k + 2 * t4 + 8 * (i >> 1));
-                    va[k][i][0] = x.x; va[k][i][1] = x.y;
-                }
+                for (int i = 0; i < 4; ++i) va[k][i] = *(const float2*)(u_s + (16 * cw + g + 8 * (i & 1)) * TP + 16 * k + 2 * t4 + 8 * (i >> 1));
         } else {
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) va[k][i][e] = v_s[(16 * k + 2 * t4 + e + 8 * (i >> 1)) * VP + 16 * cw + g + 8 * (i & 1)];
-        }
-        unsigned largest = 0, largest_w = 0;
-        float wf[2][4];                                   // w of the lane's tokens 16 k + 2 t4 (+ 1, + 8, + 9)
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) wf[k][i] = __shfl_sync(0xffffffffu, wt, 16 * k + 2 * t4 + (i & 1) + 8 * (i >> 1));
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    largest = max(largest, abs_bits(va[k][i][e]));
-                    largest_w = max(largest_w, abs_bits(va[k][i][e] * wf[k][2 * (i >> 1) + e]));
+                for (int i = 0; i < 4; ++i) {
+                    const float* v = v_s + (16 * k + 2 * t4 + 8 * (i >> 1)) * VP + 16 * cw + g + 8 * (i & 1);
+                    va[k][i] = make_float2(v[0], v[VP]);
                 }
-        largest = __reduce_max_sync(0xffffffffu, largest);
-        largest_w = __reduce_max_sync(0xffffffffu, largest_w);
-        lost |= max(largest, largest_w) >= 0x7f800000u;
-
-        // ---- the state after the chunk
+        }
+        unsigned vh[2][4], vl[2][4];                      // V split, and as it joins the state
+        float v_down;
         {
-            const Scale s = scale_of(largest_w);
-            unsigned ah[2][4], al[2][4];
+            float m = 0.f;
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    split2(va[k][i][0] * wf[k][2 * (i >> 1)] * s.up, va[k][i][1] * wf[k][2 * (i >> 1) + 1] * s.up, ah[k][i], al[k][i]);
-            const float down = s.down * k_down;
+                for (int i = 0; i < 4; ++i) m = max_abs(m, va[k][i].x, va[k][i].y);
+            const unsigned largest = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+            lost |= largest >= 0x7f800000u;
+            const Scale s = scale_of(largest);
+            const pair up = pair_of(s.up, s.up);
+            v_down = s.down;
 #pragma unroll
-            for (int n = 0; n < NK; n += 2) {
-                float main[2][4] = {}, cross[2][4] = {};
+            for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    const int row = 16 * k + 8 * ((lane >> 3) & 1) + (lane & 7), col = KPW * kw + 8 * n + 8 * (lane >> 4);
-                    unsigned bh[4], bl[4];
-                    ldsm_t(bh, k_s + tile_at<DP>(row, col));
-                    ldsm_t(bl, k_s + CT * DP + tile_at<DP>(row, col));
-                    mma3(main[0], cross[0], ah[k], al[k], bh[0], bh[1], bl[0], bl[1]);
-                    mma3(main[1], cross[1], ah[k], al[k], bh[2], bh[3], bl[2], bl[3]);
-                }
-#pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    float2 d = make_float2(decay, decay);
-                    if constexpr (MODE == KEY_DECAY) d = *(const float2*)(rec + Rec::KEYS + KPW * kw + 8 * (n + m) + 2 * t4);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) S[n + m][i] = fmaf((i & 1) ? d.y : d.x, S[n + m][i], (main[m][i] + cross[m][i]) * down);
-                }
-            }
+                for (int i = 0; i < 4; ++i) split2(pair_of(va[k][i].x, va[k][i].y), up, vh[k][i], vl[k][i]);
         }
         // ---- P V of the tokens that the warp finishes
         float o[NT][4];
         if (KW <= 4 || kw < 4) {
-            const Scale s = scale_of(largest);
-            unsigned ah[2][4], al[2][4];
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) split2(va[k][i][0] * s.up, va[k][i][1] * s.up, ah[k][i], al[k][i]);
-            const float down = s.down * p_down;
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                float main[4] = {}, cross[4] = {};
+                float acc[3][4] = {};
                 const int row = 8 * (NT * kw + n) + (lane & 7);
                 unsigned bh[4], bl[4];                    // the four groups of eight tokens s
                 ldsm(bh, p_s + score_at(row, 8 * (lane >> 3)));
                 ldsm(bl, p_s + CT * CT + score_at(row, 8 * (lane >> 3)));
-                mma3(main, cross, ah[0], al[0], bh[0], bh[1], bl[0], bl[1]);
-                mma3(main, cross, ah[1], al[1], bh[2], bh[3], bl[2], bl[3]);
+                mma3(acc, vh[0], vl[0], bh[0], bh[1], bl[0], bl[1]);
+                mma3(acc, vh[1], vl[1], bh[2], bh[3], bl[2], bl[3]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) o[n][i] = (main[i] + cross[i]) * down;
+                for (int r = 0; r < 2; ++r) {
+                    const float2 x = sum3(acc, r);
+                    o[n][2 * r] = x.x; o[n][2 * r + 1] = x.y;
+                }
             }
         }
-        if constexpr (MODE == MATRIX_MEMORY) {            // q . n of the tokens: eight lanes a token, then n after the chunk
-            const float* n_old = n_s + (c & 1) * DP;
-            float* n_new = n_s + ((c + 1) & 1) * DP;
-            float* nq_s = n_s + 2 * DP + (c & 1) * CT;
-            for (int t = tid >> 3; t < CT; t += THREADS / 8) {
-                float s = 0.f;
-                for (int d = 8 * (lane & 7); d < DP; d += 64) {
-                    const uint4 h4 = *(const uint4*)(q_s + tile_at<DP>(t, d)), l4 = *(const uint4*)(q_s + CT * DP + tile_at<DP>(t, d));
-                    const __half2* h = reinterpret_cast<const __half2*>(&h4);
-                    const __half2* l = reinterpret_cast<const __half2*>(&l4);
+        const float p_down = v_down * rec[Rec::SCALARS + P_DOWN];
+        // ---- the state after the chunk
+        if constexpr (WEIGHTED) {
+            float m = 0.f;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float2 a = __half22float2(h[i]), b = __half22float2(l[i]), n = *(const float2*)(n_old + d + 2 * i);
-                        s = fmaf(a.x + b.x, n.x, s);
-                        s = fmaf(a.y + b.y, n.y, s);
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 w = *(const float2*)(rec + Rec::W + 16 * k + 2 * t4 + 8 * (i >> 1));
+                    va[k][i].x *= w.x; va[k][i].y *= w.y;
+                    m = max_abs(m, va[k][i].x, va[k][i].y);
+                }
+            const unsigned largest = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+            lost |= largest >= 0x7f800000u;
+            const Scale s = scale_of(largest);
+            const pair up = pair_of(s.up, s.up);
+            v_down = s.down;
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) split2(pair_of(va[k][i].x, va[k][i].y), up, vh[k][i], vl[k][i]);
+        }
+        {
+            float down = v_down * rec[Rec::SCALARS + K_DOWN], decay;
+            if constexpr (MODE == MATRIX_MEMORY) { decay = fac[3 * CT]; down *= fac[3 * CT + 1]; }
+            else decay = rec[Rec::SCALARS + DECAY];
+            const pair down2 = pair_of(down, down);
+            pair decay2 = pair_of(decay, decay);
+            constexpr int NB = NK < 4 ? NK : 4;           // groups of eight keys at a time
+#pragma unroll
+            for (int n = 0; n < NK; n += NB) {
+                float acc[NB][3][4] = {};
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int j = 0; j < NB / 2; ++j) {
+                        const int at = tile_at<DP>(16 * k + 8 * ((lane >> 3) & 1) + (lane & 7), KPW * kw + 8 * (n + 2 * j) + 8 * (lane >> 4));
+                        unsigned bh[4], bl[4];
+                        ldsm_t(bh, k_s + at);
+                        ldsm_t(bl, k_s + CT * DP + at);
+                        mma3(acc[2 * j], vh[k], vl[k], bh[0], bh[1], bl[0], bl[1]);
+                        mma3(acc[2 * j + 1], vh[k], vl[k], bh[2], bh[3], bl[2], bl[3]);
+                    }
+#pragma unroll
+                for (int j = 0; j < NB; ++j) {
+                    if constexpr (MODE == KEY_DECAY) {
+                        const float2 d = *(const float2*)(rec + Rec::KEYS + KPW * kw + 8 * (n + j) + 2 * t4);
+                        decay2 = pair_of(d.x, d.y);
+                    }
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const float2 y = sum3(acc[j], r);
+                        const float2 x = floats_of(fma2(decay2, pair_of(S[n + j][2 * r], S[n + j][2 * r + 1]), mul2(pair_of(y.x, y.y), down2)));
+                        S[n + j][2 * r] = x.x; S[n + j][2 * r + 1] = x.y;
                     }
                 }
-                s += __shfl_xor_sync(0xffffffffu, s, 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
-                s += __shfl_xor_sync(0xffffffffu, s, 4);
-                if ((lane & 7) == 0) nq_s[t] = s * q_down;
             }
-            for (int d = tid; d < DP; d += THREADS) n_new[d] = fmaf(decay, n_old[d], w_more * rec[Rec::KEYS + d]);
+            mark_largest(largest_of[0][slot_next]);
         }
-        if (p.stages > 2) copy_wait<1>(); else copy_wait<0>();       // the next chunk has landed
-        float skipped[NT][4];
-        if constexpr (MODE == HEAD_DECAY) {
+        slot3 = slot_next;
+        if constexpr (MODE == MATRIX_MEMORY) {
+            // q . n of sixteen tokens over the warp's keys (n is row 0 of a left operand), then n after the chunk
+            const float* n_old = n_s + (c & 1) * DP;
+            float* n_new = n_s + ((c + 1) & 1) * DP;
+            const unsigned n_largest = largest_of[1][slot_now];
+            lost |= n_largest >= 0x7f800000u;
+            const Scale sn = scale_of(n_largest);
+            if (cw < 2) {
+                float acc[2][3][4] = {};
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+                for (int k = 0; k < KS; ++k) {
+                    unsigned ah[4] = {}, al[4] = {}, bh[4], bl[4];
+                    if (g == 0) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    skipped[n][i] = skip * v_s[(8 * (NT * kw + n) + 2 * t4 + (i & 1)) * VP + 16 * cw + g + (i >> 1) * 8];
+                        for (int i = 0; i < 2; ++i) {
+                            const float2 x = *(const float2*)(n_old + KPW * kw + 16 * k + 8 * i + 2 * t4);
+                            split2(pair_of(x.x, x.y), pair_of(sn.up, sn.up), ah[2 * i], al[2 * i]);
+                        }
+                    }
+                    ldsm(bh, q_s + at_q[k] + cw * 16 * DP);
+                    ldsm(bl, q_s + CT * DP + at_q[k] + cw * 16 * DP);
+                    mma3(acc[0], ah, al, bh[0], bh[1], bl[0], bl[1]);
+                    mma3(acc[1], ah, al, bh[2], bh[3], bl[2], bl[3]);
+                }
+                if (g == 0) {
+                    float* to = nq_s + ((c & 1) * KW + kw) * CT + 16 * cw + 2 * t4;
+                    const float down = sn.down * rec[Rec::SCALARS + Q_DOWN];
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        const float2 x = sum3(acc[n], 0);
+                        *(float2*)(to + 8 * n) = make_float2(x.x * down, x.y * down);
+                    }
+                }
+            }
+            unsigned largest = 0;
+            for (int d = tid; d < DP; d += THREADS) {
+                const float x = fmaf(fac[3 * CT], n_old[d], fac[3 * CT + 1] * rec[Rec::KEYS + d]);
+                n_new[d] = x;
+                largest = max(largest, abs_bits(x));
+            }
+            largest = __reduce_max_sync(0xffffffffu, largest);
+            if (lane == 0) atomicMax(&largest_of[1][slot_next], largest);
         }
-        const float row_sum = MODE == MATRIX_MEMORY ? rec[Rec::SUMS + lane] : 0.f;
-        if constexpr (MODE != DELTA) {                    // the sums over the keys are complete, and this chunk's stage is free
-            lost = __syncthreads_or(lost);
+        wait_for(c + 1, stage, parity);
+        // what the read-outs take from this chunk's stage
+        float2 gt[NT], row_sum[NT], skipped[NT][2];
+        if constexpr (MODE != DELTA) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const int t = 8 * (NT * kw + n) + 2 * t4;
+                if constexpr (MODE == HEAD_DECAY) {
+                    gt[n] = *(const float2*)(rec + Rec::G + t);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+                        skipped[n][r] = make_float2(skip * v_s[t * VP + 16 * cw + g + 8 * r], skip * v_s[(t + 1) * VP + 16 * cw + g + 8 * r]);
+                }
+                if constexpr (MODE == MATRIX_MEMORY) {
+                    gt[n] = *(const float2*)(fac + (t & 31));
+                    row_sum[n] = *(const float2*)(rec + Rec::SUMS + (t & 31));
+                }
+            }
+            lost = __syncthreads_or(lost);                // the sums over the keys are complete, and this chunk's stage is free
             if (lost) break;
         }
-        float den_t = 1.f;
-        if constexpr (MODE == MATRIX_MEMORY) {
-            const float nq = p.out_scale * (gt * n_s[2 * DP + (c & 1) * CT + lane] + ht * row_sum);
-            den_t = fmaxf(fabsf(nq), den) + 1e-6f;
+        if constexpr (MODE == MATRIX_MEMORY) {            // the next chunk's factors (read behind the next barrier)
+            if (warp == 0 && c + 1 < n_chunks)
+                make_factors(reinterpret_cast<const float*>(smem + (size_t)stage * SH::STAGE + REC_AT), min(CT, t1 - tb - CT),
+                             factors + ((c + 1) & 1) * SH::FACTORS);
         }
         if (KW <= 4 || kw < 4) {
             float* out = p.out + (size_t)tb * p.out_stride + (size_t)head * p.vdim + col0;
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < NT; ++n) {
+                const int t = 8 * (NT * kw + n) + 2 * t4;
+                float2 fz = make_float2(q_down * p.out_scale, q_down * p.out_scale), fo = make_float2(p_down * p.out_scale, p_down * p.out_scale);
+                if constexpr (MODE == HEAD_DECAY) { fz.x *= gt[n].x; fz.y *= gt[n].y; }
+                if constexpr (MODE == MATRIX_MEMORY) {
+                    const float2 ht = *(const float2*)(fac + CT + t), floor = *(const float2*)(fac + 2 * CT + t);
+                    float2 nq = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < KW; ++k) {
+                        const float2 a = *(const float2*)(nq_s + ((c & 1) * KW + k) * CT + t);
+                        nq.x += a.x; nq.y += a.y;
+                    }
+                    const float rx = 1.f / (fmaxf(fabsf(p.out_scale * (gt[n].x * nq.x + ht.x * row_sum[n].x)), floor.x) + 1e-6f);
+                    const float ry = 1.f / (fmaxf(fabsf(p.out_scale * (gt[n].y * nq.y + ht.y * row_sum[n].y)), floor.y) + 1e-6f);
+                    fz.x *= gt[n].x * rx; fz.y *= gt[n].y * ry; fo.x *= ht.x * rx; fo.y *= ht.y * ry;
+                }
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const int t = 8 * (NT * kw + n) + 2 * t4, col = 16 * cw + g + 8 * r;
-                    float2 z = make_float2(0.f, 0.f);
-                    if constexpr (MODE == DELTA) z = *(const float2*)(extra + (COLS + col) * TP + t);
-                    else {
+                    const int col = 16 * cw + g + 8 * r;
+                    float2 x;
+                    if constexpr (MODE == DELTA) {
+                        const float2 z = *(const float2*)(extra + (COLS + col) * TP + t);
+                        x = make_float2(fmaf(fo.x, o[n][2 * r], p.out_scale * z.x), fmaf(fo.y, o[n][2 * r + 1], p.out_scale * z.y));
+                    } else {
+                        float2 z = make_float2(0.f, 0.f);
 #pragma unroll
                         for (int k = 0; k < KW; ++k) {
                             const float2 a = *(const float2*)(sum + (k * COLS + col) * TP + t);
                             z.x += a.x; z.y += a.y;
                         }
+                        x = make_float2(fmaf(fz.x, z.x, fo.x * o[n][2 * r]), fmaf(fz.y, z.y, fo.y * o[n][2 * r + 1]));
+                        if constexpr (MODE == HEAD_DECAY) { x.x += skipped[n][r].x; x.y += skipped[n][r].y; }
                     }
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        float x;
-                        if constexpr (MODE == DELTA) x = p.out_scale * ((e ? z.y : z.x) + o[n][2 * r + e]);
-                        else {
-                            x = p.out_scale * fmaf(__shfl_sync(0xffffffffu, gt, t + e), e ? z.y : z.x,
-                                                   MODE == MATRIX_MEMORY ? __shfl_sync(0xffffffffu, ht, t + e) * o[n][2 * r + e] : o[n][2 * r + e]);
-                            if constexpr (MODE == HEAD_DECAY) x += skipped[n][2 * r + e];
-                            if constexpr (MODE == MATRIX_MEMORY) x /= __shfl_sync(0xffffffffu, den_t, t + e);
-                        }
-                        if (t + e < len && col < n_cols) out[(size_t)(t + e) * p.out_stride + col] = x;
+                    if (col < n_cols) {
+                        if (t < len) out[(size_t)t * p.out_stride + col] = x.x;
+                        if (t + 1 < len) out[(size_t)(t + 1) * p.out_stride + col] = x.y;
                     }
                 }
+            }
         }
         if constexpr (MODE == DELTA) {                    // (the stage, the sums and u are free)
             lost = __syncthreads_or(lost);
@@ -612,6 +757,10 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
     }
     copy_wait<0>();
     if (lost) {                                           // the slot is as it was, and the columns go token by token
+        if (tid == 0)                                     // (copies in flight land before the block leaves)
+            for (int x = c + 1; x < min(c + p.stages, n_chunks); ++x)
+                tc::mbar_drain(tc::smem_u32(&full[x % p.stages]), (x / p.stages) & 1, waits.limit_cycles);
+        __syncthreads();
         if (tid < CW && col0 / 16 + tid < p.column_groups) p.columns[((size_t)seg * p.heads + head) * p.column_groups + col0 / 16 + tid] = 1;
         return;
     }
@@ -632,7 +781,7 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p) 
 }
 
 template <int KPW, int KW, int CW, int MODE>
-int launch_walk(Walk p, cudaStream_t st) {
+int launch_walk(Walk p, const tc::WaitControl& waits, cudaStream_t st) {
     using SH = Shape<KPW, KW, CW, MODE>;
     dim3 grid((p.vdim + SH::COLS - 1) / SH::COLS, p.heads, p.n_segments);
     // three stages where a multiprocessor holds one block anyway, two where two blocks then fit
@@ -642,7 +791,7 @@ int launch_walk(Walk p, cudaStream_t st) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::bytes(three ? 3 : 2)) != cudaSuccess)
         return SPITE_LAUNCH_FAILED;
     // (in the ordinary way: started early, the blocks would sit on the multiprocessors of the kernel before, several to one)
-    kernel<<<grid, SH::THREADS, SH::bytes(p.stages), st>>>(p);
+    kernel<<<grid, SH::THREADS, SH::bytes(p.stages), st>>>(p, waits);
     return spite_launch_status();
 }
 

@@ -24,6 +24,8 @@
 // 1 - beta k k^T never lengthen a vector.  `delta_chunk_kernel` makes Q, K, T beta K, P and T' beta V for all chunks and heads at once.
 #include "chunk.cuh"
 
+SPITE_WAIT_CONTROLS(delta, chunk::walk_error)
+
 struct DeltaParams {
     const float* x;             // [tokens, stride]
     long long stride;
@@ -531,8 +533,8 @@ int launch_delta_chunks(const DeltaParams& p, const Made& out, int n_chunks, cud
     // 16 columns a block while that leaves every multiprocessor one block at most, else 32.  2,048 tokens, us of the walk alone: 16 heads
     // (128 blocks of 16 columns) 124, with 16 keys a warp and twice the warps 135; 32 heads (128 blocks of 32) 165.  The kernel before it: 39
     // and 70 (a block a head instead of two: 69 and 111).
-    if ((long long)((p.vdim + 15) / 16) * p.heads * p.n_segments <= 148) return launch_walk<32, DP / 32, 1, DELTA>(w, st);
-    return launch_walk<32, DP / 32, 2, DELTA>(w, st);
+    if ((long long)((p.vdim + 15) / 16) * p.heads * p.n_segments <= 148) return launch_walk<32, DP / 32, 1, DELTA>(w, s_waits, st);
+    return launch_walk<32, DP / 32, 2, DELTA>(w, s_waits, st);
 }
 
 int check_delta(const DeltaParams* p) {

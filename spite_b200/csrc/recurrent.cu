@@ -16,6 +16,8 @@
 // read and one write of the state (a lane moves 8 consecutive floats of a key row: whole 32-byte sectors).
 #include "chunk.cuh"
 
+SPITE_WAIT_CONTROLS(recurrent, chunk::walk_error)
+
 struct MlstmParams {
     const float* proj;          // [tokens, stride]: the projection's float32 output
     long long stride;
@@ -581,8 +583,8 @@ int launch_mlstm_chunk(const MlstmParams& p, float* scratch, int scratch_chunks,
 
 // ---- the same in chunks of 32 tokens on the tensor cores (chunk.cuh), for up to 256 key rows.  What a chunk needs that does not depend on
 // the state, one block a (chunk, head): q and k as split tiles; a_s, F_t and the running maximum M_t of a_s within the chunk (m0
-// joins in the walk: max(m0, M_t)); the scores exp(a_s - M_t) q_t . k_s (s <= t) as a split tile, and their sums over s; the weights
-// exp(a_s - M_last) and sum_s of them times k_s, which n takes.
+// joins in the walk: max(m0, M_t)); the scores exp(a_s - M_t) q_t . k_s (s <= t) as a split tile, and their sums over s; k_s times its
+// weight exp(a_s - M_last) as a split tile, which the state takes, and the sum of those, which n takes.
 template <int DP> struct MemoryChunkSmem {
     __half qk[4][chunk::CT * DP];
     float P[chunk::CT][36], kn[8][DP], w[chunk::CT];
@@ -726,6 +728,14 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, 
         for (int i = 0; i < 8; ++i) sum += sm.kn[i][d];
         rec[Rec::KEYS + d] = sum;
     }
+#pragma unroll
+    for (int e = 0; e < E; ++e)                           // the scores are made: k takes its weights (at most one, so the scale holds)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = warp + 8 * i, at = tile_at<DP>(t, lane + 32 * e);
+            split1(sm.w[t] * kv[i][e] * sk.up, sm.qk[2][at], sm.qk[3][at]);
+        }
+    __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(out.qk + at_head * (4 * CL * DP));
     const uint4* src = reinterpret_cast<const uint4*>(sm.qk[0]);
 #pragma unroll 4
@@ -755,7 +765,7 @@ int launch_memory_chunks(const MlstmParams& p, const chunk::Made& out, int n_chu
     w.cu_seqlens = p.cu_seqlens; w.slots = p.slots;
     w.n_segments = p.n_segments; w.heads = p.heads; w.qk_heads = p.heads; w.dim = p.dim; w.vdim = p.vdim;
     w.out_scale = p.q_scale;
-    return chunk::launch_walk<KPW, DP / KPW, 2, chunk::MATRIX_MEMORY>(w, st);
+    return chunk::launch_walk<KPW, DP / KPW, 2, chunk::MATRIX_MEMORY>(w, s_waits, st);
 }
 
 int check_mlstm(const MlstmParams* p) {

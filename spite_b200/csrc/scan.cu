@@ -28,6 +28,8 @@
 // No exponent is ever positive.  The kernels below make these for all chunks and heads of a step at once.
 #include "chunk.cuh"
 
+SPITE_WAIT_CONTROLS(scan, chunk::walk_error)
+
 struct ScanParams {
     const float* q; const float* k; const float* v;       // first element of token 0's q, k [kv_heads * dim], v [heads * vdim]
     long long q_stride, k_stride, v_stride;               // floats between two tokens' rows
@@ -810,8 +812,8 @@ int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_s
     chunk::Walk w = scan_walk(p, out);
     w.skip = p.skip;
     // 32 columns a block while that leaves every multiprocessor one block at most, else 64
-    if (one_wave(p, 32)) return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, st);
-    return launch_walk<DP / 2, 2, 4, HEAD_DECAY>(w, st);
+    if (one_wave(p, 32)) return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, s_waits, st);
+    return launch_walk<DP / 2, 2, 4, HEAD_DECAY>(w, s_waits, st);
 }
 template <int DP, bool BONUS>
 int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, cudaStream_t st) {
@@ -822,8 +824,8 @@ int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, 
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
     chunk::Walk w = scan_walk(p, out);
     w.out_scale = BONUS ? 1.f : p.out_scale;
-    if (one_wave(p, 32)) return launch_walk<32, DP / 32, 2, KEY_DECAY>(w, st);
-    return launch_walk<32, DP / 32, DP == 64 ? 4 : 2, KEY_DECAY>(w, st);
+    if (one_wave(p, 32)) return launch_walk<32, DP / 32, 2, KEY_DECAY>(w, s_waits, st);
+    return launch_walk<32, DP / 32, DP == 64 ? 4 : 2, KEY_DECAY>(w, s_waits, st);
 }
 template <bool BONUS, int WALK>
 int key_decay_in_chunks(const ScanParams& p, void* scratch, int n_chunks, int min_tokens, cudaStream_t st) {

@@ -153,7 +153,8 @@ class SampleParams(C.Structure):
 # Libraries whose kernels wait on mbarriers with a limit.  A kernel that gives up records a code in its
 # library's word of one small buffer in pinned host memory, which the device writes directly: the host
 # reads it after any point at which it has waited for a step's results, without another copy or wait.
-_WAITING_LIBRARIES = ("gemm_tc", "gemm_tc_pair", "gemm_stream", "attention_tc", "attention_decode", "gemm_tc_experts")
+_WAITING_LIBRARIES = ("gemm_tc", "gemm_tc_pair", "gemm_stream", "attention_tc", "attention_decode", "gemm_tc_experts", "delta",
+                      "recurrent", "scan")
 _error_words = None          # pinned int32 [len(_WAITING_LIBRARIES)], one per process
 _configured: set = set()
 

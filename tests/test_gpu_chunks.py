@@ -362,3 +362,33 @@ def test_scan_and_memory_entry_points_refuse_malformed_calls():
     assert tiles(dim=300, stride=1000, head_stride=1 << 14) == -2 and tiles(n_segments=0) == 0
     torch.cuda.synchronize()
     assert not t.any()
+
+
+def test_a_wait_that_runs_out_is_reported_and_the_tokens_are_walked():
+    """The first stage is announced 16 bytes more than its copies deliver, with waits of two milliseconds: every block of the walk in
+    chunks gives up, says so, and leaves its columns to the walk token by token."""
+    heads, dim, vdim, n = 2, 64, 32, 70
+    ks = kernels(torch.bfloat16)
+    g = torch.Generator().manual_seed(8)
+    batch, M = step_batch([n], [0], True)
+    cols = (0, dim * heads, 2 * dim * heads, 2 * dim * heads + heads * vdim, 2 * dim * heads + heads * vdim + heads)
+    x = torch.randn((M, cols[4] + heads), generator=g).to(DEV)
+    zero = torch.zeros(heads, device=DEV)
+
+    def run(chunked):
+        state, out = torch.zeros((1, heads * dim * vdim), device=DEV), torch.empty((M, heads * vdim), device=DEV)
+        ks.delta_scan(x, out, batch, state, heads=heads, kv_heads=heads, dim=dim, vdim=vdim, columns=cols, a_log=zero, dt_bias=zero, q_scale=1.0,
+                      chunked=chunked)
+        torch.cuda.synchronize()
+        return out, state
+    want = run(False)
+    assert ks.errors() == {}
+    ks.configure_waits("delta", limit_cycles=4_000_000, extra_tx=16)
+    try:
+        got = run(True)
+    finally:
+        ks.configure_waits("delta")
+    assert ks.errors() == {"delta": 2} and ks.errors() == {}
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    near(run(True)[0], want[0].double(), "with the default waits")
+    assert ks.errors() == {}
