@@ -781,6 +781,101 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvParams p
     }
 }
 
+// The same for segments of several tokens whose columns are whole groups of four: a thread has four columns and CONV_ROWS tokens, all of
+// whose inputs it asks for before it uses the first (the kernel above has one load of four bytes in flight a thread, which left it at a
+// third of the copy bandwidth).  The sums are the same, term by term.
+constexpr int CONV_ROWS = 8;
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128) short_conv_rows_kernel(const ShortConvParams p) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= p.channels + p.copy_columns) return;
+    const int s = blockIdx.y, t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0, i0 = blockIdx.z * CONV_ROWS;
+    if (i0 >= n) return;
+    const int slot = p.slots[s];
+    if (s > 0 && slot == p.slots[0]) return;                  // (the first row's thread writes its copies, as above)
+    const int rows = min(CONV_ROWS, n - i0);
+    const float* x = p.x + (size_t)(t0 + i0) * p.x_stride + c;
+    T* out = (T*)p.out + (size_t)(t0 + i0) * p.out_stride + c;
+    const bool conv = c < p.channels;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 in[TAPS - 1 + CONV_ROWS];                          // in[TAPS - 1 + i]: token i0 + i
+    float* st = p.state + (size_t)slot * p.slot_stride + c;
+    float4 old[TAPS > 1 ? TAPS - 1 : 1];
+#pragma unroll
+    for (int k = 0; k < TAPS - 1; ++k) {
+        old[k] = conv && i0 == 0 ? *(const float4*)(st + (size_t)k * p.channels) : zero;
+        in[k] = !conv ? zero : i0 == 0 ? old[k] : *(const float4*)(x - (size_t)(TAPS - 1 - k) * p.x_stride);
+    }
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i) in[TAPS - 1 + i] = i < rows ? *(const float4*)(x + (size_t)i * p.x_stride) : zero;
+    if (!conv) {
+#pragma unroll
+        for (int i = 0; i < CONV_ROWS; ++i)
+            if (i < rows) store4(out + (size_t)i * p.out_stride, in[TAPS - 1 + i].x, in[TAPS - 1 + i].y, in[TAPS - 1 + i].z, in[TAPS - 1 + i].w);
+    } else {
+        float w[4][TAPS];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) w[e][j] = p.w[(size_t)(c + e) * TAPS + j];
+        const float4 bias = p.bias ? make_float4(p.bias[c], p.bias[c + 1], p.bias[c + 2], p.bias[c + 3]) : zero;
+#pragma unroll
+        for (int i = 0; i < CONV_ROWS; ++i) {
+            if (i >= rows) break;
+            float4 a = zero;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                a.x = fmaf(w[0][j], in[i + j].x, a.x); a.y = fmaf(w[1][j], in[i + j].y, a.y);
+                a.z = fmaf(w[2][j], in[i + j].z, a.z); a.w = fmaf(w[3][j], in[i + j].w, a.w);
+            }
+            a.x += bias.x; a.y += bias.y; a.z += bias.z; a.w += bias.w;
+            if (p.activation == 1) {
+                a.x = a.x / (1.0f + expf(-a.x)); a.y = a.y / (1.0f + expf(-a.y));
+                a.z = a.z / (1.0f + expf(-a.z)); a.w = a.w / (1.0f + expf(-a.w));
+            }
+            store4(out + (size_t)i * p.out_stride, a.x, a.y, a.z, a.w);
+        }
+        if (i0 == 0) {                                        // the slot's next content: the last TAPS - 1 inputs of the sequence so far
+#pragma unroll
+            for (int k = 0; k < TAPS - 1; ++k) {
+                const int idx = n - (TAPS - 1) + k;
+                float4 v = zero;
+                if (idx >= 0) v = *(const float4*)(x + (size_t)idx * p.x_stride);
+                else {
+#pragma unroll
+                    for (int kk = 0; kk < TAPS - 1; ++kk) if (kk == TAPS - 1 + idx) v = old[kk];
+                }
+                *(float4*)(st + (size_t)k * p.channels) = v;
+            }
+        }
+    }
+    if (s == 0 && i0 == 0) {
+        for (int s2 = 1; s2 < p.n_segments; ++s2) {
+            if (p.slots[s2] != slot) continue;
+            const int u0 = p.cu_seqlens[s2], m = min(p.cu_seqlens[s2 + 1] - u0, rows);
+            for (int i = 0; i < m; ++i)
+                for (int e = 0; e < 4; ++e) ((T*)p.out)[(size_t)(u0 + i) * p.out_stride + c + e] = out[(size_t)i * p.out_stride + e];
+        }
+    }
+}
+// Fewer tokens than this in every segment: the kernel above, whose threads have one column each (decode steps)
+constexpr int CONV_ROWS_MIN = 4;
+template <typename T>
+static void launch_short_conv_rows(const ShortConvParams& p, dim3 grid, cudaStream_t st) {
+    switch (p.taps) {
+        case 1: SPITE_LAUNCH((short_conv_rows_kernel<T, 1>), grid, 128, 0, st, p); break;
+        case 2: SPITE_LAUNCH((short_conv_rows_kernel<T, 2>), grid, 128, 0, st, p); break;
+        case 3: SPITE_LAUNCH((short_conv_rows_kernel<T, 3>), grid, 128, 0, st, p); break;
+        case 4: SPITE_LAUNCH((short_conv_rows_kernel<T, 4>), grid, 128, 0, st, p); break;
+        case 5: SPITE_LAUNCH((short_conv_rows_kernel<T, 5>), grid, 128, 0, st, p); break;
+        case 6: SPITE_LAUNCH((short_conv_rows_kernel<T, 6>), grid, 128, 0, st, p); break;
+        case 7: SPITE_LAUNCH((short_conv_rows_kernel<T, 7>), grid, 128, 0, st, p); break;
+        default: SPITE_LAUNCH((short_conv_rows_kernel<T, 8>), grid, 128, 0, st, p);
+    }
+}
+
 SPITE_API int spite_short_conv(int out_dtype, const ShortConvParams* p, void* stream) {
     if (!p || !p->x || !p->w || !p->out || !p->state || !p->cu_seqlens || !p->slots) return SPITE_BAD_ARG;
     if (p->n_segments < 0 || p->channels < 1 || p->taps < 1 || p->copy_columns < 0 || p->max_seg_len < 0) return SPITE_BAD_ARG;
@@ -791,6 +886,14 @@ SPITE_API int spite_short_conv(int out_dtype, const ShortConvParams* p, void* st
     if (p->taps > CONV_MAX_TAPS || p->n_segments > 65535) return SPITE_UNSUPPORTED;
     if (p->n_segments == 0 || p->max_seg_len == 0) return SPITE_OK;
     const int cols = p->channels + p->copy_columns;
+    const int rows_zb = (p->max_seg_len + CONV_ROWS - 1) / CONV_ROWS;
+    if (p->max_seg_len >= CONV_ROWS_MIN && rows_zb <= 65535 && p->channels % 4 == 0 && p->copy_columns % 4 == 0 && p->x_stride % 4 == 0 &&
+        p->out_stride % 4 == 0 && p->slot_stride % 4 == 0 && (((uintptr_t)p->x | (uintptr_t)p->out | (uintptr_t)p->state) & 15) == 0) {
+        dim3 grid((cols / 4 + 127) / 128, p->n_segments, rows_zb);
+        if (out_dtype == SPITE_DT_F32) launch_short_conv_rows<float>(*p, grid, (cudaStream_t)stream);
+        else launch_short_conv_rows<__nv_bfloat16>(*p, grid, (cudaStream_t)stream);
+        return spite_launch_status();
+    }
     const int zb = (p->max_seg_len + CONV_TB - 1) / CONV_TB;
     if (zb > 65535) return SPITE_UNSUPPORTED;
     dim3 grid((cols + 127) / 128, p->n_segments, zb);
@@ -933,6 +1036,46 @@ __global__ void __launch_bounds__(256) gate_group_norm_kernel(const float* __res
     }
 }
 
+// The same with a part in registers (up to 4 x 256 x NV elements in groups of four): every load is asked for before the first is used, and
+// nothing passes through shared memory.  The sums are the same, term by term.
+template <typename T, int NV>
+__global__ void __launch_bounds__(256) gate_group_norm_reg_kernel(const float* __restrict__ x, const float* __restrict__ z, long long z_stride,
+                                                                  const float* __restrict__ gain, T* __restrict__ out, int groups, int size,
+                                                                  float eps) {
+    __shared__ float scratch[33];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int m = blockIdx.x, g = blockIdx.y;
+    const float* xr = x + ((size_t)m * groups + g) * size;
+    const float* zr = z + (size_t)m * z_stride + (size_t)g * size;
+    const float* w = gain + (size_t)g * size;
+    T* o = out + ((size_t)m * groups + g) * size;
+    float4 v[NV], b[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = 4 * (threadIdx.x + i * blockDim.x);
+        v[i] = c < size ? *(const float4*)(xr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        b[i] = c < size ? *(const float4*)(zr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        if (4 * (threadIdx.x + i * blockDim.x) >= size) break;
+        v[i].x *= b[i].x / (1.0f + expf(-b[i].x)); v[i].y *= b[i].y / (1.0f + expf(-b[i].y));
+        v[i].z *= b[i].z / (1.0f + expf(-b[i].z)); v[i].w *= b[i].w / (1.0f + expf(-b[i].w));
+        s += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+    }
+    s = block_sum(s, scratch);
+    const float mul = 1.0f / sqrtf(s / (float)size + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = 4 * (threadIdx.x + i * blockDim.x);
+        if (c >= size) break;
+        const float4 f = *(const float4*)(w + c);
+        store4(o + c, v[i].x * mul * f.x, v[i].y * mul * f.y, v[i].z * mul * f.z, v[i].w * mul * f.w);
+    }
+}
+
 template <typename K>
 static int raise_smem_limit(K kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return SPITE_OK;
@@ -953,6 +1096,18 @@ SPITE_API int spite_gate_group_norm(int out_dtype, const float* x, const float* 
     const int threads = work <= 32 ? 32 : work <= 64 ? 64 : work <= 128 ? 128 : 256;
     dim3 grid(n_tokens, groups);
     cudaStream_t st = (cudaStream_t)stream;
+    if (vec && work <= 8 * threads) {
+#define SPITE_GGN_REG(T, NV) SPITE_LAUNCH((gate_group_norm_reg_kernel<T, NV>), grid, threads, 0, st, x, z, z_stride, gain, (T*)out, groups, size, eps)
+#define SPITE_GGN_ANY(T)                                                                                                    \
+        if (work <= threads) SPITE_GGN_REG(T, 1);                                                                           \
+        else if (work <= 2 * threads) SPITE_GGN_REG(T, 2);                                                                  \
+        else if (work <= 4 * threads) SPITE_GGN_REG(T, 4);                                                                  \
+        else SPITE_GGN_REG(T, 8)
+        if (out_dtype == SPITE_DT_F32) { SPITE_GGN_ANY(float); } else { SPITE_GGN_ANY(__nv_bfloat16); }
+#undef SPITE_GGN_ANY
+#undef SPITE_GGN_REG
+        return spite_launch_status();
+    }
 #define SPITE_GGN(T, V)                                                                                                     \
     if (raise_smem_limit(gate_group_norm_kernel<T, V>, bytes) != SPITE_OK) return SPITE_LAUNCH_FAILED;                      \
     SPITE_LAUNCH((gate_group_norm_kernel<T, V>), grid, threads, bytes, st, x, z, z_stride, gain, (T*)out, groups, size, eps)

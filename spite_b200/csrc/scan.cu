@@ -609,7 +609,7 @@ template <int DP> struct KeyDecayChunkSmem {
     __half tiles[4 * CT * DP], off[2 * CT * DP];          // `off`: rows 0 .. 15 k of the first half, 16 .. 31 q of the second, brought to the border
     float q[CT][DP + 4], k[CT][DP + 4], w[CT][DP + 4];
     float P[CT][36];
-    double part[256 / DP][DP];                            // sums of log decays of a thread's tokens
+    float part[256 / DP][DP];                             // sums of log decays of a thread's tokens
     unsigned largest[5];                                  // of q and k in `tiles`, k and q in `off`, the scores
     int bad;
 };
@@ -631,8 +631,7 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
     if (tid == 5) sm.bad = 0;
     const size_t at_head = (size_t)blockIdx.x * p.heads + head;
     const int ch = tid % DP, part = tid / DP;
-    float qv[TN], kv[TN];
-    double cum[TN];                                       // sum of the log decays up to the token, within the thread's tokens at first
+    float qv[TN], kv[TN], lw[TN];                         // q, k and the log decays
     bool bad = false;
     {
         const float* q = p.q + (size_t)first * p.q_stride + (size_t)head * dim + ch;
@@ -647,37 +646,50 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
             kv[i] = on ? k[(size_t)t * p.k_stride] : 0.f;
             wv[i] = on ? w[(size_t)t * p.w_stride] : 1.f;
         }
-        double sum = 0.0;
+        float sum = 0.f;
 #pragma unroll
         for (int i = 0; i < TN; ++i) {
             const int t = part * TN + i;
             sm.q[t][ch] = qv[i]; sm.k[t][ch] = kv[i]; sm.w[t][ch] = wv[i];
             bad |= !(wv[i] >= 0.f && wv[i] <= 1.f);
-            sum += (double)bounded_log(logf(wv[i]));
-            cum[i] = sum;
+            lw[i] = bounded_log(logf(wv[i]));
+            sum += lw[i];
         }
         sm.part[part][ch] = sum;
     }
     for (int e = tid; e < CT * CT; e += 256) sm.P[e / CT][e % CT] = 0.f;
     __syncthreads();
     {
-        double before = 0.0, border = 0.0, last = 0.0;
+        // Sums of log decays from the chunk's start to a token, from behind it to the end, and between it and the border: each is made
+        // from its own end, so that a small one has no large one's rounding in it.
+        constexpr int HALF = PARTS / 2;
+        float before = 0.f, after = 0.f, inner = 0.f, last = 0.f;     // over the parts before, behind, and between this one and the border
 #pragma unroll
         for (int i = 0; i < PARTS; ++i) {
-            const double s = sm.part[i][ch];
+            const float s = sm.part[i][ch];
             if (i < part) before += s;
-            if (i < PARTS / 2) border += s;
+            if (i > part) after += s;
+            if (part < HALF ? i > part && i < HALF : i >= HALF && i < part) inner += s;
             last += s;
         }
         float qs[TN], ks[TN], os[TN];
         unsigned lq = 0, lk = 0, lo = 0;
+        float run = 0.f, back = 0.f;
+#pragma unroll
+        for (int i = 0; i < TN; ++i) {                    // (a token of the memory is read before its own decay)
+            if (!BONUS) run += lw[i];
+            qs[i] = qv[i] * expf(before + run);
+            if (part >= HALF) os[i] = qv[i] * expf(inner + run);
+            if (BONUS) run += lw[i];
+        }
+#pragma unroll
+        for (int i = TN - 1; i >= 0; --i) {
+            ks[i] = kv[i] * expf(after + back);
+            if (part < HALF) os[i] = kv[i] * expf(inner + back);
+            back += lw[i];
+        }
 #pragma unroll
         for (int i = 0; i < TN; ++i) {
-            const double c = before + cum[i];             // (a token of the memory is read before its own decay)
-            const double cq = BONUS ? before + (i ? cum[i ? i - 1 : 0] : 0.0) : c;
-            qs[i] = qv[i] * expf((float)cq);
-            ks[i] = kv[i] * expf((float)(last - c));
-            os[i] = part < PARTS / 2 ? kv[i] * expf((float)(border - c)) : qv[i] * expf((float)(cq - border));
             lq = max(lq, abs_bits(qs[i])); lk = max(lk, abs_bits(ks[i])); lo = max(lo, abs_bits(os[i]));
             bad |= max(abs_bits(qv[i]), abs_bits(kv[i])) >= 0x7f800000u;
         }
@@ -699,7 +711,7 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
             split1(os[i] * so.up, sm.off[at], sm.off[CT * DP + at]);
         }
         float* rec = out.records + at_head * Rec::FLOATS;
-        if (part == 0) rec[Rec::KEYS + ch] = ch < dim ? expf((float)last) : 0.f;
+        if (part == 0) rec[Rec::KEYS + ch] = ch < dim ? expf(last) : 0.f;
         if (tid < CT) { rec[Rec::G + tid] = 1.f; rec[Rec::W + tid] = 1.f; }
     }
     // ---- scores within a half of the chunk: a warp has four tokens s, its lanes the channels
@@ -824,8 +836,9 @@ int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, 
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
     chunk::Walk w = scan_walk(p, out);
     w.out_scale = BONUS ? 1.f : p.out_scale;
-    if (one_wave(p, 32)) return launch_walk<32, DP / 32, 2, KEY_DECAY>(w, s_waits, st);
-    return launch_walk<32, DP / 32, DP == 64 ? 4 : 2, KEY_DECAY>(w, s_waits, st);
+    // (32 columns a block; with 64, 32 heads of 64 x 128: five requests of 2,048 tokens together 68 us against 62, four of 2,048 each 205
+    // against 231)
+    return launch_walk<32, DP / 32, 2, KEY_DECAY>(w, s_waits, st);
 }
 template <bool BONUS, int WALK>
 int key_decay_in_chunks(const ScanParams& p, void* scratch, int n_chunks, int min_tokens, cudaStream_t st) {
