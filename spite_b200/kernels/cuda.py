@@ -301,11 +301,15 @@ class CudaKernels(KernelSet):
         # Scout shapes, one token 2.90 ms with (110 KiB, 2 per multiprocessor) against 3.01 with (74 KiB, 3), eight
         # tokens 7.10 against 7.02, sixty-four alike; one block per multiprocessor with 110 or 200 KiB: 3.2 and 3.1 ms
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
-        # Recurrences over prompts: segments of at least so many tokens go in chunks of 32 on the tensor cores, the others token by
-        # token.  Delta rule, 16 heads of 128 x 128, us in chunks / token by token: one prompt of 32 tokens 21 / 24, 64:
-        # 23 / 42, 512: 52 / 291, 2,048: 170 / 1,147; sixteen prompts of 16: 59 / 52, of 32: 61 / 95.
+        # Recurrences over prompts: a step whose longest segment has at least so many tokens goes in chunks of 32 on the tensor cores (its
+        # segments of fewer than 32 tokens, 8 in the matrix memory, token by token).  us in chunks / token by token.  Delta rule, 16 heads
+        # of 128 x 128: one prompt of 32 tokens 21 / 24, 64: 23 / 42, 512: 45 / 291, 2,048: 152 / 1,147; sixteen prompts of 32: 64 / 95.
+        # Matrix memory, 8 heads of 256 x 512: 16 tokens 19 / 21, 2,048: 224 / 3,150.  State space, 128 heads of 128 x 64: 64 tokens
+        # 26 / 18, 128: 31 / 30, 512: 63 / 99, 2,048: 206 / 378.  Gated linear attention, 32 heads of 64 x 128: 256 tokens 35 / 32, 512:
+        # 48 / 59, 2,048: 155 / 223; sixteen prompts of 128: 139 / 133.
+        self.chunk_from = {"delta": 32, "memory": 8, "state_space": 160, "linear_attention": 320, "decaying_memory": 1024}
         self.chunk_min_tokens = 32
-        self.memory_min_tokens = 8             # ... the matrix memory's
+        self.memory_min_tokens = 8
         # how much working memory a call may take for that (a step of 8,192 tokens of 32 heads of 128 x 128 takes 0.45 GB); a call that
         # would need more goes token by token
         self.chunk_scratch_limit = 1 << 30
@@ -1172,7 +1176,7 @@ class CudaKernels(KernelSet):
         if chunked is None:
             # Prompts and their portions go 32 tokens at a time.  The float32 set keeps the walk token by token for
             # every step, so that its results do not depend on how a prompt was cut, to the last bit.
-            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.memory_min_tokens
+            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from["memory"]
         p = MlstmParams(proj=proj.data_ptr(), stride=proj.shape[1], q_col=q_col, k_col=k_col, v_col=v_col, i_col=i_col,
                         f_col=f_col, i_bias=i_bias.data_ptr(), f_bias=f_bias.data_ptr(), out=out.data_ptr(),
                         state=state.data_ptr(), head_stride=state.shape[2], cu_seqlens=batch.cu_seqlens.data_ptr(),
@@ -1228,7 +1232,7 @@ class CudaKernels(KernelSet):
         if chunked is None:
             # Prompts and their portions go 32 tokens at a time.  The float32 set keeps the walk token by token for every step,
             # so that its results do not depend on how a prompt was cut, to the last bit.
-            chunked = split_rows is None and self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_min_tokens
+            chunked = split_rows is None and self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from["delta"]
         if chunked:
             n_chunks = (M + 31) // 32 + n_seg
             scratch = self._chunk_scratch("delta", "spite_delta_chunk_bytes", dim, vdim, heads, kv_heads, M, n_chunks, n_seg)
@@ -1269,12 +1273,12 @@ class CudaKernels(KernelSet):
                        dim=int(dim), vdim=int(vdim))
         return p, scalars
 
-    def _run_scan(self, entry, p, batch, kv_heads, per_channel, chunked, *rest):
+    def _run_scan(self, kind, entry, p, batch, kv_heads, per_channel, chunked, *rest):
         """One of the three walks: in chunks where that is asked for or pays and the sizes allow it, else token by token."""
         lib = self._lib("scan")
         if chunked is None:
             # (the float32 set keeps the walk token by token, so that its results do not depend on how a prompt was cut)
-            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_min_tokens
+            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from[kind]
         if chunked:
             n_chunks = (p.n_tokens + 31) // 32 + p.n_segments
             scratch = self._chunk_scratch("scan", "spite_scan_chunk_bytes", per_channel, p.dim, p.vdim, p.heads, kv_heads, n_chunks, p.n_segments)
@@ -1299,7 +1303,7 @@ class CudaKernels(KernelSet):
         self._t(t, torch.float32, "step")
         a = self._columns(t, column, heads, out.shape[0], "state_space_scan: step")
         p.skip = skip.data_ptr()
-        self._run_scan("spite_state_space_scan", p, batch, kv_heads, False, chunked, C.c_void_p(a), C.c_longlong(t.shape[1]),
+        self._run_scan("state_space", "spite_state_space_scan", p, batch, kv_heads, False, chunked, C.c_void_p(a), C.c_longlong(t.shape[1]),
                        C.c_void_p(a_log.data_ptr()), C.c_void_p(dt_bias.data_ptr()))
 
     def decay_scan(self, r, k, v, w, out, batch, state, *, heads, dim, vdim, w0, u, state_offset=0, chunked=None):
@@ -1312,7 +1316,7 @@ class CudaKernels(KernelSet):
             if self._t(t, torch.float32, name).numel() != heads * dim:
                 raise KernelError(f"decay_scan: {name} has one element per head and key channel")
         p.w, p.w_stride = w.data_ptr(), w.shape[1]
-        self._run_scan("spite_decay_scan", p, batch, heads, True, chunked, C.c_void_p(w0.data_ptr()), C.c_void_p(u.data_ptr()))
+        self._run_scan("decaying_memory", "spite_decay_scan", p, batch, heads, True, chunked, C.c_void_p(w0.data_ptr()), C.c_void_p(u.data_ptr()))
 
     def gated_linear_scan(self, q, k, v, a, w, out, batch, state, *, heads, dim, vdim, a2, a2_bias, tau, q_scale, state_offset=0, chunked=None):
         p, _ = self._scan("gated_linear_scan", q, k, v, out, batch, state, heads=heads, kv_heads=heads, dim=dim, vdim=vdim,
@@ -1325,7 +1329,7 @@ class CudaKernels(KernelSet):
         self._t(t, torch.float32, "a")
         at = self._columns(t, column, rank, out.shape[0], "gated_linear_scan: a")
         p.w, p.w_stride, p.out_scale = w.data_ptr(), n, float(q_scale)
-        self._run_scan("spite_gated_linear_scan", p, batch, heads, True, chunked, C.c_void_p(at), C.c_longlong(t.shape[1]),
+        self._run_scan("linear_attention", "spite_gated_linear_scan", p, batch, heads, True, chunked, C.c_void_p(at), C.c_longlong(t.shape[1]),
                        C.c_void_p(a2.data_ptr()), C.c_void_p(a2_bias.data_ptr()), int(rank), C.c_float(tau))
 
     # ------------------------------------------------------------------ mixture of experts
