@@ -714,51 +714,43 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
         if (part == 0) rec[Rec::KEYS + ch] = ch < dim ? expf(last) : 0.f;
         if (tid < CT) { rec[Rec::G + tid] = 1.f; rec[Rec::W + tid] = 1.f; }
     }
-    // ---- scores within a half of the chunk: a warp has four tokens s in a row, its lanes the channels; what a token t brings is read once
-    {
-        const int s0 = 4 * warp, end = (s0 & 16) + 16;
+    // ---- scores within a half of the chunk: a warp has four tokens s, its lanes the channels (four tokens in a row, with what
+    // a token t brings read once: 58 against 48 us for 2,048 tokens of 32 heads of 64, for its 64 sums a lane)
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const int s = warp + 8 * i, end = (s & 16) + 16;
         constexpr int C2 = DP / 64;                       // pairs of channels a lane
-        float2 kf[4][C2];                                 // k_s times the decays up to token t
-        float o[4][16];                                   // scores of token s0 + i and token (s0 & 16) + j
+        float2 kf[C2];
+        float o[16];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int c = 0; c < C2; ++c) kf[c] = *(const float2*)&sm.k[s][2 * lane + 64 * c];
 #pragma unroll
-            for (int c = 0; c < C2; ++c) kf[i][c] = *(const float2*)&sm.k[s0 + i][2 * lane + 64 * c];
+        for (int j = 0; j < 16; ++j) {                    // token s + j
+            o[j] = 0.f;
+            if (s + j < end) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int t = (s0 & 16) + j;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o[i][j] = 0.f;
-            if (t < s0) continue;
-#pragma unroll
-            for (int c = 0; c < C2; ++c) {
-                const float2 w = *(const float2*)&sm.w[t][2 * lane + 64 * c], q = *(const float2*)&sm.q[t][2 * lane + 64 * c];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const bool behind = t > s0 + i;
-                    if (!BONUS && behind) { kf[i][c].x *= w.x; kf[i][c].y *= w.y; }
-                    if (behind || (!BONUS && t == s0 + i)) { o[i][j] = fmaf(q.x, kf[i][c].x, o[i][j]); o[i][j] = fmaf(q.y, kf[i][c].y, o[i][j]); }
-                    if (BONUS && behind) { kf[i][c].x *= w.x; kf[i][c].y *= w.y; }
+                for (int c = 0; c < C2; ++c) {
+                    const float2 w = *(const float2*)&sm.w[s + j][2 * lane + 64 * c], q = *(const float2*)&sm.q[s + j][2 * lane + 64 * c];
+                    if (!BONUS && j) { kf[c].x *= w.x; kf[c].y *= w.y; }
+                    if (!BONUS || j) { o[j] = fmaf(q.x, kf[c].x, o[j]); o[j] = fmaf(q.y, kf[c].y, o[j]); }
+                    if (BONUS && j) { kf[c].x *= w.x; kf[c].y *= w.y; }
                 }
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int h = 8; h >= 1; h >>= 1) {
+            const bool up = (lane & h) != 0;
 #pragma unroll
-            for (int h = 8; h >= 1; h >>= 1) {
-                const bool up = (lane & h) != 0;
-#pragma unroll
-                for (int j = 0; j < h; ++j) {
-                    const float give = up ? o[i][j] : o[i][j + h], keep = up ? o[i][j + h] : o[i][j];
-                    o[i][j] = keep + __shfl_xor_sync(0xffffffffu, give, h);
-                }
+            for (int j = 0; j < h; ++j) {
+                const float give = up ? o[j] : o[j + h], keep = up ? o[j + h] : o[j];
+                o[j] = keep + __shfl_xor_sync(0xffffffffu, give, h);
             }
-            float x = o[i][0] + __shfl_xor_sync(0xffffffffu, o[i][0], 16);
-            const int t = (s0 & 16) + lane, s = s0 + i;
-            if (lane < 16 && t >= s && t < end) {
-                if (BONUS && t == s) x = t < len ? p.scalars[4 * ((size_t)(first + t) * p.heads + head)] : 0.f;
-                sm.P[t][s] = x;
-            }
+        }
+        float x = o[0] + __shfl_xor_sync(0xffffffffu, o[0], 16);
+        const int t = s + lane;
+        if (lane < 16 && t < end) {
+            if (BONUS && lane == 0) x = t < len ? p.scalars[4 * ((size_t)(first + t) * p.heads + head)] : 0.f;
+            sm.P[t][s] = x;
         }
     }
     __syncthreads();

@@ -306,7 +306,8 @@ class CudaKernels(KernelSet):
         # of 128 x 128: one prompt of 32 tokens 21 / 24, 64: 23 / 42, 512: 45 / 291, 2,048: 152 / 1,147; sixteen prompts of 32: 64 / 95.
         # Matrix memory, 8 heads of 256 x 512: 16 tokens 19 / 21, 2,048: 224 / 3,150.  State space, 128 heads of 128 x 64: 64 tokens
         # 26 / 18, 128: 31 / 30, 512: 63 / 99, 2,048: 206 / 378.  Gated linear attention, 32 heads of 64 x 128: 256 tokens 35 / 32, 512:
-        # 48 / 59, 2,048: 155 / 223; sixteen prompts of 128: 139 / 133.
+        # 48 / 59, 2,048: 155 / 223; sixteen prompts of 128: 139 / 133.  Decaying memory, 64 heads of 64 x 64: 512 tokens 64 / 63, 2,048:
+        # 224 / 238.
         self.chunk_from = {"delta": 32, "memory": 8, "state_space": 160, "linear_attention": 320, "decaying_memory": 1024}
         self.chunk_min_tokens = 32
         self.memory_min_tokens = 8
