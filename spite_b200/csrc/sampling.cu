@@ -518,7 +518,8 @@ __global__ void __launch_bounds__(THREADS) sample_cluster_kernel(const SamplePar
         const float want = topp * tot;
         // Largest key K with mass(key >= K) >= want, three bits of the key at a time: a pass adds up the masses above the seven values
         // that the next three bits can have.  Each of them is the sum, term by term, that a bisection bit by bit would make on its way
-        // (32 passes: 290 us for 32 rows of 202,048 logits, a pass costing as much for its barriers as for its numbers).
+        // (32 rows of 202,048 logits with temperature, top-p and penalty: 283 us in 32 passes, 220 in these 11; a pass costs as much for
+        // its barriers as for its numbers).
         unsigned K = next_bits<2>(sh, l, n, mx, want, 0u, 30);
         for (int shift = 27; shift >= 0; shift -= 3) K = next_bits<3>(sh, l, n, mx, want, K, shift);
         float cut[2] = {0.f, 0.f};                               // the mass above the cut, the logits at it
