@@ -6,7 +6,8 @@
 // many bytes a multiprocessor keeps in flight and how quickly the stream starts again after the
 // kernel before.  Here a producer warp keeps a ring of shared-memory stages full: per stage one TMA
 // box of 128 weight rows x 64 k (128-byte swizzle; for SwiGLU 64 gate and 64 up rows) and the
-// matching 64 k of the group's tokens (cp.async, same swizzle).  Eight consumer warps own 16 of the
+// matching 64 k of the group's tokens: cp.async with the same swizzle up to 16 token columns, a TMA box with 32
+// (one-group products, rows in place).  Eight consumer warps own 16 of the
 // 128 rows each and multiply with mma.sync.m16n8k16 (weights as the 16-row operand from ldmatrix,
 // tokens as the 8, 16 or 32 columns), so no sums cross warps.  Registers stay few, and two blocks (of this
 // kernel, or the last of this and the first of the next) share a multiprocessor.
@@ -51,11 +52,17 @@ __device__ int g_stream_error = 0;
 SPITE_WAIT_CONTROLS(gemm_stream, g_stream_error)
 namespace {
 
-struct Tail {
+template <int GROUPS>
+struct TailOf {
     unsigned long long full[MAX_STAGES], empty[MAX_STAGES];
     int abort_flag, n_active, last;
-    int active[MAX_GROUPS];
+    int active[GROUPS];
 };
+template <int NT>
+using TailFor = TailOf<(NT > 16 ? 1 : MAX_GROUPS)>;           // 32 token columns: one-group products only
+// The tensor map of the tokens, where they come as boxes.
+template <bool BOXES> struct TokenMap { CUtensorMap map; };
+template <> struct TokenMap<false> {};
 // After the tail, with k slices: the sums of the warps of slices 1 .. S - 1 on their way to the warps of slice 0,
 // [warp - R][lane][NT / 2] floats.
 constexpr int slices_bytes(int nt, int s) { return s > 1 ? (CONSUMERS - CONSUMERS / s) * 32 * (nt / 2) * 4 : 0; }
@@ -118,7 +125,7 @@ struct Item {
 // global memory: no scratch, no fence, no ticket, no second pass through L2.
 template <int NT, int EPI, int S, bool CL>
 __global__ void __launch_bounds__(THREADS, NT <= 16 ? 3 : 2)
-gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p, const int n_stages,
+gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ TokenMap<(NT > 16)> tokens, const GemmParams p, const int n_stages,
                    const int n_splits, float* __restrict__ scratch, int* __restrict__ tickets, const WaitControl waits) {
     constexpr bool DUAL = (EPI == EPI_SWIGLU);
     constexpr int TR = ROWS / S;                                 // weight rows of a tile
@@ -130,11 +137,17 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
     constexpr int NB = NT / 8;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    using Tail = TailFor<NT>;
     Tail* tail = (Tail*)(smem + (size_t)n_stages * STAGE);
     float* const slice_sums = (float*)(tail + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool grouped = p.group_offsets != nullptr;
+    // With 32 token columns the tokens come as boxes: the producer's 8 S copies of 16 bytes a lane and stage took longer than the
+    // weights (2048 x 8192 at 24 rows 17.2 us, now 14.6; 2048 x 2048 14.4, now 10.7).  Up to 16 columns, where rows may be gathered, they
+    // cost nothing (and boxes 0.7 us more at a few rows: 5.8 against 5.1 us for 2048 x 2048 at 8 rows).
+    constexpr bool BOXES = NT > 16;
+    constexpr unsigned STAGE_TX = W_BYTES + (BOXES ? S * X_BYTES : 0);
     const int row_tiles = (p.N + COLS - 1) / COLS;
     const int num_kb = p.K / (BK * S);                        // stages along k
     const int w_rows = DUAL ? 2 * p.N : p.N;
@@ -143,7 +156,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
     const long long wait_limit = waits.limit_cycles;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < n_stages; ++s) { mbar_init(smem_u32(&tail->full[s]), 33); mbar_init(smem_u32(&tail->empty[s]), CONSUMERS); }
+        for (int s = 0; s < n_stages; ++s) { mbar_init(smem_u32(&tail->full[s]), BOXES ? 1 : 33); mbar_init(smem_u32(&tail->empty[s]), CONSUMERS); }
         tail->abort_flag = 0;
         mbar_init_fence();
     }
@@ -151,6 +164,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
     // A one-group product's first item is known now: request its first weights before waiting for
     // the kernels before (weights are written by no kernel of the step).
     int pre = 0;
+    if constexpr (BOXES) {
+        if (threadIdx.x == 0) asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&tokens.map) : "memory");
+    }
     if (!grouped) {
         __syncthreads();
         if (warp == CONSUMERS && lane == 0 && (int)blockIdx.x < row_tiles * n_splits) {
@@ -160,7 +176,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
             pre = min(n_stages, kb1 - kb0);
             for (int j = 0; j < pre; ++j) {
                 const unsigned bar = smem_u32(&tail->full[j]), dst = smem_u32(smem + j * STAGE);
-                mbar_expect_tx(bar, W_BYTES);
+                mbar_expect_tx(bar, STAGE_TX);
 #pragma unroll
                 for (int sl = 0; sl < S; ++sl) {
                     const int kx = ((kb0 + j) * S + sl) * BK;
@@ -216,14 +232,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
         const __nv_bfloat16* X = (const __nv_bfloat16*)p.A;
         for (int i = blockIdx.x; i < total && ok; i += gridDim.x) {
             const Item it = item_at(i);
-            // this lane's 16-byte chunks of a slice's token tile: chunk q = lane + 32 j, token q / 8, k chunk q % 8.
-            // Up to 16 tokens their places are worked out once an item; with more (one-group products only, rows
-            // in place) they are cheap enough to work out again for every stage, and sixteen pointers would
-            // cost every thread of the block their registers.
+            // this lane's 16-byte chunks of a slice's token tile: chunk q = lane + 32 j, token q / 8, k chunk q % 8
             constexpr int KEPT = NT <= 16 ? NT / 4 : 1;
             const __nv_bfloat16* src[KEPT];
             unsigned off[KEPT];
-            if (NT <= 16) {
+            if (!BOXES) {
 #pragma unroll
                 for (int j = 0; j < KEPT; ++j) {
                     const int q = lane + 32 * j, t = q >> 3, c = q & 7;
@@ -241,7 +254,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
                 if (skip_tma > 0) {
                     --skip_tma;
                 } else if (lane == 0) {
-                    mbar_expect_tx(bar, W_BYTES);
+                    mbar_expect_tx(bar, STAGE_TX);
 #pragma unroll
                     for (int sl = 0; sl < S; ++sl) {
                         const int kx = (kb * S + sl) * BK;
@@ -253,28 +266,28 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
                         }
                     }
                 }
-                if (NT <= 16) {
+                if constexpr (BOXES) {
+                    // rows past the product's tokens are filled with zeros; never stored
+                    if (lane == 0) {
+#pragma unroll
+                        for (int sl = 0; sl < S; ++sl)
+                            tma_load_2d(dst + W_BYTES + sl * X_BYTES, &tokens.map, (kb * S + sl) * BK, 0, bar);
+                    }
+                } else {
 #pragma unroll
                     for (int sl = 0; sl < S; ++sl)
 #pragma unroll
                         for (int j = 0; j < KEPT; ++j)
                             cp_async16(dst + sl * X_BYTES + off[j], src[j] + ((size_t)kb * S + sl) * BK);
-                } else {
-                    const int c = lane & 7;
-#pragma unroll
-                    for (int sl = 0; sl < S; ++sl)
-#pragma unroll 4
-                        for (int j = 0; j < NT / 4; ++j) {
-                            const int t = (lane >> 3) + 4 * j;
-                            const int li = it.lo + min(t, it.m - 1);
-                            cp_async16(dst + sl * X_BYTES + W_BYTES + t * 128 + ((c ^ (t & 7)) << 4),
-                                       X + (size_t)li * p.lda + c * 8 + ((size_t)kb * S + sl) * BK);
-                        }
+                    cp_async_arrive(bar);
                 }
-                cp_async_arrive(bar);
             }
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (lane == 0 && *abort_flag)                            // boxes on their way land before the block leaves: stages before s
+            for (int j = 0; j < n_stages; ++j)                   // were asked for in this turn of the ring, the others in the last
+                mbar_drain(smem_u32(&tail->full[j]), j < s ? ph : ph ^ 1, wait_limit);
+        __syncwarp();
         if (CL && (int)blockIdx.x < total) { cluster_sync(); cluster_sync(); }     // with the consumers, see below
     } else {
         // ---- consumers: warp w works on slice w / R; it owns rows 16 r .. 16 r + 15 (r = w % R) of the tile
@@ -284,7 +297,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
         const int mrow = (lane & 7) + ((lane >> 3) & 1) * 8;     // fragment row this lane addresses for ldmatrix
         const int arow = DUAL ? (mrow < 8 ? 8 * rg + mrow : TR / 2 + 8 * rg + mrow - 8) : 16 * rg + mrow;
         const unsigned a_off = slice * BOX_BYTES + arow * 128, a_swz = arow & 7, a_k = lane >> 4;
-        const int brow = lane & 7;
+        const int brow = (lane & 7) + (NB > 1 ? (lane >> 4) * 8 : 0);   // two groups of 8 tokens a load where there are two
         const unsigned b_k = (lane >> 3) & 1;
         int s = 0;
         unsigned ph = 0;
@@ -304,12 +317,19 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const GemmParams p
                 for (int ks = 0; ks < BK / 16; ++ks) {
                     unsigned a[4];
                     ldmatrix_x4(a, wbase + a_off + (((2 * ks + a_k) ^ a_swz) << 4));
-#pragma unroll
-                    for (int j = 0; j < NB; ++j) {
-                        const int t = 8 * j + brow;
+                    if constexpr (NB == 1) {
                         unsigned b0, b1;
-                        ldmatrix_x2(b0, b1, xbase + t * 128 + (((2 * ks + b_k) ^ (t & 7)) << 4));
-                        mma16816(acc[j], a, b0, b1);
+                        ldmatrix_x2(b0, b1, xbase + brow * 128 + (((2 * ks + b_k) ^ (brow & 7)) << 4));
+                        mma16816(acc[0], a, b0, b1);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < NB; j += 2) {
+                            const int t = 8 * j + brow;
+                            unsigned b[4];
+                            ldmatrix_x4(b, xbase + t * 128 + (((2 * ks + b_k) ^ (t & 7)) << 4));
+                            mma16816(acc[j], a, b[0], b[1]);
+                            mma16816(acc[j + 1], a, b[2], b[3]);
+                        }
                     }
                 }
                 __syncwarp();
@@ -461,7 +481,14 @@ int launch(const GemmParams& p, int n_blocks, int smem_budget, int n_splits, flo
     cuuint64_t strides[1] = {(cuuint64_t)p.K * 2};
     cuuint32_t box[2] = {BK, (cuuint32_t)(DUAL ? TR / 2 : TR)};
     if (!make_map(&mw, p.W, 2, dims, strides, box)) return SPITE_LAUNCH_FAILED;
-    constexpr int FIXED = (int)sizeof(Tail) + slices_bytes(NT, S) + 1024;
+    TokenMap<(NT > 16)> mx;
+    if constexpr (NT > 16) {
+        cuuint64_t x_dims[2] = {(cuuint64_t)p.K, (cuuint64_t)p.M};
+        cuuint64_t x_strides[1] = {(cuuint64_t)p.lda * 2};
+        cuuint32_t x_box[2] = {BK, NT};
+        if (!make_map(&mx.map, p.A, 2, x_dims, x_strides, x_box)) return SPITE_LAUNCH_FAILED;
+    }
+    constexpr int FIXED = (int)sizeof(TailFor<NT>) + slices_bytes(NT, S) + 1024;
     int n_stages = (smem_budget - FIXED) / STAGE;
     if (n_stages > MAX_STAGES) n_stages = MAX_STAGES;
     if (n_stages < 2) return SPITE_UNSUPPORTED;                    // (16 tokens x 8 slices are 32 KiB a stage)
@@ -474,7 +501,7 @@ int launch(const GemmParams& p, int n_blocks, int smem_budget, int n_splits, flo
     const long long tiles = (long long)((p.N + cols - 1) / cols) * (p.group_offsets ? (p.n_groups < p.M ? p.n_groups : p.M) : 1) * n_splits;
     if (!CL) {
         const int grid = (int)(tiles < n_blocks ? tiles : n_blocks);
-        SPITE_LAUNCH(k, grid, THREADS, smem, st, mw, p, n_stages, n_splits, scratch, tickets, s_waits);
+        SPITE_LAUNCH(k, grid, THREADS, smem, st, mw, mx, p, n_stages, n_splits, scratch, tickets, s_waits);
         return spite_launch_status();
     }
     // one block per (tile, split), the splits of a tile one cluster; all of them resident at once, or the caller
@@ -513,7 +540,7 @@ int launch(const GemmParams& p, int n_blocks, int smem_budget, int n_splits, flo
     }
     if ((long long)fit * n_splits < tiles) return SPITE_UNSUPPORTED;
     cfg.numAttrs = spite_pdl_enabled() ? 2 : 1;
-    (void)cudaLaunchKernelEx(&cfg, k, mw, p, n_stages, n_splits, scratch, tickets, s_waits);
+    (void)cudaLaunchKernelEx(&cfg, k, mw, mx, p, n_stages, n_splits, scratch, tickets, s_waits);
     return spite_launch_status();
 }
 
@@ -525,10 +552,11 @@ int launch_slices(int k_slices, bool cluster, const GemmParams& p, int n_blocks,
         if (NT > 16) return SPITE_UNSUPPORTED;
         return launch<NT <= 16 ? NT : 8, EPI, 1, true>(p, n_blocks, smem_budget, n_splits, scratch, tickets, st);
     }
-    if (NT > 16) {                                             // many tokens: tiles of 128 or 64 rows (more slices, more of a
-        switch (k_slices) {                                    // stage would be tokens than weights)
+    if (NT > 16) {                                             // many tokens: tiles of 128, 64 or 32 rows (with eight slices three
+        switch (k_slices) {                                    // quarters of a stage would be tokens)
             case 1: return launch<NT, EPI, 1, false>(p, n_blocks, smem_budget, n_splits, scratch, tickets, st);
             case 2: return launch<NT, EPI, 2, false>(p, n_blocks, smem_budget, n_splits, scratch, tickets, st);
+            case 4: return launch<NT, EPI, 4, false>(p, n_blocks, smem_budget, n_splits, scratch, tickets, st);
             default: return SPITE_UNSUPPORTED;
         }
     }

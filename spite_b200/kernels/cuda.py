@@ -280,6 +280,10 @@ class CudaKernels(KernelSet):
         self.stream_split_item_cost = 6.0
         self.stream_split_cost = 1.5
         self.stream_slice_cost = 1.0
+        # the first three for one-group products that may be cut into slices.  Against the best of all (slices, splits), over 2048 x
+        # 2048, 6176 x 2048, 8192 x 2048, 2048 x 8192, 32768 x 2048, 5120 x 5120, 7168 x 5120, 4096 x 4096 and 1024 x 4096 at 4 to 32
+        # rows alone, the choice by these costs is 0.8 % slower on average, by the three above 4.5 %
+        self.stream_one_group_costs = (1.0, 2.0, 1.0)
         self.stream_max_slices = 8             # 1: tiles of 128 rows only
         self.stream_slices_min_rows = 6        # products of fewer rows keep tiles of 128 rows (see stream_cut)
         self.stream_slices_grouped = False     # ... and so do grouped products
@@ -297,9 +301,12 @@ class CudaKernels(KernelSet):
         # Decode step at 20 / 24 / 32 requests: 11.98 / 12.63 / 14.07 ms against 12.17 / 13.07 / 14.30 on tcgen05
         self.stream_max_rows = 32
         self.stream_force = None               # (k slices, k splits) for every call, for measurements
-        # (shared memory per block, resident blocks) for up to 3 tokens and for more: measured in the decode step at
+        # (shared memory per block, resident blocks) for up to 3 tokens and one-group products, and for products over groups of
+        # more tokens: measured in the decode step at
         # Scout shapes, one token 2.90 ms with (110 KiB, 2 per multiprocessor) against 3.01 with (74 KiB, 3), eight
-        # tokens 7.10 against 7.02, sixty-four alike; one block per multiprocessor with 110 or 200 KiB: 3.2 and 3.1 ms
+        # tokens 7.10 against 7.02 (both kinds of products alike), sixty-four alike; one-group products alone in the deeper ring, us
+        # against (74 KiB, 3), 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 / 17.8, 4096 x 4096 8.5 / 10.6; 16 rows 8.6 / 10.8,
+        # 16.2 / 20.6, 9.8 / 13.8; one block per multiprocessor with 110 or 200 KiB: 3.2 and 3.1 ms
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
         # Recurrences over prompts: a step whose longest segment has at least so many tokens goes in chunks of 32 on the tensor cores (its
         # segments of fewer than 32 tokens, 8 in the matrix memory, token by token).  us in chunks / token by token.  Delta rule, 16 heads
@@ -696,7 +703,7 @@ class CudaKernels(KernelSet):
         scratch for the partial sums of the splits."""
         swiglu = p.epilogue == EPI_SWIGLU
         groups = min(p.n_groups, p.M) if grouped else 1
-        smem, blocks = self.stream_shape[0 if rows <= 3 or rows > 16 else 1]      # (the tokens of many rows need the larger ring)
+        smem, blocks = self.stream_shape[0 if rows <= 3 or not grouped else 1]
         nt = 8 if max_rows_per_group <= 8 else 16 if max_rows_per_group <= 16 else 32
         slices, splits = self.stream_force or self._stream_cut(rows, p.N, p.K, groups, swiglu, blocks, smem, nt, grouped)
         tile_rows = 128 // slices
@@ -722,10 +729,11 @@ class CudaKernels(KernelSet):
 
     def _stream_cut(self, M: int, N: int, K: int, groups: int, swiglu: bool, slots: int, smem: int, nt: int,
                     grouped: bool):
-        return stream_cut(M, N, K, groups, swiglu, slots, smem, nt, item_cost=self.stream_item_cost,
-                          split_item_cost=self.stream_split_item_cost, split_cost=self.stream_split_cost,
+        item, split_item, split = (self.stream_one_group_costs if not grouped and M >= self.stream_slices_min_rows else
+                                   (self.stream_item_cost, self.stream_split_item_cost, self.stream_split_cost))
+        return stream_cut(M, N, K, groups, swiglu, slots, smem, nt, item_cost=item, split_item_cost=split_item, split_cost=split,
                           slice_cost=self.stream_slice_cost,
-                          max_slices=(min(2, self.stream_max_slices) if nt > 16 else self.stream_max_slices)
+                          max_slices=(min(4, self.stream_max_slices) if nt > 16 else self.stream_max_slices)
                           if self.stream_slices_grouped or not grouped else 1,
                           slices_min_rows=self.stream_slices_min_rows,
                           cluster_max_splits=self.stream_cluster_max_splits if M <= self.stream_cluster_max_rows else 0,
