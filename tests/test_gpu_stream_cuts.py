@@ -1,0 +1,62 @@
+"""Decode products of 17 to 32 rows (tokens that arrive as boxes, up to four k slices a stage) against float64, and the cuts that the
+kernel set chooses for one-group products."""
+import pytest
+import torch
+
+from spite_b200.kernels.cuda import stream_cut
+
+DEV = "cuda:0"
+
+
+def data(M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn((M, K), generator=g).to(torch.bfloat16)
+    w = torch.randn((N, K), generator=g).to(torch.bfloat16)
+    return x, w
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("force", [(1, 2), (2, 4), (4, 1), (4, 2), (4, 3), None], ids=str)
+@pytest.mark.parametrize("M,N,K", [(17, 40, 512), (24, 200, 1024), (32, 129, 2048), (31, 2048, 2048), (20, 96, 256)])
+def test_products_of_17_to_32_rows(force, M, N, K):
+    from spite_b200.kernels.cuda import CudaKernels
+    ks = CudaKernels(torch.bfloat16, DEV)
+    ks.stream_force = force
+    x, w = data(M, N, K)
+    before = ks.launches_by_library["gemm_stream"]
+    # rows of a larger buffer: what lies behind the tokens must not be read as a token
+    rows = torch.full((M + 40, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    rows[:M] = x.to(DEV)
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float32, device=DEV)
+    ks.linear(rows[:M], w.to(DEV), out[:M])
+    again = torch.empty((M, N), dtype=torch.float32, device=DEV)
+    ks.linear(x.to(DEV), w.to(DEV), again)
+    ref = x.double() @ w.double().t()
+    # a float32 sum of K products of magnitude |x||w|: each of its at most K roundings is below 2^-24 of the sum of magnitudes
+    bound = K * 2.0**-24 * (x.double().abs() @ w.double().abs().t())
+    assert bool(((out[:M].cpu().double() - ref).abs() <= bound).all())
+    assert bool((out[M] == 7.0).all()) and torch.equal(again, out[:M])
+    F = N // 2
+    a = torch.empty((M, F), dtype=torch.bfloat16, device=DEV)
+    ks.linear_swiglu(x.to(DEV), w[:2 * F].contiguous().to(DEV), a)
+    gate, up = ref[:, :F], ref[:, F:2 * F]
+    want = gate / (1 + torch.exp(-gate)) * up
+    # bfloat16 rounding of the result (2^-8) and the two sums' bounds through silu (slope below 1.1) and the product
+    tol = 2.0**-8 * want.abs() + 1.1 * bound[:, :F] * up.abs() + bound[:, F:2 * F] * gate.abs() + 1e-5 * want.abs() + 1e-6
+    assert bool(((a.cpu().double() - want).abs() <= tol).all())
+    assert ks.launches_by_library["gemm_stream"] == before + 3 and ks.errors() == {}
+
+
+@pytest.mark.parametrize("M", [6, 8, 9, 16, 17, 24, 32])
+@pytest.mark.parametrize("N,K,swiglu", [(40, 64, False), (200, 320, False), (104, 1024, True), (5120, 8192, False), (2048, 2048, False),
+                                        (8192, 5120, True), (129, 4096, False), (16, 64, True), (1024, 16384, False)])
+def test_cuts_of_one_group_products_are_cuts_that_the_kernel_takes(M, N, K, swiglu):
+    nt, smem, slots = (8 if M <= 8 else 16 if M <= 16 else 32), 110 * 1024, 296
+    most = 4 if M > 16 else 8
+    slices, splits = stream_cut(M, N, K, 1, swiglu, slots, smem, nt, item_cost=1.0, split_item_cost=2.0, split_cost=1.0, max_slices=most,
+                                slices_min_rows=6)
+    assert slices <= most and K % (64 * slices) == 0 and not (swiglu and slices == 8)
+    assert 1 <= splits <= max(1, K // (64 * slices) // 4)
+    groups = 1 if nt == 32 else 1024
+    fixed = 24 * 8 + 16 + 4 * groups + (8 - 8 // slices) * 64 * nt * (slices > 1) + 1024
+    assert (smem - fixed) // (16384 + max(1024, slices * nt * 128)) >= 2                      # a ring of at least two stages
