@@ -203,7 +203,10 @@ def stream_cut(M: int, N: int, K: int, groups: int, swiglu: bool, slots: int, sm
     9.53; for the experts' products only 4.76 / 5.83 / 6.63 / 8.68 / 9.60.  The experts' products are faster
     alone with slices and slower in the step: with tiles of 128 rows some blocks end early and the next
     kernel's blocks start under the rest.  So the caller allows slices for one-group products from
-    `slices_min_rows` rows on (the kernel set's defaults: six), and tiles of 128 rows otherwise."""
+    `slices_min_rows` rows on (the kernel set's defaults: six), and tiles of 128 rows otherwise.  Those products now run
+    in the deeper ring (296 blocks) with costs of their own (`stream_one_group_costs`): 8 rows, 4096 x 4096 (8, 1) 8.5, (4,
+    2) 9.2, (2, 3) 10.6; 1024 x 4096 (4, 8) 5.5, (8, 2) 5.7, (8, 1) 6.6; decode step of 16 Scout layers at 8 / 16 / 24
+    requests over 2,048 keys 6.12 / 8.81 / 11.23 ms, before 6.15 / 8.87 / 11.48."""
     best, best_cost = (1, 1), None
     for slices in (1, 2, 4, 8):
         if K % (64 * slices) or (swiglu and slices == 8):
@@ -297,8 +300,8 @@ class CudaKernels(KernelSet):
         # and down projections in seven through global memory) against 4, 2, 1 (all three in four): 2.714 against
         # 2.738, 2.727, 2.726 ms at one token
         self.stream_cluster_cost = 9.0
-        # one-group products of up to this many rows stream their weights too (16: never; the kernel takes up to 32).
-        # Decode step at 20 / 24 / 32 requests: 11.98 / 12.63 / 14.07 ms against 12.17 / 13.07 / 14.30 on tcgen05
+        # one-group products of up to this many rows stream their weights too (16: never; the kernel takes up to 32), here / on
+        # tcgen05, us, 24 rows: 2048 x 2048 7.9 / 12.6, 8192 x 2048 10.4 / 17.4, 2048 x 8192 12.8 / 40, 5120 x 5120 17.2 / 27.4
         self.stream_max_rows = 32
         self.stream_force = None               # (k slices, k splits) for every call, for measurements
         # (shared memory per block, resident blocks) for up to 3 tokens and one-group products, and for products over groups of
