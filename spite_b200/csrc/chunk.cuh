@@ -294,9 +294,10 @@ template <int KPW, int KW, int CW, int MODE> struct Shape {
     // two sets of partial sums: in turn (a chunk's are read while the next one's are written), or a delta rule's two products
     static constexpr int SUM_FLOATS = KW * COLS * TP;
     static constexpr int SUMS = 2 * SUM_FLOATS * 4;
-    // a delta rule: u, and what the read-outs start from; the memory: n, the parts of q . n of the tokens, and the tokens' factors, two of each
+    // a delta rule: u, and what the read-outs start from; the memory: n and the parts of q . n of the tokens, two of each, and the tokens'
+    // factors, three (a chunk's are written before its predecessor's barrier, while a slow warp may still read those of the one before)
     static constexpr int FACTORS = 3 * CT + 4;
-    static constexpr int EXTRA = MODE == DELTA ? 2 * COLS * TP * 4 : MODE == MATRIX_MEMORY ? 2 * (DP + KW * CT + FACTORS) * 4 : 0;
+    static constexpr int EXTRA = MODE == DELTA ? 2 * COLS * TP * 4 : MODE == MATRIX_MEMORY ? (2 * (DP + KW * CT) + 3 * FACTORS) * 4 : 0;
     static constexpr int bytes(int stages) { return stages * STAGE + SUMS + EXTRA; }
 };
 
@@ -412,9 +413,10 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
     float m_run = 0.f;                                    // MATRIX_MEMORY: the running maximum (warp 0)
     float* n_s = extra;                                   // n, then the warps' parts of q . n of the chunk's tokens
     float* nq_s = extra + 2 * DP;
-    float* factors = extra + 2 * (DP + KW * CT);          // of chunk c: g, h, the denominator's floor [CT] each, decay, the weights' factor
+    float* factors = extra + 2 * (DP + KW * CT);          // of chunk c, at c % 3: g, h, the denominator's floor [CT] each, decay, the weights' factor
     float* st_n = st + p.n_offset + (size_t)(blockIdx.x * (COLS / 32)) * p.n_stride;
-    // The memory's factors per token (a lane has token `lane`): g on Q S0, h on P V.  Warp 0 makes them a chunk ahead.
+    // The memory's factors per token (a lane has token `lane`): g on Q S0, h on P V.  Warp 0 makes them a chunk ahead, before a barrier
+    // that every warp passes before it reads them.
     const auto make_factors = [&](const float* rec, int len, float* to) {
         const double* md = reinterpret_cast<const double*>(rec);
         const double m_local = md[lane], F = md[CT + lane];
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
         const float* v_s = reinterpret_cast<const float*>(stg + REC_AT + SH::REC_BYTES);
         const int tb = t0 + c * CT, len = min(CT, t1 - tb);
         float* sum = sums + (MODE == DELTA ? 0 : (c & 1) * SH::SUM_FLOATS);
-        const float* fac = factors + (c & 1) * SH::FACTORS;
+        const float* fac = factors + slot3 * SH::FACTORS;
         const unsigned state_largest = largest_of[0][slot3], slot_now = slot3, slot_next = slot3 == 2 ? 0 : slot3 + 1;
         lost |= state_largest >= 0x7f800000u;
         if (tid < 2) largest_of[tid][slot_next == 2 ? 0 : slot_next + 1] = 0;
@@ -682,6 +684,11 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
             if (lane == 0) atomicMax(&largest_of[1][slot_next], largest);
         }
         wait_for(c + 1, stage, parity);
+        if constexpr (MODE == MATRIX_MEMORY) {            // the next chunk's factors, in front of the barrier below
+            if (warp == 0 && c + 1 < n_chunks)
+                make_factors(reinterpret_cast<const float*>(smem + (size_t)stage * SH::STAGE + REC_AT), min(CT, t1 - tb - CT),
+                             factors + slot_next * SH::FACTORS);
+        }
         // what the read-outs take from this chunk's stage
         float2 gt[NT], row_sum[NT], skipped[NT][2];
         if constexpr (MODE != DELTA) {
@@ -701,11 +708,6 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
             }
             lost = __syncthreads_or(lost);                // the sums over the keys are complete, and this chunk's stage is free
             if (lost) break;
-        }
-        if constexpr (MODE == MATRIX_MEMORY) {            // the next chunk's factors (read behind the next barrier)
-            if (warp == 0 && c + 1 < n_chunks)
-                make_factors(reinterpret_cast<const float*>(smem + (size_t)stage * SH::STAGE + REC_AT), min(CT, t1 - tb - CT),
-                             factors + ((c + 1) & 1) * SH::FACTORS);
         }
         if (KW <= 4 || kw < 4) {
             float* out = p.out + (size_t)tb * p.out_stride + (size_t)head * p.vdim + col0;

@@ -392,3 +392,62 @@ def test_a_wait_that_runs_out_is_reported_and_the_tokens_are_walked():
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     near(run(True)[0], want[0].double(), "with the default waits")
     assert ks.errors() == {}
+
+
+# ---------------------------------------------------------------------------- the order of what warps do
+def walks(kind, ks, g, counts, heads, dim, vdim, scale=lambda name, t: t):
+    """A function that makes one pass of a walk in chunks over new states: () -> (outputs [M, heads * vdim], states).  `scale` may change
+    the drawn q, k, v."""
+    rnd = lambda *s: torch.randn(s, generator=g).to(DEV)
+    batch, M = step_batch(counts, list(range(len(counts))), True)
+    q, k, v = (scale(n, rnd(M, heads, w)).reshape(M, -1) for n, w in (("q", dim), ("k", dim), ("v", vdim)))
+    a, b, par, z, chan = rnd(M, heads), rnd(M, heads), rnd(heads), rnd(M, heads * dim) - 2.0, rnd(heads * dim) - 1.0
+    a2, wide = rnd(6, heads * dim), torch.cat([q, k, v, a, b], 1).contiguous()
+    n, m = heads * dim, 2 * heads * dim + heads * vdim
+    cols = (0, n, 2 * n, m, m + heads)
+
+    def run(chunked=True):
+        out = torch.empty((M, heads * vdim), device=DEV)
+        shape = (heads, ks.mlstm_state_size(dim, vdim)) if kind == "matrix_memory" else (
+            heads * (dim * vdim if kind == "delta" else ks.scan_state_size(dim, vdim)),)
+        state = torch.zeros((len(counts),) + shape, device=DEV)
+        more = dict(heads=heads, dim=dim, vdim=vdim, chunked=chunked)
+        if kind == "matrix_memory":
+            ks.mlstm_scan(wide, out, batch, state, gate_cap=8.0, q_scale=dim ** -0.5, columns=cols, i_bias=par, f_bias=par + 3.0, **more)
+        elif kind == "delta":
+            ks.delta_scan(wide, out, batch, state, kv_heads=heads, columns=cols, a_log=par, dt_bias=par, q_scale=dim ** -0.5, **more)
+        elif kind == "state_space":
+            ks.state_space_scan((q, 0), (k, 0), (v, 0), (a, 0), out, batch, state, kv_heads=heads, a_log=par, dt_bias=par - 3.0, skip=par, **more)
+        elif kind == "decaying_memory":
+            ks.decay_scan((q, 0), (k, 0), (v, 0), z.clone(), out, batch, state, w0=chan, u=chan, **more)
+        else:
+            ks.gated_linear_scan((q, 0), (k, 0), (v, 0), (wide, m), torch.empty((M, n), device=DEV), out, batch, state, a2=a2, a2_bias=chan + 2.0,
+                                 tau=8.0, q_scale=0.2, **more)
+        return out, state
+    return run
+
+
+KINDS = ["matrix_memory", "delta", "state_space", "decaying_memory", "linear_attention"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_passes_of_the_same_input_are_the_same_bits(kind):
+    """Many chunks, heads and segments of unequal length, alone and beside products on another stream that take multiprocessors and
+    change the warps' pace: what a warp makes for others (sums, factors, scales) is ordered before their reads, whoever comes first."""
+    ks = kernels(torch.bfloat16)
+    dim = 256 if kind == "matrix_memory" else 128
+    run = walks(kind, ks, torch.Generator().manual_seed(12), [517, 97, 260, 33, 1025], 8, dim, 256)
+    want = run()
+    assert torch.isfinite(want[0]).all()
+    x, y = torch.randn((2048, 2048), device=DEV), torch.empty((2048, 2048), device=DEV)
+    side = torch.cuda.Stream()
+    for i in range(12):
+        if i % 2:
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                for _ in range(1 + i):
+                    torch.mm(x, x, out=y)
+        got = run()
+        torch.cuda.synchronize()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), f"pass {i}"
+    assert ks.errors() == {}
