@@ -759,8 +759,8 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
     }
     copy_wait<0>();
     if (lost) {                                           // the slot is as it was, and the columns go token by token
-        if (tid == 0)                                     // (copies in flight land before the block leaves)
-            for (int x = c + 1; x < min(c + p.stages, n_chunks); ++x)
+        if (tid == 0)                                     // (copies in flight land before the block leaves: chunk c's too, whose wait may
+            for (int x = c; x < min(c + p.stages, n_chunks); ++x)          // be the one that ran out)
                 tc::mbar_drain(tc::smem_u32(&full[x % p.stages]), (x / p.stages) & 1, waits.limit_cycles);
         __syncthreads();
         if (tid < CW && col0 / 16 + tid < p.column_groups) p.columns[((size_t)seg * p.heads + head) * p.column_groups + col0 / 16 + tid] = 1;

@@ -364,7 +364,7 @@ def test_scan_and_memory_entry_points_refuse_malformed_calls():
     assert not t.any()
 
 
-def test_a_wait_that_runs_out_is_reported_and_the_tokens_are_walked():
+def test_a_wait_that_runs_out_in_the_delta_rule_is_reported_and_the_tokens_are_walked():
     """The first stage is announced 16 bytes more than its copies deliver, with waits of two milliseconds: every block of the walk in
     chunks gives up, says so, and leaves its columns to the walk token by token."""
     heads, dim, vdim, n = 2, 64, 32, 70
@@ -421,7 +421,7 @@ def walks(kind, ks, g, counts, heads, dim, vdim, scale=lambda name, t: t):
         elif kind == "decaying_memory":
             ks.decay_scan((q, 0), (k, 0), (v, 0), z.clone(), out, batch, state, w0=chan, u=chan, **more)
         else:
-            ks.gated_linear_scan((q, 0), (k, 0), (v, 0), (wide, m), torch.empty((M, n), device=DEV), out, batch, state, a2=a2, a2_bias=chan + 2.0,
+            ks.gated_linear_scan((q, 0), (k, 0), (v, 0), (wide, 0), torch.empty((M, n), device=DEV), out, batch, state, a2=a2, a2_bias=chan + 2.0,
                                  tau=8.0, q_scale=0.2, **more)
         return out, state
     return run
@@ -450,4 +450,32 @@ def test_passes_of_the_same_input_are_the_same_bits(kind):
         got = run()
         torch.cuda.synchronize()
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), f"pass {i}"
+    assert ks.errors() == {}
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_block_that_gives_up_waits_for_its_first_chunk_before_it_leaves(kind):
+    """The first chunk's stage is announced 16 bytes more than its copies deliver: the wait for it runs out, and the block waits for that
+    stage's copies once more, with the same limit, since they could land in shared memory that is another block's by then."""
+    limit, library = 8_000_000, {"matrix_memory": "recurrent", "delta": "delta"}.get(kind, "scan")
+    ks = kernels(torch.bfloat16)
+    run = walks(kind, ks, torch.Generator().manual_seed(13), [70, 150], 2, 64, 32)
+    want = run(False)
+    run()
+    torch.cuda.synchronize()
+    assert ks.errors() == {}
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    ks.configure_waits(library, limit_cycles=limit, extra_tx=16)
+    try:
+        begin.record()
+        got = run()
+        end.record()
+        torch.cuda.synchronize()
+    finally:
+        ks.configure_waits(library)
+    assert ks.errors() == {library: 2} and ks.errors() == {}
+    # two limits of 8 million clocks at 2.0 GHz at most (a single one and the tokens' walk take 4.1 to 5 ms)
+    assert begin.elapsed_time(end) >= 2 * limit / 2.0e6
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    near(run()[0], want[0].double(), "with the default waits", 1e-4)
     assert ks.errors() == {}
