@@ -852,10 +852,10 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(const ShortConvPar
             }
         }
     }
-    if (s == 0 && i0 == 0) {
+    if (s == 0 && i0 < CONV_TB) {                             // copies of up to CONV_TB tokens, as above, every block its own rows of them
         for (int s2 = 1; s2 < p.n_segments; ++s2) {
             if (p.slots[s2] != slot) continue;
-            const int u0 = p.cu_seqlens[s2], m = min(p.cu_seqlens[s2 + 1] - u0, rows);
+            const int u0 = p.cu_seqlens[s2] + i0, m = min(p.cu_seqlens[s2 + 1] - u0, rows);
             for (int i = 0; i < m; ++i)
                 for (int e = 0; e < 4; ++e) ((T*)p.out)[(size_t)(u0 + i) * p.out_stride + c + e] = out[(size_t)i * p.out_stride + e];
         }

@@ -119,6 +119,29 @@ def test_padding_rows_of_a_captured_step_come_out_as_the_first_row():
     assert torch.equal(state[1].cpu(), before[1])
 
 
+@pytest.mark.parametrize("n", [3, 4, 8, 9, 12, 16])
+@pytest.mark.parametrize("channels", [70, 72])                # (72: whole groups of four columns, the kernel of several tokens a thread)
+def test_padding_rows_of_several_tokens_come_out_as_the_first_segment(channels, n):
+    ks = kernels(torch.float32)
+    taps, extra = 4, 4
+    g = torch.Generator().manual_seed(90 + n)
+    state = torch.randn((3, (taps - 1) * channels), generator=g).to(DEV)
+    before = state.cpu().clone()
+    w = torch.randn((channels, taps), generator=g)
+    x = torch.randn((3 * n + 5, channels + extra), generator=g)
+    x[n + 5:2 * n + 5] = x[:n]
+    x[2 * n + 5:] = x[:n]
+    batch, M = step_batch([n, 5, n, n], [2, 0, 2, 2])
+    out = torch.full((M, channels + extra), 7.0, device=DEV)
+    ks.short_conv(x.to(DEV), w.to(DEV), out, batch, state, channels=channels)
+    rows = torch.cat([before[2].view(taps - 1, channels), x[:n, :channels]], 0).double()
+    ref = sum(w[:, j].double() * rows[j:j + n] for j in range(taps))
+    close(out[:n, :channels], ref, 1e-6, "the first segment")
+    assert torch.equal(out[:n, channels:].cpu(), x[:n, channels:])
+    assert torch.equal(out[n + 5:2 * n + 5], out[:n]) and torch.equal(out[2 * n + 5:], out[:n])
+    assert torch.equal(state[2].cpu().view(taps - 1, channels), rows[n:].float()) and torch.equal(state[1].cpu(), before[1])
+
+
 # ---------------------------------------------------------------------------- the gated delta rule
 def delta_loops(q, k, v, zb, za, a_log, dt, q_scale, S):
     """One head, token by token, in float64: (outputs [T, vdim], S)."""
