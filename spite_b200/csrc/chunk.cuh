@@ -6,13 +6,14 @@
 // What does not depend on the state (scores, factors, W, U0) is computed by a kernel of the design's own for all chunks of a step at
 // once and left in working memory (`Record`s and operand tiles); `chunk_walk_kernel` then goes from chunk to chunk.
 //
-// Operands.  mma.sync takes 16-bit numbers.  A float32 x is split into two halves, h = fp16(s x) and l = fp16(s x - h), with a power of
-// two s that brings the tile's largest element to [2^13, 2^14): h + l then holds x to 2^-23 of itself (and no worse than 2^-38 of the
-// tile's largest element, where l leaves fp16's normal range), and a product of two splits is h h' + (h l' + l h'), three
-// instructions with float32 sums; what is left out, l l', is 2^-24 of the product.  The two kinds of terms have accumulators of
-// their own, and a chunk's sums start from zero and join the state by one float32 addition, so the tensor cores' sums are never
-// longer than a chunk (or than the keys of one warp).  Three products on the tensor cores (1,024 multiply-adds a clock and
-// multiprocessor with mma.sync, measured 960) are 2.6 times what the float32 units do (measured 122).
+// Operands.  mma.sync takes 16-bit numbers.  A float32 x is split into two halves, h = fp16(s x) and l = fp16(2^11 (s x - h)), with a
+// power of two s: the numbers that one product adds up, a column's keys or tokens on the left and a token's keys or tokens on the right,
+// share one s, which brings the largest of them to [2^13, 2^14); no column and no token shares it with another.  h + 2^-11 l then holds x
+// to 2^-23 of itself down to 2^-28 of the largest (where h leaves fp16's normal range; below that to 2^-50 of the largest).  A product of
+// two splits is h h' + 2^-11 (h l' + l h'), three instructions with float32 sums; what is left out, l l', is 2^-24 of the product.  The two
+// kinds of terms have accumulators of their own, and a chunk's sums start from zero and join the state by one float32 addition, so the
+// tensor cores' sums are never longer than a chunk (or than the keys of one warp).  Three products on the tensor cores (1,024
+// multiply-adds a clock and multiprocessor with mma.sync, measured 960) are 2.6 times what the float32 units do (measured 122).
 //
 // Work.  A block owns 16 CW value columns of one (segment, head), a warp KPW keys by 16 of those columns.  It keeps the state
 // transposed, as mma accumulators (rows: columns of S, columns: keys): split, they are the left operand of (Q S0)^T = S0^T Q^T without
@@ -33,21 +34,29 @@ enum Mode { HEAD_DECAY = 0, MATRIX_MEMORY = 1, DELTA = 2, KEY_DECAY = 3 };
 
 // ---- the split of a float32 tile into two fp16 tiles
 __device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
-struct Scale { float up, down; };                         // powers of two, up * down = 1
+constexpr float UP = 8192.f, DOWN = 1.f / 8192.f;         // what numbers of size one are scaled by
+constexpr float LOW_UP = 2048.f, LOW_DOWN = 1.f / 2048.f; // what the low half is scaled by besides
+// Powers of two: size <= |largest| < 2 size and up = UP / size.  (Zeros, and numbers below 2^-100: the size of 2^-100.)
+struct Scale { float up, size; };
 __device__ __forceinline__ Scale scale_of(unsigned largest_bits) {
-    const unsigned e = min(max(largest_bits >> 23, 14u), 254u);       // (a tile of zeros, or of numbers below 2^-113: the largest factor)
-    return {__uint_as_float((267u - e) << 23), __uint_as_float((e - 13u) << 23)};
+    const unsigned e = min(max(largest_bits >> 23, 27u), 254u);
+    return {__uint_as_float((267u - e) << 23), __uint_as_float(e << 23)};
 }
 __device__ __forceinline__ void split2(float a, float b, unsigned& high, unsigned& low) {
     const __half2 h = __floats2half2_rn(a, b);
     const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    const __half2 l = __floats2half2_rn((a - f.x) * LOW_UP, (b - f.y) * LOW_UP);
     high = *reinterpret_cast<const unsigned*>(&h);
     low = *reinterpret_cast<const unsigned*>(&l);
 }
 __device__ __forceinline__ void split1(float a, __half& high, __half& low) {
     high = __float2half_rn(a);
-    low = __float2half_rn(a - __half2float(high));
+    low = __float2half_rn((a - __half2float(high)) * LOW_UP);
+}
+// the largest of what the four lanes of a row of eight (the lanes of one g) hold
+__device__ __forceinline__ unsigned quad_max(unsigned x) {
+    x = max(x, __shfl_xor_sync(0xffffffffu, x, 1));
+    return max(x, __shfl_xor_sync(0xffffffffu, x, 2));
 }
 
 // two floats in one register pair, for the two-at-a-time multiply-adds of sm_100
@@ -72,12 +81,11 @@ __device__ __forceinline__ pair fma2(pair a, pair b, pair c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// the split of two numbers times `up`
-__device__ __forceinline__ void split2(pair x, pair up, unsigned& high, unsigned& low) {
-    x = mul2(x, up);
-    const float2 f = floats_of(x);
+// the split of two numbers times `up`; `low_up`: up times LOW_UP
+__device__ __forceinline__ void split2(pair x, pair up, pair low_up, unsigned& high, unsigned& low) {
+    const float2 f = floats_of(mul2(x, up));
     const __half2 h = __floats2half2_rn(f.x, f.y);
-    const float2 hf = __half22float2(h), r = floats_of(fma2(pair_of(hf.x, hf.y), pair_of(-1.f, -1.f), x));
+    const float2 hf = __half22float2(h), r = floats_of(fma2(pair_of(hf.x, hf.y), pair_of(-LOW_UP, -LOW_UP), mul2(x, low_up)));
     const __half2 l = __floats2half2_rn(r.x, r.y);
     high = *reinterpret_cast<const unsigned*>(&h);
     low = *reinterpret_cast<const unsigned*>(&l);
@@ -101,7 +109,7 @@ __device__ __forceinline__ void ldsm_t(unsigned (&r)[4], const __half* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
 }
-// c += (ah + al)(bh + bl) without al bl, the three terms in sums of their own; and the sum of those, elements 2 i and 2 i + 1
+// the products of two splits, without al bl, the three terms in sums of their own; and the sum of those, elements 2 i and 2 i + 1
 __device__ __forceinline__ void mma3(float (&c)[3][4], const unsigned (&ah)[4], const unsigned (&al)[4], unsigned bh0, unsigned bh1, unsigned bl0,
                                      unsigned bl1) {
     mma(c[0], al, bh0, bh1);
@@ -109,15 +117,16 @@ __device__ __forceinline__ void mma3(float (&c)[3][4], const unsigned (&ah)[4], 
     mma(c[2], ah, bh0, bh1);
 }
 __device__ __forceinline__ float2 sum3(const float (&c)[3][4], int i) {
-    return make_float2(c[2][2 * i] + (c[0][2 * i] + c[1][2 * i]), c[2][2 * i + 1] + (c[0][2 * i + 1] + c[1][2 * i + 1]));
+    return make_float2(fmaf(c[0][2 * i] + c[1][2 * i], LOW_DOWN, c[2][2 * i]), fmaf(c[0][2 * i + 1] + c[1][2 * i + 1], LOW_DOWN, c[2][2 * i + 1]));
 }
-// ... in two sums: `main` takes the first, `cross` the other two
+// ... in two sums: `main` takes the first, `cross` the other two; their sum times DOWN^2
 __device__ __forceinline__ void mma3(float (&main)[4], float (&cross)[4], const unsigned (&ah)[4], const unsigned (&al)[4],
                                      unsigned bh0, unsigned bh1, unsigned bl0, unsigned bl1) {
     mma(cross, al, bh0, bh1);
     mma(main, ah, bh0, bh1);
     mma(cross, ah, bl0, bl1);
 }
+__device__ __forceinline__ float sum2(float main, float cross) { return fmaf(cross, LOW_DOWN, main) * (DOWN * DOWN); }
 
 // An operand tile of CT rows of DP halves: the 16-byte group of element (row, col) lies at group (col / 8) ^ (row & 7) of its row, so
 // that eight rows' groups at one column fall on different banks.
@@ -182,15 +191,20 @@ __device__ __forceinline__ bool find_chunk(const int* cu_seqlens, int n_segments
     return false;
 }
 
-// What a chunk needs of one head besides operand tiles (floats; double-sized parts first).
-//   HEAD_DECAY, DELTA, KEY_DECAY: g [CT], w [CT], scalars [8]   (KEY_DECAY: and the chunk's decay per key [DP])
-//   MATRIX_MEMORY: M [CT] and F [CT] as doubles, w [CT], row sums of the scores [CT], scalars [8], sum_s w_s k_s [DP]
-enum Scalar { Q_DOWN = 0, K_DOWN = 1, P_DOWN = 2, DECAY = 3, W_DOWN = 4, BAD = 5 };
+// What a chunk needs of one head besides operand tiles (floats; double-sized parts first).  Sizes are those of the tokens' rows in the
+// tiles (Scale); a row of the tile of k is divided by its size, and `w` takes it back.
+//   HEAD_DECAY: g [CT], w [CT], sizes of q's rows [CT], of the scores' rows [CT], scalars [8]
+//   DELTA: g, w, sizes of W's rows [CT], -, scalars (the sizes of q, k and the scores are one)
+//   KEY_DECAY: -, w, sizes of q's rows, of the scores' rows, scalars, the chunk's decay per key [DP]
+//   MATRIX_MEMORY: M [CT] and F [CT] as doubles, w [CT], sizes of q's rows, of the scores' rows, row sums of the scores [CT], scalars [8],
+//   sum_s w_s k_s [DP]
+enum Scalar { DECAY = 0, BAD = 1 };
 template <int MODE, int DP> struct Record {
     static constexpr int G = 0;                           // (the memory's M, F: doubles at 0 and 2 CT)
     static constexpr int W = MODE == MATRIX_MEMORY ? 4 * CT : CT;
-    static constexpr int SUMS = 5 * CT;                   // the memory's alone
-    static constexpr int SCALARS = MODE == MATRIX_MEMORY ? 6 * CT : 2 * CT;
+    static constexpr int Q_SIZE = W + CT, W_SIZE = Q_SIZE, P_SIZE = W + 2 * CT;
+    static constexpr int SUMS = W + 3 * CT;               // the memory's alone
+    static constexpr int SCALARS = MODE == MATRIX_MEMORY ? 8 * CT : 4 * CT;
     static constexpr int KEYS = SCALARS + 8;
     static constexpr int FLOATS = KEYS + (MODE == MATRIX_MEMORY || MODE == KEY_DECAY ? DP : 0);
     static_assert(FLOATS % 4 == 0, "records are copied in 16-byte groups");
@@ -308,9 +322,7 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
     using Rec = typename SH::Rec;
     constexpr int DP = SH::DP, COLS = SH::COLS, THREADS = SH::THREADS, VP = SH::VP, TP = SH::TP, NK = KPW / 8, KS = KPW / 16;
     constexpr int NT = KW >= 4 ? 1 : 4 / KW;              // groups of eight tokens whose read-outs a warp finishes
-    constexpr bool WEIGHTED = MODE == DELTA || MODE == HEAD_DECAY;       // the values that join the state have a factor per token
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ unsigned largest_of[2][3];                 // largest magnitudes at the start of chunk c: of the state, of the memory's n; c % 3
     __shared__ __align__(8) unsigned long long full[3];   // a stage's tiles have landed
     __shared__ int abort_flag;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
@@ -330,7 +342,6 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
         return;
     }
     const int n_cols = min(COLS, p.vdim - col0), n_chunks = (t1 - t0 + CT - 1) / CT, chunk0 = chunks_before(p.cu_seqlens, seg);
-    if (tid < 3) { largest_of[0][tid] = 0; largest_of[1][tid] = 0; }
     if (tid == 0) {
         for (int i = 0; i < 3; ++i) tc::mbar_init(tc::smem_u32(&full[i]), 1);
         abort_flag = 0;
@@ -394,13 +405,6 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
         key = KPW * kw + 8 * n + 2 * t4 + (i & 1);
         return col < n_cols && key < p.dim;
     };
-    const auto mark_largest = [&](unsigned& slot_of) {    // of the warp's part of the state
-        float m = 0.f;
-#pragma unroll
-        for (int n = 0; n < NK; ++n) m = max_abs(m, max_abs(S[n][0], S[n][1], S[n][2]), S[n][3]);
-        const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-        if (lane == 0) atomicMax(&slot_of, bits);
-    };
 #pragma unroll
     for (int n = 0; n < NK; ++n)
 #pragma unroll
@@ -408,7 +412,6 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
             int col, key;
             S[n][i] = state_at(n, i, col, key) ? st[(size_t)key * p.key_stride + (size_t)(col0 + col) * p.col_stride] : 0.f;
         }
-    mark_largest(largest_of[0][0]);
     const float skip = p.skip ? p.skip[head] : 0.f;
     float m_run = 0.f;                                    // MATRIX_MEMORY: the running maximum (warp 0)
     float* n_s = extra;                                   // n, then the warps' parts of q . n of the chunk's tokens
@@ -437,10 +440,7 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
     if constexpr (MODE == MATRIX_MEMORY) {
         static_assert(COLS % 32 == 0, "a copy of n serves 32 columns");
         if (warp == 0) m_run = st_n[p.dim];
-        for (int d = tid; d < DP; d += THREADS) {
-            n_s[d] = d < p.dim ? st_n[d] : 0.f;
-            atomicMax(&largest_of[1][0], abs_bits(n_s[d]));
-        }
+        for (int d = tid; d < DP; d += THREADS) n_s[d] = d < p.dim ? st_n[d] : 0.f;
     }
     wait_for(0, 0, 0);
     __syncthreads();
@@ -471,20 +471,31 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
         const int tb = t0 + c * CT, len = min(CT, t1 - tb);
         float* sum = sums + (MODE == DELTA ? 0 : (c & 1) * SH::SUM_FLOATS);
         const float* fac = factors + slot3 * SH::FACTORS;
-        const unsigned state_largest = largest_of[0][slot3], slot_now = slot3, slot_next = slot3 == 2 ? 0 : slot3 + 1;
-        lost |= state_largest >= 0x7f800000u;
-        if (tid < 2) largest_of[tid][slot_next == 2 ? 0 : slot_next + 1] = 0;
-        const Scale ss = scale_of(state_largest);
+        const unsigned slot_next = slot3 == 2 ? 0 : slot3 + 1;
 
-        // ---- (Q S0)^T, and (W S0)^T, over the warp's keys: still scaled
+        // ---- (Q S0)^T, and (W S0)^T, over the warp's keys: still to be multiplied by the sizes of q's and W's rows
         {
-            const pair up = pair_of(ss.up, ss.up);
+            float largest[2] = {0.f, 0.f}, down[2];       // of the columns g and g + 8
+            pair up[2], low_up[2];
+#pragma unroll
+            for (int n = 0; n < NK; ++n)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) largest[i] = max_abs(largest[i], S[n][2 * i], S[n][2 * i + 1]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const unsigned bits = quad_max(__float_as_uint(largest[i]));
+                lost |= bits >= 0x7f800000u;
+                const Scale s = scale_of(bits);
+                up[i] = pair_of(s.up, s.up);
+                low_up[i] = pair_of(s.up * LOW_UP, s.up * LOW_UP);
+                down[i] = s.size * (DOWN * DOWN);
+            }
             unsigned ah[KS][4], al[KS][4];
 #pragma unroll
             for (int k = 0; k < KS; ++k)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    split2(pair_of(S[2 * k + (i >> 1)][2 * (i & 1)], S[2 * k + (i >> 1)][2 * (i & 1) + 1]), up, ah[k][i], al[k][i]);
+                    split2(pair_of(S[2 * k + (i >> 1)][2 * (i & 1)], S[2 * k + (i >> 1)][2 * (i & 1) + 1]), up[i & 1], low_up[i & 1], ah[k][i], al[k][i]);
             const auto product = [&](const __half* tile, float* to) {
                 to += (kw * COLS + 16 * cw + g) * TP + 2 * t4;
                 float acc[4][3][4] = {};                  // groups of eight tokens; the terms apart, so that no sum waits for another
@@ -501,19 +512,20 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
 #pragma unroll
                 for (int n = 0; n < 4; ++n)
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) *(float2*)(to + 8 * i * TP + 8 * n) = sum3(acc[n], i);
+                    for (int i = 0; i < 2; ++i) {
+                        const float2 x = sum3(acc[n], i);
+                        *(float2*)(to + 8 * i * TP + 8 * n) = make_float2(x.x * down[i], x.y * down[i]);
+                    }
             };
             product(q_s, sum);
             if constexpr (MODE == DELTA) product(w_s, sum + SH::SUM_FLOATS);
         }
-        const float q_down = ss.down * rec[Rec::SCALARS + Q_DOWN];
         // ---- the chunk's values as left operands (columns g, g + 8; tokens 16 k + 2 t4, + 1, + 8, + 9)
         float2 va[2][4];                                  // [sixteen tokens][register]
         if constexpr (MODE == DELTA) {                    // V <- U0 - g (W S0); what the read-outs start from beside it
             __syncthreads();
             float* u_s = extra;
             float* z_s = extra + COLS * TP;
-            const float w_down = ss.down * rec[Rec::SCALARS + W_DOWN];
             for (int e = tid; e < COLS * (CT / 4); e += THREADS) {
                 const int j = e % COLS, t = 4 * (e / COLS);
                 float4 y = make_float4(0.f, 0.f, 0.f, 0.f), z = y;
@@ -523,11 +535,11 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
                     z.x += a.x; z.y += a.y; z.z += a.z; z.w += a.w;
                     y.x += b.x; y.y += b.y; y.z += b.z; y.w += b.w;
                 }
-                const float4 gg = *(const float4*)(rec + Rec::G + t);
+                const float4 gg = *(const float4*)(rec + Rec::G + t), ws = *(const float4*)(rec + Rec::W_SIZE + t);
                 *(float4*)(u_s + j * TP + t) =
-                    make_float4(fmaf(-gg.x, y.x * w_down, v_s[t * VP + j]), fmaf(-gg.y, y.y * w_down, v_s[(t + 1) * VP + j]),
-                                fmaf(-gg.z, y.z * w_down, v_s[(t + 2) * VP + j]), fmaf(-gg.w, y.w * w_down, v_s[(t + 3) * VP + j]));
-                *(float4*)(z_s + j * TP + t) = make_float4(gg.x * (z.x * q_down), gg.y * (z.y * q_down), gg.z * (z.z * q_down), gg.w * (z.w * q_down));
+                    make_float4(fmaf(-gg.x, y.x * ws.x, v_s[t * VP + j]), fmaf(-gg.y, y.y * ws.y, v_s[(t + 1) * VP + j]),
+                                fmaf(-gg.z, y.z * ws.z, v_s[(t + 2) * VP + j]), fmaf(-gg.w, y.w * ws.w, v_s[(t + 3) * VP + j]));
+                *(float4*)(z_s + j * TP + t) = make_float4(gg.x * z.x, gg.y * z.y, gg.z * z.z, gg.w * z.w);
             }
             __syncthreads();
 #pragma unroll
@@ -544,24 +556,27 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
                 }
         }
         unsigned vh[2][4], vl[2][4];                      // V split, and as it joins the state
-        float v_down;
-        {
-            float m = 0.f;
+        float v_down[2];                                  // the columns' sizes times DOWN^2
+        const auto split_values = [&] {
+            pair up[2], low_up[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float m = max_abs(max_abs(max_abs(va[0][i].x, va[0][i].y, va[0][i + 2].x), va[0][i + 2].y, va[1][i].x),
+                                        max_abs(va[1][i].y, va[1][i + 2].x, va[1][i + 2].y), 0.f);
+                const unsigned bits = quad_max(__float_as_uint(m));
+                lost |= bits >= 0x7f800000u;
+                const Scale s = scale_of(bits);
+                up[i] = pair_of(s.up, s.up);
+                low_up[i] = pair_of(s.up * LOW_UP, s.up * LOW_UP);
+                v_down[i] = s.size * (DOWN * DOWN);
+            }
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) m = max_abs(m, va[k][i].x, va[k][i].y);
-            const unsigned largest = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-            lost |= largest >= 0x7f800000u;
-            const Scale s = scale_of(largest);
-            const pair up = pair_of(s.up, s.up);
-            v_down = s.down;
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) split2(pair_of(va[k][i].x, va[k][i].y), up, vh[k][i], vl[k][i]);
-        }
-        // ---- P V of the tokens that the warp finishes
+                for (int i = 0; i < 4; ++i) split2(pair_of(va[k][i].x, va[k][i].y), up[i & 1], low_up[i & 1], vh[k][i], vl[k][i]);
+        };
+        split_values();
+        // ---- P V of the tokens that the warp finishes (still to be multiplied by the sizes of P's rows)
         float o[NT][4];
         if (KW <= 4 || kw < 4) {
 #pragma unroll
@@ -576,37 +591,24 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float2 x = sum3(acc, r);
-                    o[n][2 * r] = x.x; o[n][2 * r + 1] = x.y;
+                    o[n][2 * r] = x.x * v_down[r]; o[n][2 * r + 1] = x.y * v_down[r];
                 }
             }
         }
-        const float p_down = v_down * rec[Rec::SCALARS + P_DOWN];
         // ---- the state after the chunk
-        if constexpr (WEIGHTED) {
-            float m = 0.f;
 #pragma unroll
-            for (int k = 0; k < 2; ++k)
+        for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 w = *(const float2*)(rec + Rec::W + 16 * k + 2 * t4 + 8 * (i >> 1));
-                    va[k][i].x *= w.x; va[k][i].y *= w.y;
-                    m = max_abs(m, va[k][i].x, va[k][i].y);
-                }
-            const unsigned largest = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-            lost |= largest >= 0x7f800000u;
-            const Scale s = scale_of(largest);
-            const pair up = pair_of(s.up, s.up);
-            v_down = s.down;
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) split2(pair_of(va[k][i].x, va[k][i].y), up, vh[k][i], vl[k][i]);
-        }
+            for (int i = 0; i < 4; ++i) {
+                const float2 w = *(const float2*)(rec + Rec::W + 16 * k + 2 * t4 + 8 * (i >> 1));
+                va[k][i].x *= w.x; va[k][i].y *= w.y;
+            }
+        split_values();
         {
-            float down = v_down * rec[Rec::SCALARS + K_DOWN], decay;
-            if constexpr (MODE == MATRIX_MEMORY) { decay = fac[3 * CT]; down *= fac[3 * CT + 1]; }
+            float decay;
+            if constexpr (MODE == MATRIX_MEMORY) { decay = fac[3 * CT]; v_down[0] *= fac[3 * CT + 1]; v_down[1] *= fac[3 * CT + 1]; }
             else decay = rec[Rec::SCALARS + DECAY];
-            const pair down2 = pair_of(down, down);
+            const pair down2[2] = {pair_of(v_down[0], v_down[0]), pair_of(v_down[1], v_down[1])};
             pair decay2 = pair_of(decay, decay);
             constexpr int NB = NK < 4 ? NK : 4;           // groups of eight keys at a time
 #pragma unroll
@@ -632,32 +634,38 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
                         const float2 y = sum3(acc[j], r);
-                        const float2 x = floats_of(fma2(decay2, pair_of(S[n + j][2 * r], S[n + j][2 * r + 1]), mul2(pair_of(y.x, y.y), down2)));
+                        const float2 x = floats_of(fma2(decay2, pair_of(S[n + j][2 * r], S[n + j][2 * r + 1]), mul2(pair_of(y.x, y.y), down2[r])));
                         S[n + j][2 * r] = x.x; S[n + j][2 * r + 1] = x.y;
                     }
                 }
             }
-            mark_largest(largest_of[0][slot_next]);
         }
         slot3 = slot_next;
         if constexpr (MODE == MATRIX_MEMORY) {
             // q . n of sixteen tokens over the warp's keys (n is row 0 of a left operand), then n after the chunk
             const float* n_old = n_s + (c & 1) * DP;
             float* n_new = n_s + ((c + 1) & 1) * DP;
-            const unsigned n_largest = largest_of[1][slot_now];
-            lost |= n_largest >= 0x7f800000u;
-            const Scale sn = scale_of(n_largest);
             if (cw < 2) {
                 float acc[2][3][4] = {};
+                float2 x[KS][2];
+                float m = 0.f;
+#pragma unroll
+                for (int k = 0; k < KS; ++k)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        x[k][i] = g == 0 ? *(const float2*)(n_old + KPW * kw + 16 * k + 8 * i + 2 * t4) : make_float2(0.f, 0.f);
+                        m = max_abs(m, x[k][i].x, x[k][i].y);
+                    }
+                const unsigned bits = quad_max(__float_as_uint(m));
+                lost |= bits >= 0x7f800000u;
+                const Scale sn = scale_of(bits);
+                const pair up = pair_of(sn.up, sn.up), low_up = pair_of(sn.up * LOW_UP, sn.up * LOW_UP);
 #pragma unroll
                 for (int k = 0; k < KS; ++k) {
                     unsigned ah[4] = {}, al[4] = {}, bh[4], bl[4];
                     if (g == 0) {
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const float2 x = *(const float2*)(n_old + KPW * kw + 16 * k + 8 * i + 2 * t4);
-                            split2(pair_of(x.x, x.y), pair_of(sn.up, sn.up), ah[2 * i], al[2 * i]);
-                        }
+                        for (int i = 0; i < 2; ++i) split2(pair_of(x[k][i].x, x[k][i].y), up, low_up, ah[2 * i], al[2 * i]);
                     }
                     ldsm(bh, q_s + at_q[k] + cw * 16 * DP);
                     ldsm(bl, q_s + CT * DP + at_q[k] + cw * 16 * DP);
@@ -666,22 +674,15 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
                 }
                 if (g == 0) {
                     float* to = nq_s + ((c & 1) * KW + kw) * CT + 16 * cw + 2 * t4;
-                    const float down = sn.down * rec[Rec::SCALARS + Q_DOWN];
+                    const float down = sn.size * (DOWN * DOWN);          // (still to be multiplied by the sizes of q's rows)
 #pragma unroll
                     for (int n = 0; n < 2; ++n) {
-                        const float2 x = sum3(acc[n], 0);
-                        *(float2*)(to + 8 * n) = make_float2(x.x * down, x.y * down);
+                        const float2 y = sum3(acc[n], 0);
+                        *(float2*)(to + 8 * n) = make_float2(y.x * down, y.y * down);
                     }
                 }
             }
-            unsigned largest = 0;
-            for (int d = tid; d < DP; d += THREADS) {
-                const float x = fmaf(fac[3 * CT], n_old[d], fac[3 * CT + 1] * rec[Rec::KEYS + d]);
-                n_new[d] = x;
-                largest = max(largest, abs_bits(x));
-            }
-            largest = __reduce_max_sync(0xffffffffu, largest);
-            if (lane == 0) atomicMax(&largest_of[1][slot_next], largest);
+            for (int d = tid; d < DP; d += THREADS) n_new[d] = fmaf(fac[3 * CT], n_old[d], fac[3 * CT + 1] * rec[Rec::KEYS + d]);
         }
         wait_for(c + 1, stage, parity);
         if constexpr (MODE == MATRIX_MEMORY) {            // the next chunk's factors, in front of the barrier below
@@ -690,13 +691,15 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
                              factors + slot_next * SH::FACTORS);
         }
         // what the read-outs take from this chunk's stage
-        float2 gt[NT], row_sum[NT], skipped[NT][2];
+        float2 gt[NT], row_sum[NT], skipped[NT][2], q_size[NT], p_size[NT];
         if constexpr (MODE != DELTA) {
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 const int t = 8 * (NT * kw + n) + 2 * t4;
+                q_size[n] = *(const float2*)(rec + Rec::Q_SIZE + (t & 31));
+                p_size[n] = *(const float2*)(rec + Rec::P_SIZE + (t & 31));
                 if constexpr (MODE == HEAD_DECAY) {
-                    gt[n] = *(const float2*)(rec + Rec::G + t);
+                    gt[n] = *(const float2*)(rec + Rec::G + (t & 31));
 #pragma unroll
                     for (int r = 0; r < 2; ++r)
                         skipped[n][r] = make_float2(skip * v_s[t * VP + 16 * cw + g + 8 * r], skip * v_s[(t + 1) * VP + 16 * cw + g + 8 * r]);
@@ -714,7 +717,10 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 const int t = 8 * (NT * kw + n) + 2 * t4;
-                float2 fz = make_float2(q_down * p.out_scale, q_down * p.out_scale), fo = make_float2(p_down * p.out_scale, p_down * p.out_scale);
+                float2 fz = make_float2(p.out_scale, p.out_scale), fo = fz;
+                if constexpr (MODE != DELTA) {
+                    fz.x *= q_size[n].x; fz.y *= q_size[n].y; fo.x *= p_size[n].x; fo.y *= p_size[n].y;
+                }
                 if constexpr (MODE == HEAD_DECAY) { fz.x *= gt[n].x; fz.y *= gt[n].y; }
                 if constexpr (MODE == MATRIX_MEMORY) {
                     const float2 ht = *(const float2*)(fac + CT + t), floor = *(const float2*)(fac + 2 * CT + t);
@@ -724,6 +730,7 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
                         const float2 a = *(const float2*)(nq_s + ((c & 1) * KW + k) * CT + t);
                         nq.x += a.x; nq.y += a.y;
                     }
+                    nq.x *= q_size[n].x; nq.y *= q_size[n].y;
                     const float rx = 1.f / (fmaxf(fabsf(p.out_scale * (gt[n].x * nq.x + ht.x * row_sum[n].x)), floor.x) + 1e-6f);
                     const float ry = 1.f / (fmaxf(fabsf(p.out_scale * (gt[n].y * nq.y + ht.y * row_sum[n].y)), floor.y) + 1e-6f);
                     fz.x *= gt[n].x * rx; fz.y *= gt[n].y * ry; fo.x *= ht.x * rx; fo.y *= ht.y * ry;

@@ -207,7 +207,8 @@ static int launch_scan(const DeltaParams& p, const Leftovers& left, cudaStream_t
 }
 
 // What the walk in chunks needs that does not depend on the state.  A block has one chunk and HB heads that share q and k, four warps a
-// head.  Left in working memory: the unit q and k and W = T beta K as split tiles (times 2^13), P alike, U0 = T' beta V in float32.
+// head.  Left in working memory: the unit q and k and P as split tiles (of size one), W = T beta K alike, its rows divided by their token's
+// beta's size (a row is no longer than its beta), U0 = T' beta V in float32.
 template <int DP, int HB>
 struct DeltaChunkSmem {
     __half qk[4][CT * DP];                                // as in working memory: q high, q low, k high, k low
@@ -216,12 +217,10 @@ struct DeltaChunkSmem {
         __half decayed[2][CT * CT], plain[2][CT * CT];    // T' beta and T beta, split
         float T[CT][36], X[16][20];
         double b[CT];
-        float beta[CT];
+        float beta[CT], size[CT];                         // `size`: of beta (Scale), by which the rows of T' beta, T beta and W are divided
     } head[HB];
     int bad[HB];
 };
-
-constexpr float UNIT_UP = 8192.f, UNIT_DOWN = 1.f / 8192.f;   // for numbers of size one at most
 
 template <int DP, int HB>
 __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams p, const Made out) {
@@ -275,6 +274,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
             gates[2 * p.kv_heads + p.heads + head] = expf(log_decay);
         }
         hd.beta[lane] = beta;
+        hd.size[lane] = scale_of(abs_bits(beta)).size;
         hd.b[lane] = prefix_sum((double)bounded_log(log_decay), lane);
     }
     // the values of the warp's first two groups of sixteen columns, as left operands: columns g, g + 8, tokens 2 t4, + 1, + 8, + 9
@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const int at = tile_at<DP>(t, lane + 32 * e);
-            split1(t < len ? qv[i][e] * rq * UNIT_UP : 0.f, sm.qk[0][at], sm.qk[1][at]);
-            split1(t < len ? kv[i][e] * rk * UNIT_UP : 0.f, sm.qk[2][at], sm.qk[3][at]);
+            split1(t < len ? qv[i][e] * rq * UP : 0.f, sm.qk[0][at], sm.qk[1][at]);
+            split1(t < len ? kv[i][e] * rk * UP : 0.f, sm.qk[2][at], sm.qk[3][at]);
         }
     }
     if (brief) return;
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
 #pragma unroll
             for (int r = 0; r < 2; ++r)
                 *(float2*)&to[16 * m + g + 8 * r][8 * (n0 + n) + 2 * t4] =
-                    make_float2((main[n][2 * r] + cross[n][2 * r]) * (UNIT_DOWN * UNIT_DOWN), (main[n][2 * r + 1] + cross[n][2 * r + 1]) * (UNIT_DOWN * UNIT_DOWN));
+                    make_float2(sum2(main[n][2 * r], cross[n][2 * r]), sum2(main[n][2 * r + 1], cross[n][2 * r + 1]));
     }
     if (head0 % group == 0) {                             // q and k of the group's heads are the same
         uint4* dst = reinterpret_cast<uint4*>(out.qk + ((size_t)blockIdx.x * p.kv_heads + kvh) * (4 * CT * DP));
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
             const int t = e >> 4, s = 2 * (e & 15);
             float x[2];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) x[i] = s + i <= t && t < len ? sm.qk_scores[t][s + i] * expf((float)(hd.b[t] - hd.b[s + i])) * UNIT_UP : 0.f;
+            for (int i = 0; i < 2; ++i) x[i] = s + i <= t && t < len ? sm.qk_scores[t][s + i] * expf((float)(hd.b[t] - hd.b[s + i])) * UP : 0.f;
             unsigned h, l;
             split2(x[0], x[1], h, l);
             *(unsigned*)(scores + score_at(t, s)) = h;
@@ -411,10 +411,11 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int e = tt + 128 * r, t = e >> 4, s = 2 * (e & 15), at = score_at(t, s);
+        const float up = UP / hd.size[t];                 // (a power of two)
         float x[2], y[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            x[i] = s + i <= t ? hd.T[t][s + i] * hd.beta[s + i] * UNIT_UP : 0.f;
+            x[i] = s + i <= t ? hd.T[t][s + i] * hd.beta[s + i] * up : 0.f;
             y[i] = s + i <= t ? x[i] * expf((float)(hd.b[t] - hd.b[s + i])) : 0.f;
         }
         split2(x[0], x[1], *(unsigned*)&hd.plain[0][at], *(unsigned*)&hd.plain[1][at]);
@@ -423,19 +424,23 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
     __syncthreads();
     // ---- U0^T = V^T (T' beta)^T, sixteen columns at a time
     const auto u0_tile = [&](int tile, const float (&v)[2][4][2]) {
-        unsigned largest = 0;
+        Scale sc[2];                                      // of the columns g and g + 8
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+        for (int c = 0; c < 2; ++c) {
+            unsigned largest = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) largest = max(largest, max(abs_bits(v[k][i][0]), abs_bits(v[k][i][1])));
-        largest = __reduce_max_sync(0xffffffffu, largest);
-        bad |= largest >= 0x7f800000u;
-        const Scale s = scale_of(largest);
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int i = c; i < 4; i += 2) largest = max(largest, max(abs_bits(v[k][i][0]), abs_bits(v[k][i][1])));
+            largest = quad_max(largest);
+            bad |= largest >= 0x7f800000u;
+            sc[c] = scale_of(largest);
+        }
         unsigned ah[2][4], al[2][4];
 #pragma unroll
         for (int k = 0; k < 2; ++k)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) split2(v[k][i][0] * s.up, v[k][i][1] * s.up, ah[k][i], al[k][i]);
+            for (int i = 0; i < 4; ++i) split2(v[k][i][0] * sc[i & 1].up, v[k][i][1] * sc[i & 1].up, ah[k][i], al[k][i]);
         float* u0 = out.u0 + (size_t)first * p.heads * vdim + (size_t)head * vdim;
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int t = 8 * n + 2 * t4 + (i & 1), col = 16 * tile + g + 8 * (i >> 1);
-                if (t < len && col < vdim) u0[(size_t)t * p.heads * vdim + col] = (main[i] + cross[i]) * (s.down * UNIT_DOWN);
+                if (t < len && col < vdim) u0[(size_t)t * p.heads * vdim + col] = sum2(main[i], cross[i]) * sc[i >> 1].size * hd.size[t];
             }
         }
     };
@@ -485,7 +490,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
             for (int r = 0; r < 2; ++r) {
                 const int at = tile_at<DP>(16 * m + g + 8 * r, DP / 4 * tw + 8 * n + 2 * t4);
                 unsigned h, l;
-                split2((main[n][2 * r] + cross[n][2 * r]) * UNIT_DOWN, (main[n][2 * r + 1] + cross[n][2 * r + 1]) * UNIT_DOWN, h, l);
+                split2(sum2(main[n][2 * r], cross[n][2 * r]) * UP, sum2(main[n][2 * r + 1], cross[n][2 * r + 1]) * UP, h, l);
                 *(unsigned*)(w + at) = h;
                 *(unsigned*)(w + CT * DP + at) = l;
             }
@@ -496,10 +501,11 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
         const double last = hd.b[len - 1];
         rec[Rec::G + lane] = lane < len ? expf((float)hd.b[lane]) : 0.f;
         rec[Rec::W + lane] = lane < len ? expf((float)(last - hd.b[lane])) : 0.f;
+        rec[Rec::W_SIZE + lane] = hd.size[lane];
         if (lane < 8) {
             bool any = false;
             for (int h = 0; h < HB; ++h) any |= sm.bad[h] != 0;       // (a block's heads share q and k)
-            rec[Rec::SCALARS + lane] = lane == DECAY ? expf((float)last) : lane == BAD ? (any ? 1.f : 0.f) : UNIT_DOWN;
+            rec[Rec::SCALARS + lane] = lane == DECAY ? expf((float)last) : lane == BAD && any ? 1.f : 0.f;
         }
     }
 }

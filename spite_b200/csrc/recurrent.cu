@@ -583,13 +583,14 @@ int launch_mlstm_chunk(const MlstmParams& p, float* scratch, int scratch_chunks,
 
 // ---- the same in chunks of 32 tokens on the tensor cores (chunk.cuh), for up to 256 key rows.  What a chunk needs that does not depend on
 // the state, one block a (chunk, head): q and k as split tiles; a_s, F_t and the running maximum M_t of a_s within the chunk (m0
-// joins in the walk: max(m0, M_t)); the scores exp(a_s - M_t) q_t . k_s (s <= t) as a split tile, and their sums over s; k_s times its
-// weight exp(a_s - M_last) as a split tile, which the state takes, and the sum of those, which n takes.
+// joins in the walk: max(m0, M_t)); the scores exp(a_s - M_t) q_t . k_s (s <= t) as a split tile, and their sums over s; the weights
+// exp(a_s - M_last), with which the state takes k_s v_s, and the sum of the weighted k_s, which n takes.
 template <int DP> struct MemoryChunkSmem {
     __half qk[4][chunk::CT * DP];
     float P[chunk::CT][36], kn[8][DP], w[chunk::CT];
     double a[chunk::CT], M[chunk::CT];
-    unsigned largest[3], bad;                             // of q, k and the scores
+    float q_size[chunk::CT], k_size[chunk::CT];           // of the tokens' rows (Scale)
+    unsigned bad;
 };
 
 template <int DP>
@@ -610,8 +611,7 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, 
     const float* rows = p.proj + (size_t)first * p.stride;
     const size_t at_head = (size_t)blockIdx.x * p.heads + head;
     float* rec = out.records + at_head * Rec::FLOATS;
-    if (tid < 3) sm.largest[tid] = 0;
-    if (tid == 3) sm.bad = 0;
+    if (tid == 0) sm.bad = 0;
 
     // a warp has the tokens warp, warp + 8, ..., a lane the elements lane, lane + 32, ...
     constexpr int E = DP / 32;
@@ -645,28 +645,28 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, 
         sm.a[lane] = a; sm.M[lane] = M; sm.w[lane] = w;
         double* md = reinterpret_cast<double*>(rec);
         md[lane] = M; md[CL + lane] = F;
-        rec[Rec::W + lane] = w;
     }
-    unsigned lq = 0, lk = 0;
+    Scale sq[4], sk[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        unsigned lq = 0, lk = 0;
 #pragma unroll
         for (int e = 0; e < E; ++e) { lq = max(lq, abs_bits(qv[i][e])); lk = max(lk, abs_bits(kv[i][e])); }
-    lq = __reduce_max_sync(0xffffffffu, lq);
-    lk = __reduce_max_sync(0xffffffffu, lk);
+        lq = __reduce_max_sync(0xffffffffu, lq);
+        lk = __reduce_max_sync(0xffffffffu, lk);
+        bad |= max(lq, lk) >= 0x7f800000u;
+        sq[i] = scale_of(lq); sk[i] = scale_of(lk);
+        if (lane == 0) { sm.q_size[warp + 8 * i] = sq[i].size; sm.k_size[warp + 8 * i] = sk[i].size; }
+    }
     __syncthreads();
-    if (lane == 0) { atomicMax(&sm.largest[0], lq); atomicMax(&sm.largest[1], lk); }
-    __syncthreads();
-    const Scale sq = scale_of(sm.largest[0]), sk = scale_of(sm.largest[1]);
-    bad |= max(sm.largest[0], sm.largest[1]) >= 0x7f800000u;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         float sum = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int t = warp + 8 * i, at = tile_at<DP>(t, lane + 32 * e);
-            split1(qv[i][e] * sq.up, sm.qk[0][at], sm.qk[1][at]);
-            split1(kv[i][e] * sk.up, sm.qk[2][at], sm.qk[3][at]);
+            split1(qv[i][e] * sq[i].up, sm.qk[0][at], sm.qk[1][at]);
+            split1(kv[i][e] * sk[i].up, sm.qk[2][at], sm.qk[3][at]);
             sum = fmaf(sm.w[t], kv[i][e], sum);
         }
         sm.kn[warp][lane + 32 * e] = sum;
@@ -690,52 +690,43 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, 
                 mma3(main, cross, ah, al, bh[2], bh[3], bl[2], bl[3]);
             }
         }
-        unsigned largest = 0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int t = 16 * m + g + 8 * (i >> 1), s = 8 * n + 2 * t4 + (i & 1);
-            const float x = s <= t ? (main[i] + cross[i]) * sq.down * sk.down * expf((float)(sm.a[s] - sm.M[t])) : 0.f;
-            sm.P[t][s] = x;
-            largest = max(largest, abs_bits(x));
+            sm.P[t][s] = s <= t ? sum2(main[i], cross[i]) * sm.q_size[t] * sm.k_size[s] * expf((float)(sm.a[s] - sm.M[t])) : 0.f;
         }
-        largest = __reduce_max_sync(0xffffffffu, largest);
-        if (lane == 0) atomicMax(&sm.largest[2], largest);
         if (bad) sm.bad = 1;
     }
     __syncthreads();
+    bool lost;
     {   // a thread has a token and four tokens s
         const int t = tid >> 3, s = 4 * (tid & 7);
-        const Scale sp = scale_of(sm.largest[2]);
         const float4 x = *(const float4*)&sm.P[t][s];
+        unsigned largest = quad_max(max(max(abs_bits(x.x), abs_bits(x.y)), max(abs_bits(x.z), abs_bits(x.w))));
+        largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 4));
+        const Scale sp = scale_of(largest);
+        lost = largest >= 0x7f800000u;
         float sum = (x.x + x.y) + (x.z + x.w);
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-        if ((tid & 7) == 0) rec[Rec::SUMS + t] = sum;
+        if ((tid & 7) == 0) { rec[Rec::SUMS + t] = sum; rec[Rec::P_SIZE + t] = sp.size; }
         uint2 h, l;
         split2(x.x * sp.up, x.y * sp.up, h.x, l.x);
         split2(x.z * sp.up, x.w * sp.up, h.y, l.y);
         __half* scores = out.scores + at_head * (2 * CL * CL) + score_at(t, s);
         *(uint2*)scores = h;
         *(uint2*)(scores + CL * CL) = l;
-        if (tid < 8)
-            rec[Rec::SCALARS + tid] = tid == Q_DOWN ? sq.down : tid == K_DOWN ? sk.down : tid == P_DOWN ? sp.down
-                                    : tid == BAD ? (sm.bad || sm.largest[2] >= 0x7f800000u ? 1.f : 0.f) : 0.f;
+        if (tid < CL) { rec[Rec::Q_SIZE + tid] = sm.q_size[tid]; rec[Rec::W + tid] = sm.w[tid] * sm.k_size[tid]; }
     }
+    lost = __syncthreads_or(lost);
+    if (tid < 8) rec[Rec::SCALARS + tid] = tid == BAD && (sm.bad || lost) ? 1.f : 0.f;
     for (int d = tid; d < DP; d += 256) {
         float sum = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) sum += sm.kn[i][d];
         rec[Rec::KEYS + d] = sum;
     }
-#pragma unroll
-    for (int e = 0; e < E; ++e)                           // the scores are made: k takes its weights (at most one, so the scale holds)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = warp + 8 * i, at = tile_at<DP>(t, lane + 32 * e);
-            split1(sm.w[t] * kv[i][e] * sk.up, sm.qk[2][at], sm.qk[3][at]);
-        }
-    __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(out.qk + at_head * (4 * CL * DP));
     const uint4* src = reinterpret_cast<const uint4*>(sm.qk[0]);
 #pragma unroll 4

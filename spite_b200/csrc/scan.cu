@@ -448,14 +448,14 @@ int choose_scan(const ScanParams& p, cudaStream_t st, const Leftovers& left = {}
 
 // ---- what the walk in chunks needs that does not depend on the state
 // q and k of a chunk (a warp has the tokens warp, warp + 8, ..., a lane the elements lane, lane + 32, ...; 256 threads) into split tiles;
-// q_t . k_s into `scores`.  Returns the tiles' scales, and whether a number is not finite.  `largest`: two zeroed words.
+// q_t . k_s into `scores`, the sizes of the tokens' rows into `q_size`, `k_size`.  Returns whether a number is not finite (of the warp's).
 template <int DP>
 __device__ __forceinline__ bool split_tiles(const float* q, long long q_stride, const float* k, long long k_stride, int len, int dim, __half* tiles,
-                                            float (*scores)[36], unsigned* largest, Scale& sq, Scale& sk) {
+                                            float (*scores)[36], float* q_size, float* k_size) {
     constexpr int E = DP / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
     float qv[4][E], kv[4][E];
-    unsigned lq = 0, lk = 0;
+    bool bad = false;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -466,23 +466,22 @@ __device__ __forceinline__ bool split_tiles(const float* q, long long q_stride, 
             kv[i][e] = on ? k[t * k_stride + d] : 0.f;
         }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        unsigned lq = 0, lk = 0;
 #pragma unroll
         for (int e = 0; e < E; ++e) { lq = max(lq, abs_bits(qv[i][e])); lk = max(lk, abs_bits(kv[i][e])); }
-    lq = __reduce_max_sync(0xffffffffu, lq);
-    lk = __reduce_max_sync(0xffffffffu, lk);
-    if (lane == 0) { atomicMax(&largest[0], lq); atomicMax(&largest[1], lk); }
-    __syncthreads();
-    sq = scale_of(largest[0]);
-    sk = scale_of(largest[1]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
+        lq = __reduce_max_sync(0xffffffffu, lq);
+        lk = __reduce_max_sync(0xffffffffu, lk);
+        bad |= max(lq, lk) >= 0x7f800000u;
+        const Scale sq = scale_of(lq), sk = scale_of(lk);
+        if (lane == 0) { q_size[warp + 8 * i] = sq.size; k_size[warp + 8 * i] = sk.size; }
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const int at = tile_at<DP>(warp + 8 * i, lane + 32 * e);
             split1(qv[i][e] * sq.up, tiles[at], tiles[CT * DP + at]);
             split1(kv[i][e] * sk.up, tiles[2 * CT * DP + at], tiles[3 * CT * DP + at]);
         }
+    }
     __syncthreads();
     const int m = warp & 1, n = warp >> 1;                // sixteen tokens t and eight tokens s a warp
     float main[4] = {}, cross[4] = {};
@@ -500,11 +499,14 @@ __device__ __forceinline__ bool split_tiles(const float* q, long long q_stride, 
             mma3(main, cross, ah, al, bh[2], bh[3], bl[2], bl[3]);
         }
     }
+    const float2 ks = *(const float2*)(k_size + 8 * n + 2 * t4);
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
-        *(float2*)&scores[16 * m + g + 8 * r][8 * n + 2 * t4] = make_float2((main[2 * r] + cross[2 * r]) * sq.down * sk.down,
-                                                                             (main[2 * r + 1] + cross[2 * r + 1]) * sq.down * sk.down);
-    return max(largest[0], largest[1]) >= 0x7f800000u;
+    for (int r = 0; r < 2; ++r) {
+        const float qs = q_size[16 * m + g + 8 * r];
+        *(float2*)&scores[16 * m + g + 8 * r][8 * n + 2 * t4] = make_float2(sum2(main[2 * r], cross[2 * r]) * qs * ks.x,
+                                                                             sum2(main[2 * r + 1], cross[2 * r + 1]) * qs * ks.y);
+    }
+    return bad;
 }
 template <int DP> __device__ __forceinline__ void store_tiles(__half* to, const __half* tiles) {
     uint4* dst = reinterpret_cast<uint4*>(to);
@@ -519,8 +521,7 @@ template <int DP> struct StateSpaceChunkSmem {
     __half tiles[4 * CT * DP];
     float scores[CT][36];
     double b[8][CT];
-    float dt[8][CT];
-    unsigned largest[2];
+    float dt[8][CT], q_size[CT], k_size[CT];
 };
 template <int DP>
 __global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams p, const float* __restrict__ a, long long a_stride,
@@ -540,15 +541,12 @@ __global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams
     const bool brief = p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens;     // walked token by token: the tokens' scalars alone
     if (first == p.cu_seqlens[seg])
         for (int h = h0 + warp; h < h1; h += 8) clear_marks(out.columns, out.column_groups, seg, h, p.heads, lane, 32);
-    Scale sq, sk;
     bool bad = false;
     if (!brief) {
-        if (tid < 2) sm.largest[tid] = 0;
-        __syncthreads();
         bad = split_tiles<DP>(p.q + (size_t)first * p.q_stride + (size_t)kvh * p.dim, p.q_stride, p.k + (size_t)first * p.k_stride + (size_t)kvh * p.dim,
-                              p.k_stride, len, p.dim, sm.tiles, sm.scores, sm.largest, sq, sk);
+                              p.k_stride, len, p.dim, sm.tiles, sm.scores, sm.q_size, sm.k_size);
         if (slice == 0) store_tiles<DP>(out.qk + ((size_t)blockIdx.x * p.kv_heads + kvh) * (4 * CT * DP), sm.tiles);
-        __syncthreads();
+        bad = __syncthreads_or(bad);
     }
     for (int h = h0 + warp; h < h1; h += 8) {             // a lane a token
         float dt = 0.f, log_decay = 0.f;
@@ -566,39 +564,38 @@ __global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams
         sm.b[warp][lane] = b;
         sm.dt[warp][lane] = dt;
         __syncwarp();
-        const int s = 2 * (lane & 15);
-        const double b0 = sm.b[warp][s], b1 = sm.b[warp][s + 1];
-        const float d0 = sm.dt[warp][s], d1 = sm.dt[warp][s + 1];
-        float2 x[CT / 2];
+        float x[CT];                                      // a lane has a row of scores
         unsigned largest = 0;
 #pragma unroll
-        for (int i = 0; i < CT / 2; ++i) {
-            const int t = 2 * i + (lane >> 4);
-            const double bt = sm.b[warp][t];
-            const float2 gs = *(const float2*)&sm.scores[t][s];
-            x[i].x = s <= t ? gs.x * expf((float)(bt - b0)) * d0 : 0.f;
-            x[i].y = s + 1 <= t ? gs.y * expf((float)(bt - b1)) * d1 : 0.f;
-            largest = max(largest, max(abs_bits(x[i].x), abs_bits(x[i].y)));
+        for (int s = 0; s < CT; s += 4) {
+            const float4 gs = *(const float4*)&sm.scores[lane][s];
+            const float row[4] = {gs.x, gs.y, gs.z, gs.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                x[s + i] = s + i <= lane ? row[i] * expf((float)(b - sm.b[warp][s + i])) * sm.dt[warp][s + i] : 0.f;
+                largest = max(largest, abs_bits(x[s + i]));
+            }
         }
-        largest = __reduce_max_sync(0xffffffffu, largest);
         const Scale sp = scale_of(largest);
         const size_t at_head = (size_t)blockIdx.x * p.heads + h;
         __half* scores = out.scores + at_head * (2 * CT * CT);
 #pragma unroll
-        for (int i = 0; i < CT / 2; ++i) {
-            unsigned hi, lo;
-            split2(x[i].x * sp.up, x[i].y * sp.up, hi, lo);
-            const int at = score_at(2 * i + (lane >> 4), s);
-            *(unsigned*)(scores + at) = hi;
-            *(unsigned*)(scores + CT * CT + at) = lo;
+        for (int s = 0; s < CT; s += 8) {
+            uint4 hi, lo;
+            split2(x[s] * sp.up, x[s + 1] * sp.up, hi.x, lo.x);
+            split2(x[s + 2] * sp.up, x[s + 3] * sp.up, hi.y, lo.y);
+            split2(x[s + 4] * sp.up, x[s + 5] * sp.up, hi.z, lo.z);
+            split2(x[s + 6] * sp.up, x[s + 7] * sp.up, hi.w, lo.w);
+            *(uint4*)(scores + score_at(lane, s)) = hi;
+            *(uint4*)(scores + CT * CT + score_at(lane, s)) = lo;
         }
         lost = __any_sync(0xffffffffu, lost || bad || largest >= 0x7f800000u);
         float* rec = out.records + at_head * Rec::FLOATS;
         rec[Rec::G + lane] = expf((float)b);
-        rec[Rec::W + lane] = dt * expf((float)(last - b));          // (beyond the chunk's tokens dt is zero)
-        if (lane < 8)
-            rec[Rec::SCALARS + lane] = lane == Q_DOWN ? sq.down : lane == K_DOWN ? sk.down : lane == P_DOWN ? sp.down
-                                     : lane == DECAY ? expf((float)last) : lane == BAD ? (lost ? 1.f : 0.f) : 0.f;
+        rec[Rec::W + lane] = dt * expf((float)(last - b)) * sm.k_size[lane];          // (beyond the chunk's tokens dt is zero)
+        rec[Rec::Q_SIZE + lane] = sm.q_size[lane];
+        rec[Rec::P_SIZE + lane] = sp.size;
+        if (lane < 8) rec[Rec::SCALARS + lane] = lane == DECAY ? expf((float)last) : lane == BAD && lost ? 1.f : 0.f;
     }
 }
 
@@ -610,7 +607,7 @@ template <int DP> struct KeyDecayChunkSmem {
     float q[CT][DP + 4], k[CT][DP + 4], w[CT][DP + 4];
     float P[CT][36];
     float part[256 / DP][DP];                             // sums of log decays of a thread's tokens
-    unsigned largest[5];                                  // of q and k in `tiles`, k and q in `off`, the scores
+    unsigned largest[3][CT];                              // of the rows of q and of k in `tiles`, of those of `off`
     int bad;
 };
 template <int DP, bool BONUS>
@@ -627,8 +624,8 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
     if (first == p.cu_seqlens[seg]) clear_marks(out.columns, out.column_groups, seg, head, p.heads, tid, 256);
     if (p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens) return;
     const int len = min(CT, p.cu_seqlens[seg + 1] - first);
-    if (tid < 5) sm.largest[tid] = 0;
-    if (tid == 5) sm.bad = 0;
+    if (tid < 3 * CT) sm.largest[tid / CT][tid % CT] = 0;
+    if (tid == 0) sm.bad = 0;
     const size_t at_head = (size_t)blockIdx.x * p.heads + head;
     const int ch = tid % DP, part = tid / DP;
     float qv[TN], kv[TN], lw[TN];                         // q, k and the log decays
@@ -673,7 +670,6 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
             last += s;
         }
         float qs[TN], ks[TN], os[TN];
-        unsigned lq = 0, lk = 0, lo = 0;
         float run = 0.f, back = 0.f;
 #pragma unroll
         for (int i = 0; i < TN; ++i) {                    // (a token of the memory is read before its own decay)
@@ -690,29 +686,23 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
         }
 #pragma unroll
         for (int i = 0; i < TN; ++i) {
-            lq = max(lq, abs_bits(qs[i])); lk = max(lk, abs_bits(ks[i])); lo = max(lo, abs_bits(os[i]));
+            const unsigned lq = __reduce_max_sync(0xffffffffu, abs_bits(qs[i])), lk = __reduce_max_sync(0xffffffffu, abs_bits(ks[i])),
+                           lo = __reduce_max_sync(0xffffffffu, abs_bits(os[i]));
             bad |= max(abs_bits(qv[i]), abs_bits(kv[i])) >= 0x7f800000u;
-        }
-        lq = __reduce_max_sync(0xffffffffu, lq);
-        lk = __reduce_max_sync(0xffffffffu, lk);
-        lo = __reduce_max_sync(0xffffffffu, lo);
-        if (lane == 0) {
-            atomicMax(&sm.largest[0], lq); atomicMax(&sm.largest[1], lk);
-            atomicMax(&sm.largest[part < PARTS / 2 ? 2 : 3], lo);
+            if (lane < 3) atomicMax(&sm.largest[lane][part * TN + i], lane == 0 ? lq : lane == 1 ? lk : lo);
         }
         if (bad) sm.bad = 1;
         __syncthreads();
-        const Scale sq = scale_of(sm.largest[0]), sk = scale_of(sm.largest[1]), so = scale_of(sm.largest[part < PARTS / 2 ? 2 : 3]);
 #pragma unroll
         for (int i = 0; i < TN; ++i) {
-            const int at = tile_at<DP>(part * TN + i, ch);
-            split1(qs[i] * sq.up, sm.tiles[at], sm.tiles[CT * DP + at]);
-            split1(ks[i] * sk.up, sm.tiles[2 * CT * DP + at], sm.tiles[3 * CT * DP + at]);
-            split1(os[i] * so.up, sm.off[at], sm.off[CT * DP + at]);
+            const int t = part * TN + i, at = tile_at<DP>(t, ch);
+            split1(qs[i] * scale_of(sm.largest[0][t]).up, sm.tiles[at], sm.tiles[CT * DP + at]);
+            split1(ks[i] * scale_of(sm.largest[1][t]).up, sm.tiles[2 * CT * DP + at], sm.tiles[3 * CT * DP + at]);
+            split1(os[i] * scale_of(sm.largest[2][t]).up, sm.off[at], sm.off[CT * DP + at]);
         }
         float* rec = out.records + at_head * Rec::FLOATS;
         if (part == 0) rec[Rec::KEYS + ch] = ch < dim ? expf(last) : 0.f;
-        if (tid < CT) { rec[Rec::G + tid] = 1.f; rec[Rec::W + tid] = 1.f; }
+        if (tid < CT) { rec[Rec::Q_SIZE + tid] = scale_of(sm.largest[0][tid]).size; rec[Rec::W + tid] = scale_of(sm.largest[1][tid]).size; }
     }
     // ---- scores within a half of the chunk: a warp has four tokens s, its lanes the channels (four tokens in a row, with what
     // a token t brings read once: 58 against 48 us for 2,048 tokens of 32 heads of 64, for its 64 sums a lane)
@@ -756,7 +746,8 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
     __syncthreads();
     // ---- scores of the second half with the first: two warps, eight tokens s each
     if (warp < 2) {
-        const Scale s0 = scale_of(sm.largest[2]), s1 = scale_of(sm.largest[3]);
+        const int s = 8 * warp + 2 * (lane & 3);
+        const float s0 = scale_of(sm.largest[2][s]).size, s1 = scale_of(sm.largest[2][s + 1]).size;
         float main[4] = {}, cross[4] = {};
 #pragma unroll
         for (int k = 0; k < DP / 16; k += 2) {
@@ -771,28 +762,29 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
             mma3(main, cross, ah, al, bh[2], bh[3], bl[2], bl[3]);
         }
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
-            *(float2*)&sm.P[16 + (lane >> 2) + 8 * r][8 * warp + 2 * (lane & 3)] =
-                make_float2((main[2 * r] + cross[2 * r]) * s0.down * s1.down, (main[2 * r + 1] + cross[2 * r + 1]) * s0.down * s1.down);
+        for (int r = 0; r < 2; ++r) {
+            const int t = 16 + (lane >> 2) + 8 * r;
+            const float st = scale_of(sm.largest[2][t]).size;
+            *(float2*)&sm.P[t][s] = make_float2(sum2(main[2 * r], cross[2 * r]) * st * s0, sum2(main[2 * r + 1], cross[2 * r + 1]) * st * s1);
+        }
     }
     store_tiles<DP>(out.qk + at_head * (4 * CT * DP), sm.tiles);
     __syncthreads();
     const int t = tid >> 3, s = 4 * (tid & 7);
     const float4 x = *(const float4*)&sm.P[t][s];
-    const unsigned largest = __reduce_max_sync(0xffffffffu, max(max(abs_bits(x.x), abs_bits(x.y)), max(abs_bits(x.z), abs_bits(x.w))));
-    if (lane == 0) atomicMax(&sm.largest[4], largest);
-    __syncthreads();
-    const Scale sp = scale_of(sm.largest[4]);
+    unsigned largest = quad_max(max(max(abs_bits(x.x), abs_bits(x.y)), max(abs_bits(x.z), abs_bits(x.w))));
+    largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 4));
+    const Scale sp = scale_of(largest);
     uint2 h, l;
     split2(x.x * sp.up, x.y * sp.up, h.x, l.x);
     split2(x.z * sp.up, x.w * sp.up, h.y, l.y);
     __half* scores = out.scores + at_head * (2 * CT * CT) + score_at(t, s);
     *(uint2*)scores = h;
     *(uint2*)(scores + CT * CT) = l;
-    if (tid < 8)
-        out.records[at_head * Rec::FLOATS + Rec::SCALARS + tid] =
-            tid == Q_DOWN ? scale_of(sm.largest[0]).down : tid == K_DOWN ? scale_of(sm.largest[1]).down : tid == P_DOWN ? sp.down
-          : tid == BAD ? (sm.bad || sm.largest[4] >= 0x7f800000u ? 1.f : 0.f) : 0.f;
+    float* rec = out.records + at_head * Rec::FLOATS;
+    if ((tid & 7) == 0) rec[Rec::P_SIZE + t] = sp.size;
+    const bool lost = __syncthreads_or(largest >= 0x7f800000u);
+    if (tid < 8) rec[Rec::SCALARS + tid] = tid == BAD && (sm.bad || lost) ? 1.f : 0.f;
 }
 
 inline Layout scan_layout(bool per_channel, int dim, int vdim, int heads, int kv_heads, int n_chunks, int n_segments) {

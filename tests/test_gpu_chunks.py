@@ -3,7 +3,8 @@ segments short enough for the walk token by token beside long ones, sizes that f
 that erase everything, numbers that are not finite.
 
 The tolerance: float32 walked token by token is within 2e-5 of float64 in these cases (the other recurrence tests), and a split
-operand holds 2^-23 of a number, so the chunks get the same."""
+operand holds 2^-23 of a number down to 2^-28 of the largest in its sum, so the chunks get the same.  Numbers of very different size
+have a test of their own, with errors relative to each column, token and key."""
 import ctypes as C
 
 import pytest
@@ -424,7 +425,58 @@ def walks(kind, ks, g, counts, heads, dim, vdim, scale=lambda name, t: t):
             ks.gated_linear_scan((q, 0), (k, 0), (v, 0), (wide, 0), torch.empty((M, n), device=DEV), out, batch, state, a2=a2, a2_bias=chan + 2.0,
                                  tau=8.0, q_scale=0.2, **more)
         return out, state
+
+    def reference():
+        """The same in float64, token by token: outputs [M, heads, vdim] and, per segment, the matrices [heads, vdim, dim]."""
+        f = lambda t: t.double().view(M, heads, -1)
+        qd, kd, vd, ad, bd, pd = f(q), f(k), f(v), a.double(), b.double(), par.double()
+        outs, states, off = [], [], 0
+        for n_tokens in counts:
+            part = slice(off, off + n_tokens)
+            off += n_tokens
+            if kind == "delta":
+                out, S = delta_reference(wide[part], cols, heads, heads, dim, vdim, par, par, dim ** -0.5,
+                                         torch.zeros((heads, dim, vdim), dtype=torch.float64, device=DEV))
+                S = S.transpose(1, 2)
+            elif kind == "matrix_memory":
+                out, S = memory_reference(qd[part] * dim ** -0.5, kd[part], vd[part], 8.0 * torch.tanh((ad[part] + pd) / 8.0),
+                                          torch.nn.functional.logsigmoid(8.0 * torch.tanh((bd[part] + pd + 3.0) / 8.0)))
+            else:
+                S, qs, ks_, extra = torch.zeros((heads, vdim, dim), dtype=torch.float64, device=DEV), qd[part], kd[part], None
+                if kind == "state_space":
+                    step = torch.nn.functional.softplus(ad[part] + pd - 3.0)
+                    w, ks_ = torch.exp(-torch.exp(pd) * step)[:, :, None, None], ks_ * step[:, :, None]
+                elif kind == "decaying_memory":
+                    w, extra = torch.exp(-torch.exp(z[part].double() + chan.double())).view(-1, heads, 1, dim), chan.double().view(heads, dim)
+                else:
+                    w = torch.sigmoid(wide[part, :6].double() @ a2.double() + chan.double() + 2.0).pow(0.125).view(-1, heads, 1, dim)
+                    qs = qs * 0.2
+                out, S = scan_reference("memory" if kind == "decaying_memory" else kind, qs, ks_, vd[part], w, extra, S)
+                if kind == "state_space":
+                    out = out + pd[:, None] * vd[part]
+            outs.append(out)
+            states.append(S)
+        return torch.cat(outs), torch.stack(states)
+
+    def matrices(state):
+        """The matrices [segments, heads, vdim, dim] of the states."""
+        if kind in ("matrix_memory", "delta"):
+            return state.view(len(counts), heads, -1)[:, :, :dim * vdim].view(len(counts), heads, dim, vdim).transpose(2, 3)
+        return state.view(len(counts), heads, vdim, dim)
+    run.reference, run.matrices = reference, matrices
     return run
+
+
+def memory_reference(q, k, v, gi, gf):
+    T, H, _ = q.shape
+    S, n, m, out = (torch.zeros(s, dtype=torch.float64, device=q.device) for s in ((H, v.shape[2], q.shape[2]), (H, q.shape[2]), (H,), v.shape))
+    for t in range(T):
+        new = torch.maximum(gf[t] + m, gi[t])
+        keep, take = torch.exp(gf[t] + m - new)[:, None], torch.exp(gi[t] - new)[:, None] * k[t]
+        m = new
+        S, n = keep[:, :, None] * S + v[t][:, :, None] * take[:, None, :], keep * n + take
+        out[t] = torch.einsum("hvk,hk->hv", S, q[t]) / (torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+    return out, S
 
 
 KINDS = ["matrix_memory", "delta", "state_space", "decaying_memory", "linear_attention"]
@@ -479,3 +531,40 @@ def test_a_block_that_gives_up_waits_for_its_first_chunk_before_it_leaves(kind):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     near(run()[0], want[0].double(), "with the default waits", 1e-4)
     assert ks.errors() == {}
+
+
+# ---------------------------------------------------------------------------- numbers of very different size
+@pytest.mark.parametrize("uneven", ["even", "columns", "tokens", "keys"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_columns_tokens_and_keys_of_different_size_keep_their_bits(kind, uneven):
+    """Value columns that differ by 10^12, tokens and keys by 10^6: every column, token and key is held as the walk token by token holds
+    it.  The error against float64, relative to the largest element of the column, the token or the key's row of the state, is at most
+    three times that walk's, plus 40 units of 2^-23 for the sums' other order (128 terms a product, a few products)."""
+    heads, dim, vdim, counts = 2, 128, 64, [100, 300]
+    ks = kernels(torch.bfloat16)
+    g = torch.Generator().manual_seed(21)
+    r = lambda n, span: 10.0 ** ((torch.rand(n, generator=g) * 2.0 - 1.0) * span).to(DEV)
+    by_column, by_key, M = r(vdim, 6.0), r(dim, 3.0), sum(counts)
+    by_token = {n: r(M, 3.0)[:, None, None] for n in "qkv"}
+
+    def scale(name, t):
+        if uneven == "tokens":
+            return t * by_token[name]
+        if uneven == "columns" and name == "v":
+            return t * by_column
+        # (a key's part of every q . k stays what it was, while q, k and the state differ from key to key)
+        return t * by_key if uneven == "keys" and name == "q" else t / by_key if uneven == "keys" and name == "k" else t
+    run = walks(kind, ks, g, counts, heads, dim, vdim, scale)
+    want, want_state = run.reference()
+
+    def errors(chunked):
+        out, state = run(chunked)
+        e, es = (out.double().view_as(want) - want).abs(), (run.matrices(state).double() - want_state).abs()
+        out_axes = {"tokens": 2}.get(uneven, 0)                          # the axis over which the largest element is looked for
+        state_axes = {"keys": 2}.get(uneven, 3)
+        rel = lambda e, w, axis: float((e.amax(axis) / w.abs().amax(axis)).max())
+        return rel(e, want, out_axes), rel(es, want_state, state_axes)
+    chunks, tokens = errors(True), errors(False)
+    print(f"{kind} {uneven}: output {chunks[0]:.2e} ({tokens[0]:.2e} token by token), state {chunks[1]:.2e} ({tokens[1]:.2e})")
+    for c, t in zip(chunks, tokens):
+        assert c <= 3.0 * t + 40 * 2.0**-23
