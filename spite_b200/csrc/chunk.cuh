@@ -176,17 +176,43 @@ __device__ __forceinline__ double prefix_max(double v, int lane) {
 __device__ __forceinline__ float bounded_log(float x) { return fmaxf(x, -1000.f); }
 
 // ---- chunks are numbered segment by segment
-__device__ __forceinline__ int chunks_before(const int* cu_seqlens, int seg) {
+__device__ __forceinline__ int chunks_of(int tokens) { return (tokens + CT - 1) / CT; }
+// Which segments go in chunks: those of at least `min_tokens` tokens whose chunks have their places in working memory, which has `chunks`.
+struct Numbering { int min_tokens, chunks; };
+// The number of a segment's first chunk, or -1: it goes token by token.  All lanes of a warp ask together.
+__device__ __forceinline__ int first_chunk(const Numbering& nb, const int* cu_seqlens, int seg) {
+    const int lane = threadIdx.x & 31, tokens = cu_seqlens[seg + 1] - cu_seqlens[seg];
+    if (tokens < nb.min_tokens) return -1;
     int n = 0;
-    for (int s = 0; s < seg; ++s) n += (cu_seqlens[s + 1] - cu_seqlens[s] + CT - 1) / CT;
-    return n;
+    for (int s = lane; s < seg; s += 32) n += chunks_of(cu_seqlens[s + 1] - cu_seqlens[s]);
+    n = __reduce_add_sync(0xffffffffu, n);
+    return n + chunks_of(tokens) <= nb.chunks ? n : -1;
 }
-// the segment of a chunk and the chunk's first token; false: the step has no such chunk
-__device__ __forceinline__ bool find_chunk(const int* cu_seqlens, int n_segments, int id, int& seg, int& first) {
-    for (seg = 0; seg < n_segments; ++seg) {
-        const int n = (cu_seqlens[seg + 1] - cu_seqlens[seg] + CT - 1) / CT;
-        if (id < n) { first = cu_seqlens[seg] + id * CT; return true; }
-        id -= n;
+// A chunk of the step: its segment, the segment's bounds, the chunk's first token and its place, or -1: its tokens are walked one by one.
+struct Place { int seg, begin, end, first, at; };
+// The id-th chunk of the step; false: it has no such chunk.  All lanes of a warp ask together.
+__device__ __forceinline__ bool find_chunk(const Numbering& nb, const int* cu_seqlens, int n_segments, int id, Place& p) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;                                       // chunks of the segments before s0
+    for (int s0 = 0; s0 < n_segments; s0 += 32) {
+        const int s = s0 + lane, a = cu_seqlens[min(s, n_segments)], b = cu_seqlens[min(s + 1, n_segments)], n = chunks_of(b - a);
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        const unsigned beyond = __ballot_sync(0xffffffffu, before + upto > id);
+        if (beyond) {
+            const int src = __ffs(beyond) - 1, base = before + __shfl_sync(0xffffffffu, upto - n, src);
+            p.seg = s0 + src;
+            p.begin = __shfl_sync(0xffffffffu, a, src);
+            p.end = __shfl_sync(0xffffffffu, b, src);
+            p.first = p.begin + (id - base) * CT;
+            p.at = p.end - p.begin >= nb.min_tokens && base + chunks_of(p.end - p.begin) <= nb.chunks ? id : -1;
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
     }
     return false;
 }
@@ -216,17 +242,19 @@ template <int MODE, int DP> struct Record {
 struct Leftovers {
     const float* bad;                                     // null: everything is the kernel's own
     long long chunk_stride;                               // floats between two chunks' marks
-    int head_stride, min_tokens;
+    int head_stride;
+    Numbering numbering;
     const int* columns; int column_groups;
 };
 enum Left { NOTHING = 0, MARKED_COLUMNS = 1, WHOLE = 2 };
 // All threads of the block ask together, for the columns col0 .. col0 + n - 1.
 __device__ __forceinline__ int left_over(const Leftovers& l, const int* cu_seqlens, int seg, int head, int heads, int col0, int n) {
     const int tokens = cu_seqlens[seg + 1] - cu_seqlens[seg];
-    if (l.bad == nullptr || tokens < l.min_tokens) return WHOLE;
-    const int first = chunks_before(cu_seqlens, seg);
+    if (l.bad == nullptr) return WHOLE;
+    const int first = first_chunk(l.numbering, cu_seqlens, seg);
+    if (first < 0) return WHOLE;
     bool bad = false, marked = false;
-    for (int c = threadIdx.x; c < (tokens + CT - 1) / CT; c += blockDim.x)
+    for (int c = threadIdx.x; c < chunks_of(tokens); c += blockDim.x)
         bad |= l.bad[(first + c) * l.chunk_stride + (long long)head * l.head_stride] != 0.f;
     const int* columns = l.columns + ((size_t)seg * heads + head) * l.column_groups;
     for (int c = col0 / 16 + threadIdx.x; c < l.column_groups && 16 * c < col0 + n; c += blockDim.x) marked |= columns[c] != 0;
@@ -256,7 +284,7 @@ struct Walk {
     const int* cu_seqlens; const int* slots;
     int n_segments, heads, qk_heads, dim, vdim;
     float out_scale;                                      // on the read-out
-    int min_tokens;                                       // shorter segments are another kernel's
+    Numbering numbering;                                  // the other segments are another kernel's
     int* columns; int column_groups;                      // see Leftovers
     int stages;                                           // of the ring of chunks (2 or 3)
 };
@@ -280,21 +308,21 @@ inline Layout layout_of(int dp, int record, int heads, int qk_heads, int vdim, i
     return l;
 }
 // where the kernel before the walk leaves its results
-struct Made { __half* qk; __half* w; __half* scores; float* records; float* u0; int* columns; int column_groups, min_tokens; };
-inline Made made_at(void* scratch, const Layout& l, int min_tokens) {
+struct Made { __half* qk; __half* w; __half* scores; float* records; float* u0; int* columns; int column_groups; Numbering numbering; };
+inline Made made_at(void* scratch, const Layout& l, int min_tokens, int n_chunks) {
     unsigned char* b = (unsigned char*)scratch;
     return {(__half*)(b + l.qk), (__half*)(b + l.w), (__half*)(b + l.scores), (float*)(b + l.records), (float*)(b + l.u0),
-            (int*)(b + l.columns), l.column_groups, min_tokens};
+            (int*)(b + l.columns), l.column_groups, {min_tokens, n_chunks}};
 }
 inline Walk walk_of(const Made& m) {
     Walk w = {};
     w.qk = m.qk; w.w = m.w; w.scores = m.scores; w.records = m.records;
-    w.columns = m.columns; w.column_groups = m.column_groups; w.min_tokens = m.min_tokens;
+    w.columns = m.columns; w.column_groups = m.column_groups; w.numbering = m.numbering;
     w.out_scale = 1.f;
     return w;
 }
 inline Leftovers leftovers_of(const Made& m, const Layout& l, int heads, int scalars) {
-    return {m.records + scalars + BAD, (long long)heads * l.record, l.record, m.min_tokens, m.columns, l.column_groups};
+    return {m.records + scalars + BAD, (long long)heads * l.record, l.record, m.numbering, m.columns, l.column_groups};
 }
 
 template <int KPW, int KW, int CW, int MODE> struct Shape {
@@ -334,14 +362,15 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
     int* const error_word = waits.error_word ? waits.error_word : &walk_error;
     pdl_wait();
     const int t0 = p.cu_seqlens[seg], t1 = p.cu_seqlens[seg + 1];
-    if (t1 - t0 < p.min_tokens) return;
+    const int chunk0 = first_chunk(p.numbering, p.cu_seqlens, seg);
+    if (chunk0 < 0) return;
     const int slot = p.slots[seg];
     if (seg > 0 && slot == p.slots[0]) {                  // a padding row of a captured step: its results are never read
         for (int e = tid; e < (t1 - t0) * COLS; e += THREADS)
             if (col0 + e % COLS < p.vdim) p.out[(size_t)(t0 + e / COLS) * p.out_stride + (size_t)head * p.vdim + col0 + e % COLS] = 0.f;
         return;
     }
-    const int n_cols = min(COLS, p.vdim - col0), n_chunks = (t1 - t0 + CT - 1) / CT, chunk0 = chunks_before(p.cu_seqlens, seg);
+    const int n_cols = min(COLS, p.vdim - col0), n_chunks = chunks_of(t1 - t0);
     if (tid == 0) {
         for (int i = 0; i < 3; ++i) tc::mbar_init(tc::smem_u32(&full[i]), 1);
         abort_flag = 0;

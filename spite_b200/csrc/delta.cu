@@ -236,13 +236,13 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
     typename SM::Head& hd = sm.head[team];
     pdl_wait();
     pdl_launch_dependents();
-    int seg, first;
-    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
-    const int len = min(CT, p.cu_seqlens[seg + 1] - first), dim = p.dim, vdim = p.vdim;
-    const bool brief = p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens;     // walked token by token: the tokens' scalars alone
+    Place pl;
+    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl)) return;
+    const int first = pl.first, len = min(CT, pl.end - first), dim = p.dim, vdim = p.vdim;
+    const bool brief = pl.at < 0;                         // walked token by token: the tokens' scalars alone
     const float* rows = p.x + (size_t)first * p.stride;
     const int n_gates = 2 * p.kv_heads + 2 * p.heads;
-    if (first == p.cu_seqlens[seg]) clear_marks(out.columns, out.column_groups, seg, head, p.heads, tt, 128);
+    if (!brief && first == pl.begin) clear_marks(out.columns, out.column_groups, pl.seg, head, p.heads, tt, 128);
     if (tid < HB) sm.bad[tid] = 0;
 
     // ---- unit vectors: a warp has the tokens warp, warp + WARPS, ..., a lane the elements lane, lane + 32, ...
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
     float va[2][2][4][2];
     load_values(tw, va[0]);
     load_values(tw + 4, va[1]);
-    const size_t at_head = (size_t)blockIdx.x * p.heads + head;
+    const size_t at_head = (size_t)pl.at * p.heads + head;
     float* rec = out.records + at_head * Rec::FLOATS;
     __syncthreads();
 
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
                     make_float2(sum2(main[n][2 * r], cross[n][2 * r]), sum2(main[n][2 * r + 1], cross[n][2 * r + 1]));
     }
     if (head0 % group == 0) {                             // q and k of the group's heads are the same
-        uint4* dst = reinterpret_cast<uint4*>(out.qk + ((size_t)blockIdx.x * p.kv_heads + kvh) * (4 * CT * DP));
+        uint4* dst = reinterpret_cast<uint4*>(out.qk + ((size_t)pl.at * p.kv_heads + kvh) * (4 * CT * DP));
         const uint4* src = reinterpret_cast<const uint4*>(sm.qk[0]);
 #pragma unroll 4
         for (int e = tid; e < 4 * CT * DP / 8; e += THREADS) dst[e] = src[e];
@@ -516,17 +516,18 @@ inline Layout delta_layout(int dim, int vdim, int heads, int kv_heads, int n_tok
 }
 
 template <int DP, int HB>
-int launch_delta_prepare(const DeltaParams& p, const Made& out, int n_chunks, cudaStream_t st) {
+int launch_delta_prepare(const DeltaParams& p, const Made& out, cudaStream_t st) {
     auto kernel = delta_chunk_kernel<DP, HB>;
     constexpr int bytes = (int)sizeof(DeltaChunkSmem<DP, HB>);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return SPITE_LAUNCH_FAILED;
-    SPITE_LAUNCH(kernel, dim3(n_chunks, p.heads / HB), 128 * HB, bytes, st, p, out);
+    // (every chunk of the step, also of segments that go token by token: their tokens' scalars come from here)
+    SPITE_LAUNCH(kernel, dim3(p.n_tokens / CT + p.n_segments, p.heads / HB), 128 * HB, bytes, st, p, out);
     return spite_launch_status();
 }
 
 template <int DP>
-int launch_delta_chunks(const DeltaParams& p, const Made& out, int n_chunks, cudaStream_t st) {
-    const int rc = p.heads / p.kv_heads % 2 == 0 ? launch_delta_prepare<DP, 2>(p, out, n_chunks, st) : launch_delta_prepare<DP, 1>(p, out, n_chunks, st);
+int launch_delta_chunks(const DeltaParams& p, const Made& out, cudaStream_t st) {
+    const int rc = p.heads / p.kv_heads % 2 == 0 ? launch_delta_prepare<DP, 2>(p, out, st) : launch_delta_prepare<DP, 1>(p, out, st);
     if (rc != SPITE_OK) return rc;
     Walk w = walk_of(out);
     w.v = out.u0; w.v_stride = (long long)p.heads * p.vdim;
@@ -594,7 +595,8 @@ SPITE_API long long spite_delta_chunk_bytes(int dim, int vdim, int heads, int kv
     return delta_layout(dim, vdim, heads, kv_heads, n_tokens, n_chunks, n_segments).bytes;
 }
 
-// Segments of at least `min_tokens` tokens in chunks of 32, the others token by token.
+// Segments of at least `min_tokens` tokens in chunks of 32, the others token by token, and those that the working memory, made for
+// `n_chunks` chunks, has no place for.
 SPITE_API int spite_delta_scan_chunked(const DeltaParams* p, void* scratch, int n_chunks, int min_tokens, void* stream) {
     const int chk = check_delta(p);
     if (chk != SPITE_OK) return chk;
@@ -603,8 +605,8 @@ SPITE_API int spite_delta_scan_chunked(const DeltaParams* p, void* scratch, int 
     if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const Layout l = delta_layout(p->dim, p->vdim, p->heads, p->kv_heads, p->n_tokens, n_chunks, p->n_segments);
-    const Made out = made_at(scratch, l, min_tokens);
-    const int rc = p->dim <= 64 ? launch_delta_chunks<64>(*p, out, n_chunks, st) : launch_delta_chunks<128>(*p, out, n_chunks, st);
+    const Made out = made_at(scratch, l, min_tokens, n_chunks);
+    const int rc = p->dim <= 64 ? launch_delta_chunks<64>(*p, out, st) : launch_delta_chunks<128>(*p, out, st);
     if (rc != SPITE_OK) return rc;
     return launch_token_walk(p, leftovers_of(out, l, p->heads, Record<DELTA, 64>::SCALARS), 0, st);
 }

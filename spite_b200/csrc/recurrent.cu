@@ -603,13 +603,12 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, head = blockIdx.y;
     pdl_wait();
     pdl_launch_dependents();
-    int seg, first;
-    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
-    if (first == p.cu_seqlens[seg]) clear_marks(out.columns, out.column_groups, seg, head, p.heads, tid, 256);
-    if (p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens) return;
-    const int len = min(CL, p.cu_seqlens[seg + 1] - first), dim = p.dim;
+    Place pl;
+    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl) || pl.at < 0) return;
+    const int first = pl.first, len = min(CL, pl.end - first), dim = p.dim;
+    if (first == pl.begin) clear_marks(out.columns, out.column_groups, pl.seg, head, p.heads, tid, 256);
     const float* rows = p.proj + (size_t)first * p.stride;
-    const size_t at_head = (size_t)blockIdx.x * p.heads + head;
+    const size_t at_head = (size_t)pl.at * p.heads + head;
     float* rec = out.records + at_head * Rec::FLOATS;
     if (tid == 0) sm.bad = 0;
 
@@ -817,7 +816,8 @@ SPITE_API long long spite_mlstm_tiles_bytes(int dim, int vdim, int heads, int n_
     return memory_layout(dim, vdim, heads, n_chunks, n_segments).bytes;
 }
 
-// Segments of at least `min_tokens` tokens in chunks of 32 on the tensor cores, the others token by token.
+// Segments of at least `min_tokens` tokens in chunks of 32 on the tensor cores, the others token by token, and those that the working
+// memory, made for `n_chunks` chunks, has no place for.
 SPITE_API int spite_mlstm_scan_tiles(const MlstmParams* p, void* scratch, int n_chunks, int min_tokens, void* stream) {
     const int chk = check_mlstm(p);
     if (chk != SPITE_OK) return chk;
@@ -827,7 +827,7 @@ SPITE_API int spite_mlstm_scan_tiles(const MlstmParams* p, void* scratch, int n_
     cudaStream_t st = (cudaStream_t)stream;
     const int dp = memory_dp(p->dim);
     const chunk::Layout l = memory_layout(p->dim, p->vdim, p->heads, n_chunks, p->n_segments);
-    const chunk::Made out = chunk::made_at(scratch, l, min_tokens);
+    const chunk::Made out = chunk::made_at(scratch, l, min_tokens, n_chunks);
     const int rc = dp == 64 ? launch_memory_chunks<64, 32>(*p, out, n_chunks, st) : dp == 128 ? launch_memory_chunks<128, 32>(*p, out, n_chunks, st)
                                                                                             : launch_memory_chunks<256, 64>(*p, out, n_chunks, st);
     if (rc != SPITE_OK) return rc;

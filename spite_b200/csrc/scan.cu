@@ -535,17 +535,17 @@ __global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams
     const int h0 = kvh * group + slice * SSM_HEADS, h1 = min(h0 + SSM_HEADS, (kvh + 1) * group);
     pdl_wait();
     pdl_launch_dependents();
-    int seg, first;
-    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
-    const int len = min(CT, p.cu_seqlens[seg + 1] - first);
-    const bool brief = p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens;     // walked token by token: the tokens' scalars alone
-    if (first == p.cu_seqlens[seg])
-        for (int h = h0 + warp; h < h1; h += 8) clear_marks(out.columns, out.column_groups, seg, h, p.heads, lane, 32);
+    Place pl;
+    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl)) return;
+    const int first = pl.first, len = min(CT, pl.end - first);
+    const bool brief = pl.at < 0;                         // walked token by token: the tokens' scalars alone
+    if (!brief && first == pl.begin)
+        for (int h = h0 + warp; h < h1; h += 8) clear_marks(out.columns, out.column_groups, pl.seg, h, p.heads, lane, 32);
     bool bad = false;
     if (!brief) {
         bad = split_tiles<DP>(p.q + (size_t)first * p.q_stride + (size_t)kvh * p.dim, p.q_stride, p.k + (size_t)first * p.k_stride + (size_t)kvh * p.dim,
                               p.k_stride, len, p.dim, sm.tiles, sm.scores, sm.q_size, sm.k_size);
-        if (slice == 0) store_tiles<DP>(out.qk + ((size_t)blockIdx.x * p.kv_heads + kvh) * (4 * CT * DP), sm.tiles);
+        if (slice == 0) store_tiles<DP>(out.qk + ((size_t)pl.at * p.kv_heads + kvh) * (4 * CT * DP), sm.tiles);
         bad = __syncthreads_or(bad);
     }
     for (int h = h0 + warp; h < h1; h += 8) {             // a lane a token
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams
             }
         }
         const Scale sp = scale_of(largest);
-        const size_t at_head = (size_t)blockIdx.x * p.heads + h;
+        const size_t at_head = (size_t)pl.at * p.heads + h;
         __half* scores = out.scores + at_head * (2 * CT * CT);
 #pragma unroll
         for (int s = 0; s < CT; s += 8) {
@@ -619,14 +619,13 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, dim = p.dim;
     pdl_wait();
     pdl_launch_dependents();
-    int seg, first;
-    if (!find_chunk(p.cu_seqlens, p.n_segments, blockIdx.x, seg, first)) return;
-    if (first == p.cu_seqlens[seg]) clear_marks(out.columns, out.column_groups, seg, head, p.heads, tid, 256);
-    if (p.cu_seqlens[seg + 1] - p.cu_seqlens[seg] < out.min_tokens) return;
-    const int len = min(CT, p.cu_seqlens[seg + 1] - first);
+    Place pl;
+    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl) || pl.at < 0) return;
+    const int first = pl.first, len = min(CT, pl.end - first);
+    if (first == pl.begin) clear_marks(out.columns, out.column_groups, pl.seg, head, p.heads, tid, 256);
     if (tid < 3 * CT) sm.largest[tid / CT][tid % CT] = 0;
     if (tid == 0) sm.bad = 0;
-    const size_t at_head = (size_t)blockIdx.x * p.heads + head;
+    const size_t at_head = (size_t)pl.at * p.heads + head;
     const int ch = tid % DP, part = tid / DP;
     float qv[TN], kv[TN], lw[TN];                         // q, k and the log decays
     bool bad = false;
@@ -807,12 +806,13 @@ inline bool one_wave(const ScanParams& p, int cols) { return (long long)((p.vdim
 
 template <int DP>
 int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_stride, const float* a_log, const float* dt_bias, const Made& out,
-                              int n_chunks, cudaStream_t st) {
+                              cudaStream_t st) {
     auto prep = state_space_chunk_kernel<DP>;
     constexpr int bytes = (int)sizeof(StateSpaceChunkSmem<DP>);
     if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return SPITE_LAUNCH_FAILED;
     const int slices = (p.heads / p.kv_heads + SSM_HEADS - 1) / SSM_HEADS;
-    SPITE_LAUNCH(prep, dim3(n_chunks, p.kv_heads * slices), 256, bytes, st, p, a, a_stride, a_log, dt_bias, (float*)p.scalars, out, slices);
+    // (every chunk of the step, also of segments that go token by token: their tokens' scalars come from here)
+    SPITE_LAUNCH(prep, dim3(p.n_tokens / CT + p.n_segments, p.kv_heads * slices), 256, bytes, st, p, a, a_stride, a_log, dt_bias, (float*)p.scalars, out, slices);
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
     chunk::Walk w = scan_walk(p, out);
     w.skip = p.skip;
@@ -836,7 +836,7 @@ int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, 
 template <bool BONUS, int WALK>
 int key_decay_in_chunks(const ScanParams& p, void* scratch, int n_chunks, int min_tokens, cudaStream_t st) {
     const Layout l = scan_layout(true, p.dim, p.vdim, p.heads, p.heads, n_chunks, p.n_segments);
-    const Made out = made_at(scratch, l, min_tokens);
+    const Made out = made_at(scratch, l, min_tokens, n_chunks);
     const int rc = p.dim <= 64 ? launch_key_decay_chunks<64, BONUS>(p, out, n_chunks, st) : launch_key_decay_chunks<128, BONUS>(p, out, n_chunks, st);
     if (rc != SPITE_OK) return rc;
     return choose_scan<WALK>(p, st, leftovers_of(out, l, p.heads, Record<KEY_DECAY, 64>::SCALARS));
@@ -875,7 +875,8 @@ static int check_state_space(const ScanParams* p, const float* a, long long a_st
     if (chk != SPITE_OK) return chk;
     return !a || !a_log || !dt_bias || !p->scalars || p->w || a_stride < p->heads ? SPITE_BAD_ARG : SPITE_OK;
 }
-// Segments of at least `min_tokens` tokens in chunks of 32, the others token by token.
+// Segments of at least `min_tokens` tokens in chunks of 32, the others token by token, and those that the working memory, made for
+// `n_chunks` chunks, has no place for (in all three).
 SPITE_API int spite_state_space_scan_chunked(const ScanParams* p, const float* a, long long a_stride, const float* a_log, const float* dt_bias,
                                              void* scratch, int n_chunks, int min_tokens, void* stream) {
     int chk = check_state_space(p, a, a_stride, a_log, dt_bias);
@@ -884,9 +885,9 @@ SPITE_API int spite_state_space_scan_chunked(const ScanParams* p, const float* a
     if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const Layout l = scan_layout(false, p->dim, p->vdim, p->heads, p->kv_heads, n_chunks, p->n_segments);
-    const Made out = made_at(scratch, l, min_tokens);
-    const int rc = p->dim <= 64 ? launch_state_space_chunks<64>(*p, a, a_stride, a_log, dt_bias, out, n_chunks, st)
-                                : launch_state_space_chunks<128>(*p, a, a_stride, a_log, dt_bias, out, n_chunks, st);
+    const Made out = made_at(scratch, l, min_tokens, n_chunks);
+    const int rc = p->dim <= 64 ? launch_state_space_chunks<64>(*p, a, a_stride, a_log, dt_bias, out, st)
+                                : launch_state_space_chunks<128>(*p, a, a_stride, a_log, dt_bias, out, st);
     if (rc != SPITE_OK) return rc;
     return choose_scan<PER_HEAD>(*p, st, leftovers_of(out, l, p->heads, Record<HEAD_DECAY, 64>::SCALARS));
 }

@@ -568,3 +568,47 @@ def test_columns_tokens_and_keys_of_different_size_keep_their_bits(kind, uneven)
     print(f"{kind} {uneven}: output {chunks[0]:.2e} ({tokens[0]:.2e} token by token), state {chunks[1]:.2e} ({tokens[1]:.2e})")
     for c, t in zip(chunks, tokens):
         assert c <= 3.0 * t + 40 * 2.0**-23
+
+
+# ---------------------------------------------------------------------------- working memory
+class _Fewer:
+    """A kernel library whose walks in chunks are told of `n` chunks."""
+
+    def __init__(self, lib, n):
+        self.lib, self.n = lib, n
+
+    def __getattr__(self, name):
+        f = getattr(self.lib, name)
+        return (lambda *a: f(*a[:-3], self.n, *a[-2:])) if name.endswith(("_chunked", "_tiles")) else f
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 6, 7])
+@pytest.mark.parametrize("kind", KINDS)
+def test_working_memory_for_fewer_chunks_than_the_step_has(kind, n):
+    """Segments that a caller's working memory has no place for go token by token, and nothing is written behind it."""
+    counts, heads, dim, vdim = [40, 70, 3, 64], 2, 64, 32
+    library = {"matrix_memory": "recurrent", "delta": "delta"}.get(kind, "scan")
+    ks = kernels(torch.bfloat16)
+    run = walks(kind, ks, torch.Generator().manual_seed(14), counts, heads, dim, vdim)
+    want, whole = run(False), run()
+    buffers = []
+
+    def scratch(library, query, *sizes):
+        f = getattr(ks._lib(library).lib, query)
+        f.restype = C.c_longlong
+        need = f(*(int(x) for x in sizes[:-2]), n, int(sizes[-1]))
+        buffers.append((torch.full((need + (1 << 16),), 0x5a, dtype=torch.uint8, device=DEV), need))
+        return buffers[-1][0]
+    ks._chunk_scratch = scratch
+    ks._libs[library] = _Fewer(ks._lib(library), n)
+    out, state = run()
+    # (segments of fewer than 32 tokens, 8 in the matrix memory, have no chunks)
+    at, off = 0, 0
+    for s, tokens in enumerate(counts):
+        chunks = -(-tokens // 32)
+        part = slice(off, off + tokens)
+        off += tokens
+        ref = whole if tokens >= 32 and at + chunks <= n else want
+        assert torch.equal(out[part], ref[0][part]) and torch.equal(state[s], ref[1][s]), f"segment {s}"
+        at += chunks
+    assert buffers and all(bool((b[need:] == 0x5a).all()) for b, need in buffers)
