@@ -175,44 +175,67 @@ __device__ __forceinline__ double prefix_max(double v, int lane) {
 // keeps its other terms.
 __device__ __forceinline__ float bounded_log(float x) { return fmaxf(x, -1000.f); }
 
-// ---- chunks are numbered segment by segment
+// ---- Which segments go in chunks: the first `segments` ones of at least `min_tokens` tokens, as far as their chunks have their places in
+// working memory, which has `chunks`.  Only these segments' chunks are numbered, segment by segment: a decoded token beside a prompt's
+// portion takes no memory, no block of the walk and no turn of a search.
+struct Numbering { int min_tokens, chunks, segments; };
 __device__ __forceinline__ int chunks_of(int tokens) { return (tokens + CT - 1) / CT; }
-// Which segments go in chunks: those of at least `min_tokens` tokens whose chunks have their places in working memory, which has `chunks`.
-struct Numbering { int min_tokens, chunks; };
-// The number of a segment's first chunk, or -1: it goes token by token.  All lanes of a warp ask together.
-__device__ __forceinline__ int first_chunk(const Numbering& nb, const int* cu_seqlens, int seg) {
-    const int lane = threadIdx.x & 31, tokens = cu_seqlens[seg + 1] - cu_seqlens[seg];
-    if (tokens < nb.min_tokens) return -1;
-    int n = 0;
-    for (int s = lane; s < seg; s += 32) n += chunks_of(cu_seqlens[s + 1] - cu_seqlens[s]);
-    n = __reduce_add_sync(0xffffffffu, n);
-    return n + chunks_of(tokens) <= nb.chunks ? n : -1;
+__device__ __forceinline__ int upto_lane(int x) {         // the sum over the lanes up to this one
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += u;
+    }
+    return x;
 }
-// A chunk of the step: its segment, the segment's bounds, the chunk's first token and its place, or -1: its tokens are walked one by one.
+// The number of a segment's first chunk, or -1: it goes token by token.  All lanes of a warp ask together (in all three).
+__device__ __forceinline__ int first_chunk(const Numbering& nb, const int* cu_seqlens, int seg) {
+    const int tokens = cu_seqlens[seg + 1] - cu_seqlens[seg];
+    if (tokens < nb.min_tokens) return -1;
+    int chunks = 0, segments = 0;
+    for (int s = threadIdx.x & 31; s < seg; s += 32) {
+        const int n = cu_seqlens[s + 1] - cu_seqlens[s];
+        if (n >= nb.min_tokens) { chunks += chunks_of(n); ++segments; }
+    }
+    chunks = __reduce_add_sync(0xffffffffu, chunks);
+    segments = __reduce_add_sync(0xffffffffu, segments);
+    return segments < nb.segments && chunks + chunks_of(tokens) <= nb.chunks ? chunks : -1;
+}
+// A chunk of the step: its segment, the segment's bounds, the chunk's first token and its number, or -1: its tokens are walked one by one.
 struct Place { int seg, begin, end, first, at; };
-// The id-th chunk of the step; false: it has no such chunk.  All lanes of a warp ask together.
+// The id-th of all chunks of the step, also of those that have no number (ALL), the id-th numbered one, or the first chunk of the id-th
+// segment whose chunks are (SEGMENTS); false: the step has no such chunk.
+enum Search { ALL, NUMBERED, SEGMENTS };
+template <int WHAT>
 __device__ __forceinline__ bool find_chunk(const Numbering& nb, const int* cu_seqlens, int n_segments, int id, Place& p) {
     const int lane = threadIdx.x & 31;
-    int before = 0;                                       // chunks of the segments before s0
+    int all = 0, chunks = 0, segments = 0;                // of the segments before s0
     for (int s0 = 0; s0 < n_segments; s0 += 32) {
-        const int s = s0 + lane, a = cu_seqlens[min(s, n_segments)], b = cu_seqlens[min(s + 1, n_segments)], n = chunks_of(b - a);
-        int upto = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += u;
-        }
-        const unsigned beyond = __ballot_sync(0xffffffffu, before + upto > id);
+        const int s = s0 + lane, a = cu_seqlens[min(s, n_segments)], b = cu_seqlens[min(s + 1, n_segments)];
+        const bool in = s < n_segments && b - a >= nb.min_tokens;
+        const int n = chunks_of(b - a), upto_chunks = upto_lane(in ? n : 0);
+        const int upto_all = WHAT == ALL ? upto_lane(n) : 0;
+        const unsigned mask = __ballot_sync(0xffffffffu, in);
+        const int upto_segments = __popc(mask & (0xffffffffu >> (31 - lane)));
+        const unsigned beyond = __ballot_sync(0xffffffffu, (WHAT == ALL ? all + upto_all : WHAT == NUMBERED ? chunks + upto_chunks
+                                                                                                             : segments + upto_segments) > id);
         if (beyond) {
-            const int src = __ffs(beyond) - 1, base = before + __shfl_sync(0xffffffffu, upto - n, src);
+            const int src = __ffs(beyond) - 1;
+            const int chunks_before = chunks + __shfl_sync(0xffffffffu, upto_chunks - (in ? n : 0), src);
+            const int segments_before = segments + __shfl_sync(0xffffffffu, upto_segments - (in ? 1 : 0), src);
+            const int before = WHAT == ALL ? all + __shfl_sync(0xffffffffu, upto_all - n, src) : WHAT == NUMBERED ? chunks_before : id;
             p.seg = s0 + src;
             p.begin = __shfl_sync(0xffffffffu, a, src);
             p.end = __shfl_sync(0xffffffffu, b, src);
-            p.first = p.begin + (id - base) * CT;
-            p.at = p.end - p.begin >= nb.min_tokens && base + chunks_of(p.end - p.begin) <= nb.chunks ? id : -1;
+            p.first = p.begin + (id - before) * CT;
+            p.at = (mask >> src & 1) && segments_before < nb.segments && chunks_before + chunks_of(p.end - p.begin) <= nb.chunks
+                       ? chunks_before + id - before : -1;
             return true;
         }
-        before += __shfl_sync(0xffffffffu, upto, 31);
+        if (WHAT == ALL) all += __shfl_sync(0xffffffffu, upto_all, 31);
+        chunks += __shfl_sync(0xffffffffu, upto_chunks, 31);
+        segments += __popc(mask);
     }
     return false;
 }
@@ -309,10 +332,11 @@ inline Layout layout_of(int dp, int record, int heads, int qk_heads, int vdim, i
 }
 // where the kernel before the walk leaves its results
 struct Made { __half* qk; __half* w; __half* scores; float* records; float* u0; int* columns; int column_groups; Numbering numbering; };
-inline Made made_at(void* scratch, const Layout& l, int min_tokens, int n_chunks) {
+// `n_long`: how many segments have at least min_tokens tokens, 0 if the caller does not know (each has a chunk at least)
+inline Made made_at(void* scratch, const Layout& l, int min_tokens, int n_chunks, int n_segments, int n_long) {
     unsigned char* b = (unsigned char*)scratch;
     return {(__half*)(b + l.qk), (__half*)(b + l.w), (__half*)(b + l.scores), (float*)(b + l.records), (float*)(b + l.u0),
-            (int*)(b + l.columns), l.column_groups, {min_tokens, n_chunks}};
+            (int*)(b + l.columns), l.column_groups, {min_tokens, n_chunks, n_long > 0 ? n_long : n_chunks < n_segments ? n_chunks : n_segments}};
 }
 inline Walk walk_of(const Made& m) {
     Walk w = {};
@@ -343,7 +367,7 @@ template <int KPW, int KW, int CW, int MODE> struct Shape {
     static constexpr int bytes(int stages) { return stages * STAGE + SUMS + EXTRA; }
 };
 
-// grid (ceil(vdim / COLS), heads, segments)
+// grid (ceil(vdim / COLS), heads, segments that go in chunks)
 template <int KPW, int KW, int CW, int MODE>
 __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, const tc::WaitControl waits) {
     using SH = Shape<KPW, KW, CW, MODE>;
@@ -355,15 +379,15 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
     __shared__ int abort_flag;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
     const int kw = warp % KW, cw = warp / KW;             // the warp's keys and columns
-    const int seg = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * COLS;
+    const int head = blockIdx.y, col0 = blockIdx.x * COLS;
     float* sums = reinterpret_cast<float*>(smem + (size_t)p.stages * SH::STAGE);
     float* extra = sums + SH::SUMS / 4;
     bool lost = false;                                    // a number that is not finite, or a wait that ran out
     int* const error_word = waits.error_word ? waits.error_word : &walk_error;
     pdl_wait();
-    const int t0 = p.cu_seqlens[seg], t1 = p.cu_seqlens[seg + 1];
-    const int chunk0 = first_chunk(p.numbering, p.cu_seqlens, seg);
-    if (chunk0 < 0) return;
+    Place place;
+    if (!find_chunk<SEGMENTS>(p.numbering, p.cu_seqlens, p.n_segments, blockIdx.z, place) || place.at < 0) return;
+    const int seg = place.seg, t0 = place.begin, t1 = place.end, chunk0 = place.at;
     const int slot = p.slots[seg];
     if (seg > 0 && slot == p.slots[0]) {                  // a padding row of a captured step: its results are never read
         for (int e = tid; e < (t1 - t0) * COLS; e += THREADS)
@@ -821,7 +845,7 @@ __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, 
 template <int KPW, int KW, int CW, int MODE>
 int launch_walk(Walk p, const tc::WaitControl& waits, cudaStream_t st) {
     using SH = Shape<KPW, KW, CW, MODE>;
-    dim3 grid((p.vdim + SH::COLS - 1) / SH::COLS, p.heads, p.n_segments);
+    dim3 grid((p.vdim + SH::COLS - 1) / SH::COLS, p.heads, p.numbering.segments);
     // three stages where a multiprocessor holds one block anyway, two where two blocks then fit
     constexpr bool three = SH::bytes(3) <= 227 * 1024;
     p.stages = three && (long long)grid.x * grid.y * grid.z <= 148 ? 3 : 2;

@@ -42,6 +42,7 @@ struct DeltaParams {
     float* gates;               // scratch [tokens, 2 * kv_heads + 2 * heads]: per q/k head the factors that make k and q unit
                                 // vectors (q's with q_scale), per head beta and the decay; written before the walk
     int n_tokens;
+    int n_long;                 // the walk in chunks: how many segments it takes, if that is known (else 0)
 };
 
 namespace {
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(128 * HB) delta_chunk_kernel(const DeltaParams
     pdl_wait();
     pdl_launch_dependents();
     Place pl;
-    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl)) return;
+    if (!find_chunk<ALL>(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl)) return;
     const int first = pl.first, len = min(CT, pl.end - first), dim = p.dim, vdim = p.vdim;
     const bool brief = pl.at < 0;                         // walked token by token: the tokens' scalars alone
     const float* rows = p.x + (size_t)first * p.stride;
@@ -540,7 +541,7 @@ int launch_delta_chunks(const DeltaParams& p, const Made& out, cudaStream_t st) 
     // 16 columns a block while that leaves every multiprocessor one block at most, else 32.  2,048 tokens, us of the walk alone: 16 heads
     // (128 blocks of 16 columns) 124, with 16 keys a warp and twice the warps 135; 32 heads (128 blocks of 32) 165.  The kernel before it: 39
     // and 70 (a block a head instead of two: 69 and 111).
-    if ((long long)((p.vdim + 15) / 16) * p.heads * p.n_segments <= 148) return launch_walk<32, DP / 32, 1, DELTA>(w, s_waits, st);
+    if ((long long)((p.vdim + 15) / 16) * p.heads * out.numbering.segments <= 148) return launch_walk<32, DP / 32, 1, DELTA>(w, s_waits, st);
     return launch_walk<32, DP / 32, 2, DELTA>(w, s_waits, st);
 }
 
@@ -587,7 +588,7 @@ SPITE_API int spite_delta_scan(const DeltaParams* p, int split_rows, void* strea
     return launch_token_walk(p, Leftovers{}, split_rows, st);
 }
 
-// Bytes of working memory that `spite_delta_scan_chunked` needs for a step of `n_chunks` chunks of 32 tokens (the sum over the segments
+// Bytes of working memory that `spite_delta_scan_chunked` needs for a step of `n_chunks` chunks of 32 tokens (the sum over the long segments
 // of ceil(tokens / 32), or more); -2: sizes that it does not take.
 SPITE_API long long spite_delta_chunk_bytes(int dim, int vdim, int heads, int kv_heads, int n_tokens, int n_chunks, int n_segments) {
     if (dim < 1 || vdim < 1 || heads < 1 || kv_heads < 1 || n_tokens < 0 || n_chunks < 0 || n_segments < 0) return SPITE_BAD_ARG;
@@ -605,7 +606,7 @@ SPITE_API int spite_delta_scan_chunked(const DeltaParams* p, void* scratch, int 
     if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const Layout l = delta_layout(p->dim, p->vdim, p->heads, p->kv_heads, p->n_tokens, n_chunks, p->n_segments);
-    const Made out = made_at(scratch, l, min_tokens, n_chunks);
+    const Made out = made_at(scratch, l, min_tokens, n_chunks, p->n_segments, p->n_long);
     const int rc = p->dim <= 64 ? launch_delta_chunks<64>(*p, out, st) : launch_delta_chunks<128>(*p, out, st);
     if (rc != SPITE_OK) return rc;
     return launch_token_walk(p, leftovers_of(out, l, p->heads, Record<DELTA, 64>::SCALARS), 0, st);

@@ -35,6 +35,7 @@ struct MlstmParams {
     int n_segments, heads, dim, vdim;
     float gate_cap, q_scale;
     int chunked;                // not 0: segments are walked 32 tokens at a time (prompts and their portions)
+    int n_long;                 // the walk in chunks on the tensor cores: how many segments it takes, if that is known (else 0)
 };
 
 namespace {
@@ -604,7 +605,7 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(const MlstmParams p, 
     pdl_wait();
     pdl_launch_dependents();
     Place pl;
-    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl) || pl.at < 0) return;
+    if (!find_chunk<NUMBERED>(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl) || pl.at < 0) return;
     const int first = pl.first, len = min(CL, pl.end - first), dim = p.dim;
     if (first == pl.begin) clear_marks(out.columns, out.column_groups, pl.seg, head, p.heads, tid, 256);
     const float* rows = p.proj + (size_t)first * p.stride;
@@ -827,7 +828,7 @@ SPITE_API int spite_mlstm_scan_tiles(const MlstmParams* p, void* scratch, int n_
     cudaStream_t st = (cudaStream_t)stream;
     const int dp = memory_dp(p->dim);
     const chunk::Layout l = memory_layout(p->dim, p->vdim, p->heads, n_chunks, p->n_segments);
-    const chunk::Made out = chunk::made_at(scratch, l, min_tokens, n_chunks);
+    const chunk::Made out = chunk::made_at(scratch, l, min_tokens, n_chunks, p->n_segments, p->n_long);
     const int rc = dp == 64 ? launch_memory_chunks<64, 32>(*p, out, n_chunks, st) : dp == 128 ? launch_memory_chunks<128, 32>(*p, out, n_chunks, st)
                                                                                             : launch_memory_chunks<256, 64>(*p, out, n_chunks, st);
     if (rc != SPITE_OK) return rc;

@@ -42,6 +42,7 @@ struct ScanParams {
     const int* cu_seqlens; const int* slots;
     int n_segments, n_tokens, heads, kv_heads, dim, vdim;
     float out_scale;                                      // gated linear attention: the factor c on the read-out
+    int n_long;                                           // the walks in chunks: how many segments they take, if that is known
 };
 
 namespace {
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(256) state_space_chunk_kernel(const ScanParams
     pdl_wait();
     pdl_launch_dependents();
     Place pl;
-    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl)) return;
+    if (!find_chunk<ALL>(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl)) return;
     const int first = pl.first, len = min(CT, pl.end - first);
     const bool brief = pl.at < 0;                         // walked token by token: the tokens' scalars alone
     if (!brief && first == pl.begin)
@@ -620,7 +621,7 @@ __global__ void __launch_bounds__(256) key_decay_chunk_kernel(const ScanParams p
     pdl_wait();
     pdl_launch_dependents();
     Place pl;
-    if (!find_chunk(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl) || pl.at < 0) return;
+    if (!find_chunk<NUMBERED>(out.numbering, p.cu_seqlens, p.n_segments, blockIdx.x, pl) || pl.at < 0) return;
     const int first = pl.first, len = min(CT, pl.end - first);
     if (first == pl.begin) clear_marks(out.columns, out.column_groups, pl.seg, head, p.heads, tid, 256);
     if (tid < 3 * CT) sm.largest[tid / CT][tid % CT] = 0;
@@ -802,7 +803,9 @@ inline chunk::Walk scan_walk(const ScanParams& p, const Made& out) {
     w.n_segments = p.n_segments; w.heads = p.heads; w.qk_heads = p.kv_heads; w.dim = p.dim; w.vdim = p.vdim;
     return w;
 }
-inline bool one_wave(const ScanParams& p, int cols) { return (long long)((p.vdim + cols - 1) / cols) * p.heads * p.n_segments <= 148; }
+inline bool one_wave(const ScanParams& p, const Made& out, int cols) {
+    return (long long)((p.vdim + cols - 1) / cols) * p.heads * out.numbering.segments <= 148;
+}
 
 template <int DP>
 int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_stride, const float* a_log, const float* dt_bias, const Made& out,
@@ -817,7 +820,7 @@ int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_s
     chunk::Walk w = scan_walk(p, out);
     w.skip = p.skip;
     // 32 columns a block while that leaves every multiprocessor one block at most, else 64
-    if (one_wave(p, 32)) return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, s_waits, st);
+    if (one_wave(p, out, 32)) return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, s_waits, st);
     return launch_walk<DP / 2, 2, 4, HEAD_DECAY>(w, s_waits, st);
 }
 template <int DP, bool BONUS>
@@ -836,7 +839,7 @@ int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, 
 template <bool BONUS, int WALK>
 int key_decay_in_chunks(const ScanParams& p, void* scratch, int n_chunks, int min_tokens, cudaStream_t st) {
     const Layout l = scan_layout(true, p.dim, p.vdim, p.heads, p.heads, n_chunks, p.n_segments);
-    const Made out = made_at(scratch, l, min_tokens, n_chunks);
+    const Made out = made_at(scratch, l, min_tokens, n_chunks, p.n_segments, p.n_long);
     const int rc = p.dim <= 64 ? launch_key_decay_chunks<64, BONUS>(p, out, n_chunks, st) : launch_key_decay_chunks<128, BONUS>(p, out, n_chunks, st);
     if (rc != SPITE_OK) return rc;
     return choose_scan<WALK>(p, st, leftovers_of(out, l, p.heads, Record<KEY_DECAY, 64>::SCALARS));
@@ -885,7 +888,7 @@ SPITE_API int spite_state_space_scan_chunked(const ScanParams* p, const float* a
     if (p->n_segments == 0 || p->n_tokens == 0) return SPITE_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const Layout l = scan_layout(false, p->dim, p->vdim, p->heads, p->kv_heads, n_chunks, p->n_segments);
-    const Made out = made_at(scratch, l, min_tokens, n_chunks);
+    const Made out = made_at(scratch, l, min_tokens, n_chunks, p->n_segments, p->n_long);
     const int rc = p->dim <= 64 ? launch_state_space_chunks<64>(*p, a, a_stride, a_log, dt_bias, out, st)
                                 : launch_state_space_chunks<128>(*p, a, a_stride, a_log, dt_bias, out, st);
     if (rc != SPITE_OK) return rc;

@@ -109,7 +109,7 @@ class ScanParams(C.Structure):
                 ("w", C.c_void_p), ("w_stride", C.c_longlong), ("scalars", C.c_void_p), ("skip", C.c_void_p),
                 ("out", C.c_void_p), ("out_stride", C.c_longlong), ("state", C.c_void_p), ("slot_stride", C.c_longlong),
                 ("cu_seqlens", C.c_void_p), ("slots", C.c_void_p), ("n_segments", C.c_int), ("n_tokens", C.c_int),
-                ("heads", C.c_int), ("kv_heads", C.c_int), ("dim", C.c_int), ("vdim", C.c_int), ("out_scale", C.c_float)]
+                ("heads", C.c_int), ("kv_heads", C.c_int), ("dim", C.c_int), ("vdim", C.c_int), ("out_scale", C.c_float), ("n_long", C.c_int)]
 
 
 class DeltaParams(C.Structure):
@@ -118,7 +118,8 @@ class DeltaParams(C.Structure):
                 ("a_log", C.c_void_p), ("dt_bias", C.c_void_p), ("out", C.c_void_p), ("state", C.c_void_p),
                 ("slot_stride", C.c_longlong), ("cu_seqlens", C.c_void_p), ("slots", C.c_void_p),
                 ("n_segments", C.c_int), ("heads", C.c_int), ("kv_heads", C.c_int), ("dim", C.c_int), ("vdim", C.c_int),
-                ("q_scale", C.c_float), ("unit_eps", C.c_float), ("gates", C.c_void_p), ("n_tokens", C.c_int)]
+                ("q_scale", C.c_float), ("unit_eps", C.c_float), ("gates", C.c_void_p), ("n_tokens", C.c_int),
+                ("n_long", C.c_int)]
 
 
 class MlstmParams(C.Structure):
@@ -127,7 +128,7 @@ class MlstmParams(C.Structure):
                 ("i_bias", C.c_void_p), ("f_bias", C.c_void_p), ("out", C.c_void_p), ("state", C.c_void_p),
                 ("head_stride", C.c_longlong), ("cu_seqlens", C.c_void_p), ("slots", C.c_void_p),
                 ("n_segments", C.c_int), ("heads", C.c_int), ("dim", C.c_int), ("vdim", C.c_int),
-                ("gate_cap", C.c_float), ("q_scale", C.c_float), ("chunked", C.c_int)]
+                ("gate_cap", C.c_float), ("q_scale", C.c_float), ("chunked", C.c_int), ("n_long", C.c_int)]
 
 
 class AttnMmaExtra(C.Structure):
@@ -1199,7 +1200,7 @@ class CudaKernels(KernelSet):
                         slots=batch.slots.data_ptr(), n_segments=n_seg, heads=int(heads), dim=int(dim), vdim=int(vdim),
                         gate_cap=float(gate_cap), q_scale=float(q_scale), chunked=int(bool(chunked)))
         if chunked:
-            n_chunks = (M + 31) // 32 + n_seg
+            p.n_long, n_chunks = self._long_segments(batch, self.memory_min_tokens)
             scratch = self._chunk_scratch("recurrent", "spite_mlstm_tiles_bytes", dim, vdim, heads, n_chunks, n_seg)
             if scratch is not None:
                 st = self._lib("recurrent").spite_mlstm_scan_tiles(C.byref(p), C.c_void_p(scratch.data_ptr()), n_chunks,
@@ -1210,12 +1211,20 @@ class CudaKernels(KernelSet):
             # (more than 256 key rows: the chunks' products on the float32 units)
             # working memory for what the chunks need ahead of the state (scores, sums of the gates): a record for every
             # chunk and head; the segments' chunks are at most tokens / 32 + segments
+            n_chunks = (M + 31) // 32 + n_seg
             scratch = torch.empty((n_chunks, heads, 1152), dtype=torch.float32, device=proj.device)
             st = self._lib("recurrent").spite_mlstm_scan_chunked(C.byref(p), C.c_void_p(scratch.data_ptr()), C.c_int(n_chunks), self._stream())
         else:
             st = self._lib("recurrent").spite_mlstm_scan(C.byref(p), self._stream())
         self._count("recurrent", 2 if chunked else 1)
         _check(st, "mlstm_scan")
+
+    @staticmethod
+    def _long_segments(batch, least):
+        """How many segments of a step have at least `least` tokens, and how many chunks of 32 these are (for none: as if for one, a
+        size that the entry points take)."""
+        chunks = [(s.n_tokens + 31) // 32 for s in batch.segments if s.n_tokens >= least]
+        return len(chunks), max(1, sum(chunks))
 
     def _chunk_scratch(self, library, query, *sizes):
         """Working memory of a walk in chunks, or None: sizes that it does not take, or more memory than the limit."""
@@ -1250,7 +1259,7 @@ class CudaKernels(KernelSet):
             # so that its results do not depend on how a prompt was cut, to the last bit.
             chunked = split_rows is None and self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from["delta"]
         if chunked:
-            n_chunks = (M + 31) // 32 + n_seg
+            p.n_long, n_chunks = self._long_segments(batch, self.chunk_min_tokens)
             scratch = self._chunk_scratch("delta", "spite_delta_chunk_bytes", dim, vdim, heads, kv_heads, M, n_chunks, n_seg)
             if scratch is not None:
                 st = self._lib("delta").spite_delta_scan_chunked(C.byref(p), C.c_void_p(scratch.data_ptr()), n_chunks, self.chunk_min_tokens,
@@ -1296,7 +1305,7 @@ class CudaKernels(KernelSet):
             # (the float32 set keeps the walk token by token, so that its results do not depend on how a prompt was cut)
             chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from[kind]
         if chunked:
-            n_chunks = (p.n_tokens + 31) // 32 + p.n_segments
+            p.n_long, n_chunks = self._long_segments(batch, self.chunk_min_tokens)
             scratch = self._chunk_scratch("scan", "spite_scan_chunk_bytes", per_channel, p.dim, p.vdim, p.heads, kv_heads, n_chunks, p.n_segments)
             if scratch is not None:
                 st = getattr(lib, entry + "_chunked")(C.byref(p), *rest, C.c_void_p(scratch.data_ptr()), n_chunks, self.chunk_min_tokens,

@@ -610,5 +610,36 @@ def test_working_memory_for_fewer_chunks_than_the_step_has(kind, n):
         off += tokens
         ref = whole if tokens >= 32 and at + chunks <= n else want
         assert torch.equal(out[part], ref[0][part]) and torch.equal(state[s], ref[1][s]), f"segment {s}"
-        at += chunks
+        at += chunks if tokens >= 32 else 0
     assert buffers and all(bool((b[need:] == 0x5a).all()) for b, need in buffers)
+
+
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("kind", KINDS)
+def test_decode_tokens_beside_portions_take_no_chunks(kind, known):
+    """Portions among many decoded tokens: the tokens' rows are the walk token by token's, the portions' the walk in chunks' alone, and
+    working memory is asked for the portions only.  `known`: the entry points are told how many portions there are."""
+    counts, heads, dim, vdim = [1] * 40 + [70] + [1] * 33 + [32, 1, 200] + [2] * 3, 2, 64, 48
+    ks = kernels(torch.bfloat16)
+    ks.memory_min_tokens = 32
+    run = walks(kind, ks, torch.Generator().manual_seed(15), counts, heads, dim, vdim)
+    asked, inner, of_batch = [], ks._chunk_scratch, ks._long_segments
+
+    def scratch(library, query, *sizes):
+        asked.append(sizes[-2])
+        return inner(library, query, *sizes)
+    ks._chunk_scratch = scratch
+    if not known:
+        ks._long_segments = lambda batch, least: (0, of_batch(batch, least)[1])
+    want, got = run(False), run()
+    assert asked == [3 + 1 + 7]
+    off = 0
+    for s, n in enumerate(counts):
+        part = slice(off, off + n)
+        off += n
+        if n < 32:
+            assert torch.equal(got[0][part], want[0][part]) and torch.equal(got[1][s], want[1][s]), f"segment {s}"
+        else:
+            near(got[0][part], want[0][part].double(), f"segment {s}", 1e-4)
+            near(got[1][s], want[1][s].double(), f"state of segment {s}", 1e-4)
+    assert ks.errors() == {}
