@@ -323,7 +323,8 @@ class CudaKernels(KernelSet):
         self.chunk_min_tokens = 32
         self.memory_min_tokens = 8
         # how much working memory a call may take for that (a step of 8,192 tokens of 32 heads of 128 x 128 takes 0.45 GB); a call that
-        # would need more goes token by token
+        # would need more goes as before: token by token, the matrix memory in chunks on the float32 units (which need 4.6 KB a chunk and
+        # head: 2,048 tokens of 8 heads of 256 x 512 599 us, token by token 3,150)
         self.chunk_scratch_limit = 1 << 30
         # arrival counters of the splits (zero between calls), one set per stream, since calls that share a set must not
         # overlap.  The sets are made ahead: one made while a CUDA graph is captured would lie in the graphs' memory
@@ -1208,7 +1209,7 @@ class CudaKernels(KernelSet):
                 self._count("recurrent", 3)
                 _check(st, "mlstm_scan")
                 return
-            # (more than 256 key rows: the chunks' products on the float32 units)
+            # (more than 256 key rows, or more working memory than the limit: the chunks' products on the float32 units)
             # working memory for what the chunks need ahead of the state (scores, sums of the gates): a record for every
             # chunk and head; the segments' chunks are at most tokens / 32 + segments
             n_chunks = (M + 31) // 32 + n_seg

@@ -643,3 +643,24 @@ def test_decode_tokens_beside_portions_take_no_chunks(kind, known):
             near(got[0][part], want[0][part].double(), f"segment {s}", 1e-4)
             near(got[1][s], want[1][s].double(), f"state of segment {s}", 1e-4)
     assert ks.errors() == {}
+
+
+@pytest.mark.parametrize("dim", [40, 100, 200])
+@pytest.mark.parametrize("kind", KINDS)
+def test_calls_beyond_the_limit_of_working_memory(kind, dim):
+    """The matrix memory goes in chunks on the float32 units, the other walks token by token."""
+    if kind != "matrix_memory" and dim > 128:
+        pytest.skip("no walk in chunks: always token by token")
+    ks = kernels(torch.bfloat16)
+    ks.chunk_scratch_limit = 1 << 10
+    library = {"matrix_memory": "recurrent", "delta": "delta"}.get(kind, "scan")
+    run = walks(kind, ks, torch.Generator().manual_seed(16), [70, 33, 1], 2, dim, 40)
+    want, want_state = run.reference()
+    before = ks.launches_by_library[library]
+    out, state = run()
+    assert ks.launches_by_library[library] == before + 2
+    near(out.view_as(want), want, "outputs", 1e-4)
+    near(run.matrices(state), want_state, "states")
+    if kind != "matrix_memory":
+        tokens = run(False)
+        assert torch.equal(out, tokens[0]) and torch.equal(state, tokens[1])
