@@ -384,9 +384,15 @@ class CudaKernels(KernelSet):
         return out
 
     @staticmethod
+    def _raw_stream() -> int:
+        # The handle by a name that torch's own compiler uses but does not document: a Stream object for each of a step's launches takes
+        # about 1.5 us more.  A torch without the name gets the object.
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
+
+    @staticmethod
     def _stream():
-        # (the raw handle: a Stream object for each of a step's launches takes about 1.5 us more)
-        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+        return C.c_void_p(CudaKernels._raw_stream())
 
     def _t(self, t, dtype=None, name="tensor"):
         if t.device.type != "cuda" or not t.is_contiguous():
@@ -718,7 +724,7 @@ class CudaKernels(KernelSet):
         tile_rows = 128 // slices
         tiles = -(-p.N // (tile_rows // 2 if swiglu else tile_rows)) * groups
         lib = self._lib("gemm_stream")
-        stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        stream = self._raw_stream()
         if slices == 1 and 2 <= splits <= self.stream_cluster_max_splits and rows <= self.stream_cluster_max_rows:
             # the k splits of a tile as one thread-block cluster: their sums meet in shared memory
             st = lib.spite_gemm_stream(C.byref(p), max_rows_per_group, 1, 1, blocks, smem, splits, None, C.c_longlong(0),

@@ -60,3 +60,14 @@ def test_cuts_of_one_group_products_are_cuts_that_the_kernel_takes(M, N, K, swig
     groups = 1 if nt == 32 else 1024
     fixed = 24 * 8 + 16 + 4 * groups + (8 - 8 // slices) * 64 * nt * (slices > 1) + 1024
     assert (smem - fixed) // (16384 + max(1024, slices * nt * 128)) >= 2                      # a ring of at least two stages
+
+
+def test_stream_handles_without_the_undocumented_name(monkeypatch):
+    from types import SimpleNamespace
+    from spite_b200.kernels.cuda import CudaKernels
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 100 + device, raising=False)
+    assert CudaKernels._raw_stream() == 103
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=77))
+    assert CudaKernels._raw_stream() == 77
