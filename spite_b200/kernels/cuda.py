@@ -312,14 +312,24 @@ class CudaKernels(KernelSet):
         # against (74 KiB, 3), 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 / 17.8, 4096 x 4096 8.5 / 10.6; 16 rows 8.6 / 10.8,
         # 16.2 / 20.6, 9.8 / 13.8; one block per multiprocessor with 110 or 200 KiB: 3.2 and 3.1 ms
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
-        # Recurrences over prompts: a step whose longest segment has at least so many tokens goes in chunks of 32 on the tensor cores (its
-        # segments of fewer than 32 tokens, 8 in the matrix memory, token by token).  us in chunks / token by token.  Delta rule, 16 heads
-        # of 128 x 128: one prompt of 32 tokens 21 / 24, 64: 23 / 42, 512: 45 / 291, 2,048: 152 / 1,147; sixteen prompts of 32: 64 / 95.
-        # Matrix memory, 8 heads of 256 x 512: 16 tokens 19 / 21, 2,048: 224 / 3,150.  State space, 128 heads of 128 x 64: 64 tokens
-        # 26 / 18, 128: 31 / 30, 512: 63 / 99, 2,048: 206 / 378.  Gated linear attention, 32 heads of 64 x 128: 256 tokens 35 / 32, 512:
-        # 48 / 59, 2,048: 155 / 223; sixteen prompts of 128: 139 / 133.  Decaying memory, 64 heads of 64 x 64: 512 tokens 64 / 63, 2,048:
-        # 224 / 238.
-        self.chunk_from = {"delta": 32, "memory": 8, "state_space": 160, "linear_attention": 320, "decaying_memory": 1024}
+        # Recurrences over prompts: a step whose longest segment has at least so many tokens, `chunk_from` (`chunk_from_few` where its long
+        # segments have fewer than 32 heads together), and `chunk_per_brief` more for each of its segments of fewer than 32 tokens (8 in
+        # the matrix memory), goes in chunks of 32 on the tensor cores, those short segments token by token behind them.  The token walk alone takes all segments of a step side by side, so its walk over a portion
+        # hides behind many decode tokens' states; the chunks and the short segments follow one another.  us in chunks / token by token:
+        #   delta rule, 16 heads of 128 x 128: one prompt of 32 tokens 24 / 25, 64: 26 / 44, 2,000: 169 / 1,150; four of 32 31 / 30, of 40
+        #     36 / 36; beside 48 decode tokens 64: 54 / 51, 128: 59 / 87; beside 384 256: 286 / 226, 1,024: 346 / 652; 32 heads: beside 128
+        #     128: 194 / 163, 256: 207 / 216, beside 384 512: 569 / 491, 1,024: 628 / 810
+        #   matrix memory, 8 heads of 256 x 512 (in chunks of float32 products 31 from 8 tokens on): 8: 20 / 13, 16: 20 / 21, 2,000:
+        #     246 / 3,056; beside 128 decode tokens 64: 345 / 347 (2,036), 256: 366 / 525 (2,068)
+        #   state space, 128 heads of 128 x 64: 160: 38 / 36, 192: 41 / 42, 256: 46 / 53, 2,000: 226 / 368; beside 16 256: 77 / 74, 512: 101 /
+        #     140; beside 128 512: 297 / 297, 1,024: 348 / 372; 64 heads: 160: 31 / 33; beside 128 1,024: 202 / 193, 2,000: 263 / 368; beside
+        #     384 2,000: 490 / 454
+        #   gated linear attention, 32 heads of 64 x 128: 320: 42 / 39, 384: 45 / 46, 512: 52 / 59, 2,000: 170 / 218; four of 384 110 / 111;
+        #     16 heads: 512: 50 / 47, beside 4 512: 51 / 52; 32 heads beside 128 512: 119 / 95, 1,024: 156 / 168; beside 384 2,000: 360 / 337
+        #   decaying memory, 64 heads of 64 x 64: 512: 69 / 63, 2,048: 243 / 238, four of 2,048 783 / 690: never unless it is asked for
+        self.chunk_from = {"delta": 40, "memory": 8, "state_space": 192, "linear_attention": 384, "decaying_memory": None}
+        self.chunk_from_few = {"linear_attention": 560}
+        self.chunk_per_brief = {"delta": 1.3, "memory": 0.0, "state_space": 6.6, "linear_attention": 4.5, "decaying_memory": 0.0}
         self.chunk_min_tokens = 32
         self.memory_min_tokens = 8
         # how much working memory a call may take for that (a step of 8,192 tokens of 32 heads of 128 x 128 takes 0.45 GB); a call that
@@ -1198,9 +1208,7 @@ class CudaKernels(KernelSet):
             raise KernelError("mlstm_scan: the columns lie outside the projection's rows")
         n_seg = batch.cu_seqlens.numel() - 1
         if chunked is None:
-            # Prompts and their portions go 32 tokens at a time.  The float32 set keeps the walk token by token for
-            # every step, so that its results do not depend on how a prompt was cut, to the last bit.
-            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from["memory"]
+            chunked = self._pays_in_chunks("memory", batch, self.memory_min_tokens, heads)
         p = MlstmParams(proj=proj.data_ptr(), stride=proj.shape[1], q_col=q_col, k_col=k_col, v_col=v_col, i_col=i_col,
                         f_col=f_col, i_bias=i_bias.data_ptr(), f_bias=f_bias.data_ptr(), out=out.data_ptr(),
                         state=state.data_ptr(), head_stride=state.shape[2], cu_seqlens=batch.cu_seqlens.data_ptr(),
@@ -1226,10 +1234,24 @@ class CudaKernels(KernelSet):
         self._count("recurrent", 2 if chunked else 1)
         _check(st, "mlstm_scan")
 
+    def _pays_in_chunks(self, kind, batch, least, heads):
+        """Whether a step's segments of at least `least` tokens go in chunks where the caller leaves it open."""
+        start = self.chunk_from[kind]
+        # (the float32 set keeps the walk token by token, so that its results do not depend on how a prompt was cut)
+        if self.dtype == torch.float32 or start is None or batch.max_seg_len < start:
+            return False
+        brief = sum(s.n_tokens < least for s in batch.segments)
+        if heads * max(1, len(batch.segments) - brief) < 32:
+            start = self.chunk_from_few.get(kind, start)
+        return batch.max_seg_len >= start + self.chunk_per_brief[kind] * brief
+
     @staticmethod
     def _long_segments(batch, least):
         """How many segments of a step have at least `least` tokens, and how many chunks of 32 these are (for none: as if for one, a
-        size that the entry points take)."""
+        size that the entry points take).  A batch that does not name its segments: not known, and as many as they can be."""
+        n_seg = batch.cu_seqlens.numel() - 1
+        if len(batch.segments) != n_seg:
+            return 0, batch.n_tokens // 32 + n_seg
         chunks = [(s.n_tokens + 31) // 32 for s in batch.segments if s.n_tokens >= least]
         return len(chunks), max(1, sum(chunks))
 
@@ -1262,9 +1284,7 @@ class CudaKernels(KernelSet):
                         vdim=int(vdim), q_scale=float(q_scale), unit_eps=float(unit_eps), gates=gates.data_ptr(), n_tokens=M)
         n_seg = batch.cu_seqlens.numel() - 1
         if chunked is None:
-            # Prompts and their portions go 32 tokens at a time.  The float32 set keeps the walk token by token for every step,
-            # so that its results do not depend on how a prompt was cut, to the last bit.
-            chunked = split_rows is None and self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from["delta"]
+            chunked = split_rows is None and self._pays_in_chunks("delta", batch, self.chunk_min_tokens, heads)
         if chunked:
             p.n_long, n_chunks = self._long_segments(batch, self.chunk_min_tokens)
             scratch = self._chunk_scratch("delta", "spite_delta_chunk_bytes", dim, vdim, heads, kv_heads, M, n_chunks, n_seg)
@@ -1309,8 +1329,7 @@ class CudaKernels(KernelSet):
         """One of the three walks: in chunks where that is asked for or pays and the sizes allow it, else token by token."""
         lib = self._lib("scan")
         if chunked is None:
-            # (the float32 set keeps the walk token by token, so that its results do not depend on how a prompt was cut)
-            chunked = self.dtype != torch.float32 and batch.max_seg_len >= self.chunk_from[kind]
+            chunked = self._pays_in_chunks(kind, batch, self.chunk_min_tokens, p.heads)
         if chunked:
             p.n_long, n_chunks = self._long_segments(batch, self.chunk_min_tokens)
             scratch = self._chunk_scratch("scan", "spite_scan_chunk_bytes", per_channel, p.dim, p.vdim, p.heads, kv_heads, n_chunks, p.n_segments)

@@ -664,3 +664,27 @@ def test_calls_beyond_the_limit_of_working_memory(kind, dim):
     if kind != "matrix_memory":
         tokens = run(False)
         assert torch.equal(out, tokens[0]) and torch.equal(state, tokens[1])
+
+
+# (walk, heads, segments, in chunks): a portion beside decode tokens whose states hide the token walk's chain goes token by token
+ROUTES = [("delta", 16, [40], True), ("delta", 16, [39], False), ("delta", 16, [64] + [1] * 16, True), ("delta", 16, [64] + [1] * 48, False),
+          ("delta", 16, [1] * 100 + [256], True), ("state_space", 64, [192], True), ("state_space", 64, [191], False),
+          ("state_space", 64, [256] + [1] * 16, False), ("state_space", 64, [512] + [1] * 16, True), ("linear_attention", 32, [384], True),
+          ("linear_attention", 16, [384], False), ("linear_attention", 16, [300, 384], True), ("linear_attention", 32, [512] + [1] * 64, False),
+          ("decaying_memory", 8, [2048], False), ("matrix_memory", 2, [8], True), ("matrix_memory", 2, [7], False),
+          ("matrix_memory", 2, [1] * 50 + [9], True)]
+
+
+@pytest.mark.parametrize("case", range(len(ROUTES)))
+def test_which_steps_go_in_chunks_where_the_caller_leaves_it_open(case):
+    kind, heads, counts, in_chunks = ROUTES[case]
+    ks, exact = kernels(torch.bfloat16), kernels(torch.float32)
+    library = {"matrix_memory": "recurrent", "delta": "delta"}.get(kind, "scan")
+    for k, want in ((ks, in_chunks), (exact, False)):
+        run = walks(kind, k, torch.Generator().manual_seed(17), counts, heads, 32, 16)
+        before = k.launches_by_library[library]
+        out, state = run(None)
+        assert k.launches_by_library[library] - before == (1 if library == "recurrent" else 2) + want * (
+            2 if kind in ("matrix_memory", "linear_attention") else 1)
+        forced = run(want)
+        assert torch.equal(out, forced[0]) and torch.equal(state, forced[1])
