@@ -314,22 +314,23 @@ class CudaKernels(KernelSet):
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
         # Recurrences over prompts: a step whose longest segment has at least so many tokens, `chunk_from` (`chunk_from_few` where its long
         # segments have fewer than 32 heads together), and `chunk_per_brief` more for each of its segments of fewer than 32 tokens (8 in
-        # the matrix memory), goes in chunks of 32 on the tensor cores, those short segments token by token behind them.  The token walk alone takes all segments of a step side by side, so its walk over a portion
-        # hides behind many decode tokens' states; the chunks and the short segments follow one another.  us in chunks / token by token:
+        # the matrix memory), goes in chunks of 32 on the tensor cores, those short segments token by token behind them.  The token walk
+        # alone takes all segments of a step side by side, so its walk over a portion hides behind many decode tokens' states; the chunks
+        # and the short segments follow one another.  us in chunks / token by token:
         #   delta rule, 16 heads of 128 x 128: one prompt of 32 tokens 24 / 25, 64: 26 / 44, 2,000: 169 / 1,150; four of 32 31 / 30, of 40
         #     36 / 36; beside 48 decode tokens 64: 54 / 51, 128: 59 / 87; beside 384 256: 286 / 226, 1,024: 346 / 652; 32 heads: beside 128
-        #     128: 194 / 163, 256: 207 / 216, beside 384 512: 569 / 491, 1,024: 628 / 810
+        #     128: 194 / 163, 256: 207 / 216, beside 200 300: 306 / 269, 400: 317 / 334, beside 384 512: 569 / 491, 1,024: 628 / 810
         #   matrix memory, 8 heads of 256 x 512 (in chunks of float32 products 31 from 8 tokens on): 8: 20 / 13, 16: 20 / 21, 2,000:
         #     246 / 3,056; beside 128 decode tokens 64: 345 / 347 (2,036), 256: 366 / 525 (2,068)
         #   state space, 128 heads of 128 x 64: 160: 38 / 36, 192: 41 / 42, 256: 46 / 53, 2,000: 226 / 368; beside 16 256: 77 / 74, 512: 101 /
         #     140; beside 128 512: 297 / 297, 1,024: 348 / 372; 64 heads: 160: 31 / 33; beside 128 1,024: 202 / 193, 2,000: 263 / 368; beside
         #     384 2,000: 490 / 454
         #   gated linear attention, 32 heads of 64 x 128: 320: 42 / 39, 384: 45 / 46, 512: 52 / 59, 2,000: 170 / 218; four of 384 110 / 111;
-        #     16 heads: 512: 50 / 47, beside 4 512: 51 / 52; 32 heads beside 128 512: 119 / 95, 1,024: 156 / 168; beside 384 2,000: 360 / 337
+        #     16 heads: 512: 50 / 47, 600: 55 / 54, 1,000: 76 / 86; 32 heads beside 128 512: 119 / 95, 1,024: 156 / 168; beside 384 2,000: 360 / 337
         #   decaying memory, 64 heads of 64 x 64: 512: 69 / 63, 2,048: 243 / 238, four of 2,048 783 / 690: never unless it is asked for
         self.chunk_from = {"delta": 40, "memory": 8, "state_space": 192, "linear_attention": 384, "decaying_memory": None}
-        self.chunk_from_few = {"linear_attention": 560}
-        self.chunk_per_brief = {"delta": 1.3, "memory": 0.0, "state_space": 6.6, "linear_attention": 4.5, "decaying_memory": 0.0}
+        self.chunk_from_few = {"linear_attention": 640}
+        self.chunk_per_brief = {"delta": 1.7, "memory": 0.0, "state_space": 6.6, "linear_attention": 4.5, "decaying_memory": 0.0}
         self.chunk_min_tokens = 32
         self.memory_min_tokens = 8
         # how much working memory a call may take for that (a step of 8,192 tokens of 32 heads of 128 x 128 takes 0.45 GB); a call that

@@ -667,7 +667,7 @@ def test_calls_beyond_the_limit_of_working_memory(kind, dim):
 
 
 # (walk, heads, segments, in chunks): a portion beside decode tokens whose states hide the token walk's chain goes token by token
-ROUTES = [("delta", 16, [40], True), ("delta", 16, [39], False), ("delta", 16, [64] + [1] * 16, True), ("delta", 16, [64] + [1] * 48, False),
+ROUTES = [("delta", 16, [40], True), ("delta", 16, [39], False), ("delta", 16, [72] + [1] * 16, True), ("delta", 16, [72] + [1] * 48, False),
           ("delta", 16, [1] * 100 + [256], True), ("state_space", 64, [192], True), ("state_space", 64, [191], False),
           ("state_space", 64, [256] + [1] * 16, False), ("state_space", 64, [512] + [1] * 16, True), ("linear_attention", 32, [384], True),
           ("linear_attention", 16, [384], False), ("linear_attention", 16, [300, 384], True), ("linear_attention", 32, [512] + [1] * 64, False),
