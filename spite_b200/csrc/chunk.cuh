@@ -335,8 +335,9 @@ struct Made { __half* qk; __half* w; __half* scores; float* records; float* u0; 
 // `n_long`: how many segments have at least min_tokens tokens, 0 if the caller does not know (each has a chunk at least)
 inline Made made_at(void* scratch, const Layout& l, int min_tokens, int n_chunks, int n_segments, int n_long) {
     unsigned char* b = (unsigned char*)scratch;
+    const int most = n_chunks < n_segments ? n_chunks : n_segments;
     return {(__half*)(b + l.qk), (__half*)(b + l.w), (__half*)(b + l.scores), (float*)(b + l.records), (float*)(b + l.u0),
-            (int*)(b + l.columns), l.column_groups, {min_tokens, n_chunks, n_long > 0 ? n_long : n_chunks < n_segments ? n_chunks : n_segments}};
+            (int*)(b + l.columns), l.column_groups, {min_tokens, n_chunks, n_long > 0 && n_long < most ? n_long : most}};
 }
 inline Walk walk_of(const Made& m) {
     Walk w = {};
@@ -367,6 +368,10 @@ template <int KPW, int KW, int CW, int MODE> struct Shape {
     static constexpr int bytes(int stages) { return stages * STAGE + SUMS + EXTRA; }
 };
 
+// What bounds it: the dependent instructions of the two warps a scheduler holds (8 x 256 x 512, 2,048 tokens: 228 us; tensor pipe 27 % of
+// the time, issue slots 42 %, memory 5 %; a warp waits for the instruction before 1.5, for shared memory and shuffles 0.5, for the tensor
+// pipe 0.5, at the barrier 0.3 of the 4.8 clocks between two of its instructions).  A scale per column and token instead of one a tile
+// with a block-wide maximum: 201 -> 228 us; 128 x 128, 16 heads 114 -> 130; 128 x 64, 128 heads 181 -> 200; 64 x 128, 32 heads 92 -> 103.
 // grid (ceil(vdim / COLS), heads, segments that go in chunks)
 template <int KPW, int KW, int CW, int MODE>
 __global__ void __launch_bounds__(32 * KW * CW) chunk_walk_kernel(const Walk p, const tc::WaitControl waits) {

@@ -539,8 +539,8 @@ int launch_delta_chunks(const DeltaParams& p, const Made& out, cudaStream_t st) 
     w.n_segments = p.n_segments; w.heads = p.heads; w.qk_heads = p.kv_heads; w.dim = p.dim; w.vdim = p.vdim;
     w.out_scale = p.q_scale;
     // 16 columns a block while that leaves every multiprocessor one block at most, else 32.  2,048 tokens, us of the walk alone: 16 heads
-    // (128 blocks of 16 columns) 124, with 16 keys a warp and twice the warps 135; 32 heads (128 blocks of 32) 165.  The kernel before it: 39
-    // and 70 (a block a head instead of two: 69 and 111).
+    // (128 blocks of 16 columns) 130, 32 heads (128 blocks of 32) 176.  The kernel before it: 41 and 74.  Measured with one scale a tile:
+    // 124, with 16 keys a warp and twice the warps 135; the kernel before it 39 and 70, with a block a head instead of two 69 and 111.
     if ((long long)((p.vdim + 15) / 16) * p.heads * out.numbering.segments <= 148) return launch_walk<32, DP / 32, 1, DELTA>(w, s_waits, st);
     return launch_walk<32, DP / 32, 2, DELTA>(w, s_waits, st);
 }

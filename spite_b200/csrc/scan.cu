@@ -832,8 +832,8 @@ int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, 
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
     chunk::Walk w = scan_walk(p, out);
     w.out_scale = BONUS ? 1.f : p.out_scale;
-    // (32 columns a block; with 64, 32 heads of 64 x 128: five requests of 2,048 tokens together 68 us against 62, four of 2,048 each 205
-    // against 231)
+    // (32 columns a block: 32 heads of 64 x 128, five requests of 2,048 tokens together 73 us, four of 2,048 each 258; measured with one
+    // scale a tile 62 and 231, with 64 columns 68 and 205)
     return launch_walk<32, DP / 32, 2, KEY_DECAY>(w, s_waits, st);
 }
 template <bool BONUS, int WALK>
