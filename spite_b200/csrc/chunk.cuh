@@ -122,9 +122,12 @@ __device__ __forceinline__ float2 sum3(const float (&c)[3][4], int i) {
 // ... in two sums: `main` takes the first, `cross` the other two; their sum times DOWN^2
 __device__ __forceinline__ void mma3(float (&main)[4], float (&cross)[4], const unsigned (&ah)[4], const unsigned (&al)[4],
                                      unsigned bh0, unsigned bh1, unsigned bl0, unsigned bl1) {
+    float p[4] = {};                                      // (the tensor cores cut their sums off; float32 additions round them)
     mma(cross, al, bh0, bh1);
-    mma(main, ah, bh0, bh1);
+    mma(p, ah, bh0, bh1);
     mma(cross, ah, bl0, bl1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) main[i] += p[i];
 }
 __device__ __forceinline__ float sum2(float main, float cross) { return fmaf(cross, LOW_DOWN, main) * (DOWN * DOWN); }
 
