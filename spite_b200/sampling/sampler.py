@@ -10,8 +10,10 @@ token, so what a request samples does not depend on what else is in the batch.
 """
 from __future__ import annotations
 
+import struct
 from dataclasses import dataclass, field
 
+import numpy
 import torch
 
 DEFAULT_SEED = 0x1234_5678_9ABC_DEF0        # the constant of crates/spite-cli/src/main.rs:606
@@ -54,10 +56,6 @@ def lcg_advance(state: int) -> int:
     return (state * 6364136223846793005 + 1442695040888963407) & _MASK64
 
 
-def _signed(x: int) -> int:
-    return x - (1 << 64) if x >= (1 << 63) else x
-
-
 @dataclass
 class SampleRow:
     params: SamplingParams
@@ -94,9 +92,10 @@ class Sampler:
 
     def _staged(self, dev):
         if dev.type == "cuda":
-            ev = torch.cuda.Event()
-            ev.record()
-            self._buffers[self._turn][1] = ev
+            slot = self._buffers[self._turn]
+            if slot[1] is None:
+                slot[1] = torch.cuda.Event()
+            slot[1].record()
 
     def greedy_on_device(self, logits: torch.Tensor) -> torch.Tensor:
         """The argmax of every row as int32 on the device; nothing is read back."""
@@ -121,14 +120,14 @@ class Sampler:
             return self.k.argmax(logits), [r.rng_state for r in rows]
         ctx, offs, holes, sources = [], [0], [], []
         for i, r in enumerate(rows):
-            c = r.context
+            c, params = r.context, r.params
             late = pending is not None and pending[1][i] >= 0
             if late:
                 c = c + [0]                                  # the place of the token that is still on the device
-            n = r.params.repeat_last_n
+            n = params.repeat_last_n
             if n and n < len(c):
                 c = c[-n:]
-            if abs(r.params.repetition_penalty - 1.0) < 1.2e-7:
+            if abs(params.repetition_penalty - 1.0) < 1.2e-7:
                 c = []
             ctx += c
             offs.append(len(ctx))
@@ -147,17 +146,20 @@ class Sampler:
         a_state = (a_late + 2 * len(holes) + 1) // 2 * 2          # 64-bit states on an 8-byte boundary
         n_words = a_state + 2 * R
         host = self._staging(n_words, dev)
-        fl = host.view(torch.float32)
-        fl[0:R] = torch.tensor([r.params.temperature for r in rows], dtype=torch.float32)
-        host[R:2 * R] = torch.tensor([r.params.top_k for r in rows], dtype=torch.int32)
-        fl[2 * R:3 * R] = torch.tensor([r.params.top_p for r in rows], dtype=torch.float32)
-        fl[3 * R:4 * R] = torch.tensor([r.params.min_p for r in rows], dtype=torch.float32)
-        fl[4 * R:5 * R] = torch.tensor([r.params.repetition_penalty for r in rows], dtype=torch.float32)
-        host[a_off:a_ctx] = torch.tensor(offs, dtype=torch.int32)
-        host[a_ctx:a_late] = torch.tensor(ctx, dtype=torch.int32)
+        # Filled as numbers in memory: with a torch tensor made from each list first a call for 32 rows with up to 64 tokens of context takes 239
+        # us of host, this way 88 (the kernel behind it 63).
+        ints = host.numpy()
+        floats = ints.view(numpy.float32)
+        settings = [r.params for r in rows]
+        floats[0:R] = [p.temperature for p in settings]
+        ints[R:2 * R] = [p.top_k for p in settings]
+        floats[2 * R:3 * R] = [p.top_p for p in settings]
+        floats[3 * R:4 * R] = [p.min_p for p in settings]
+        floats[4 * R:5 * R] = [p.repetition_penalty for p in settings]
+        struct.pack_into(f"{len(offs) + len(ctx)}i", ints, 4 * a_off, *offs, *ctx)
         if holes:
-            host[a_late:a_late + 2 * len(holes)] = torch.tensor(holes + sources, dtype=torch.int32)
-        host[a_state:n_words].view(torch.int64)[:] = torch.tensor([_signed(r.rng_state & _MASK64) for r in rows], dtype=torch.int64)
+            struct.pack_into(f"{2 * len(holes)}i", ints, 4 * a_late, *holes, *sources)
+        struct.pack_into(f"{R}Q", ints, 4 * a_state, *[r.rng_state & _MASK64 for r in rows])
         words = torch.empty(n_words, dtype=torch.int32, device=dev)
         words.copy_(host[:n_words], non_blocking=True)
         self._staged(dev)
