@@ -26,7 +26,8 @@
 // products.  (A kernel that allocates tensor memory gets one block per multiprocessor, so the
 // overlap has to come from within the block.)  Blocks are persistent, one per multiprocessor:
 // the work items (pair of row tiles, kv head) are dealt out round by round in alternating
-// direction, heaviest first, and between items the block renews its barriers.
+// direction, heaviest first, or cut along the keys into equal shares (see Cut), and between items the
+// block renews its barriers.
 // The output accumulates in tensor memory.  A row's reference maximum moves only when the
 // tile's maximum exceeds it by more than 8 (in log2 units): then the row's part of O and its
 // sum are multiplied by 2^(old - new) before the next product is added.  P stays below 2^8, and
@@ -58,6 +59,19 @@ __device__ int g_attn_tc_error = 0;
 // (`extra_tx` is not used here.)
 SPITE_WAIT_CONTROLS(attention_tc, g_attn_tc_error)
 namespace {
+
+// Work cut along the keys.  An item (pair of row tiles, kv head) costs its key tiles and CUT_ITEM more (to start and to end, about 7 us);
+// the items laid end to end are one line, and every block takes an equal stretch of it.  What a stretch holds of an item that it shares
+// with others is a part: its rows' output before the division, their maximum and their sum go to `partial`, and a kernel behind this one
+// adds an item's parts up, in the order of the keys.
+constexpr int CUT_PAIRS = 1024;         // most pairs of row tiles
+constexpr int CUT_ITEM = 6;
+constexpr int CUT_PIECE = 4;            // a part is no shorter than this many key tiles: a cut so close to an item's end moves there
+constexpr int CUT_SHARE = 8;            // nor is a block's share
+struct Cut {
+    float* partial;                     // [blocks][2: a block's first part, its last][2 row tiles x (HD + 2) x 128], or null: items are not cut
+    int4* items;                        // [blocks]: the item whose first cut is where block i begins (item, parts, first token, tokens); no parts: none
+};
 
 struct GroupBarriers {
     unsigned long long s_full[2], p_ready, pv_done, exp_done;
@@ -97,18 +111,32 @@ __device__ __forceinline__ unsigned pack_bf16(float a, float b) {
     return *(unsigned*)&v;
 }
 
+__host__ __device__ constexpr size_t slot_floats(int head_dim) { return 2 * (size_t)(head_dim + 2) * BM; }     // of a part
+
+// What a row's output is multiplied by in the end: one over its sum, which the sink joins first; m is the row's reference in log2 units.
+__device__ __forceinline__ float inverse_sum(const AttentionParams& p, int tok, int head, float m, float l) {
+    float shrink = 1.f;
+    if (p.has_sink) {                              // the sink's score in this kernel's units (powers of two)
+        const float sink2 = sink_of(p, head) * LOG2E, m2 = fmaxf(m, sink2);
+        shrink = (m == -INFINITY) ? 0.f : exp2f(m - m2);
+        l = l * shrink + exp2f(sink2 - m2);
+    }
+    return shrink * gate_of(p, tok, head) / fmaxf(l, 1e-30f);
+}
+
 // NKB = head_dim / 64.  grid (blocks over (request, pair of token tiles), kv heads).
 template <int NKB, int FORM>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const AttentionParams p, const StepTokens b,
-               const PagedCache c, const AttnMmaExtra x, const int q_box_tokens, const int n_tile_pairs,
+               const PagedCache c, const AttnMmaExtra x, const int q_box_tokens, const int n_tile_pairs, const Cut cut,
                const WaitControl waits) {
     constexpr int HD = 64 * NKB;
     constexpr int Q_BYTES = NKB * BM * 128;              // q of one row tile
     constexpr int KT_BYTES = NKB * BN * 128;             // one K tile, one V tile
     extern __shared__ __align__(1024) unsigned char smem[];   // [Q0][Q1][K ring][V ring], each 1024-byte aligned
     __shared__ Barriers bars;
+    __shared__ int line[CUT_PAIRS + 1];                       // what the pairs before cost (for one kv head)
     __shared__ __align__(16) float key_scales[FORM == FORM_ANY ? 8 : 1][BN];    // a softmax warp's copy of its tile's keys' factors
     pdl_wait();
     pdl_launch_dependents();
@@ -147,6 +175,29 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         init_barriers(false);
     }
     if (warp == 1) tmem_alloc(&bars.tmem_base, TMEM_COLS);
+    // The pair of row tiles `idx`: its request, first token, number of tokens (seg < 0: the caller counted more pairs than there are),
+    // first key and key tiles, from the first key that its first token sees to its last token's own.
+    struct Pair { int seg, t0, nt, k_begin, n_tiles; };
+    auto pair_of = [&](int idx) {
+        Pair r{-1, 0, 0, 0, 0};
+        for (int s = 0; s < x.n_segments; ++s) {
+            const int lo = x.cu_seqlens[s], n = x.cu_seqlens[s + 1] - lo;
+            if (n < x.seg_min_tokens || n > x.seg_max_tokens) continue;   // another kernel serves this segment
+            const int blocks = (n + 2 * tpt - 1) / (2 * tpt);
+            if (idx < blocks) { r.seg = s; r.t0 = lo + idx * 2 * tpt; r.nt = min(2 * tpt, lo + n - r.t0); break; }
+            idx -= blocks;
+        }
+        if (r.seg >= 0) {
+            r.k_begin = (window_lowest(p.window_kind, p.window_size, b.positions[r.t0]) / BN) * BN;
+            r.n_tiles = (b.positions[r.t0 + r.nt - 1] - r.k_begin) / BN + 1;
+        }
+        return r;
+    };
+    if (cut.partial)
+        for (int j = threadIdx.x; j < n_tile_pairs; j += THREADS) {
+            const int n = pair_of(n_tile_pairs - 1 - j).n_tiles;
+            line[j + 1] = n ? n + CUT_ITEM : 0;
+        }
     if (warp >= 3) {
         // rows of a q tile that the TMA box does not write: zero, so that their scores are plain numbers
         const int g = (warp - 3) >> 2, r = (warp & 3) * 32 + lane;
@@ -164,27 +215,97 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     fence_after();
     const unsigned tmem = bars.tmem_base;
 
+    // The line: item (pair n_tile_pairs - 1 - j, kv head h) begins at nkv * line[j] + h * its length.  Block i's stretch goes from cut i to
+    // cut i + 1; cut i is at i equal shares, or at the item's start or end if it leaves less than CUT_PIECE key tiles on that side.
+    long long line_end = 0, at = 0, stretch_end = 0;
+    int sharers = 0;
+    struct Place { int j, kvh, off, len; };
+    auto place_of = [&](long long t) {                        // 0 <= t < line_end
+        int lo = 0, hi = n_tile_pairs;                        // nkv * line[lo] <= t < nkv * line[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if ((long long)nkv * line[mid] <= t) lo = mid; else hi = mid;
+        }
+        const int len = line[lo + 1] - line[lo], rest = (int)(t - (long long)nkv * line[lo]);
+        return Place{lo, rest / len, rest % len, len};
+    };
+    auto cut_at = [&](int i) {
+        if (i >= sharers) return line_end;
+        const long long t = line_end * i / sharers;
+        if (t == 0) return t;
+        const Place q = place_of(t);
+        return q.off < CUT_ITEM + CUT_PIECE ? t - q.off : q.len - q.off < CUT_PIECE ? t + q.len - q.off : t;
+    };
+    if (cut.partial) {
+        if (warp == 0) {
+            int sum = 0;
+            for (int j0 = 0; j0 < n_tile_pairs; j0 += 32) {
+                int v = j0 + lane < n_tile_pairs ? line[j0 + lane + 1] : 0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, v, o);
+                    if (lane >= o) v += u;
+                }
+                if (j0 + lane < n_tile_pairs) line[j0 + lane + 1] = sum + v;
+                sum += __shfl_sync(0xffffffffu, v, 31);
+            }
+            if (lane == 0) line[0] = 0;
+        }
+        __syncthreads();
+        line_end = (long long)nkv * line[n_tile_pairs];
+        sharers = (int)min((long long)gridDim.x, max(1ll, line_end / CUT_SHARE));
+        if (line_end > 0 && blockIdx.x < sharers) { at = cut_at(blockIdx.x); stretch_end = cut_at(blockIdx.x + 1); }
+        if (threadIdx.x == 0) {
+            int4 mine = make_int4(0, 0, 0, 0);
+            if (at < stretch_end) {
+                const Place q = place_of(at);
+                if (q.off > 0) {                              // the cuts within the item: those that leave CUT_PIECE tiles on either side
+                    const long long t0 = at - q.off;
+                    int first = -1, n = 0;
+                    for (int i = (int)(t0 * sharers / line_end); i < sharers; ++i) {
+                        const long long t = line_end * i / sharers;
+                        if (t > t0 + q.len - CUT_PIECE) break;
+                        if (i == 0 || t < t0 + CUT_ITEM + CUT_PIECE) continue;
+                        if (n++ == 0) first = i;
+                    }
+                    if (first == blockIdx.x) {
+                        const Pair r = pair_of(n_tile_pairs - 1 - q.j);
+                        mine = make_int4(q.j * nkv + q.kvh, n + 1, r.t0, r.nt);
+                    }
+                }
+            }
+            cut.items[blockIdx.x] = mine;
+        }
+    }
+
     // Work items: (pair of row tiles of a request, kv head), numbered so that the work falls with the
-    // number (later tokens see more keys).  Blocks are persistent; round r deals items r * blocks ..
+    // number (later tokens see more keys).  Blocks are persistent.  Uncut, round r deals items r * blocks ..
     // (r + 1) * blocks - 1 to the blocks, in alternating direction, so that the shares come out alike.
     const int n_items = n_tile_pairs * nkv;
     for (int round = 0;; ++round) {
-        const int item = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-        if (item >= n_items) break;
-        const int kvh = item % nkv;
-        int idx = n_tile_pairs - 1 - item / nkv, seg = -1, t0 = 0, nt = 0;
-        for (int s = 0; s < x.n_segments; ++s) {
-            const int lo = x.cu_seqlens[s], n = x.cu_seqlens[s + 1] - lo;
-            if (n < x.seg_min_tokens || n > x.seg_max_tokens) continue;   // another kernel serves this segment
-            const int blocks = (n + 2 * tpt - 1) / (2 * tpt);
-            if (idx < blocks) { seg = s; t0 = lo + idx * 2 * tpt; nt = min(2 * tpt, lo + n - t0); break; }
-            idx -= blocks;
+        int kvh, from = 0;
+        bool part = false;
+        Pair pair;
+        if (cut.partial) {
+            if (at >= stretch_end) break;
+            const Place q = place_of(at);
+            const int to = (int)min((long long)q.len, q.off + (stretch_end - at));
+            kvh = q.kvh;
+            at += to - q.off;
+            from = max(0, q.off - CUT_ITEM);
+            part = from > 0 || to < q.len;
+            pair = pair_of(n_tile_pairs - 1 - q.j);
+            pair.k_begin += from * BN;
+            pair.n_tiles = to - CUT_ITEM - from;
+        } else {
+            const int item = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+            if (item >= n_items) break;
+            kvh = item % nkv;
+            pair = pair_of(n_tile_pairs - 1 - item / nkv);
+            if (pair.seg < 0) break;
         }
-        if (seg < 0) break;                                   // the caller counted more tile pairs than there are
+        const int seg = pair.seg, t0 = pair.t0, nt = pair.nt, k_begin = pair.k_begin, n_tiles = pair.n_tiles;
         const int* table = b.block_table + (size_t)seg * b.table_width;
-        // key tiles of the item: from the first key the first token sees to the last token's own
-        const int k_begin = (window_lowest(p.window_kind, p.window_size, b.positions[t0]) / BN) * BN;
-        const int n_tiles = (b.positions[t0 + nt - 1] - k_begin) / BN + 1;
 
         if (warp == 0) {
             if (lane == 0) {
@@ -235,14 +356,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             GroupBarriers& gb = bars.g[g];
             const int tg0 = t0 + g * tpt;
             const int ntg = max(0, min(tpt, nt - g * tpt));
-            // this row tile's own key tiles, [first, last] among the block's; the second tile of a block may hold no token
+            // the key tiles from the first that a row tile's first token sees to its last token's own, [lo, hi] among the block's
+            auto own_tiles = [&](int pos_first, int pos_last, int& lo, int& hi) {
+                lo = max(0, window_lowest(p.window_kind, p.window_size, pos_first) / BN - k_begin / BN);
+                hi = min(n_tiles, pos_last / BN - k_begin / BN + 1) - 1;
+                if (hi < lo) { lo = 0; hi = -1; }
+            };
+            // this row tile's own; the second tile of a block may hold no token, and a part may hold none of a row tile's keys
             int first = 0, last = -1, p_first = 0, lo_last = 0;
             if (ntg > 0) {
                 p_first = b.positions[tg0];
                 const int p_last = b.positions[tg0 + ntg - 1];
                 lo_last = window_lowest(p.window_kind, p.window_size, p_last);
-                first = (window_lowest(p.window_kind, p.window_size, p_first) / BN * BN - k_begin) / BN;
-                last = (p_last - k_begin) / BN;
+                own_tiles(p_first, p_last, first, last);
             }
             const int n_own = last - first + 1;
             // the key tiles that both row tiles own, [shared_lo, shared_hi] among the block's: there the two take
@@ -252,8 +378,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 const int og = g ^ 1, otg0 = t0 + og * tpt, ontg = max(0, min(tpt, nt - og * tpt));
                 if (ontg > 0 && ntg > 0) {
                     const int op_first = b.positions[otg0], op_last = b.positions[otg0 + ontg - 1];
-                    shared_lo = max(first, (window_lowest(p.window_kind, p.window_size, op_first) / BN * BN - k_begin) / BN);
-                    shared_hi = min(last, (op_last - k_begin) / BN);
+                    int olo, ohi;
+                    own_tiles(op_first, op_last, olo, ohi);
+                    shared_lo = max(first, olo);
+                    shared_hi = min(last, ohi);
                 }
             }
             const unsigned tmem_g = tmem + g * GROUP_COLS;
@@ -479,25 +607,28 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&gb.pv_done), (n_own - 1) & 1, abort_flag, err_word, 3, wait_limit));
                 if (ok && n_own > 0) {
                     fence_after();
-                    float shrink = 1.f;
-                    if (p.has_sink) {                              // the sink's score in this kernel's units (powers of two)
-                        const float sink2 = sink_of(p, head) * LOG2E, m2 = fmaxf(m_ref, sink2);
-                        shrink = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m2);
-                        l = l * shrink + exp2f(sink2 - m2);
-                    }
-                    const float inv = shrink * gate_of(p, tok, head) / fmaxf(l, 1e-30f);
+                    const float inv = part ? 0.f : inverse_sum(p, tok, head, m_ref, l);
                     __nv_bfloat16* dst = (__nv_bfloat16*)p.out + out_row_of(p, tok, head) * HD;
+                    float* to = cut.partial + (size_t)(2 * blockIdx.x + (from == 0)) * slot_floats(HD) + g * HD * BM + r;
 #pragma unroll 1
                     for (int c0 = 0; c0 < HD; c0 += 32) {
                         float o[32];
                         ld32(o, lane_base + 2 * BN + c0);          // warp-collective: every lane takes part
                         if (!row_ok) continue;
+                        if (part) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) __stcg(to + (c0 + e) * BM, o[e]);    // a column's rows side by side
+                            continue;
+                        }
 #pragma unroll
                         for (int e = 0; e < 32; e += 8)
                             *(uint4*)(dst + c0 + e) = make_uint4(pack_bf16(o[e] * inv, o[e + 1] * inv), pack_bf16(o[e + 2] * inv, o[e + 3] * inv),
                                                                  pack_bf16(o[e + 4] * inv, o[e + 5] * inv), pack_bf16(o[e + 6] * inv, o[e + 7] * inv));
                     }
                 }
+                if (part)
+                    __stcg((float2*)(cut.partial + (size_t)(2 * blockIdx.x + (from == 0)) * slot_floats(HD) + 2 * HD * BM) + g * BM + r,
+                           make_float2(n_own > 0 ? m_ref : -INFINITY, n_own > 0 ? l : 0.f));
             }
         }
         // end of the item: everything asynchronous has been waited for; renew the barriers
@@ -516,9 +647,67 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
 }
 
+// Adds up the parts of the items that were cut.  grid (cuts, head_dim / JOIN_COLS), a thread a row; part 0 of an item is the last of the
+// block before its first cut, part k the first of the block behind its cut k.
+constexpr int JOIN_COLS = 16;                                 // a thread's elements of a row
+template <int N> struct Count { static constexpr int value = N; };
+__global__ void __launch_bounds__(2 * BM) attn_tc_join_kernel(const AttentionParams p, const Cut cut, int nkv, int tpt, int hd) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int4 item = __ldcg(cut.items + blockIdx.x);
+    if (item.y < 2) return;
+    const int G = p.num_heads / nkv, g = threadIdx.x / BM, r = threadIdx.x % BM, c0 = blockIdx.y * JOIN_COLS;
+    if (r >= min(tpt, item.w - g * tpt) * G) return;
+    const int tok = item.z + g * tpt + r / G, head = (item.x % nkv) * G + r % G;
+    auto slot = [&](int k) { return cut.partial + (2 * (size_t)blockIdx.x + 2 * k - (k ? 2 : 1)) * slot_floats(hd); };
+    float m = -INFINITY, l = 0.f, o[JOIN_COLS];
+#pragma unroll
+    for (int e = 0; e < JOIN_COLS; ++e) o[e] = 0.f;
+    // N parts from part k0 on: their loads are asked for together
+    auto add = [&](auto n, int k0) {
+        constexpr int N = decltype(n)::value;
+        float2 ml[N];
+        float v[N][JOIN_COLS];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const float* from = slot(min(k0 + k, item.y - 1));
+            ml[k] = __ldcg((const float2*)(from + 2 * hd * BM) + threadIdx.x);
+#pragma unroll
+            for (int e = 0; e < JOIN_COLS; ++e) v[k][e] = __ldcg(from + (size_t)(g * hd + c0 + e) * BM + r);
+        }
+        float top = m;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (k0 + k >= item.y) ml[k].x = -INFINITY;
+            top = fmaxf(top, ml[k].x);
+        }
+        const float keep = m == -INFINITY ? 0.f : exp2f(m - top);
+        m = top;
+        l *= keep;
+#pragma unroll
+        for (int e = 0; e < JOIN_COLS; ++e) o[e] *= keep;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (ml[k].x == -INFINITY) continue;               // (a part without a key for this row has left nothing there)
+            const float w = exp2f(ml[k].x - m);
+            l = fmaf(w, ml[k].y, l);
+#pragma unroll
+            for (int e = 0; e < JOIN_COLS; ++e) o[e] = fmaf(w, v[k][e], o[e]);
+        }
+    };
+    if (item.y == 2) add(Count<2>{}, 0);
+    else for (int k0 = 0; k0 < item.y; k0 += 4) add(Count<4>{}, k0);
+    const float inv = inverse_sum(p, tok, head, m, l);
+    __nv_bfloat16* dst = (__nv_bfloat16*)p.out + out_row_of(p, tok, head) * hd + c0;
+#pragma unroll
+    for (int e = 0; e < JOIN_COLS; e += 8)
+        *(uint4*)(dst + e) = make_uint4(pack_bf16(o[e] * inv, o[e + 1] * inv), pack_bf16(o[e + 2] * inv, o[e + 3] * inv),
+                                        pack_bf16(o[e + 4] * inv, o[e + 5] * inv), pack_bf16(o[e + 6] * inv, o[e + 7] * inv));
+}
+
 template <int NKB>
 int launch(const AttentionParams& p, const StepTokens& b, const PagedCache& c, const AttnMmaExtra& x, int n_blocks,
-           int n_sm, cudaStream_t st) {
+           int n_sm, const Cut& cut, cudaStream_t st) {
     const int hd = 64 * NKB, nq = p.num_heads, nkv = c.num_kv_heads, G = nq / nkv;
     const int box_tokens = x.tokens_per_block < b.n_tokens ? x.tokens_per_block : b.n_tokens;
     CUtensorMap mq, mk, mv;
@@ -541,18 +730,16 @@ int launch(const AttentionParams& p, const StepTokens& b, const PagedCache& c, c
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return SPITE_LAUNCH_FAILED;
     const long long items = (long long)n_blocks * nkv;
-    const int grid = (int)(items < n_sm ? items : n_sm);
-    SPITE_LAUNCH(k, grid, THREADS, smem, st, mq, mk, mv, p, b, c, x, box_tokens, n_blocks, s_waits);
+    const int grid = (int)(items < n_sm && !cut.partial ? items : n_sm);
+    SPITE_LAUNCH(k, grid, THREADS, smem, st, mq, mk, mv, p, b, c, x, box_tokens, n_blocks, cut, s_waits);
+    if (cut.partial) SPITE_LAUNCH(attn_tc_join_kernel, dim3(grid, hd / JOIN_COLS), 2 * BM, 0, st, p, cut, nkv, x.tokens_per_block, hd);
     return spite_launch_status();
 }
 
 }  // namespace
 
-// `tokens_per_block`: tokens of one row tile, tokens_per_block * (query heads per kv head) <= 128; a block
-// serves two row tiles.  `n_blocks` = sum over the served segments of ceil(tokens / (2 tokens_per_block)),
-// computed by the caller; `n_sm`: number of multiprocessors (one persistent block each).
-SPITE_API int spite_paged_attention_tc(const AttentionParams* p, const StepTokens* b, const PagedCache* c,
-                                       const AttnMmaExtra* x, int n_blocks, int n_sm, void* stream) {
+static int paged_attention_tc(const AttentionParams* p, const StepTokens* b, const PagedCache* c, const AttnMmaExtra* x, int n_blocks, int n_sm,
+                              const Cut& cut, void* stream) {
     if (n_sm < 1) return SPITE_BAD_ARG;
     if (!p || !b || !c || !x || !p->q || !p->out || !x->cu_seqlens || !c->kv) return SPITE_BAD_ARG;
     if (!b->positions || !b->block_table || b->n_tokens < 0 || b->table_width < 1) return SPITE_BAD_ARG;
@@ -569,5 +756,23 @@ SPITE_API int spite_paged_attention_tc(const AttentionParams* p, const StepToken
     if ((((uintptr_t)p->q | (uintptr_t)p->out | (uintptr_t)c->kv | (uintptr_t)c->key_scale) & 15) || (c->v_offset & 7)) return SPITE_UNSUPPORTED;
     if (b->n_tokens == 0 || n_blocks == 0) return SPITE_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    return c->head_dim == 64 ? launch<1>(*p, *b, *c, *x, n_blocks, n_sm, st) : launch<2>(*p, *b, *c, *x, n_blocks, n_sm, st);
+    return c->head_dim == 64 ? launch<1>(*p, *b, *c, *x, n_blocks, n_sm, cut, st) : launch<2>(*p, *b, *c, *x, n_blocks, n_sm, cut, st);
+}
+
+// `tokens_per_block`: tokens of one row tile, tokens_per_block * (query heads per kv head) <= 128; a block
+// serves two row tiles.  `n_blocks` = sum over the served segments of ceil(tokens / (2 tokens_per_block)),
+// computed by the caller; `n_sm`: number of multiprocessors (one persistent block each).
+SPITE_API int spite_paged_attention_tc(const AttentionParams* p, const StepTokens* b, const PagedCache* c,
+                                       const AttnMmaExtra* x, int n_blocks, int n_sm, void* stream) {
+    return paged_attention_tc(p, b, c, x, n_blocks, n_sm, Cut{nullptr, nullptr}, stream);
+}
+
+// The same with the work cut along the keys into n_sm equal shares, and a second kernel that adds the parts up.  `scratch`: n_sm * (4 * (head_dim +
+// 2) * 128 + 4) floats.
+SPITE_API int spite_paged_attention_tc_cut(const AttentionParams* p, const StepTokens* b, const PagedCache* c,
+                                           const AttnMmaExtra* x, int n_blocks, int n_sm, float* scratch, long long n_floats, void* stream) {
+    if (!scratch || n_sm < 1 || !c || c->head_dim < 1) return SPITE_BAD_ARG;
+    const long long slots = 2ll * n_sm * (long long)slot_floats(c->head_dim);
+    if (n_blocks > CUT_PAIRS || ((uintptr_t)scratch & 15) || slots + 4ll * n_sm > n_floats) return SPITE_UNSUPPORTED;
+    return paged_attention_tc(p, b, c, x, n_blocks, n_sm, Cut{scratch, (int4*)(scratch + slots)}, stream);
 }

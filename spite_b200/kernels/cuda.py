@@ -235,6 +235,42 @@ def stream_cut(M: int, N: int, K: int, groups: int, swiglu: bool, slots: int, sm
     return best
 
 
+def attention_cut_pays(segments, window, pair_tokens: int, kv_heads: int, blocks: int) -> bool:
+    """Whether the prompt portions (first position, tokens) of a step are faster on the tcgen05 attention kernel with its work cut along the keys
+    into equal shares than with whole items (a pair of row tiles, `pair_tokens` tokens, and a kv head) dealt out round by round.
+
+    Both are estimated in tiles of 64 keys (1.2 us).  An item costs its tiles and 6 more; items are dealt out from the last portion's end backwards,
+    one a block and round, in alternating direction, and the longest of five blocks' sums counts; a share costs its part of all that and
+    24 for the parts that begin and end in it (another start 6, their outputs 3, the line that is cut 3) and for adding the parts up behind
+    them (6 to 12).  us, whole / cut, 40 heads, 8 kv heads of 128: 2,048 tokens behind 6,144 410 / 350, 1,000 behind 7,192 287 / 199, 500 behind
+    7,692 163 / 112, 100 behind 8,092 160 / 41, 50 behind 8,142 158 / 37, three portions of 683 behind 7,500 470 / 390; 2,048 from the start 75 / 92,
+    1,048 behind 1,000 64 / 75, 500 behind 500 31 / 40.  Of 80 shapes (four kinds of heads) the rule takes the slower one twice, by 0 and 7 %."""
+    runs, items, tiles = [], 0, 0.0                          # (items up to the run's end, tiles of its first, of its last)
+    for start, n in reversed(segments):
+        pairs, end, near = -(-n // pair_tokens), start + n - 1, start + min(n, pair_tokens) - 1
+        longest = (end - window.lowest_visible(max(start, end - pair_tokens + 1))) / 64 + 1
+        shortest = (near - window.lowest_visible(start)) / 64 + 1
+        items += pairs * kv_heads
+        tiles += pairs * kv_heads * (longest + shortest) / 2
+        runs.append((items, longest, shortest))
+    if items <= blocks:
+        whole = 6 + max((max(a, b) for _, a, b in runs), default=0.0)
+    else:
+        sums = [0.0] * 5
+        for round_, first in enumerate(range(0, items, blocks)):
+            run, begin = 0, 0
+            for i in range(5):
+                at = first + (blocks - 1) * i // 4
+                if at >= items:
+                    break
+                while at >= runs[run][0]:
+                    run, begin = run + 1, runs[run][0]
+                end, longest, shortest = runs[run]
+                sums[4 - i if round_ & 1 else i] += 6 + longest - (longest - shortest) * (at - begin) / (end - begin)
+        whole = max(sums)
+    return max(8.0, (tiles + 6 * items) / blocks) + 24 < whole
+
+
 class CudaKernels(KernelSet):
     def __init__(self, dtype: torch.dtype, device="cuda:0"):
         if dtype not in _DT:
@@ -1064,9 +1100,19 @@ class CudaKernels(KernelSet):
                 x = AttnMmaExtra(cu_seqlens=batch.cu_seqlens.data_ptr(), o_part=None, ml_part=None,
                                  n_segments=len(batch.segments), tokens_per_block=tpb_tc, n_splits=1,
                                  seg_min_tokens=tc_from, seg_max_tokens=0x7fffffff)
-                st = self._lib("attention_tc").spite_paged_attention_tc(
-                    C.byref(p), C.byref(b), C.byref(c), C.byref(x), n_tc, self.sm_count, self._stream())
-                self._count("attention_tc", 1)
+                lib, st, cut = self._lib("attention_tc"), -2, False
+                if attention_cut_pays([(s.start_pos, s.n_tokens) for s in batch.segments if s.n_tokens >= tc_from], window, 2 * tpb_tc,
+                                      c.num_kv_heads, self.sm_count):
+                    n_floats = self.sm_count * (4 * (c.head_dim + 2) * 128 + 4)
+                    part = torch.empty(n_floats, dtype=torch.float32, device=q.device)
+                    self.attention_scratch_bytes = n_floats * 4
+                    st = lib.spite_paged_attention_tc_cut(
+                        C.byref(p), C.byref(b), C.byref(c), C.byref(x), n_tc, self.sm_count, C.c_void_p(part.data_ptr()), C.c_longlong(n_floats),
+                        self._stream())
+                    cut = st == 0
+                if st == -2:
+                    st = lib.spite_paged_attention_tc(C.byref(p), C.byref(b), C.byref(c), C.byref(x), n_tc, self.sm_count, self._stream())
+                self._count("attention_tc", 1 + cut)
                 _check(st, "paged_attention (tcgen05, prompt portions)")
             if n_big:
                 x = AttnMmaExtra(cu_seqlens=batch.cu_seqlens.data_ptr(), o_part=None, ml_part=None,
