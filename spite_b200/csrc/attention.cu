@@ -196,6 +196,145 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(const QkPrepareParams p
     }
 }
 
+template <int N> struct Int { static constexpr int value = N; };
+
+// The same for bfloat16 heads of 64 or 128 elements in rows that 16-byte words divide, without what few layers ask for (blended or rotated
+// values, keys that are the values): a lane holds eight neighbouring elements of a head, HD / 8 lanes a head, so a warp works on two or four
+// heads at a time, and a thread asks for its part of ITER heads before anything else: the angles and the way to the page (three
+// loads in a row) follow under them.  grid (tokens, ceil(heads / (256 / (HD / 8) * ITER))).
+// What bounds it is that chain of loads (58 MB at 2,048 tokens are 9 us).  In a layer, us: 2,048 tokens of 56 heads of 128 54 -> 20, 8 tokens
+// 5.3 -> 3.0.
+template <int HD, bool HALVES, int ITER>
+__global__ void __launch_bounds__(256) qk_prepare_vec_kernel(const QkPrepareParams p, const StepTokens b, const PagedCache c) {
+    constexpr int LANES = HD / 8, SLOTS = 256 / LANES, ANGLES = HALVES ? 8 : 4;      // lanes a head, heads at a time, angles a lane needs
+    pdl_wait();
+    pdl_launch_dependents();
+    const int t = blockIdx.x, l = threadIdx.x % LANES;
+    const int nq = p.num_heads, nkv = c.num_kv_heads;
+    const int heads_total = p.q_only ? nq : nq + 2 * nkv;
+    const int head0 = blockIdx.y * SLOTS * ITER + threadIdx.x / LANES;
+    const __nv_bfloat16* row = (const __nv_bfloat16*)p.qkv + (size_t)t * p.qkv_stride;
+    uint4 raw[ITER];
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) {
+        const int head = head0 + it * SLOTS;
+        raw[it] = head < heads_total ? *(const uint4*)(row + (size_t)head * HD + 8 * l) : make_uint4(0, 0, 0, 0);
+    }
+    const int pos = b.positions[t];
+    int page = -1;
+    if (p.write_cache && !p.q_only) {
+        const int at = pos / c.page_size;
+        page = b.block_table[(size_t)b.seg_of_token[t] * b.table_width + at];
+        if (page >= c.n_pages) page = -1;                     // the host never lets this happen
+        // copies of a captured step's first row append nothing (see qk_prepare_kernel)
+        if (t > 0 && pos == b.positions[0] && page == b.block_table[(size_t)b.seg_of_token[0] * b.table_width + at]) page = -1;
+    }
+    const int rot = p.inv_freq ? p.rotary_dim : 0;
+    __shared__ __align__(16) float cs_s[HD / 2], sn_s[HD / 2];
+    for (int i = threadIdx.x; 2 * i < rot; i += 256) {
+        turn_of((float)pos, p.inv_freq, p.inv_freq_low, i, cs_s[i], sn_s[i]);
+        sn_s[i] *= p.rot_amplitude; cs_s[i] *= p.rot_amplitude;
+    }
+    if (p.gates_out && blockIdx.y == 0)                      // the gate columns behind the heads
+        for (int h = threadIdx.x; h < nq; h += 256)
+            p.gates_out[(size_t)t * nq + h] = 1.0f / (1.0f + expf(-__bfloat162float(row[(size_t)heads_total * HD + h])));
+    float temp = 1.f;
+    if (p.temperature_floor > 0) temp = logf((float)((pos + 1) / p.temperature_floor) + 1.0f) * p.temperature_scale + 1.0f;
+    __syncthreads();
+    // the lane's angles: of its four pairs of neighbours, or of its eight elements, whose partners are another lane's
+    float cs[ANGLES], sn[ANGLES];
+    const bool turns = 8 * l < rot;                           // (halves: a lane's elements rotate together; neighbours: see below)
+    const bool upper = HALVES && 16 * l >= rot;               // of the two halves
+    const int partner = !turns ? l : upper ? l - rot / 16 : l + rot / 16;
+#pragma unroll
+    for (int j = 0; j < ANGLES; ++j) {
+        const int i = HALVES ? 8 * l + j - (upper ? rot / 2 : 0) : 4 * l + j;
+        const bool yes = HALVES ? turns : 2 * i < rot;
+        cs[j] = yes ? cs_s[i] : 1.f;
+        sn[j] = yes ? sn_s[i] : 0.f;
+    }
+    const bool norm = p.qk_norm_eps > 0.f;
+    const bool norm_first = norm && p.norm_before_rotation;
+    const float norm_n = (float)(p.norm_dim > 0 ? p.norm_dim : HD);
+    auto head_sum = [&](const float (&x)[8]) {
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss = fmaf(x[j], x[j], ss);
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        return ss;
+    };
+    auto multiply = [&](float (&x)[8], const float* by) {
+        const float4 u = *(const float4*)by, v = *(const float4*)(by + 4);
+        x[0] *= u.x; x[1] *= u.y; x[2] *= u.z; x[3] *= u.w;
+        x[4] *= v.x; x[5] *= v.y; x[6] *= v.z; x[7] *= v.w;
+    };
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) {
+        const int head = head0 + it * SLOTS;
+        const bool is_q = head < nq, is_v = head >= nq + nkv;
+        float x[8];
+        {
+            const unsigned w[4] = {raw[it].x, raw[it].y, raw[it].z, raw[it].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { x[2 * j] = __uint_as_float(w[j] << 16); x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
+        }
+        if (p.bias && head < heads_total) {
+            const float4 u = *(const float4*)(p.bias + (size_t)head * HD + 8 * l), v = *(const float4*)(p.bias + (size_t)head * HD + 8 * l + 4);
+            x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
+            x[4] += v.x; x[5] += v.y; x[6] += v.z; x[7] += v.w;
+        }
+        if (!__all_sync(0xffffffffu, is_v)) {                 // (the lanes of a head, and the heads of a warp, go through the sums together)
+            const float* gain = is_q ? p.q_gain : p.k_gain;
+            float y[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) y[j] = x[j];
+            if (norm_first) {
+                const float mul = 1.0f / sqrtf(head_sum(y) / norm_n + p.qk_norm_eps);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] *= mul;
+                if (gain) multiply(y, gain + 8 * l);
+            }
+            if constexpr (HALVES) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float other = __shfl_sync(0xffffffffu, y[j], partner, LANES);
+                    if (turns) y[j] = upper ? other * sn[j] + y[j] * cs[j] : y[j] * cs[j] - other * sn[j];
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (2 * (4 * l + j) < rot) {
+                        const float ra = y[2 * j] * cs[j] - y[2 * j + 1] * sn[j], rb = y[2 * j] * sn[j] + y[2 * j + 1] * cs[j];
+                        y[2 * j] = ra; y[2 * j + 1] = rb;
+                    }
+            }
+            float mul = 1.f;
+            if (norm && !norm_first) mul = 1.0f / sqrtf(head_sum(y) / norm_n + p.qk_norm_eps);
+            if (is_q) mul *= temp;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) y[j] *= mul;
+            if (gain && norm && !norm_first) multiply(y, gain + 8 * l);
+            if (!is_v)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = y[j];
+        }
+        if (head >= heads_total || (!is_q && page < 0)) continue;        // nothing to append (or no page)
+        __nv_bfloat16* dst;
+        if (is_q) dst = (__nv_bfloat16*)p.q_out + ((size_t)t * nq + head) * HD;
+        else
+            dst = (__nv_bfloat16*)c.kv + (is_v ? c.v_offset : 0) +
+                  (((size_t)page * nkv + (is_v ? head - nq - nkv : head - nq)) * c.page_size + pos % c.page_size) * HD;
+        unsigned w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat162 two = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+            w[j] = *(const unsigned*)&two;
+        }
+        *(uint4*)(dst + 8 * l) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 // out[t, h * size + e] = scale * x[t, h, e] for e < size, the pairs of the first `rot` elements turned back by the
 // token's position: the pair (u, v) becomes (u cos a + v sin a, v cos a - u sin a), a = pos * inv_freq[i].  x has rows of
 // heads * head_dim elements, out rows of out_stride.  grid (tokens, head chunks): a block computes the angles once.
@@ -357,6 +496,21 @@ SPITE_API int spite_qk_prepare(int dtype, const QkPrepareParams* given, const St
     cudaStream_t st = (cudaStream_t)stream;
     const bool halves = p->pairing == SPITE_PAIR_HALVES && p->inv_freq;
     if (dtype != SPITE_DT_F32 && dtype != SPITE_DT_BF16) return SPITE_BAD_ARG;
+    const uintptr_t words = (uintptr_t)p->qkv | (uintptr_t)p->q_out | (uintptr_t)c->kv | (uintptr_t)p->bias | (uintptr_t)p->q_gain | (uintptr_t)p->k_gain;
+    if (dtype == SPITE_DT_BF16 && (c->head_dim == 64 || c->head_dim == 128) && (words & 15) == 0 && p->qkv_stride % 8 == 0 && c->v_offset % 8 == 0 &&
+        !p->v_other && !p->v_inv_freq && !p->values_are_keys && (!halves || p->rotary_dim % 16 == 0)) {
+        // a block per token where there are enough of them to fill the device, else a block for as many heads as it works on at a time
+        const bool all = b->n_tokens >= 256;
+        const int at_once = 256 / (c->head_dim / 8) * (all ? 4 : 1);
+        const dim3 blocks(b->n_tokens, (heads + at_once - 1) / at_once);
+        auto launch = [&](auto hd, auto pairs, auto iter) {
+            SPITE_LAUNCH((qk_prepare_vec_kernel<decltype(hd)::value, decltype(pairs)::value, decltype(iter)::value>), blocks, 256, 0, st, *p, *b, *c);
+        };
+        auto by_iter = [&](auto hd, auto pairs) { if (all) launch(hd, pairs, Int<4>{}); else launch(hd, pairs, Int<1>{}); };
+        auto by_pairs = [&](auto hd) { if (halves) by_iter(hd, Int<1>{}); else by_iter(hd, Int<0>{}); };
+        if (c->head_dim == 64) by_pairs(Int<64>{}); else by_pairs(Int<128>{});
+        return spite_launch_status();
+    }
     if (dtype == SPITE_DT_F32) {
         if (halves) SPITE_LAUNCH((qk_prepare_kernel<float, true>), grid, threads, 0, st, *p, *b, *c, heads_per_block);
         else SPITE_LAUNCH((qk_prepare_kernel<float, false>), grid, threads, 0, st, *p, *b, *c, heads_per_block);
