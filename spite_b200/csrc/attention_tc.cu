@@ -89,6 +89,7 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
 }
+template <int N> struct Count { static constexpr int value = N; };
 typedef unsigned long long f2;                            // two packed floats
 __device__ __forceinline__ f2 pack2(float lo, float hi) {
     f2 v;
@@ -105,6 +106,32 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
     f2 v;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
     return v;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+// 2^x for two numbers on the multiply-add units, x at least -126 (smaller ones give 2^-126): x = n + f with n whole and |f| <= 1/2, a
+// polynomial of degree 5 for 2^f (least worst relative error over [-1/2, 1/2], fitted by Lawson's iteration: 7.5e-8, 2.1e-7 with the
+// roundings, as much as the special-function unit's), and n added to its exponent.
+__device__ __forceinline__ void ex2_pair(f2 x, float& a, float& b) {
+    auto both = [](float v) { return pack2(v, v); };
+    float xa, xb;
+    unpack2(x, xa, xb);
+    x = pack2(fmaxf(xa, -126.f), fmaxf(xb, -126.f));
+    const f2 n = add2(x, both(12582912.f));                // 1.5 * 2^23: n stands in the low bits
+    const f2 f = fma2(add2(n, both(-12582912.f)), both(-1.f), x);
+    f2 p = fma2(both(0.00132764445f), f, both(0.00967553724f));
+    p = fma2(p, f, both(0.0555071346f));
+    p = fma2(p, f, both(0.240221202f));
+    p = fma2(p, f, both(0.693146944f));
+    p = fma2(p, f, both(1.00000012f));
+    float pa, pb, na, nb;
+    unpack2(p, pa, pb);
+    unpack2(n, na, nb);
+    a = __int_as_float(__float_as_int(pa) + (__float_as_int(na) << 23));
+    b = __int_as_float(__float_as_int(pb) + (__float_as_int(nb) << 23));
 }
 __device__ __forceinline__ unsigned pack_bf16(float a, float b) {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
@@ -568,17 +595,38 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.g[g ^ 1].exp_done), before & 1, abort_flag, err_word, 3, wait_limit));
                         if (!ok) break;
                     }
+                    // Three of sixteen pairs go through the multiply-add units instead (not on a window's edge or the diagonal, where a
+                    // masked key must get 0), and the turn is passed on a quarter before the end, so that the other row tile's first
+                    // exponentials follow the last ones here.  us, 2,048 tokens behind 6,144, 40 heads: 343; turn passed early 336;
+                    // one pair in 4 317; both 310; 3 in 16 307; one pair in 2, 3 328, 327; without turns 324.
                     unsigned packed[BN / 2];
-                    float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+                    f2 sum2[4] = {0ull, 0ull, 0ull, 0ull};
+                    const f2 scale2 = pack2(scale, scale), neg_m2 = pack2(neg_m, neg_m);
+                    auto weights = [&](auto mixed) {
 #pragma unroll
-                    for (int e = 0; e < BN; e += 2) {
-                        const float a = ex2(fmaf(s[e], scale, neg_m)), bb = ex2(fmaf(s[e + 1], scale, neg_m));
-                        sum4[(e >> 1) & 3] += a + bb;
-                        packed[e / 2] = pack_bf16(a, bb);
-                    }
-                    __syncwarp();
-                    if (takes_turns && lane == 0) mbar_arrive(smem_u32(&gb.exp_done));
-                    const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+                        for (int e = 0; e < BN; e += 2) {
+                            if (e == BN * 3 / 4) {
+                                __syncwarp();
+                                if (takes_turns && lane == 0) mbar_arrive(smem_u32(&gb.exp_done));
+                            }
+                            const f2 x = fma2(pack2(s[e], s[e + 1]), scale2, neg_m2);
+                            float a, bb;
+                            if (decltype(mixed)::value && ((e / 2) % 16 == 3 || (e / 2) % 16 == 8 || (e / 2) % 16 == 13)) {
+                                ex2_pair(x, a, bb);
+                            } else {
+                                unpack2(x, a, bb);
+                                a = ex2(a);
+                                bb = ex2(bb);
+                            }
+                            sum2[(e >> 1) & 3] = add2(sum2[(e >> 1) & 3], pack2(a, bb));
+                            packed[e / 2] = pack_bf16(a, bb);
+                        }
+                    };
+                    if (open) weights(Count<1>{}); else weights(Count<0>{});
+                    const f2 sums = add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3]));
+                    float sum_a, sum_b;
+                    unpack2(sums, sum_a, sum_b);
+                    const float sum = sum_a + sum_b;
                     l += sum;
                     if (li > 0) {
                         // The product of the tile before must have left O before its rows are rescaled.  The wait is
@@ -650,7 +698,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 // Adds up the parts of the items that were cut.  grid (cuts, head_dim / JOIN_COLS), a thread a row; part 0 of an item is the last of the
 // block before its first cut, part k the first of the block behind its cut k.
 constexpr int JOIN_COLS = 16;                                 // a thread's elements of a row
-template <int N> struct Count { static constexpr int value = N; };
 __global__ void __launch_bounds__(2 * BM) attn_tc_join_kernel(const AttentionParams p, const Cut cut, int nkv, int tpt, int hd) {
     pdl_wait();
     pdl_launch_dependents();

@@ -239,12 +239,12 @@ def attention_cut_pays(segments, window, pair_tokens: int, kv_heads: int, blocks
     """Whether the prompt portions (first position, tokens) of a step are faster on the tcgen05 attention kernel with its work cut along the keys
     into equal shares than with whole items (a pair of row tiles, `pair_tokens` tokens, and a kv head) dealt out round by round.
 
-    Both are estimated in tiles of 64 keys (1.2 us).  An item costs its tiles and 6 more; items are dealt out from the last portion's end backwards,
+    Both are estimated in tiles of 64 keys (1.1 us).  An item costs its tiles and 6 more; items are dealt out from the last portion's end backwards,
     one a block and round, in alternating direction, and the longest of five blocks' sums counts; a share costs its part of all that and
     24 for the parts that begin and end in it (another start 6, their outputs 3, the line that is cut 3) and for adding the parts up behind
-    them (6 to 12).  us, whole / cut, 40 heads, 8 kv heads of 128: 2,048 tokens behind 6,144 410 / 350, 1,000 behind 7,192 287 / 199, 500 behind
-    7,692 163 / 112, 100 behind 8,092 160 / 41, 50 behind 8,142 158 / 37, three portions of 683 behind 7,500 470 / 390; 2,048 from the start 75 / 92,
-    1,048 behind 1,000 64 / 75, 500 behind 500 31 / 40.  Of 80 shapes (four kinds of heads) the rule takes the slower one twice, by 0 and 7 %."""
+    them (6 to 12).  us, whole / cut, 40 heads, 8 kv heads of 128: 2,048 tokens behind 6,144 361 / 306, 1,000 behind 7,192 254 / 173, 500 behind
+    7,692 142 / 100, 100 behind 8,092 141 / 39, 50 behind 8,142 140 / 36, three portions of 683 behind 7,500 410 / 344; 2,048 from the start 70 / 87,
+    1,048 behind 1,000 60 / 67, 500 behind 500 27 / 35.  Of 80 shapes (four kinds of heads) the rule takes the slower one three times, by 0, 1 and 8 %."""
     runs, items, tiles = [], 0, 0.0                          # (items up to the run's end, tiles of its first, of its last)
     for start, n in reversed(segments):
         pairs, end, near = -(-n // pair_tokens), start + n - 1, start + min(n, pair_tokens) - 1
