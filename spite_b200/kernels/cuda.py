@@ -128,7 +128,7 @@ class MlstmParams(C.Structure):
                 ("i_bias", C.c_void_p), ("f_bias", C.c_void_p), ("out", C.c_void_p), ("state", C.c_void_p),
                 ("head_stride", C.c_longlong), ("cu_seqlens", C.c_void_p), ("slots", C.c_void_p),
                 ("n_segments", C.c_int), ("heads", C.c_int), ("dim", C.c_int), ("vdim", C.c_int),
-                ("gate_cap", C.c_float), ("q_scale", C.c_float), ("chunked", C.c_int), ("n_long", C.c_int)]
+                ("gate_cap", C.c_float), ("q_scale", C.c_float), ("chunked", C.c_int), ("n_long", C.c_int), ("one_token", C.c_int)]
 
 
 class AttnMmaExtra(C.Structure):
@@ -1260,7 +1260,9 @@ class CudaKernels(KernelSet):
                         f_col=f_col, i_bias=i_bias.data_ptr(), f_bias=f_bias.data_ptr(), out=out.data_ptr(),
                         state=state.data_ptr(), head_stride=state.shape[2], cu_seqlens=batch.cu_seqlens.data_ptr(),
                         slots=batch.slots.data_ptr(), n_segments=n_seg, heads=int(heads), dim=int(dim), vdim=int(vdim),
-                        gate_cap=float(gate_cap), q_scale=float(q_scale), chunked=int(bool(chunked)))
+                        gate_cap=float(gate_cap), q_scale=float(q_scale), chunked=int(bool(chunked)),
+                        # (the float32 set adds a token's sums as the walk over a prompt does, however the tokens were cut)
+                        one_token=int(self.dtype == torch.bfloat16 and batch.max_seg_len == 1 and n_seg == M))
         if chunked:
             p.n_long, n_chunks = self._long_segments(batch, self.memory_min_tokens)
             scratch = self._chunk_scratch("recurrent", "spite_mlstm_tiles_bytes", dim, vdim, heads, n_chunks, n_seg)
