@@ -783,24 +783,43 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvParams p
 
 // The same for segments of several tokens whose columns are whole groups of four: a thread has four columns and CONV_ROWS tokens, all of
 // whose inputs it asks for before it uses the first (the kernel above has one load of four bytes in flight a thread, which left it at a
-// third of the copy bandwidth).  The sums are the same, term by term.  8,448 channels of 4 taps, 2,048 tokens: 75 us above, 47 us here;
-// eight prompts of 2,048 tokens: 530 and 307 us.
+// third of the copy bandwidth).  The sums are the same, term by term.  The weights are asked for before the wait for the kernel in front,
+// and seven blocks fit a multiprocessor: what is left is a round trip to memory and the gate's exponential and division, block after block.
+// 8,448 channels of 4 taps, 2,048 tokens (138 MB: 21 us): 75 us above, 37 here (47 with the weights behind the inputs and 96 registers;
+// 42 with the weights in front, 38 with six blocks, 40 with eight; 4, 12, 16 tokens a thread 43, 40, 40).
 constexpr int CONV_ROWS = 8;
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) short_conv_rows_kernel(const ShortConvParams p) {
+__global__ void __launch_bounds__(128, 7) short_conv_rows_kernel(const ShortConvParams p) {
+    const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool conv = c < p.channels;
+    float w[4][TAPS];                                         // (weights: no kernel of the step writes them)
+    float4 bias = zero;
+    if (conv) {
+        if (TAPS % 4 == 0 && (((uintptr_t)p.w) & 15) == 0) {  // (the taps of four channels lie side by side)
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const float4 v = *(const float4*)(p.w + (size_t)c * TAPS + 4 * j);
+                w[(4 * j) / TAPS][(4 * j) % TAPS] = v.x; w[(4 * j + 1) / TAPS][(4 * j + 1) % TAPS] = v.y;
+                w[(4 * j + 2) / TAPS][(4 * j + 2) % TAPS] = v.z; w[(4 * j + 3) / TAPS][(4 * j + 3) % TAPS] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) w[e][j] = p.w[(size_t)(c + e) * TAPS + j];
+        }
+        if (p.bias) bias = make_float4(p.bias[c], p.bias[c + 1], p.bias[c + 2], p.bias[c + 3]);
+    }
     pdl_wait();
     pdl_launch_dependents();
-    const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (c >= p.channels + p.copy_columns) return;
-    const int s = blockIdx.y, t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0, i0 = blockIdx.z * CONV_ROWS;
+    const int s = blockIdx.y, t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0, i0 = blockIdx.z * CONV_ROWS, slot = p.slots[s], slot0 = p.slots[0];
     if (i0 >= n) return;
-    const int slot = p.slots[s];
-    if (s > 0 && slot == p.slots[0]) return;                  // (the first row's thread writes its copies, as above)
+    if (s > 0 && slot == slot0) return;                       // (the first row's thread writes its copies, as above)
     const int rows = min(CONV_ROWS, n - i0);
     const float* x = p.x + (size_t)(t0 + i0) * p.x_stride + c;
     T* out = (T*)p.out + (size_t)(t0 + i0) * p.out_stride + c;
-    const bool conv = c < p.channels;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 in[TAPS - 1 + CONV_ROWS];                          // in[TAPS - 1 + i]: token i0 + i
     float* st = p.state + (size_t)slot * p.slot_stride + c;
     float4 old[TAPS > 1 ? TAPS - 1 : 1];
@@ -816,12 +835,6 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(const ShortConvPar
         for (int i = 0; i < CONV_ROWS; ++i)
             if (i < rows) store4(out + (size_t)i * p.out_stride, in[TAPS - 1 + i].x, in[TAPS - 1 + i].y, in[TAPS - 1 + i].z, in[TAPS - 1 + i].w);
     } else {
-        float w[4][TAPS];
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int j = 0; j < TAPS; ++j) w[e][j] = p.w[(size_t)(c + e) * TAPS + j];
-        const float4 bias = p.bias ? make_float4(p.bias[c], p.bias[c + 1], p.bias[c + 2], p.bias[c + 3]) : zero;
 #pragma unroll
         for (int i = 0; i < CONV_ROWS; ++i) {
             if (i >= rows) break;
