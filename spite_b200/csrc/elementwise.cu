@@ -111,19 +111,40 @@ __global__ void pack_pair_vec_kernel(float* __restrict__ a, const float* __restr
 
 // y[i, :] = x[r, :] * rsqrt(mean(x[r]^2) + eps) * gain      r = rows ? rows[i] : i
 // (crates/spite-models/src/dense.rs:175-181; the sum runs in float32)
+// The sum of block_sum, bit by bit, with one barrier instead of three: every warp adds up the warps' sums.  `scratch`: 32 floats that
+// nothing else uses in the kernel.
+__device__ __forceinline__ float block_sum_once(float v, float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v = warp_sum(v);
+    if (lane == 0) scratch[warp] = v;
+    __syncthreads();
+    return warp_sum(lane < (int)((blockDim.x + 31) >> 5) ? scratch[lane] : 0.f);
+}
+// The thread's part of a gain vector, asked for before the wait for the kernel in front (no kernel of a step writes gains): behind a norm's
+// sum it was another round trip to memory.
+template <int VPT>
+__device__ __forceinline__ void load_gain(float4 (&g)[VPT], const float* gain, int d4) {
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        g[k] = gain && c < d4 ? ((const float4*)gain)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
 // One block per row.  The row stays in registers between the sum and the scaling: every thread
 // holds up to VPT groups of four elements, loaded with one 16-byte read each.
 template <typename T, int VPT>
 __global__ void rms_norm_vec_kernel(const float* __restrict__ x, const float* __restrict__ gain,
                                     const int* __restrict__ rows, T* __restrict__ y, int d, float eps) {
+    __shared__ float scratch[32];
+    const int d4 = d >> 2;
+    float4 v[VPT], g[VPT];
+    load_gain(g, gain, d4);
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ float scratch[33];
     const int i = blockIdx.x;
     const int r = rows ? rows[i] : i;
     const float4* in = (const float4*)(x + (size_t)r * d);
-    const int d4 = d >> 2;
-    float4 v[VPT];
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
@@ -132,16 +153,13 @@ __global__ void rms_norm_vec_kernel(const float* __restrict__ x, const float* __
     }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) s += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-    s = block_sum(s, scratch);
+    s = block_sum_once(s, scratch);
     const float scale = 1.0f / sqrtf(s / (float)d + eps);
     T* out = y + (size_t)i * d;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
-        if (c < d4) {
-            const float4 g = ((const float4*)gain)[c];
-            store4(out + 4 * c, v[k].x * scale * g.x, v[k].y * scale * g.y, v[k].z * scale * g.z, v[k].w * scale * g.w);
-        }
+        if (c < d4) store4(out + 4 * c, v[k].x * scale * g[k].x, v[k].y * scale * g[k].y, v[k].z * scale * g[k].z, v[k].w * scale * g[k].w);
     }
 }
 
@@ -350,14 +368,16 @@ template <typename T, int VPT>
 __global__ void rms_norm_residual_vec_kernel(const float* __restrict__ y, const float* __restrict__ gain, float* __restrict__ h,
                                              const float* __restrict__ next_gain, T* __restrict__ next_out, int d, float eps,
                                              float mult) {
+    __shared__ float scratch[2][32];
+    const int d4 = d >> 2;
+    float4 v[VPT], r[VPT], g[VPT], ng[VPT];
+    load_gain(g, gain, d4);
+    load_gain(ng, next_gain, d4);
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ float scratch[33];
     const size_t m = blockIdx.x;
     const float4* in = (const float4*)(y + m * d);
     float4* hr = (float4*)(h + m * d);
-    const int d4 = d >> 2;
-    float4 v[VPT], r[VPT];
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
@@ -367,16 +387,15 @@ __global__ void rms_norm_residual_vec_kernel(const float* __restrict__ y, const 
     }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) s += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-    s = block_sum(s, scratch);
+    s = block_sum_once(s, scratch[0]);
     const float scale = 1.0f / sqrtf(s / (float)d + eps);
     float s2 = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
         if (c < d4) {
-            const float4 g = ((const float4*)gain)[c];
-            r[k].x += mult * (v[k].x * scale * g.x); r[k].y += mult * (v[k].y * scale * g.y);
-            r[k].z += mult * (v[k].z * scale * g.z); r[k].w += mult * (v[k].w * scale * g.w);
+            r[k].x += mult * (v[k].x * scale * g[k].x); r[k].y += mult * (v[k].y * scale * g[k].y);
+            r[k].z += mult * (v[k].z * scale * g[k].z); r[k].w += mult * (v[k].w * scale * g[k].w);
             hr[c] = r[k];
             s2 += (r[k].x * r[k].x + r[k].y * r[k].y) + (r[k].z * r[k].z + r[k].w * r[k].w);
         }
@@ -391,15 +410,12 @@ __global__ void rms_norm_residual_vec_kernel(const float* __restrict__ y, const 
         }
         return;
     }
-    s2 = block_sum(s2, scratch);
+    s2 = block_sum_once(s2, scratch[1]);
     const float scale2 = 1.0f / sqrtf(s2 / (float)d + eps);
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
-        if (c < d4) {
-            const float4 g = ((const float4*)next_gain)[c];
-            store4(out + 4 * c, r[k].x * scale2 * g.x, r[k].y * scale2 * g.y, r[k].z * scale2 * g.z, r[k].w * scale2 * g.w);
-        }
+        if (c < d4) store4(out + 4 * c, r[k].x * scale2 * ng[k].x, r[k].y * scale2 * ng[k].y, r[k].z * scale2 * ng[k].z, r[k].w * scale2 * ng[k].w);
     }
 }
 
