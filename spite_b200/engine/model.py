@@ -52,6 +52,9 @@ class Model:
         self.embed_table = None
         self.head_weight = None
         self.position_table = None
+        self._logit_scales = None
+        if plan.logit_scale != 1.0 and plan.logit_softcap is None:
+            self._logit_scales = torch.full((4096,), plan.logit_scale, dtype=torch.float32, device=self.device)
         self._ones = None if plan.streams is None else torch.ones(plan.streams, dtype=torch.float32, device=self.device)
         #: if set, called as `layer_tap(i, h)` after the i-th layer run of the order with the float32 residual
         #: stream (the sum of the streams, if there are several; for comparing a model layer by layer; the step then cannot be captured in a graph)
@@ -214,12 +217,22 @@ class Model:
         if self.junctions:                       # the embedding's output, which the junctions mix back in
             h0 = torch.empty_like(h)
             h0.copy_(h)
-        runs = 0
-        for call in p.order:
+        runs, entered = 0, None
+        for i, call in enumerate(p.order):
             if isinstance(call, JunctionCall):
                 self.junctions[call.junction].forward(h, h0, batch, call.step)
                 continue
-            self.blocks[call.layer].forward(h, batch, storage.layer_cache(call.cache, call.write_cache))
+            # what the next layer begins with is made by this one's last kernel where both know how (a tap may change the stream between)
+            block, after, more = self.blocks[call.layer], p.order[i + 1] if i + 1 < len(p.order) else None, {}
+            if entered is not None:
+                more["entered"] = entered
+            entered = None
+            if after is not None and not isinstance(after, JunctionCall) and self.layer_tap is None:
+                entry = self.blocks[after.layer].entry()
+                if block.leaves(entry):
+                    entered = torch.empty(h.shape, dtype=self.dtype, device=self.device)
+                    more["leave"] = (entry[0], entered)
+            block.forward(h, batch, storage.layer_cache(call.cache, call.write_cache), **more)
             if self.layer_tap is not None:
                 self.layer_tap(runs, h if p.streams is None else h.total())
             runs += 1
@@ -231,6 +244,10 @@ class Model:
                 self.final_norm.forward(h, x, rows=batch.logit_rows)
             else:
                 h.enter(self._ones, self.final_norm, x, rows=batch.logit_rows, last=True)
+            if self._logit_scales is not None and R <= self._logit_scales.numel():
+                # a factor alone is the product's own: the same number as of the stored sums, without a pass over the logits
+                k.linear(x, self.head_weight, logits, row_scale=self._logit_scales[:R])
+                return logits
             k.linear(x, self.head_weight, logits)
             if p.logit_scale != 1.0 or p.logit_softcap is not None:
                 k.transform_logits(logits, scale=p.logit_scale, softcap=p.logit_softcap)

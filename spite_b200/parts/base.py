@@ -260,5 +260,15 @@ class Block(Part):
             raise ConfigError(f"block {self.kind!r}: more than one part asks for a cache")
         return wants[0] if wants else (None, None)
 
+    def entry(self):
+        """What the block's first kernel makes of the stream, if the last kernel of the block before may make it instead: (gain, eps) of an
+        RMS norm, (None, None) for the stream in the activation type, or None: nothing of that kind."""
+        return None
+
+    def leaves(self, entry) -> bool:
+        """Can the block's last kernel make that?  Then `forward(..., leave=(gain, out))` writes it into `out` [M, hidden] (T), and the
+        next block gets it as `forward(..., entered=out)`."""
+        return False
+
     def forward(self, h, batch, cache):
         raise NotImplementedError

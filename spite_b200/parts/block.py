@@ -18,6 +18,9 @@ a feed-forward follows, writes the norm that the feed-forward reads.
 The sublayers read the stream itself (in the activation type: a copy for bfloat16 products, the stream in place for
 float32 ones); the kernel that norms the mixer's output and adds it to the stream also writes the copy that the
 feed-forward reads.
+
+The last kernel of a sandwich or postnorm layer also writes what the next layer of either kind begins with (its first norm, or the
+copy), which was a kernel of its own: a decode step of a request is a chain of kernels of two to seven us.
 """
 from __future__ import annotations
 
@@ -92,6 +95,18 @@ class SandwichResidual(Block):
             if n is not None and (n.kind != "rms_norm" or n.eps != self.mixer_norm.eps):
                 raise ConfigError("sandwich_residual fuses its norms into one kernel: RMS norms with one epsilon")
 
+    # (a class that runs the sublayers in its own way neither takes nor leaves anything)
+    def entry(self):
+        return (self.mixer_norm.weight, self.mixer_norm.eps) if type(self).forward is SandwichResidual.forward else None
+
+    def leaves(self, entry):
+        return type(self).forward is SandwichResidual.forward and entry is not None and entry[1] in (None, self.mixer_norm.eps)
+
+    def _last(self, y, norm, eps, h, leave):
+        """The block's last kernel: norm, factor and sum, and what the next block's first kernel would make of the stream."""
+        more = {} if leave is None else dict(next_gain=leave[0], next_out=leave[1])
+        self.k.rms_norm_residual(y, norm.weight, eps, self.mult, h, **more)
+
     def _run(self, part, x, y, *args):
         if part.can_store:
             part.forward(x, y, *args, accumulate=False)
@@ -99,19 +114,20 @@ class SandwichResidual(Block):
             y.zero_()
             part.forward(x, y, *args)
 
-    def forward(self, h, batch, cache):
+    def forward(self, h, batch, cache, entered=None, leave=None):
         k = self.k
-        x = torch.empty(h.shape, dtype=self.ctx.dtype, device=h.device)
+        x = torch.empty(h.shape, dtype=self.ctx.dtype, device=h.device) if entered is None else entered
         y = torch.empty_like(h)
-        self.mixer_norm.forward(h, x)
+        if entered is None:
+            self.mixer_norm.forward(h, x)
         self._run(self.mixer, x, y, batch, cache)
         eps = self.mixer_norm.eps
         if self.ffn is None:
-            k.rms_norm_residual(y, self.mixer_out_norm.weight, eps, self.mult, h)
+            self._last(y, self.mixer_out_norm, eps, h, leave)
             return
         k.rms_norm_residual(y, self.mixer_out_norm.weight, eps, self.mult, h, next_gain=self.ffn_norm.weight, next_out=x)
         self._run(self.ffn, x, y, batch)
-        k.rms_norm_residual(y, self.ffn_out_norm.weight, eps, self.mult, h)
+        self._last(y, self.ffn_out_norm, eps, h, leave)
 
 
 @register_block("postnorm_residual")
@@ -129,20 +145,26 @@ class PostNormResidual(Block):
             if n is not None and (n.kind != "rms_norm" or n.eps != self.mixer_out_norm.eps):
                 raise ConfigError("postnorm_residual fuses its norms into one kernel: RMS norms with one epsilon")
 
-    _run = SandwichResidual._run
+    _run, _last = SandwichResidual._run, SandwichResidual._last
 
-    def forward(self, h, batch, cache):
+    def entry(self):
+        return (None, None) if type(self).forward is PostNormResidual.forward and self.ctx.dtype != torch.float32 else None
+
+    def leaves(self, entry):
+        return type(self).forward is PostNormResidual.forward and entry is not None and entry[1] in (None, self.mixer_out_norm.eps)
+
+    def forward(self, h, batch, cache, entered=None, leave=None):
         k = self.k
         same = self.ctx.dtype == torch.float32        # float32 products read the stream in place
-        x = h if same else torch.empty(h.shape, dtype=self.ctx.dtype, device=h.device)
+        x = h if same else torch.empty(h.shape, dtype=self.ctx.dtype, device=h.device) if entered is None else entered
         y = torch.empty_like(h)
-        if not same:
+        if not same and entered is None:
             k.cast_rows(h, x)
         self._run(self.mixer, x, y, batch, cache)
         eps = self.mixer_out_norm.eps
         if self.ffn is None:
-            k.rms_norm_residual(y, self.mixer_out_norm.weight, eps, self.mult, h)
+            self._last(y, self.mixer_out_norm, eps, h, leave)
             return
         k.rms_norm_residual(y, self.mixer_out_norm.weight, eps, self.mult, h, next_out=None if same else x)
         self._run(self.ffn, x, y, batch)
-        k.rms_norm_residual(y, self.ffn_out_norm.weight, eps, self.mult, h)
+        self._last(y, self.ffn_out_norm, eps, h, leave)
