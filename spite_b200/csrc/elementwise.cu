@@ -1312,3 +1312,24 @@ SPITE_API int spite_streams(int out_dtype, const StreamsParams* p, void* stream)
     SPITE_STREAMS_T(__nv_bfloat16)
 #undef SPITE_STREAMS_T
 }
+
+// ---------------------------------------------------------------------------------------------------------------
+// A step's integer inputs from pinned host memory, read where they lie, in 16-byte words and the rest one by one.  The copy engine's copy
+// between two steps' graphs costs the two changes of engine: 11 us of a decode step of 220 for 1,024 to 16,384 words, this one 4 to 5.
+__global__ void __launch_bounds__(256) upload_words_kernel(const int* host, int* out, long long n) {
+    const long long i = 4 * ((long long)blockIdx.x * 256 + threadIdx.x);
+    if (i + 4 <= n) *(int4*)(out + i) = *(const int4*)(host + i);
+    else
+        for (long long j = i; j < n; ++j) out[j] = host[j];
+}
+
+// `host`: pinned memory of this process, 16-byte aligned, as `out`; it must stay as it is until the kernel has run.
+SPITE_API int spite_upload_words(const int* host, int* out, long long n, void* stream) {
+    if (!host || !out || n < 0) return SPITE_BAD_ARG;
+    if (((uintptr_t)host | (uintptr_t)out) & 15) return SPITE_UNSUPPORTED;
+    if (n == 0) return SPITE_OK;
+    const long long blocks = (n + 1023) / 1024;
+    if (blocks > 0x7fffffff) return SPITE_UNSUPPORTED;
+    upload_words_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(host, out, n);
+    return spite_launch_status();
+}

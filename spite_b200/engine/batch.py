@@ -103,8 +103,10 @@ class StaticDecodeBatch:
     computes and writes the same keys and values to the same place, so it changes
     nothing and reads no weight or page that the step would not read anyway."""
 
-    def __init__(self, n_requests: int, table_widths: list, device, context_bucket: int):
+    def __init__(self, n_requests: int, table_widths: list, device, context_bucket: int, upload=None):
+        """`upload(host, dev)`, if given, launches the copy of the inputs as a kernel, or says that it does not (False)."""
         S = self.S = n_requests
+        self.upload = upload
         self.widths = list(table_widths)
         total = 3 * S + (S + 1) + S + S + sum(S * w for w in self.widths)
         self.host = torch.empty(total, dtype=torch.int32)
@@ -132,6 +134,11 @@ class StaticDecodeBatch:
             max_seg_len=1, context_bucket=context_bucket)
         self._copied = None
 
+    def __del__(self):
+        # a kernel reads the pinned buffer itself, which the allocator of pinned memory does not know of: it goes when that has run
+        if getattr(self, "_copied", None) is not None:
+            self._copied.synchronize()
+
     def fill(self, segments, tokens, tables_per_group):
         """Write this step's tokens, positions, slots and block tables and start the copy."""
         if self._copied is not None:
@@ -154,8 +161,10 @@ class StaticDecodeBatch:
         first = segments[0]
         self.batch.segments = list(segments) + [
             Segment(first.req_id, first.slot, first.start_pos, 1, n + i, first.fresh) for i in range(pad)]
-        self.dev.copy_(self.host, non_blocking=True)
+        if self.upload is None or not self.upload(self.host, self.dev):
+            self.dev.copy_(self.host, non_blocking=True)
         if self.dev.is_cuda:
-            self._copied = torch.cuda.Event()
+            if self._copied is None:
+                self._copied = torch.cuda.Event()
             self._copied.record()
         return self.batch

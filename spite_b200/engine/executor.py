@@ -216,7 +216,8 @@ class Engine:
                 # a replay of the graph that goes may still be running, and its buffers are about to be freed
                 torch.cuda.current_stream(self.model.device).synchronize()
                 self._graphs.popitem(last=False)
-            st = _GraphState(StaticDecodeBatch(S, [self._table_width] * self.storage.n_groups, self.model.device, bucket))
+            st = _GraphState(StaticDecodeBatch(S, [self._table_width] * self.storage.n_groups, self.model.device, bucket,
+                                               getattr(self.model.kernels, "upload_words", None)))
             self._graphs[key] = st
         else:
             self._graphs.move_to_end(key)
