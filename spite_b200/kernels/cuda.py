@@ -442,7 +442,7 @@ class CudaKernels(KernelSet):
         return C.c_void_p(CudaKernels._raw_stream())
 
     def _t(self, t, dtype=None, name="tensor"):
-        if t.device.type != "cuda" or not t.is_contiguous():
+        if not t.is_cuda or not t.is_contiguous():            # (is_cuda: half of what device.type takes, four times a launch)
             raise KernelError(f"{name} must be a contiguous CUDA tensor")
         if dtype is not None and t.dtype != dtype:
             raise KernelError(f"{name} must be {dtype}, is {t.dtype}")
