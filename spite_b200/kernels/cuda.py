@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import collections
 import ctypes as C
+import functools
 import math
 import os
 
@@ -176,38 +177,26 @@ def _check(status, what):
         raise KernelError(f"{what}: {_STATUS.get(status, f'status {status}')}")
 
 
-def stream_cut(M: int, N: int, K: int, groups: int, swiglu: bool, slots: int, smem: int, nt: int, *,
-               item_cost: float = 2.0, split_item_cost: float = 6.0, split_cost: float = 1.5, slice_cost: float = 1.0,
-               max_slices: int = 8, slices_min_rows: int = 4, cluster_max_splits: int = 0, cluster_cost: float = 0.0):
+@functools.lru_cache(maxsize=4096)
+def stream_cut(M: int, N: int, K: int, groups: float, swiglu: bool, slots: int, smem: int, nt: int, *,
+               item_cost: float = 2.0, split_item_cost: float = 6.0, split_cost: float = 1.5, slice_cost: float = 1.0, slice_each: float = 0.0,
+               max_slices: int = 8, slices_min_rows: int = 4, min_stages: int = 4, lone_rate: float = 1.0, cluster_max_splits: int = 0,
+               cluster_cost: float = 0.0, most_groups: int | None = None):
     """(k slices inside a block, k splits across blocks) of the weight-streaming kernel for a product of M rows,
     N output columns (per group) and depth K on `slots` resident blocks of `smem` bytes, `nt` token columns.
 
-    A product of few tiles of 128 rows (a dense projection at a few tokens: 40 to 128 tiles for 296 to 444
+    A product of few tiles of 128 rows (a dense projection at a few tokens: 16 to 128 tiles for 296 or 444
     resident blocks) would leave most multiprocessors without work, and the ones that have some are then
     bound by what a single one can pull; so the items are made smaller until they fill the resident blocks
     about once: lower tiles with the k blocks of a stage side by side (the sums meet in shared memory), or k
     splits across blocks (partial sums through global memory, a ticket, a second pass over as many partial
-    tiles as there are splits).  The cost of a choice is its rounds of items times (stages an item + what an
-    item costs besides, in stages of 16 KiB: `item_cost` for any item, `split_item_cost` + `split_cost` a split
-    if its sums cross blocks through global memory, `cluster_cost` if the splits, no more than
-    `cluster_max_splits`, can be one thread-block cluster with all clusters resident at once, `slice_cost` if
-    its slices meet in shared memory); at least four stages stay together.
-
-    Measured on B200, us, (slices, splits) forced, each product alone.  Eight tokens (444 blocks): qkv 7168 x
-    5120: (1, 5) 19.6, (2, 1) 20.9, (4, 1) 17.3, (8, 1) 21.3, (2, 2) 18.9; output projection 5120 x 5120: (1, 7)
-    16.5, (4, 1) 14.2, (8, 1) 13.0, (4, 2) 13.1; shared down 5120 x 8192: (1, 7) 21.6, (4, 1) 20.8, (8, 1) 18.6;
-    seven experts' gate/up: (1, 1) 220, (1, 2) 199.5, (2, 1) 197.4, (4, 1) 195.5; their down product: (1, 1)
-    117.6, (2, 1) 113.5, (4, 1) 107.3, (8, 1) 113.4.  One token (296 blocks with rings twice as deep): slices
-    bring nothing, qkv (1, 5) 17.5, (2, 2) 17.0, (4, 1) 19.5; output projection (1, 7) 13.9, (2, 2) 14.1, (4, 1)
-    17.1.  In the decode step (ms at 4 / 6 / 8 / 12 / 16 tokens): no slices 4.64 / 5.64 / 6.63 / 8.38 / 9.67;
-    slices everywhere 4.89 / 5.85 / 6.51 / 8.68 / 9.45; for one-group products only 4.73 / 5.62 / 6.52 / 8.41 /
-    9.53; for the experts' products only 4.76 / 5.83 / 6.63 / 8.68 / 9.60.  The experts' products are faster
-    alone with slices and slower in the step: with tiles of 128 rows some blocks end early and the next
-    kernel's blocks start under the rest.  So the caller allows slices for one-group products from
-    `slices_min_rows` rows on (the kernel set's defaults: six), and tiles of 128 rows otherwise.  Those products now run
-    in the deeper ring (296 blocks) with costs of their own (`stream_one_group_costs`): 8 rows, 4096 x 4096 (8, 1) 8.5, (4,
-    2) 9.2, (2, 3) 10.6; 1024 x 4096 (4, 8) 5.5, (8, 2) 5.7, (8, 1) 6.6; decode step of 16 Scout layers at 8 / 16 / 24
-    requests over 2,048 keys 6.12 / 8.81 / 11.23 ms, before 6.15 / 8.87 / 11.48."""
+    tiles as there are splits).  The cost of a choice, in stages of 16 KiB on all blocks: the stages of its full rounds of
+    items; those of its last round, which cost as much less as there are fewer items, since a block that shares the memory with fewer
+    others pulls up to `lone_rate` times as much; and for every round what an item costs besides its stages: `item_cost` for any,
+    `split_item_cost` + `split_cost` a split if its sums cross blocks through global memory, `cluster_cost` if the splits, no more than
+    `cluster_max_splits`, can be one thread-block cluster with all clusters resident at once (of `most_groups` groups, where `groups`
+    is how many are expected to have tokens), `slice_cost` + `slice_each` a slice if slices meet in shared memory.  At least
+    `min_stages` stages stay together.  (The defaults are costs of products alone; the kernel set's own are `stream_costs`.)"""
     best, best_cost = (1, 1), None
     for slices in (1, 2, 4, 8):
         if K % (64 * slices) or (swiglu and slices == 8):
@@ -218,16 +207,18 @@ def stream_cut(M: int, N: int, K: int, groups: int, swiglu: bool, slots: int, sm
         if slices > 1 and (smem - 5504 - (8 - 8 // slices) * 64 * nt) // stage_bytes < 2:
             continue                                          # a ring of one stage
         rows = 128 // slices
-        tiles = -(-N // (rows // 2 if swiglu else rows)) * groups
+        row_tiles = -(-N // (rows // 2 if swiglu else rows))
+        tiles = row_tiles * groups
         stages = K // (64 * slices)
-        for s in range(1, max(1, min(32, stages // 4)) + 1):
-            rounds = -(-tiles * s // slots)
-            fixed = item_cost + (slice_cost if slices > 1 else 0.0)
-            if s > 1 and slices == 1 and s <= cluster_max_splits and tiles * s <= slots:
+        for s in range(1, max(1, min(32, stages // min_stages)) + 1):
+            full = tiles * s // slots
+            rest = tiles * s - full * slots
+            fixed = item_cost + (slice_cost + slice_each * slices if slices > 1 else 0.0)
+            if s > 1 and slices == 1 and s <= cluster_max_splits and row_tiles * (most_groups or groups) * s <= slots:
                 fixed += cluster_cost                         # the splits as one cluster: their sums meet in shared memory
             elif s > 1:
                 fixed += split_item_cost + split_cost * s
-            cost = rounds * (-(-stages // s) + fixed)
+            cost = (full + (max(rest / slots, 1.0 / lone_rate) if rest else 0.0)) * -(-stages // s) + (full + (rest > 0)) * fixed
             if best_cost is None or cost < best_cost:
                 best, best_cost = (slices, s), cost
             if tiles * s >= 4 * slots:
@@ -272,6 +263,15 @@ def attention_cut_pays(segments, window, pair_tokens: int, kv_heads: int, blocks
 
 
 class CudaKernels(KernelSet):
+    #: What a work item costs besides its stages, and what is left of them where blocks are alone (see stream_cut), in stages of 16 KiB.
+    #: Found by search over 240 one-group products (1024 x 1024 to 5120 x 16384, with and without SwiGLU, 1 to 32 rows, each after a
+    #: norm in a graph, against every cut): the choice is 1.3 % slower than the best cut on average; the costs before, with slices
+    #: from six rows and clusters to three only, 7.4 %.  us, before / now: 2048 x 2048 at 1 / 4 / 8 rows 7.5 / 6.2, 8.9 / 6.4, 6.4 /
+    #: 6.4; 4096 x 2048 7.8 / 6.6, 9.0 / 6.8, 6.9 / 6.9; 1024 x 4096 9.8 / 7.1, 9.9 / 7.1, 9.2 / 7.1; 5120 x 16384 at 24 rows 58.5 / 50.3.
+    #: The same costs over 45 products of grouped rows (16 or 32 experts, 1 to 16 rows): 1.0 % from the best, before 7.1 %.
+    stream_costs = dict(item_cost=4.0, split_item_cost=1.5, split_cost=0.5, slice_cost=0.0, slice_each=0.25, min_stages=1, lone_rate=1.25,
+                        cluster_cost=8.0)
+
     def __init__(self, dtype: torch.dtype, device="cuda:0"):
         if dtype not in _DT:
             raise KernelError(f"no kernel set for {dtype}; use torch.bfloat16 or torch.float32")
@@ -314,39 +314,19 @@ class CudaKernels(KernelSet):
         self.tc_experts_down_min_groups = 64
         # the TMA weight-streaming kernel for decode products
         self.use_stream = True
-        # what a work item costs besides its stages, in stages of 16 KiB: any item; one whose sums cross blocks (a
-        # fence, a ticket, a second pass: about 2.7 us) and every k split of it; one whose k slices meet in shared memory
-        self.stream_item_cost = 2.0
-        self.stream_split_item_cost = 6.0
-        self.stream_split_cost = 1.5
-        self.stream_slice_cost = 1.0
-        # the first three for one-group products that may be cut into slices.  Against the best of all (slices, splits), over 2048 x
-        # 2048, 6176 x 2048, 8192 x 2048, 2048 x 8192, 32768 x 2048, 5120 x 5120, 7168 x 5120, 4096 x 4096 and 1024 x 4096 at 4 to 32
-        # rows alone, the choice by these costs is 0.8 % slower on average, by the three above 4.5 %
-        self.stream_one_group_costs = (1.0, 2.0, 1.0)
-        self.stream_max_slices = 8             # 1: tiles of 128 rows only
-        self.stream_slices_min_rows = 6        # products of fewer rows keep tiles of 128 rows (see stream_cut)
-        self.stream_slices_grouped = False     # ... and so do grouped products
-        self.stream_cluster_max_rows = 3       # up to this many rows the k splits of a tile are a thread-block cluster (0: never)
-        # ... if they are no more than this (the hardware takes up to 8).  Measured in the decode step at one / two /
-        # three tokens: no clusters 2.780 / 3.348 / 4.114 ms, clusters of two (the gate/up products) 2.748 / 3.335 /
-        # 4.079, up to four 2.749 / 3.313 / 4.082, up to eight 2.753 / 3.316 / 4.083; clusters of seven (the 40 tiles of
-        # an output projection) are not all resident at once and are refused by the kernel's launcher
+        # up to this many rows two to four k splits of a tile are a thread-block cluster (0: never), if all are resident at once:
+        # 8192 x 2048 in four splits at 4 rows 10.1 us, through global memory 11.5; six and more splits gain nothing over slices
+        self.stream_cluster_max_rows = 16
         self.stream_cluster_max_splits = 4
-        # what such an item costs besides its stages (see stream_cut).  9 (qkv in four splits as clusters, the output
-        # and down projections in seven through global memory) against 4, 2, 1 (all three in four): 2.714 against
-        # 2.738, 2.727, 2.726 ms at one token
-        self.stream_cluster_cost = 9.0
         # one-group products of up to this many rows stream their weights too (16: never; the kernel takes up to 32), here / on
         # tcgen05, us, 24 rows: 2048 x 2048 7.9 / 12.6, 8192 x 2048 10.4 / 17.4, 2048 x 8192 12.8 / 40, 5120 x 5120 17.2 / 27.4
         self.stream_max_rows = 32
         self.stream_force = None               # (k slices, k splits) for every call, for measurements
-        # (shared memory per block, resident blocks) for up to 3 tokens and one-group products, and for products over groups of
-        # more tokens: measured in the decode step at
-        # Scout shapes, one token 2.90 ms with (110 KiB, 2 per multiprocessor) against 3.01 with (74 KiB, 3), eight
-        # tokens 7.10 against 7.02 (both kinds of products alike), sixty-four alike; one-group products alone in the deeper ring, us
-        # against (74 KiB, 3), 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 / 17.8, 4096 x 4096 8.5 / 10.6; 16 rows 8.6 / 10.8,
-        # 16.2 / 20.6, 9.8 / 13.8; one block per multiprocessor with 110 or 200 KiB: 3.2 and 3.1 ms
+        # (shared memory per block, resident blocks): one-group products and grouped ones of up to 3 rows, or of up to 8 whose weights
+        # are few (`stream_deep_bytes`), in the deeper ring.  us, deeper / other, 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 /
+        # 17.8; 16 rows 8.6 / 10.8, 16.2 / 20.6; seven experts of 2 x 1024 x 2048 (59 MB) 14.7 / 15.9, six of 2 x 8192 x 5120 (1 GB)
+        # 161 / 157; one block per multiprocessor with 110 or 200 KiB is slower throughout
+        self.stream_deep_bytes = 80e6
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
         # Recurrences over prompts: a step whose longest segment has at least so many tokens, `chunk_from` (`chunk_from_few` where its long
         # segments have fewer than 32 heads together), and `chunk_per_brief` more for each of its segments of fewer than 32 tokens (8 in
@@ -705,7 +685,7 @@ class CudaKernels(KernelSet):
             # ... and a one-group product of up to 32 rows in place (the dense projections of a larger decode batch)
             more = (not grouped and not p.a_rows and 16 < p.M <= self.stream_max_rows and p.N < 65536)
             if (few or more) and self.use_stream and p.K % 64 == 0 and max_rows_per_group <= (32 if more else 16):
-                st = self._gemm_stream(p, int(max_rows_per_group), grouped, int(max_rows_per_group) if even_groups else p.M)
+                st = self._gemm_stream(p, int(max_rows_per_group), grouped, even_groups)
                 if st != -2:
                     self._count("gemm_stream", 1)
                     _check(st, what + " (streaming)")
@@ -776,15 +756,19 @@ class CudaKernels(KernelSet):
             return p.n_groups >= self.tc_experts_down_min_groups and 32 <= avg <= self.tc_experts_max_group_rows
         return False
 
-    def _gemm_stream(self, p, max_rows_per_group, grouped, rows):
+    def _gemm_stream(self, p, max_rows_per_group, grouped, even_groups):
         """The TMA weight-streaming kernel for decode steps: picks the tile height (k slices inside the block)
         and the k splits across blocks so that the work items are many enough to spread evenly, and lends the
         scratch for the partial sums of the splits."""
         swiglu = p.epilogue == EPI_SWIGLU
         groups = min(p.n_groups, p.M) if grouped else 1
-        smem, blocks = self.stream_shape[0 if rows <= 3 or not grouped else 1]
+        rows = max_rows_per_group if even_groups else p.M
+        # how many groups have tokens: all of them, or as many as rows that fall on them at random reach
+        likely = groups if even_groups or groups == 1 else p.n_groups * (1.0 - (1.0 - 1.0 / p.n_groups) ** p.M)
+        deep = not grouped or rows <= 3 or (rows <= 8 and likely * p.N * p.K * (4 if swiglu else 2) < self.stream_deep_bytes)
+        smem, blocks = self.stream_shape[0 if deep else 1]
         nt = 8 if max_rows_per_group <= 8 else 16 if max_rows_per_group <= 16 else 32
-        slices, splits = self.stream_force or self._stream_cut(rows, p.N, p.K, groups, swiglu, blocks, smem, nt, grouped)
+        slices, splits = self.stream_force or self._stream_cut(rows, p.N, p.K, likely, groups, swiglu, blocks, smem, nt)
         tile_rows = 128 // slices
         tiles = -(-p.N // (tile_rows // 2 if swiglu else tile_rows)) * groups
         lib = self._lib("gemm_stream")
@@ -806,17 +790,9 @@ class CudaKernels(KernelSet):
             C.byref(p), max_rows_per_group, slices, 0, blocks, smem, splits, C.c_void_p(_ptr(scratch)),
             C.c_longlong(n_floats), C.c_void_p(_ptr(tickets)), self._tickets_n, C.c_void_p(stream))
 
-    def _stream_cut(self, M: int, N: int, K: int, groups: int, swiglu: bool, slots: int, smem: int, nt: int,
-                    grouped: bool):
-        item, split_item, split = (self.stream_one_group_costs if not grouped and M >= self.stream_slices_min_rows else
-                                   (self.stream_item_cost, self.stream_split_item_cost, self.stream_split_cost))
-        return stream_cut(M, N, K, groups, swiglu, slots, smem, nt, item_cost=item, split_item_cost=split_item, split_cost=split,
-                          slice_cost=self.stream_slice_cost,
-                          max_slices=(min(4, self.stream_max_slices) if nt > 16 else self.stream_max_slices)
-                          if self.stream_slices_grouped or not grouped else 1,
-                          slices_min_rows=self.stream_slices_min_rows,
-                          cluster_max_splits=self.stream_cluster_max_splits if M <= self.stream_cluster_max_rows else 0,
-                          cluster_cost=self.stream_cluster_cost)
+    def _stream_cut(self, M: int, N: int, K: int, groups: float, most_groups: int, swiglu: bool, slots: int, smem: int, nt: int):
+        return stream_cut(M, N, K, groups, swiglu, slots, smem, nt, max_slices=4 if nt > 16 else 8, slices_min_rows=1, most_groups=most_groups,
+                          cluster_max_splits=self.stream_cluster_max_splits if M <= self.stream_cluster_max_rows else 0, **self.stream_costs)
 
     def attention_tc_error(self) -> int:
         """Error code left by a tcgen05 attention block that gave up waiting (0: none); clears it. Synchronises."""
