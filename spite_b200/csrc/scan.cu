@@ -803,10 +803,6 @@ inline chunk::Walk scan_walk(const ScanParams& p, const Made& out) {
     w.n_segments = p.n_segments; w.heads = p.heads; w.qk_heads = p.kv_heads; w.dim = p.dim; w.vdim = p.vdim;
     return w;
 }
-inline bool one_wave(const ScanParams& p, const Made& out, int cols) {
-    return (long long)((p.vdim + cols - 1) / cols) * p.heads * out.numbering.segments <= 148;
-}
-
 template <int DP>
 int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_stride, const float* a_log, const float* dt_bias, const Made& out,
                               cudaStream_t st) {
@@ -819,9 +815,10 @@ int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_s
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
     chunk::Walk w = scan_walk(p, out);
     w.skip = p.skip;
-    // 32 columns a block while that leaves every multiprocessor one block at most, else 64
-    if (one_wave(p, out, 32)) return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, s_waits, st);
-    return launch_walk<DP / 2, 2, 4, HEAD_DECAY>(w, s_waits, st);
+    // 32 columns a block: two blocks of four warps on a multiprocessor wait for each other's barriers less than one of eight with 64
+    // columns does.  us, 64 / 32 columns, the same bits: 128 heads of 128 x 64, one request of 2,048 tokens 199 / 175, five of 410
+    // 224 / 195; 64 heads, five of 410 134 / 117; 64 x 64, 64 heads, three of 666 79 / 61; 16 columns 253 in the first
+    return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, s_waits, st);
 }
 template <int DP, bool BONUS>
 int launch_key_decay_chunks(const ScanParams& p, const Made& out, int n_chunks, cudaStream_t st) {
