@@ -112,14 +112,21 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
     return v;
 }
-// 2^x for two numbers on the multiply-add units, x at least -126 (smaller ones give 2^-126): x = n + f with n whole and |f| <= 1/2, a
-// polynomial of degree 5 for 2^f (least worst relative error over [-1/2, 1/2], fitted by Lawson's iteration: 7.5e-8, 2.1e-7 with the
-// roundings, as much as the special-function unit's), and n added to its exponent.
+// The larger of two numbers, or NaN where one of them is NaN (fmaxf gives the other).
+__device__ __forceinline__ float max_or_nan(float a, float b) {
+    float v;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(v) : "f"(a), "f"(b));
+    return v;
+}
+// 2^x for two numbers on the multiply-add units, x at most 127: x = n + f with n whole and |f| <= 1/2, a polynomial of degree 5 for 2^f
+// (least worst relative error over [-1/2, 1/2], fitted by Lawson's iteration: 7.5e-8, 2.1e-7 with the roundings, as much as the
+// special-function unit's) times 2^n.  As with the unit, NaN gives NaN, and what lies below -127 gives 0 (n = -127 makes the factor's
+// bits all zero).  (n is not added to the polynomial's exponent, which would be one multiplication less: on a NaN's bits that gives a number.)
 __device__ __forceinline__ void ex2_pair(f2 x, float& a, float& b) {
     auto both = [](float v) { return pack2(v, v); };
     float xa, xb;
     unpack2(x, xa, xb);
-    x = pack2(fmaxf(xa, -126.f), fmaxf(xb, -126.f));
+    x = pack2(max_or_nan(xa, -127.f), max_or_nan(xb, -127.f));
     const f2 n = add2(x, both(12582912.f));                // 1.5 * 2^23: n stands in the low bits
     const f2 f = fma2(add2(n, both(-12582912.f)), both(-1.f), x);
     f2 p = fma2(both(0.00132764445f), f, both(0.00967553724f));
@@ -127,11 +134,10 @@ __device__ __forceinline__ void ex2_pair(f2 x, float& a, float& b) {
     p = fma2(p, f, both(0.240221202f));
     p = fma2(p, f, both(0.693146944f));
     p = fma2(p, f, both(1.00000012f));
-    float pa, pb, na, nb;
-    unpack2(p, pa, pb);
+    float na, nb;
     unpack2(n, na, nb);
-    a = __int_as_float(__float_as_int(pa) + (__float_as_int(na) << 23));
-    b = __int_as_float(__float_as_int(pb) + (__float_as_int(nb) << 23));
+    const f2 two_n = pack2(__int_as_float((__float_as_int(na) << 23) + 0x3f800000), __int_as_float((__float_as_int(nb) << 23) + 0x3f800000));
+    unpack2(mul2(p, two_n), a, b);
 }
 __device__ __forceinline__ unsigned pack_bf16(float a, float b) {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
@@ -783,7 +789,22 @@ int launch(const AttentionParams& p, const StepTokens& b, const PagedCache& c, c
     return spite_launch_status();
 }
 
+// 2^x of pairs, for tests of ex2_pair
+__global__ void ex2_pairs_kernel(const float2* x, float2* y, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) ex2_pair(pack2(x[i].x, x[i].y), y[i].x, y[i].y);
+}
+
 }  // namespace
+
+// y = 2^x for n_pairs pairs of floats as the attention's weights in unmasked key tiles are made
+SPITE_API int spite_attention_exp2_pairs(const float* x, float* y, int n_pairs, void* stream) {
+    if (!x || !y || n_pairs < 0) return SPITE_BAD_ARG;
+    if (((uintptr_t)x | (uintptr_t)y) & 7) return SPITE_UNSUPPORTED;
+    if (n_pairs == 0) return SPITE_OK;
+    ex2_pairs_kernel<<<(n_pairs - 1) / 256 + 1, 256, 0, (cudaStream_t)stream>>>((const float2*)x, (float2*)y, n_pairs);
+    return spite_launch_status();
+}
 
 static int paged_attention_tc(const AttentionParams* p, const StepTokens* b, const PagedCache* c, const AttnMmaExtra* x, int n_blocks, int n_sm,
                               const Cut& cut, void* stream) {

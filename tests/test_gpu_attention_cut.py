@@ -1,5 +1,6 @@
 """Prompt-portion attention on the tcgen05 kernel with its work cut along the keys: whole items and cut ones against float64, in every form the
 kernel has.  The tolerance is the one of the kernel's other tests (weights and outputs in bfloat16)."""
+import ctypes as C
 import math
 
 import pytest
@@ -94,3 +95,57 @@ def test_every_form_cut_as_whole(case, form, monkeypatch):
     whole, none = run(ks, monkeypatch, False, *args, **kw)
     assert scratch >= ks.sm_count * 4 * (hd + 2) * 128 * 4 > none or len(specs) > 1
     close(cut, whole, TOL[torch.bfloat16], form)
+
+
+@pytest.mark.parametrize("cut", [False, True], ids=["whole", "cut"])
+@pytest.mark.parametrize("kind", ["nan", "inf", "-inf"])
+@pytest.mark.parametrize("place", [0, 6, 17, 30, 39, 48, 59, 63])
+def test_a_score_that_is_no_number(place, kind, cut, monkeypatch):
+    """A key whose score is NaN or +inf must show in every row that sees it, one whose score is -inf must weigh nothing, wherever in a tile of
+    64 keys it stands: the weights of the places 6, 7, 16, 17, 26, 27 of every 32 are made on the multiply-add units, the others on the
+    special-function units."""
+    nq, nkv, hd, P, specs = 4, 2, 128, 64, [(900, 200)]
+    ks, win, n_pages = cuda_kernels.CudaKernels(torch.bfloat16, DEV), Window("full", 0), 20
+    batch, tables = make_batch(specs, P, n_pages, 7, DEV)
+    M, g = batch.n_tokens, torch.Generator().manual_seed(place + len(kind))
+    k, v = (torch.randn((1100, nkv, hd), generator=g).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn((M, nq, hd), generator=g).to(torch.bfloat16)
+    q[:, :2] = -q[:, :2].abs() if kind == "-inf" else q[:, :2].abs()
+    ref = dense_attention_reference(q[:, 2:], [k[:, 1:]], [v[:, 1:]], specs, 2, 1, win, hd ** -0.5)
+    j = 256 + place
+    others = torch.arange(1100) != j
+    k[j, 0], v[j, 0] = float("nan") if kind == "nan" else 3e38, 1e38
+    kv = torch.zeros((2, n_pages, nkv, P, hd), dtype=torch.bfloat16)
+    fill_cache(kv, tables, [(1100, 0)], [k], [v], P)
+    out = torch.empty((M, nq * hd), dtype=torch.bfloat16, device=DEV)
+    got, _ = run(ks, monkeypatch, cut, q.reshape(M, nq * hd).to(DEV), out, batch, LayerCache(0, kv.to(DEV), None, P, False), num_heads=nq, window=win,
+                 softmax_scale=hd ** -0.5)
+    got = got.view(M, nq, hd)
+    close(got[:, 2:], ref, TOL[torch.bfloat16], "heads without that key")
+    if kind != "-inf":
+        assert bool(got[:, :2].isnan().all())
+        return
+    sc = torch.einsum("mhd,jd->hmj", q[:, :2].double(), k[others, 0].double()) * hd ** -0.5
+    seen = torch.arange(1100)[others][None, :] <= 900 + torch.arange(M)[:, None]
+    want = torch.softmax(sc.masked_fill(~seen, float("-inf")), -1) @ v[others, 0].double()
+    close(got[:, :2], want.transpose(0, 1), TOL[torch.bfloat16], "without the key")
+
+
+def test_powers_of_two():
+    """The weights made on the multiply-add units.  The polynomial is within 7.5e-8 of 2^f and each of its five multiply-adds rounds by at most
+    2^-24 of a result near 1, the first ones of a small part of it: 2.2e-7 in all over the range that weights have; below 2^-126 they may be
+    off by half the smallest number, and what is no number stays none."""
+    ks = cuda_kernels.CudaKernels(torch.bfloat16, DEV)
+    x = torch.cat([torch.linspace(-126, 8, 1 << 20), torch.linspace(8, 127, 1 << 16)])
+    special = torch.tensor([float("nan"), -float("inf"), -127.0, -1e30, -3e38, 0.0, 1.0, -126.0, float("inf"), float("nan"), 5.0, float("nan")])
+    for given in (x, special):
+        dev, y = given.to(DEV), torch.empty(given.numel(), device=DEV)
+        assert ks._lib("attention_tc").spite_attention_exp2_pairs(C.c_void_p(dev.data_ptr()), C.c_void_p(y.data_ptr()), given.numel() // 2,
+                                                                  ks._stream()) == 0
+        y = y.cpu()
+        if given is x:
+            want = torch.exp2(x.double())
+            assert float((y.double() / want - 1).abs().max()) <= 2.2e-7
+        else:
+            assert y.isnan().tolist() == [True] + 7 * [False] + [True, True, False, True]
+            assert y[1:5].tolist() == [0.0] * 4 and bool(((y[5:8] / torch.tensor([1.0, 2.0, 2.0 ** -126]) - 1).abs() <= 2.2e-7).all())
