@@ -120,8 +120,8 @@ __device__ __forceinline__ float block_sum_once(float v, float* scratch) {
     __syncthreads();
     return warp_sum(lane < (int)((blockDim.x + 31) >> 5) ? scratch[lane] : 0.f);
 }
-// The thread's part of a gain vector, asked for before the wait for the kernel in front (no kernel of a step writes gains): behind a norm's
-// sum it was another round trip to memory.
+// The thread's part of a gain vector, asked for together with the row: behind a norm's sum it was another round trip to memory.  (Not before
+// the wait for the kernel in front, which may be the one that makes the gain.)
 template <int VPT>
 __device__ __forceinline__ void load_gain(float4 (&g)[VPT], const float* gain, int d4) {
 #pragma unroll
@@ -139,9 +139,9 @@ __global__ void rms_norm_vec_kernel(const float* __restrict__ x, const float* __
     __shared__ float scratch[32];
     const int d4 = d >> 2;
     float4 v[VPT], g[VPT];
-    load_gain(g, gain, d4);
     pdl_wait();
     pdl_launch_dependents();
+    load_gain(g, gain, d4);
     const int i = blockIdx.x;
     const int r = rows ? rows[i] : i;
     const float4* in = (const float4*)(x + (size_t)r * d);
@@ -371,10 +371,10 @@ __global__ void rms_norm_residual_vec_kernel(const float* __restrict__ y, const 
     __shared__ float scratch[2][32];
     const int d4 = d >> 2;
     float4 v[VPT], r[VPT], g[VPT], ng[VPT];
-    load_gain(g, gain, d4);
-    load_gain(ng, next_gain, d4);
     pdl_wait();
     pdl_launch_dependents();
+    load_gain(g, gain, d4);
+    load_gain(ng, next_gain, d4);
     const size_t m = blockIdx.x;
     const float4* in = (const float4*)(y + m * d);
     float4* hr = (float4*)(h + m * d);
@@ -799,17 +799,19 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvParams p
 
 // The same for segments of several tokens whose columns are whole groups of four: a thread has four columns and CONV_ROWS tokens, all of
 // whose inputs it asks for before it uses the first (the kernel above has one load of four bytes in flight a thread, which left it at a
-// third of the copy bandwidth).  The sums are the same, term by term.  The weights are asked for before the wait for the kernel in front,
-// and seven blocks fit a multiprocessor: what is left is a round trip to memory and the gate's exponential and division, block after block.
+// third of the copy bandwidth).  The sums are the same, term by term.  The weights are asked for ahead of the inputs, and seven
+// blocks fit a multiprocessor: what is left is a round trip to memory and the gate's exponential and division, block after block.
 // 8,448 channels of 4 taps, 2,048 tokens (138 MB: 21 us): 75 us above, 37 here (47 with the weights behind the inputs and 96 registers;
 // 42 with the weights in front, 38 with six blocks, 40 with eight; 4, 12, 16 tokens a thread 43, 40, 40).
 constexpr int CONV_ROWS = 8;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128, 7) short_conv_rows_kernel(const ShortConvParams p) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool conv = c < p.channels;
-    float w[4][TAPS];                                         // (weights: no kernel of the step writes them)
+    float w[4][TAPS];
     float4 bias = zero;
     if (conv) {
         if (TAPS % 4 == 0 && (((uintptr_t)p.w) & 15) == 0) {  // (the taps of four channels lie side by side)
@@ -827,8 +829,6 @@ __global__ void __launch_bounds__(128, 7) short_conv_rows_kernel(const ShortConv
         }
         if (p.bias) bias = make_float4(p.bias[c], p.bias[c + 1], p.bias[c + 2], p.bias[c + 3]);
     }
-    pdl_wait();
-    pdl_launch_dependents();
     if (c >= p.channels + p.copy_columns) return;
     const int s = blockIdx.y, t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0, i0 = blockIdx.z * CONV_ROWS, slot = p.slots[s], slot0 = p.slots[0];
     if (i0 >= n) return;

@@ -64,7 +64,10 @@ class DistanceBias:
 
 
 class KernelSet:
-    """Interface; see `CudaKernels` for the product implementation."""
+    """Interface; see `CudaKernels` for the product implementation.
+
+    Arguments may come from the call right before, with two exceptions: the weights `w` of the products and the coefficients
+    of `streams` (mix, w_out, w_in) may be read while the kernel before still runs, so they must not be what it writes."""
 
     dtype: torch.dtype
     device: torch.device
