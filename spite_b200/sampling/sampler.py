@@ -13,7 +13,6 @@ from __future__ import annotations
 import struct
 from dataclasses import dataclass, field
 
-import numpy
 import torch
 
 DEFAULT_SEED = 0x1234_5678_9ABC_DEF0        # the constant of crates/spite-cli/src/main.rs:606
@@ -54,6 +53,16 @@ def run_sampling_params(temperature: float, *, seed: int = DEFAULT_SEED, max_tok
 def lcg_advance(state: int) -> int:
     """One step of the generator (crates/spite-sampling/src/lib.rs:343-348)."""
     return (state * 6364136223846793005 + 1442695040888963407) & _MASK64
+
+
+def _put(words, at: int, code: str, values: list):
+    """words[at : at + len(values)] (an int32 array) = the values as float32 ("f") or int32 ("i"): those that torch makes a tensor of."""
+    try:
+        struct.pack_into(f"{len(values)}{code}", words, 4 * at, *values)
+    except (struct.error, OverflowError, TypeError):
+        # not the plain numbers that these are in use (whole numbers given as floats, infinite or missing settings): torch's tensor, or its error
+        dtype = torch.float32 if code == "f" else torch.int32
+        torch.from_numpy(words)[at:at + len(values)].view(dtype)[:] = torch.tensor(values, dtype=dtype)
 
 
 @dataclass
@@ -146,19 +155,15 @@ class Sampler:
         a_state = (a_late + 2 * len(holes) + 1) // 2 * 2          # 64-bit states on an 8-byte boundary
         n_words = a_state + 2 * R
         host = self._staging(n_words, dev)
-        # Filled as numbers in memory: with a torch tensor made from each list first a call for 32 rows with up to 64 tokens of context takes 239
-        # us of host, this way 88 (the kernel behind it 63).
-        ints = host.numpy()
-        floats = ints.view(numpy.float32)
-        settings = [r.params for r in rows]
-        floats[0:R] = [p.temperature for p in settings]
-        ints[R:2 * R] = [p.top_k for p in settings]
-        floats[2 * R:3 * R] = [p.top_p for p in settings]
-        floats[3 * R:4 * R] = [p.min_p for p in settings]
-        floats[4 * R:5 * R] = [p.repetition_penalty for p in settings]
-        struct.pack_into(f"{len(offs) + len(ctx)}i", ints, 4 * a_off, *offs, *ctx)
+        # Written as numbers into the buffer: with a torch tensor made from each list first a call for 32 rows with up to 64 tokens of context takes
+        # 239 us of host, this way 88 (the kernel behind it 63).
+        ints, settings = host.numpy(), [r.params for r in rows]
+        _put(ints, 0, "f", [p.temperature for p in settings])
+        _put(ints, R, "i", [p.top_k for p in settings])
+        _put(ints, 2 * R, "f", [p.top_p for p in settings] + [p.min_p for p in settings] + [p.repetition_penalty for p in settings])
+        _put(ints, a_off, "i", offs + ctx)
         if holes:
-            struct.pack_into(f"{2 * len(holes)}i", ints, 4 * a_late, *holes, *sources)
+            _put(ints, a_late, "i", holes + sources)
         struct.pack_into(f"{R}Q", ints, 4 * a_state, *[r.rng_state & _MASK64 for r in rows])
         words = torch.empty(n_words, dtype=torch.int32, device=dev)
         words.copy_(host[:n_words], non_blocking=True)
