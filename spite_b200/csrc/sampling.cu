@@ -13,6 +13,9 @@
 // 247-265).  Sums are float32 and are added in a fixed order (a thread's elements, the threads of
 // a warp, the warps of a block, the blocks of a cluster by rank), so a row's result does not depend on
 // the other rows or on timing.
+#include <cmath>
+#include <cstring>
+
 #include "common.cuh"
 
 namespace {
@@ -422,8 +425,17 @@ __device__ __forceinline__ float row_max(const Part<PAD> row, float by, bool& na
 // lo.  An element's bin never falls as the element falls; below 0 are the elements above the bins, from BINS on those below.
 struct Bins {
     float lo, scale;                                         // scale: a power of two
-    __device__ __forceinline__ int of(float d) const {       // (the integer part of 2^23 + t stands in the low bits)
-        return (int)(__float_as_uint(fmaf(d - lo, scale, 8388608.f)) - 0x4b000000u);
+    __host__ __device__ __forceinline__ int of(float d) const {
+        // The integer part of 2^23 + t stands in the low bits; more than 2^23 steps above the bins the sum is negative, whose bits
+        // would be a number above all others.
+        const float sum = fmaxf(fmaf(d - lo, scale, 8388608.f), 0.f);
+#ifdef __CUDA_ARCH__
+        const unsigned bits = __float_as_uint(sum);
+#else
+        unsigned bits;
+        memcpy(&bits, &sum, sizeof bits);
+#endif
+        return (int)(bits - 0x4b000000u);
     }
 };
 
@@ -1067,6 +1079,15 @@ SPITE_API int spite_argmax(const float* logits, int rows, int vocab, int* out, v
 
 // Both entry points launch through here, so they give the same tokens: a cluster of eight blocks per row where
 // a row fits their shared memory (`p.work` is not touched then), else one block per row on `p.work`.
+// bins[i] = the bin of a logit `distances[i]` below its row's maximum in a pass whose bins begin at `lo`, `scale` bins a unit (on the host,
+// for tests)
+SPITE_API int spite_sample_bins(const float* distances, int n, float lo, float scale, int* bins) {
+    if (!distances || !bins || n < 0) return SPITE_BAD_ARG;
+    const Bins b{lo, scale};
+    for (int i = 0; i < n; ++i) bins[i] = b.of(distances[i]);
+    return SPITE_OK;
+}
+
 static int launch_sample(const SampleParams& p, int rows, cudaStream_t st) {
     int per = ((p.vocab + CL - 1) / CL + 31) / 32 * 32;
     if (per <= CLUSTER_MAX_PER_BLOCK && rows <= 0x7fffffff / CL) {
