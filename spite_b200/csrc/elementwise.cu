@@ -803,9 +803,12 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvParams p
 // blocks fit a multiprocessor: what is left is a round trip to memory and the gate's exponential and division, block after block.
 // 8,448 channels of 4 taps, 2,048 tokens (138 MB: 21 us): 75 us above, 37 here (47 with the weights behind the inputs and 96 registers;
 // 42 with the weights in front, 38 with six blocks, 40 with eight; 4, 12, 16 tokens a thread 43, 40, 40).
+// More taps hold more inputs and weights, and seven blocks leave 72 registers.  The same size with cold caches, us, 4 / 5 / 6 / 7 / 8 blocks, float32 out:
+// 4 taps 50 / 48 / 44 / 42 / 46, 5 59 / 53 / 49 / 53 / 55, 6 68 / 60 / 62 / 66 / 68, 7 71 / 65 / 64 / 72 / 78, 8 78 / 72 / 84 / 94 / 108.
 constexpr int CONV_ROWS = 8;
+constexpr int conv_blocks(int taps) { return taps <= 4 ? 7 : taps == 5 ? 6 : 5; }
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128, 7) short_conv_rows_kernel(const ShortConvParams p) {
+__global__ void __launch_bounds__(128, conv_blocks(TAPS)) short_conv_rows_kernel(const ShortConvParams p) {
     pdl_wait();
     pdl_launch_dependents();
     const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
