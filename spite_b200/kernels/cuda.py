@@ -1098,12 +1098,13 @@ class CudaKernels(KernelSet):
                                       c.num_kv_heads, self.sm_count):
                     n_floats = self.sm_count * (4 * (c.head_dim + 2) * 128 + 4)
                     part = torch.empty(n_floats, dtype=torch.float32, device=q.device)
-                    self.attention_scratch_bytes = n_floats * 4
                     st = lib.spite_paged_attention_tc_cut(
                         C.byref(p), C.byref(b), C.byref(c), C.byref(x), n_tc, self.sm_count, C.c_void_p(part.data_ptr()), C.c_longlong(n_floats),
                         self._stream())
                     cut = st == 0
-                if st == -2:
+                    if cut:
+                        self.attention_scratch_bytes = n_floats * 4
+                if st == -2:                                          # not cut, or more pairs of row tiles than that form takes
                     st = lib.spite_paged_attention_tc(C.byref(p), C.byref(b), C.byref(c), C.byref(x), n_tc, self.sm_count, self._stream())
                 self._count("attention_tc", 1 + cut)
                 _check(st, "paged_attention (tcgen05, prompt portions)")

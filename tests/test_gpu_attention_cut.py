@@ -25,15 +25,16 @@ CASES = [
 ]
 
 
-def run(ks, monkeypatch, cut, *args, **kw):
+def run(ks, monkeypatch, cut, *args, takes=True, **kw):
+    """One call with the choice made: a cut call launches a second kernel that adds the parts up (unless the cut form does not take the call)."""
     monkeypatch.setattr(cuda_kernels, "attention_cut_pays", lambda *a: cut)
     q, out, batch, cache = args
     out.fill_(float("nan"))
-    ks.attention_scratch_bytes = 0
+    before = ks.launches_by_library["attention_tc"]
     ks.paged_attention(q, out, batch, cache, **kw)
     torch.cuda.synchronize()
-    assert not ks.errors()
-    return out.clone(), ks.attention_scratch_bytes
+    assert not ks.errors() and ks.launches_by_library["attention_tc"] == before + 1 + (cut and takes)
+    return out.clone()
 
 
 @pytest.mark.parametrize("case", range(len(CASES)))
@@ -53,11 +54,10 @@ def test_cut_along_the_keys(case, monkeypatch):
     out, scale = torch.empty((M, nq * hd), dtype=torch.bfloat16, device=DEV), 1.0 / math.sqrt(hd)
     args = (q.reshape(M, nq * hd).to(DEV), out, batch, LayerCache(0, kv.to(DEV), None, P, False))
     kw = dict(num_heads=nq, window=win, softmax_scale=scale)
-    cut, scratch = run(ks, monkeypatch, True, *args, **kw)
-    assert scratch >= ks.sm_count * 4 * (hd + 2) * 128 * 4
-    again, _ = run(ks, monkeypatch, True, *args, **kw)                 # the parts are added in one order
-    assert torch.equal(cut, again)
-    whole, _ = run(ks, monkeypatch, False, *args, **kw)
+    cut = run(ks, monkeypatch, True, *args, **kw)
+    assert len(specs) > 1 or ks.attention_scratch_bytes >= ks.sm_count * 4 * (hd + 2) * 128 * 4     # (other kernels set their own behind it)
+    assert torch.equal(cut, run(ks, monkeypatch, True, *args, **kw))         # the parts are added in one order
+    whole = run(ks, monkeypatch, False, *args, **kw)
     ref = dense_attention_reference(q, k_all, v_all, specs, nq, nkv, win, scale)
     close(whole.view(M, nq, hd), ref, TOL[torch.bfloat16], "whole items")
     close(cut.view(M, nq, hd), ref, TOL[torch.bfloat16], "cut items")
@@ -91,10 +91,43 @@ def test_every_form_cut_as_whole(case, form, monkeypatch):
     out = torch.empty((M, nq * hd), dtype=torch.bfloat16, device=DEV)
     args = (q, out, batch, LayerCache(0, kv, None, P, False, factors))
     kw = dict(kw, num_heads=nq, window=win, softmax_scale=1.0 / math.sqrt(hd))
-    cut, scratch = run(ks, monkeypatch, True, *args, **kw)
-    whole, none = run(ks, monkeypatch, False, *args, **kw)
-    assert scratch >= ks.sm_count * 4 * (hd + 2) * 128 * 4 > none or len(specs) > 1
+    cut = run(ks, monkeypatch, True, *args, **kw)
+    whole = run(ks, monkeypatch, False, *args, **kw)
     close(cut, whole, TOL[torch.bfloat16], form)
+
+
+def one_portion(ks, start, n, nq=40, nkv=8, hd=128, P=64):
+    n_pages = -(-(start + n) // P) + 1
+    batch, _ = make_batch([(start, n)], P, n_pages, 3, DEV)
+    g = torch.Generator(device=DEV).manual_seed(start + n)
+    rnd = lambda *shape: torch.randn(shape, generator=g, device=DEV).to(torch.bfloat16)
+    out = torch.empty((n, nq * hd), dtype=torch.bfloat16, device=DEV)
+    return (rnd(n, nq * hd), out, batch, LayerCache(0, rnd(2, n_pages, nkv, P, hd), None, P, False)), \
+        dict(num_heads=nq, window=Window("full", 0), softmax_scale=hd ** -0.5)
+
+
+@pytest.mark.parametrize("start,n,cut", [(8092, 100, True), (7192, 1000, True), (0, 600, False), (500, 500, False)])
+def test_the_rule_chooses(start, n, cut):
+    """Without the choice made for it: the call asks the rule (whose answers are tested on the host) and follows it."""
+    ks = cuda_kernels.CudaKernels(torch.bfloat16, DEV)
+    args, kw = one_portion(ks, start, n)
+    ks.paged_attention(*args, **kw)
+    assert ks.launches_by_library["attention_tc"] == 1 + cut and (ks.attention_scratch_bytes > 0) == cut
+    torch.cuda.synchronize()
+    assert torch.isfinite(args[1]).all() and not ks.errors()
+
+
+@pytest.mark.parametrize("n", [16384, 16385])
+def test_more_pairs_of_row_tiles_than_are_cut(n, monkeypatch):
+    """16 heads a kv head: 8 tokens a row tile, 1,024 pairs of them at 16,384 tokens; one more goes whole."""
+    ks = cuda_kernels.CudaKernels(torch.bfloat16, DEV)
+    args, kw = one_portion(ks, 0, n, nq=16, nkv=1, hd=64)
+    takes = n <= 16384
+    cut = run(ks, monkeypatch, True, *args, takes=takes, **kw)
+    assert (ks.attention_scratch_bytes > 0) == takes
+    whole = run(ks, monkeypatch, False, *args, **kw)
+    close(cut, whole, TOL[torch.bfloat16], "cut")
+    assert takes or torch.equal(cut, whole)
 
 
 @pytest.mark.parametrize("cut", [False, True], ids=["whole", "cut"])
@@ -118,7 +151,7 @@ def test_a_score_that_is_no_number(place, kind, cut, monkeypatch):
     kv = torch.zeros((2, n_pages, nkv, P, hd), dtype=torch.bfloat16)
     fill_cache(kv, tables, [(1100, 0)], [k], [v], P)
     out = torch.empty((M, nq * hd), dtype=torch.bfloat16, device=DEV)
-    got, _ = run(ks, monkeypatch, cut, q.reshape(M, nq * hd).to(DEV), out, batch, LayerCache(0, kv.to(DEV), None, P, False), num_heads=nq, window=win,
+    got = run(ks, monkeypatch, cut, q.reshape(M, nq * hd).to(DEV), out, batch, LayerCache(0, kv.to(DEV), None, P, False), num_heads=nq, window=win,
                  softmax_scale=hd ** -0.5)
     got = got.view(M, nq, hd)
     close(got[:, 2:], ref, TOL[torch.bfloat16], "heads without that key")
