@@ -324,9 +324,11 @@ class CudaKernels(KernelSet):
         self.stream_force = None               # (k slices, k splits) for every call, for measurements
         # (shared memory per block, resident blocks): one-group products and grouped ones of up to 3 rows, or of up to 8 whose weights
         # are few (`stream_deep_bytes`), in the deeper ring.  us, deeper / other, 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 /
-        # 17.8; 16 rows 8.6 / 10.8, 16.2 / 20.6; seven experts of 2 x 1024 x 2048 (59 MB) 14.7 / 15.9, six of 2 x 8192 x 5120 (1 GB)
-        # 161 / 157; one block per multiprocessor with 110 or 200 KiB is slower throughout
-        self.stream_deep_bytes = 80e6
+        # 17.8; 16 rows 8.6 / 10.8, 16.2 / 20.6; one block per multiprocessor with 110 or 200 KiB is slower throughout.
+        # Grouped products of 4, 6 and 8 rows (19 layers of 8 to 128 experts, weights of 12 MB to 1.1 GB; both products of each, in a graph
+        # over several layers' weights), deeper / other, mean of the ratios by the weights' size: to 60 MB 0.96 (36 products), 60 to
+        # 125 0.97 (36), 125 to 300 1.00 (29), more 1.015 (13); single ones lie 0.79 to 1.30 around that, as their last rounds come out
+        self.stream_deep_bytes = 125e6
         self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
         # Recurrences over prompts: a step whose longest segment has at least so many tokens, `chunk_from` (`chunk_from_few` where its long
         # segments have fewer than 32 heads together), and `chunk_per_brief` more for each of its segments of fewer than 32 tokens (8 in
