@@ -178,12 +178,10 @@ def _check(status, what):
 
 
 @functools.lru_cache(maxsize=4096)
-def stream_cut(M: int, N: int, K: int, groups: float, swiglu: bool, slots: int, smem: int, nt: int, *,
-               item_cost: float = 2.0, split_item_cost: float = 6.0, split_cost: float = 1.5, slice_cost: float = 1.0, slice_each: float = 0.0,
-               max_slices: int = 8, slices_min_rows: int = 4, min_stages: int = 4, lone_rate: float = 1.0, cluster_max_splits: int = 0,
-               cluster_cost: float = 0.0, most_groups: int | None = None):
-    """(k slices inside a block, k splits across blocks) of the weight-streaming kernel for a product of M rows,
-    N output columns (per group) and depth K on `slots` resident blocks of `smem` bytes, `nt` token columns.
+def stream_cut(N: int, K: int, groups: float, most_groups: int, swiglu: bool, slots: int, smem: int, nt: int, max_slices: int, cluster_max_splits: int, *,
+               item_cost: float, split_item_cost: float, split_cost: float, slice_each: float, lone_rate: float, cluster_cost: float):
+    """(k slices inside a block, k splits across blocks) of the weight-streaming kernel for a product of N output columns
+    (per group) and depth K on `slots` resident blocks of `smem` bytes, `nt` token columns.
 
     A product of few tiles of 128 rows (a dense projection at a few tokens: 16 to 128 tiles for 296 or 444
     resident blocks) would leave most multiprocessors without work, and the ones that have some are then
@@ -195,13 +193,13 @@ def stream_cut(M: int, N: int, K: int, groups: float, swiglu: bool, slots: int, 
     others pulls up to `lone_rate` times as much; and for every round what an item costs besides its stages: `item_cost` for any,
     `split_item_cost` + `split_cost` a split if its sums cross blocks through global memory, `cluster_cost` if the splits, no more than
     `cluster_max_splits`, can be one thread-block cluster with all clusters resident at once (of `most_groups` groups, where `groups`
-    is how many are expected to have tokens), `slice_cost` + `slice_each` a slice if slices meet in shared memory.  At least
-    `min_stages` stages stay together.  (The defaults are costs of products alone; the kernel set's own are `stream_costs`.)"""
+    is how many are expected to have tokens), `slice_each` a slice if slices meet in shared memory.  (The kernel set's costs are
+    `CudaKernels.stream_costs`.)"""
     best, best_cost = (1, 1), None
     for slices in (1, 2, 4, 8):
         if K % (64 * slices) or (swiglu and slices == 8):
             continue
-        if slices > 1 and (M < slices_min_rows or slices > max_slices):
+        if slices > max_slices:
             continue
         stage_bytes = 16384 + max(1024, slices * nt * 128)
         if slices > 1 and (smem - 5504 - (8 - 8 // slices) * 64 * nt) // stage_bytes < 2:
@@ -210,11 +208,11 @@ def stream_cut(M: int, N: int, K: int, groups: float, swiglu: bool, slots: int, 
         row_tiles = -(-N // (rows // 2 if swiglu else rows))
         tiles = row_tiles * groups
         stages = K // (64 * slices)
-        for s in range(1, max(1, min(32, stages // min_stages)) + 1):
+        for s in range(1, min(32, stages) + 1):
             full = tiles * s // slots
             rest = tiles * s - full * slots
-            fixed = item_cost + (slice_cost + slice_each * slices if slices > 1 else 0.0)
-            if s > 1 and slices == 1 and s <= cluster_max_splits and row_tiles * (most_groups or groups) * s <= slots:
+            fixed = item_cost + (slice_each * slices if slices > 1 else 0.0)
+            if s > 1 and slices == 1 and s <= cluster_max_splits and row_tiles * most_groups * s <= slots:
                 fixed += cluster_cost                         # the splits as one cluster: their sums meet in shared memory
             elif s > 1:
                 fixed += split_item_cost + split_cost * s
@@ -269,8 +267,24 @@ class CudaKernels(KernelSet):
     #: from six rows and clusters to three only, 7.4 %.  us, before / now: 2048 x 2048 at 1 / 4 / 8 rows 7.5 / 6.2, 8.9 / 6.4, 6.4 /
     #: 6.4; 4096 x 2048 7.8 / 6.6, 9.0 / 6.8, 6.9 / 6.9; 1024 x 4096 9.8 / 7.1, 9.9 / 7.1, 9.2 / 7.1; 5120 x 16384 at 24 rows 58.5 / 50.3.
     #: The same costs over 45 products of grouped rows (16 or 32 experts, 1 to 16 rows): 1.0 % from the best, before 7.1 %.
-    stream_costs = dict(item_cost=4.0, split_item_cost=1.5, split_cost=0.5, slice_cost=0.0, slice_each=0.25, min_stages=1, lone_rate=1.25,
-                        cluster_cost=8.0)
+    stream_costs = dict(item_cost=4.0, split_item_cost=1.5, split_cost=0.5, slice_each=0.25, lone_rate=1.25, cluster_cost=8.0)
+    #: Up to this many rows two to four k splits of a tile are a thread-block cluster (0: never), if all are resident at once:
+    #: 8192 x 2048 in four splits at 4 rows 10.1 us, through global memory 11.5; six and more splits gain nothing over slices.
+    stream_cluster_max_rows = 16
+    stream_cluster_max_splits = 4
+
+    #: One-group products and grouped ones of up to 3 rows, or of up to 8 whose weights are few (this many bytes), run in the deeper ring.  us, deeper /
+    #: other, 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 / 17.8; 16 rows 8.6 / 10.8, 16.2 / 20.6; one block per multiprocessor with 110
+    #: or 200 KiB is slower throughout.  Grouped products of 4, 6 and 8 rows (19 layers of 8 to 128 experts, weights of 12 MB to 1.1 GB; both
+    #: products of each, in a graph over several layers' weights), deeper / other, mean of the ratios by the weights' size: to 60 MB 0.96
+    #: (36 products), 60 to 125 0.97 (36), 125 to 300 1.00 (29), more 1.015 (13); single ones lie 0.79 to 1.30 around that, as their last
+    #: rounds come out.
+    stream_deep_bytes = 125e6
+
+    @staticmethod
+    def stream_rings(sm_count: int) -> list:
+        """(shared memory per block, resident blocks) of the weight-streaming kernel: the deeper ring, the other."""
+        return [(110 * 1024, 2 * sm_count), (74 * 1024, 3 * sm_count)]
 
     def __init__(self, dtype: torch.dtype, device="cuda:0"):
         if dtype not in _DT:
@@ -314,22 +328,11 @@ class CudaKernels(KernelSet):
         self.tc_experts_down_min_groups = 64
         # the TMA weight-streaming kernel for decode products
         self.use_stream = True
-        # up to this many rows two to four k splits of a tile are a thread-block cluster (0: never), if all are resident at once:
-        # 8192 x 2048 in four splits at 4 rows 10.1 us, through global memory 11.5; six and more splits gain nothing over slices
-        self.stream_cluster_max_rows = 16
-        self.stream_cluster_max_splits = 4
         # one-group products of up to this many rows stream their weights too (16: never; the kernel takes up to 32), here / on
         # tcgen05, us, 24 rows: 2048 x 2048 7.9 / 12.6, 8192 x 2048 10.4 / 17.4, 2048 x 8192 12.8 / 40, 5120 x 5120 17.2 / 27.4
         self.stream_max_rows = 32
         self.stream_force = None               # (k slices, k splits) for every call, for measurements
-        # (shared memory per block, resident blocks): one-group products and grouped ones of up to 3 rows, or of up to 8 whose weights
-        # are few (`stream_deep_bytes`), in the deeper ring.  us, deeper / other, 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 /
-        # 17.8; 16 rows 8.6 / 10.8, 16.2 / 20.6; one block per multiprocessor with 110 or 200 KiB is slower throughout.
-        # Grouped products of 4, 6 and 8 rows (19 layers of 8 to 128 experts, weights of 12 MB to 1.1 GB; both products of each, in a graph
-        # over several layers' weights), deeper / other, mean of the ratios by the weights' size: to 60 MB 0.96 (36 products), 60 to
-        # 125 0.97 (36), 125 to 300 1.00 (29), more 1.015 (13); single ones lie 0.79 to 1.30 around that, as their last rounds come out
-        self.stream_deep_bytes = 125e6
-        self.stream_shape = [(110 * 1024, 2 * self.sm_count), (74 * 1024, 3 * self.sm_count)]
+        self.stream_shape = self.stream_rings(self.sm_count)
         # Recurrences over prompts: a step whose longest segment has at least so many tokens, `chunk_from` (`chunk_from_few` where its long
         # segments have fewer than 32 heads together), and `chunk_per_brief` more for each of its segments of fewer than 32 tokens (8 in
         # the matrix memory), goes in chunks of 32 on the tensor cores, those short segments token by token behind them.  The token walk
@@ -763,14 +766,8 @@ class CudaKernels(KernelSet):
         and the k splits across blocks so that the work items are many enough to spread evenly, and lends the
         scratch for the partial sums of the splits."""
         swiglu = p.epilogue == EPI_SWIGLU
-        groups = min(p.n_groups, p.M) if grouped else 1
-        rows = max_rows_per_group if even_groups else p.M
-        # how many groups have tokens: all of them, or as many as rows that fall on them at random reach
-        likely = groups if even_groups or groups == 1 else p.n_groups * (1.0 - (1.0 - 1.0 / p.n_groups) ** p.M)
-        deep = not grouped or rows <= 3 or (rows <= 8 and likely * p.N * p.K * (4 if swiglu else 2) < self.stream_deep_bytes)
-        smem, blocks = self.stream_shape[0 if deep else 1]
-        nt = 8 if max_rows_per_group <= 8 else 16 if max_rows_per_group <= 16 else 32
-        slices, splits = self.stream_force or self._stream_cut(rows, p.N, p.K, likely, groups, swiglu, blocks, smem, nt)
+        groups, rows = min(p.n_groups, p.M) if grouped else 1, max_rows_per_group if even_groups else p.M
+        smem, blocks, nt, slices, splits = self._stream_plan(p.M, p.N, p.K, p.n_groups, swiglu, max_rows_per_group, grouped, even_groups)
         tile_rows = 128 // slices
         tiles = -(-p.N // (tile_rows // 2 if swiglu else tile_rows)) * groups
         lib = self._lib("gemm_stream")
@@ -792,9 +789,18 @@ class CudaKernels(KernelSet):
             C.byref(p), max_rows_per_group, slices, 0, blocks, smem, splits, C.c_void_p(_ptr(scratch)),
             C.c_longlong(n_floats), C.c_void_p(_ptr(tickets)), self._tickets_n, C.c_void_p(stream))
 
-    def _stream_cut(self, M: int, N: int, K: int, groups: float, most_groups: int, swiglu: bool, slots: int, smem: int, nt: int):
-        return stream_cut(M, N, K, groups, swiglu, slots, smem, nt, max_slices=4 if nt > 16 else 8, slices_min_rows=1, most_groups=most_groups,
-                          cluster_max_splits=self.stream_cluster_max_splits if M <= self.stream_cluster_max_rows else 0, **self.stream_costs)
+    def _stream_plan(self, M: int, N: int, K: int, n_groups: int, swiglu: bool, max_rows_per_group: int, grouped: bool, even_groups: bool):
+        """(shared memory per block, resident blocks, token columns, k slices, k splits) for a product of M rows (in `n_groups` groups if `grouped`)."""
+        groups, rows = min(n_groups, M) if grouped else 1, max_rows_per_group if even_groups else M
+        # how many groups have tokens: all of them, or as many as rows that fall on them at random reach
+        likely = groups if even_groups or groups == 1 else n_groups * (1.0 - (1.0 - 1.0 / n_groups) ** M)
+        deep = not grouped or rows <= 3 or (rows <= 8 and likely * N * K * (4 if swiglu else 2) < self.stream_deep_bytes)
+        smem, blocks = self.stream_shape[0 if deep else 1]
+        nt = 8 if max_rows_per_group <= 8 else 16 if max_rows_per_group <= 16 else 32
+        slices, splits = self.stream_force or stream_cut(
+            N, K, likely, groups, swiglu, blocks, smem, nt, 4 if nt > 16 else 8,
+            self.stream_cluster_max_splits if rows <= self.stream_cluster_max_rows else 0, **self.stream_costs)
+        return smem, blocks, nt, slices, splits
 
     def attention_tc_error(self) -> int:
         """Error code left by a tcgen05 attention block that gave up waiting (0: none); clears it. Synchronises."""

@@ -1,9 +1,6 @@
-"""Decode products of 17 to 32 rows (tokens that arrive as boxes, up to four k slices a stage) against float64, and the cuts that the
-kernel set chooses for one-group products."""
+"""Decode products of 17 to 32 rows (tokens that arrive as boxes, up to four k slices a stage) against float64."""
 import pytest
 import torch
-
-from spite_b200.kernels.cuda import stream_cut
 
 DEV = "cuda:0"
 
@@ -45,21 +42,6 @@ def test_products_of_17_to_32_rows(force, M, N, K):
     tol = 2.0**-8 * want.abs() + 1.1 * bound[:, :F] * up.abs() + bound[:, F:2 * F] * gate.abs() + 1e-5 * want.abs() + 1e-6
     assert bool(((a.cpu().double() - want).abs() <= tol).all())
     assert ks.launches_by_library["gemm_stream"] == before + 3 and ks.errors() == {}
-
-
-@pytest.mark.parametrize("M", [6, 8, 9, 16, 17, 24, 32])
-@pytest.mark.parametrize("N,K,swiglu", [(40, 64, False), (200, 320, False), (104, 1024, True), (5120, 8192, False), (2048, 2048, False),
-                                        (8192, 5120, True), (129, 4096, False), (16, 64, True), (1024, 16384, False)])
-def test_cuts_of_one_group_products_are_cuts_that_the_kernel_takes(M, N, K, swiglu):
-    nt, smem, slots = (8 if M <= 8 else 16 if M <= 16 else 32), 110 * 1024, 296
-    most = 4 if M > 16 else 8
-    slices, splits = stream_cut(M, N, K, 1, swiglu, slots, smem, nt, item_cost=1.0, split_item_cost=2.0, split_cost=1.0, max_slices=most,
-                                slices_min_rows=6)
-    assert slices <= most and K % (64 * slices) == 0 and not (swiglu and slices == 8)
-    assert 1 <= splits <= max(1, K // (64 * slices) // 4)
-    groups = 1 if nt == 32 else 1024
-    fixed = 24 * 8 + 16 + 4 * groups + (8 - 8 // slices) * 64 * nt * (slices > 1) + 1024
-    assert (smem - fixed) // (16384 + max(1024, slices * nt * 128)) >= 2                      # a ring of at least two stages
 
 
 def test_stream_handles_without_the_undocumented_name(monkeypatch):

@@ -1,28 +1,14 @@
-"""Decode products of one to sixteen rows as the kernel set cuts them: cuts that the kernel takes, sums against float64, and token columns that
-nobody asks for (they hold whatever lay in shared memory) kept out of the others."""
+"""Decode products of one to sixteen rows as the kernel set cuts them: sums against float64, and token columns that nobody asks for (they hold
+whatever lay in shared memory) kept out of the others."""
 import pytest
 import torch
 
-from spite_b200.kernels.cuda import CudaKernels, stream_cut
+from spite_b200.kernels.cuda import CudaKernels
 
+pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("N,K", [(16, 64), (40, 128), (129, 192), (1024, 1024), (2048, 2048), (5120, 8192), (32768, 2048), (200, 16384)])
-@pytest.mark.parametrize("swiglu", [False, True])
-@pytest.mark.parametrize("groups,most", [(1, 1), (1.9, 2), (6.3, 8), (12.2, 16)])
-def test_cuts_are_cuts_that_the_kernel_takes(N, K, swiglu, groups, most):
-    for M in (1, 2, 3, 4, 8, 9, 16) + ((24, 32) if most == 1 else ()):
-        nt = 8 if M <= 8 else 16 if M <= 16 else 32
-        for slots, smem in ((296, 110 * 1024), (444, 74 * 1024)):
-            slices, splits = stream_cut(M, N, K, groups, swiglu, slots, smem, nt, max_slices=4 if nt > 16 else 8, slices_min_rows=1, most_groups=most,
-                                        cluster_max_splits=4, **CudaKernels.stream_costs)
-            assert slices in (1, 2, 4, 8) and K % (64 * slices) == 0 and not (swiglu and slices == 8) and (nt < 32 or slices < 8)
-            assert 1 <= splits <= min(32, K // (64 * slices))                  # no split without a stage
-            assert (smem - 5504 - (8 - 8 // slices) * 64 * nt) // (16384 + max(1024, slices * nt * 128)) >= 2 or slices == 1
-
-
-@pytest.mark.gpu
 @pytest.mark.parametrize("N,K", [(40, 64), (129, 192), (1024, 4096), (2048, 2048), (4096, 1024)])
 def test_few_rows_against_float64(N, K):
     """A float32 sum of K products: each of its at most K roundings is below 2^-24 of the sum of magnitudes."""

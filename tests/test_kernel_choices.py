@@ -1,64 +1,87 @@
-"""How the weight-streaming kernel's work is cut (k slices inside a block, k splits across blocks): the host-side
-choice alone, at the shapes it was measured on and at its borders.  The kernel itself with every cut:
+"""How the weight-streaming kernel's work is cut (ring, k slices inside a block, k splits across blocks): the kernel set's own choice on the host,
+at shapes it was measured on and at its borders.  The kernel itself with every cut:
 test_gpu_kernels.py::test_streaming_products_with_k_slices_and_k_splits."""
 import pytest
 
-from spite_b200.kernels.cuda import stream_cut
+from spite_b200.kernels.cuda import CudaKernels, stream_cut
 
-FEW = dict(slots=296, smem=110 * 1024)        # up to three tokens: two blocks a multiprocessor
-MORE = dict(slots=444, smem=74 * 1024)        # more: three
-
-
-def cut(M, N, K, groups=1, swiglu=False, **kw):
-    shape = dict(FEW if M <= 3 else MORE)
-    shape.update(kw)
-    return stream_cut(M, N, K, groups, swiglu, shape.pop("slots"), shape.pop("smem"), 8 if M <= 8 else 16, **shape)
+DEEP, OTHER = CudaKernels.stream_rings(148)
 
 
-def test_the_measured_shapes_get_the_cuts_that_were_fastest():
-    # eight tokens at Scout's layer shapes: slices, no partial sums through global memory
-    assert cut(8, 7168, 5120) == (4, 1)                       # qkv: 224 tiles of 32 rows
-    assert cut(8, 5120, 5120) == (8, 1)                       # output projection: 320 tiles of 16 rows
-    assert cut(8, 5120, 8192) == (8, 1)                       # shared expert, down
-    assert cut(8, 8192, 5120, groups=7, swiglu=True)[1] == 1  # seven experts' gate/up: tiles enough without k splits
-    assert cut(8, 5120, 8192, groups=7) == (4, 1)             # (if the caller allows slices for grouped products)
-    assert cut(8, 5120, 8192, groups=7, max_slices=1)[0] == 1
-    # one token: tiles of 128 rows, k splits that fill 296 blocks about once
-    assert cut(1, 7168, 5120) == (1, 5)
-    assert cut(1, 5120, 5120) == (1, 7)
-    assert cut(1, 8192, 5120, swiglu=True) == (1, 2)
-    # the output head has tiles enough as it is
-    assert cut(1, 202048, 5120) == (1, 1) and cut(8, 202048, 5120)[1] == 1
+def chooser(**changed):
+    ks = object.__new__(CudaKernels)                          # the choice alone: no device
+    ks.stream_shape, ks.stream_force = ks.stream_rings(148), None
+    for name, value in changed.items():
+        assert hasattr(ks, name)
+        setattr(ks, name, value)
+    return ks
 
 
-@pytest.mark.parametrize("M", [1, 2, 3, 4, 8, 13, 16])
-@pytest.mark.parametrize("N,K,swiglu", [(40, 64, False), (200, 320, False), (104, 1024, True), (5120, 8192, False),
-                                        (8192, 5120, True), (129, 4096, False), (16, 64, True)])
-@pytest.mark.parametrize("groups", [1, 5])
-def test_every_cut_is_one_the_kernel_takes(M, N, K, swiglu, groups):
-    slices, splits = cut(M, N, K, groups=min(groups, M), swiglu=swiglu)
+def plan(M, N, K, swiglu=False, experts=0, ks=None):
+    return (ks or chooser())._stream_plan(M, N, K, experts or 1, swiglu, M, experts > 0, False)
+
+
+def cut(*args, **kw):
+    return plan(*args, **kw)[3:]
+
+
+# rows, N, K, SwiGLU, experts: the cuts within 5 % of the fastest of all, each measured behind a norm in a graph over several layers' weights
+MEASURED = [
+    ((1, 7168, 5120, False, 0), {(4, 1), (1, 4), (1, 3), (2, 2)}), ((8, 7168, 5120, False, 0), {(4, 1), (1, 4)}),
+    ((1, 5120, 5120, False, 0), {(1, 6), (1, 7), (2, 3), (1, 3)}), ((8, 5120, 5120, False, 0), {(1, 4), (1, 3), (2, 3)}),
+    ((8, 5120, 8192, False, 0), {(1, 4), (2, 3), (1, 3)}), ((8, 4096, 4096, False, 0), {(8, 1), (4, 2), (1, 4)}),
+    ((4, 8192, 2048, False, 0), {(4, 1), (1, 4)}), ((16, 8192, 2048, False, 0), {(4, 1)}),
+    ((1, 2048, 2048, False, 0), {(1, 8), (8, 1), (1, 7), (2, 4), (2, 8), (4, 4)}), ((4, 2048, 2048, False, 0), {(2, 4), (4, 4), (2, 8), (4, 2), (8, 1)}),
+    ((24, 2048, 2048, False, 0), {(4, 4), (4, 3)}), ((24, 5120, 16384, False, 0), {(2, 3)}), ((24, 8192, 2048, True, 0), {(2, 1)}),
+    ((1, 8192, 5120, True, 0), {(2, 1), (1, 2)}), ((8, 8192, 5120, True, 0), {(2, 1), (1, 2)}), ((3, 4864, 8192, True, 0), {(1, 3)}),
+    ((8, 12544, 12288, False, 0), {(2, 1), (1, 2), (1, 3)}),
+    ((8, 1024, 2048, True, 32), {(2, 1)}), ((8, 2048, 1024, False, 32), {(2, 1)}), ((16, 2048, 2048, False, 16), {(2, 1), (1, 2), (4, 1)}),
+    ((3, 1024, 2048, True, 16), {(4, 1), (1, 4), (1, 3), (2, 3)}), ((1, 8192, 5120, True, 16), {(2, 1), (1, 2)}),
+    ((8, 8192, 5120, True, 16), {(2, 1), (1, 1), (4, 1), (1, 2), (2, 2)}), ((8, 5120, 8192, False, 16), {(4, 1), (1, 4), (2, 3), (1, 3)})]
+
+
+@pytest.mark.parametrize("shape,fast", MEASURED, ids=lambda v: "x".join(str(int(x)) for x in v) if isinstance(v, tuple) else "")
+def test_the_measured_shapes_get_a_cut_among_the_fastest(shape, fast):
+    assert cut(*shape) in fast
+
+
+def test_the_ring():
+    """One-group products and few rows run in the deeper ring, experts' products of four to eight rows while their weights are few."""
+    ring = lambda *a, **kw: plan(*a, **kw)[:2]
+    assert all(ring(M, 7168, 5120) == DEEP for M in (1, 8, 16, 24, 32))
+    assert all(ring(M, 8192, 5120, True, 16) == (DEEP if M <= 3 else OTHER) for M in range(1, 17))
+    assert all(ring(M, 1024, 2048, True, 32) == (DEEP if M <= 8 else OTHER) for M in range(1, 17))          # 60 MB at eight rows
+    likely = 16 * (1 - (15 / 16) ** 8)                        # experts that eight rows reach of 16
+    at_line = int(CudaKernels.stream_deep_bytes / (likely * 4096 * 2))
+    assert ring(8, at_line, 4096, False, 16) == DEEP and ring(8, at_line + 1, 4096, False, 16) == OTHER
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 6, 8, 9, 13, 16, 17, 24, 32])
+@pytest.mark.parametrize("N,K,swiglu", [(40, 64, False), (200, 320, False), (104, 1024, True), (5120, 8192, False), (2048, 2048, False),
+                                        (8192, 5120, True), (129, 4096, False), (16, 64, True), (1024, 16384, False), (202048, 5120, False)])
+@pytest.mark.parametrize("experts", [0, 2, 8, 128])
+def test_every_cut_is_one_the_kernel_takes(M, N, K, swiglu, experts):
+    if experts and M > 16:
+        return                                                 # grouped products of more rows go elsewhere
+    smem, blocks, nt, slices, splits = plan(M, N, K, swiglu, experts)
+    assert (smem, blocks) in (DEEP, OTHER) and nt == (8 if M <= 8 else 16 if M <= 16 else 32)
     assert slices in (1, 2, 4, 8) and K % (64 * slices) == 0          # a stage is `slices` k blocks of 64
-    assert not (swiglu and slices == 8)                                # tiles of 8 gate and 8 up rows are not built
-    assert slices == 1 or M >= 4                                       # few rows keep tiles of 128 rows (the function's default)
-    stages = K // (64 * slices)
-    assert 1 <= splits <= max(1, stages // 4)                          # at least four stages stay together
-    nt = 8 if M <= 8 else 16
-    smem = (FEW if M <= 3 else MORE)["smem"]
-    ring = (smem - 5504 - (8 - 8 // slices) * 64 * nt) // (16384 + max(1024, slices * nt * 128))
-    assert ring >= 2                                                   # a ring of at least two stages fits
+    assert not (swiglu and slices == 8) and not (nt == 32 and slices == 8)     # tiles that are not built
+    assert 1 <= splits <= min(32, K // (64 * slices))                  # no split without a stage
+    fixed = 24 * 8 + 16 + 4 * (1 if nt == 32 else 1024) + (8 - 8 // slices) * 64 * nt * (slices > 1) + 1024
+    assert (smem - fixed) // (16384 + max(1024, slices * nt * 128)) >= 2       # a ring of at least two stages fits
 
 
-def test_splits_that_can_be_a_cluster_are_preferred_when_the_caller_offers_clusters():
-    assert cut(1, 7168, 5120, cluster_max_splits=4, cluster_cost=9.0) == (1, 4)      # qkv: 224 blocks, 56 clusters of four
-    assert cut(1, 5120, 5120, cluster_max_splits=4, cluster_cost=9.0) == (1, 7)      # too few blocks in fours
-    assert cut(1, 8192, 5120, swiglu=True, cluster_max_splits=4, cluster_cost=9.0) == (1, 2)
-    # never more blocks than are resident at once: 128 tiles in four splits are 512 blocks for 296 places
-    assert cut(1, 8192, 5120, swiglu=True, cluster_max_splits=4, cluster_cost=0.0) == (1, 2)
+def test_splits_that_can_be_a_cluster():
+    """The cost of a cluster is asked only of two to four splits without slices whose blocks are all resident at once."""
+    kw = dict(CudaKernels.stream_costs, split_item_cost=1000.0, cluster_cost=0.0, slice_each=1000.0)
+    one = lambda N, groups=1, most=1, clusters=4: stream_cut(N, 5120, groups, most, False, 296, DEEP[0], 8, 8, clusters, **kw)
+    assert one(7168) == (1, 4) and one(7168, clusters=3) == (1, 3) and one(7168, clusters=0) == (1, 1)
+    assert one(128 * 75) == (1, 3)                                     # 75 tiles in fours are 300 blocks for 296 places
+    assert one(128 * 37, 1.9, 2) == (1, 4) and one(128 * 38, 1.9, 2) == (1, 3)        # ... of all groups that there may be
+    # the kernel set offers clusters up to stream_cluster_max_rows rows
+    assert cut(1, 5120, 2048, True) == (2, 1) and cut(1, 5120, 2048, True, ks=chooser(stream_cluster_max_rows=0)) == (1, 3)
 
 
-def test_the_costs_move_the_choice():
-    assert cut(8, 5120, 5120, max_slices=1)[0] == 1                    # tiles of 128 rows only: k splits again
-    assert cut(8, 5120, 5120, max_slices=1)[1] > 1
-    assert cut(2, 5120, 5120, slices_min_rows=1)[0] > 1                # slices allowed at two rows
-    assert cut(8, 5120, 5120, slice_cost=100.0)[0] == 1                # slices made expensive
-    assert cut(1, 5120, 5120, split_item_cost=1000.0) == (1, 1)        # splits made expensive
+def test_a_choice_made_for_every_call():
+    assert cut(8, 5120, 5120, ks=chooser(stream_force=(4, 2))) == (4, 2)
