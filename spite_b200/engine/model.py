@@ -31,6 +31,10 @@ def resolve_dtype(dtype) -> torch.dtype:
 
 
 class Model:
+    #: most rows of logits whose factor is multiplied in by the head's product (it reads the factor from a vector of so many copies, 16 KB): decode steps
+    #: and prompt portions ask for one row a request; a step that asks for more, all of a long prompt's, takes a pass over the logits
+    scaled_logit_rows = 4096
+
     def __init__(self, plan: ModelPlan, *, dtype="bfloat16", device="cuda:0", kernels=None, config=None):
         self.plan = plan.validate()
         self.config = config
@@ -54,7 +58,7 @@ class Model:
         self.position_table = None
         self._logit_scales = None
         if plan.logit_scale != 1.0 and plan.logit_softcap is None:
-            self._logit_scales = torch.full((4096,), plan.logit_scale, dtype=torch.float32, device=self.device)
+            self._logit_scales = torch.full((self.scaled_logit_rows,), plan.logit_scale, dtype=torch.float32, device=self.device)
         self._ones = None if plan.streams is None else torch.ones(plan.streams, dtype=torch.float32, device=self.device)
         #: if set, called as `layer_tap(i, h)` after the i-th layer run of the order with the float32 residual
         #: stream (the sum of the streams, if there are several; for comparing a model layer by layer; the step then cannot be captured in a graph)
@@ -244,7 +248,7 @@ class Model:
                 self.final_norm.forward(h, x, rows=batch.logit_rows)
             else:
                 h.enter(self._ones, self.final_norm, x, rows=batch.logit_rows, last=True)
-            if self._logit_scales is not None and R <= self._logit_scales.numel():
+            if self._logit_scales is not None and R <= self.scaled_logit_rows:
                 # a factor alone is the product's own: the same number as of the stored sums, without a pass over the logits
                 k.linear(x, self.head_weight, logits, row_scale=self._logit_scales[:R])
                 return logits
