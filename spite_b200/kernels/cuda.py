@@ -224,7 +224,8 @@ def stream_cut(N: int, K: int, groups: float, most_groups: int, swiglu: bool, sl
     return best
 
 
-def attention_cut_pays(segments, window, pair_tokens: int, kv_heads: int, blocks: int) -> bool:
+@functools.lru_cache(maxsize=256)
+def attention_cut_pays(segments: tuple, window, pair_tokens: int, kv_heads: int, blocks: int) -> bool:
     """Whether the prompt portions (first position, tokens) of a step are faster on the tcgen05 attention kernel with its work cut along the keys
     into equal shares than with whole items (a pair of row tiles, `pair_tokens` tokens, and a kv head) dealt out round by round.
 
@@ -233,7 +234,10 @@ def attention_cut_pays(segments, window, pair_tokens: int, kv_heads: int, blocks
     24 for the parts that begin and end in it (another start 6, their outputs 3, the line that is cut 3) and for adding the parts up behind
     them (6 to 12).  us, whole / cut, 40 heads, 8 kv heads of 128: 2,048 tokens behind 6,144 361 / 306, 1,000 behind 7,192 254 / 173, 500 behind
     7,692 142 / 100, 100 behind 8,092 141 / 39, 50 behind 8,142 140 / 36, three portions of 683 behind 7,500 410 / 344; 2,048 from the start 70 / 87,
-    1,048 behind 1,000 60 / 67, 500 behind 500 27 / 35.  Of 80 shapes (four kinds of heads) the rule takes the slower one three times, by 0, 1 and 8 %."""
+    1,048 behind 1,000 60 / 67, 500 behind 500 27 / 35.  Of 80 shapes (four kinds of heads) the rule takes the slower one three times, by 0, 1 and 8 %.
+
+    The layers of a step ask the same, so the last answers are kept by the numbers they follow from: 64 portions cost the host 55 to 85 us, asked
+    again 6."""
     runs, items, tiles = [], 0, 0.0                          # (items up to the run's end, tiles of its first, of its last)
     for start, n in reversed(segments):
         pairs, end, near = -(-n // pair_tokens), start + n - 1, start + min(n, pair_tokens) - 1
@@ -1102,7 +1106,7 @@ class CudaKernels(KernelSet):
                                  n_segments=len(batch.segments), tokens_per_block=tpb_tc, n_splits=1,
                                  seg_min_tokens=tc_from, seg_max_tokens=0x7fffffff)
                 lib, st, cut = self._lib("attention_tc"), -2, False
-                if attention_cut_pays([(s.start_pos, s.n_tokens) for s in batch.segments if s.n_tokens >= tc_from], window, 2 * tpb_tc,
+                if attention_cut_pays(tuple([(s.start_pos, s.n_tokens) for s in batch.segments if s.n_tokens >= tc_from]), window, 2 * tpb_tc,
                                       c.num_kv_heads, self.sm_count):
                     n_floats = self.sm_count * (4 * (c.head_dim + 2) * 128 + 4)
                     part = torch.empty(n_floats, dtype=torch.float32, device=q.device)

@@ -13,13 +13,13 @@ BLOCKS = 148
     ([(0, 2048)], False), ([(1000, 1048)], False), ([(500, 500)], False), ([], False)])
 @pytest.mark.parametrize("window", [Window("full", 0), Window("chunk", 8192)], ids=["full", "chunk"])
 def test_the_faster_form(segments, cut, window):
-    assert attention_cut_pays(segments, window, 50, 8, BLOCKS) is cut
+    assert attention_cut_pays(tuple(segments), window, 50, 8, BLOCKS) is cut
 
 
 def test_a_window_bounds_what_a_cut_can_give():
     """128 keys a token are three tiles: no item is long enough to share."""
-    assert attention_cut_pays([(8092, 100)], Window("full", 0), 50, 8, BLOCKS)
-    assert not attention_cut_pays([(8092, 100)], Window("sliding", 128), 50, 8, BLOCKS)
+    assert attention_cut_pays(((8092, 100),), Window("full", 0), 50, 8, BLOCKS)
+    assert not attention_cut_pays(((8092, 100),), Window("sliding", 128), 50, 8, BLOCKS)
 
 
 @pytest.mark.parametrize("segments", [[(0, 1)], [(0, 33), (4000, 900), (7, 129)], [(100, 2048)] * 30, [(131000, 2048)], [(0, 16400)]])
@@ -39,4 +39,15 @@ def test_against_every_item_dealt_out(segments, window, pair, heads):
         sums[BLOCKS - 1 - at if round_ & 1 else at] += cost
     whole, cut = max(sums), max(8.0, sum(items) / BLOCKS) + 24
     if not 0.8 < whole / cut < 1.25:
-        assert attention_cut_pays(segments, window, pair, heads, BLOCKS) is (cut < whole)
+        assert attention_cut_pays(tuple(segments), window, pair, heads, BLOCKS) is (cut < whole)
+
+
+def test_the_layers_of_a_step_ask_once():
+    """48 layers, three of four with another window: two answers are made, and other portions make others."""
+    segments = tuple((100 + i, 40 + i) for i in range(64))
+    attention_cut_pays.cache_clear()
+    for layer in range(48):
+        attention_cut_pays(tuple(segments), Window("chunk", 8192) if layer % 4 else Window("full", 0), 50, 8, BLOCKS)
+    assert attention_cut_pays.cache_info().misses == 2
+    attention_cut_pays(segments[:-1] + ((163, 104),), Window("full", 0), 50, 8, BLOCKS)
+    assert attention_cut_pays.cache_info().misses == 3
