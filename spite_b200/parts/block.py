@@ -28,6 +28,13 @@ import torch
 
 from ..config.specs import ConfigError
 from .base import Block, register_block, side_stream
+from .norm import RmsNorm
+
+
+def _runs(part, cls) -> bool:
+    """Does the part run `cls.forward` itself?  A class derived from it with a forward of its own, and a part whose forward somebody has wrapped,
+    neither take nor leave anything between layers."""
+    return getattr(part.forward, "__func__", None) is cls.forward
 
 
 @register_block("prenorm_residual")
@@ -95,12 +102,11 @@ class SandwichResidual(Block):
             if n is not None and (n.kind != "rms_norm" or n.eps != self.mixer_norm.eps):
                 raise ConfigError("sandwich_residual fuses its norms into one kernel: RMS norms with one epsilon")
 
-    # (a class that runs the sublayers in its own way neither takes nor leaves anything)
     def entry(self):
-        return (self.mixer_norm.weight, self.mixer_norm.eps) if type(self).forward is SandwichResidual.forward else None
+        return (self.mixer_norm.weight, self.mixer_norm.eps) if _runs(self, SandwichResidual) and _runs(self.mixer_norm, RmsNorm) else None
 
     def leaves(self, entry):
-        return type(self).forward is SandwichResidual.forward and entry is not None and entry[1] in (None, self.mixer_norm.eps)
+        return _runs(self, SandwichResidual) and entry is not None and entry[1] in (None, self.mixer_norm.eps)
 
     def _last(self, y, norm, eps, h, leave):
         """The block's last kernel: norm, factor and sum, and what the next block's first kernel would make of the stream."""
@@ -148,10 +154,10 @@ class PostNormResidual(Block):
     _run, _last = SandwichResidual._run, SandwichResidual._last
 
     def entry(self):
-        return (None, None) if type(self).forward is PostNormResidual.forward and self.ctx.dtype != torch.float32 else None
+        return (None, None) if _runs(self, PostNormResidual) and self.ctx.dtype != torch.float32 else None
 
     def leaves(self, entry):
-        return type(self).forward is PostNormResidual.forward and entry is not None and entry[1] in (None, self.mixer_out_norm.eps)
+        return _runs(self, PostNormResidual) and entry is not None and entry[1] in (None, self.mixer_out_norm.eps)
 
     def forward(self, h, batch, cache, entered=None, leave=None):
         k = self.k
