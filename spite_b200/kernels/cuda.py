@@ -225,26 +225,34 @@ def stream_cut(N: int, K: int, groups: float, most_groups: int, swiglu: bool, sl
 
 
 @functools.lru_cache(maxsize=256)
-def attention_cut_pays(segments: tuple, window, pair_tokens: int, kv_heads: int, blocks: int) -> bool:
+def attention_cut_pays(segments: tuple, window, pair_tokens: int, kv_heads: int, blocks: int, key_bytes: int) -> bool:
     """Whether the prompt portions (first position, tokens) of a step are faster on the tcgen05 attention kernel with its work cut along the keys
     into equal shares than with whole items (a pair of row tiles, `pair_tokens` tokens, and a kv head) dealt out round by round.
 
     Both are estimated in tiles of 64 keys (1.1 us).  An item costs its tiles and 6 more; items are dealt out from the last portion's end backwards,
     one a block and round, in alternating direction, and the longest of five blocks' sums counts; a share costs its part of all that and
     24 for the parts that begin and end in it (another start 6, their outputs 3, the line that is cut 3) and for adding the parts up behind
-    them (6 to 12).  us, whole / cut, 40 heads, 8 kv heads of 128: 2,048 tokens behind 6,144 361 / 306, 1,000 behind 7,192 254 / 173, 500 behind
+    them (6 to 12).  us, whole / cut, 40 heads, 8 kv heads of 128: 2,048 tokens behind 6,144 403 / 343, 1,000 behind 7,192 279 / 198, 500 behind
     7,692 142 / 100, 100 behind 8,092 141 / 39, 50 behind 8,142 140 / 36, three portions of 683 behind 7,500 410 / 344; 2,048 from the start 70 / 87,
-    1,048 behind 1,000 60 / 67, 500 behind 500 27 / 35.  Of 80 shapes (four kinds of heads) the rule takes the slower one three times, by 0, 1 and 8 %.
+    1,048 behind 1,000 60 / 67, 500 behind 500 27 / 35.
+
+    Blocks with whole items walk the same keys at about the same time and share them in L2; shares begin anywhere.  Once the portions see more
+    keys than L2 holds (about 100 MB; `key_bytes`: of a position of one kv head, its value included) what each block fetches for itself comes
+    from memory: a tile costs up to 17 % more with 512 bytes a key (2 x 128 bfloat16), as good as nothing with 256.  8,192 tokens at a context of 16,384 / 32,768
+    / 65,536 / 131,072 (67 to 537 MB), whole / cut, ms: 1.98 / 1.99, 4.46 / 4.74, 9.49 / 10.57, 19.6 / 22.2; 2,048 tokens at 131,072 6.64 / 5.74.
+    Over 83 such shapes (1,000 to 8,192 tokens, 8,192 to 131,072 keys, four kinds of heads) the choice takes 0.04 % more than the faster form of each;
+    of 38 others (three more kinds of heads, several portions, one plane) it takes the slower form four times, by 3 to 5 %.
 
     The layers of a step ask the same, so the last answers are kept by the numbers they follow from: 64 portions cost the host 55 to 85 us, asked
     again 6."""
-    runs, items, tiles = [], 0, 0.0                          # (items up to the run's end, tiles of its first, of its last)
+    runs, items, tiles, keys = [], 0, 0.0, 0                 # (items up to the run's end, tiles of its first, of its last)
     for start, n in reversed(segments):
         pairs, end, near = -(-n // pair_tokens), start + n - 1, start + min(n, pair_tokens) - 1
         longest = (end - window.lowest_visible(max(start, end - pair_tokens + 1))) / 64 + 1
         shortest = (near - window.lowest_visible(start)) / 64 + 1
         items += pairs * kv_heads
         tiles += pairs * kv_heads * (longest + shortest) / 2
+        keys += end + 1 - window.lowest_visible(start)
         runs.append((items, longest, shortest))
     if items <= blocks:
         whole = 6 + max((max(a, b) for _, a, b in runs), default=0.0)
@@ -261,7 +269,11 @@ def attention_cut_pays(segments: tuple, window, pair_tokens: int, kv_heads: int,
                 end, longest, shortest = runs[run]
                 sums[4 - i if round_ & 1 else i] += 6 + longest - (longest - shortest) * (at - begin) / (end - begin)
         whole = max(sums)
-    return max(8.0, (tiles + 6 * items) / blocks) + 24 < whole
+    share = max(8.0, (tiles + 6 * items) / blocks)
+    seen = keys * kv_heads * key_bytes
+    if key_bytes > 256 and seen > 100e6:
+        share *= 1 + 0.17 * (1 - 100e6 / seen)
+    return share + 24 < whole
 
 
 class CudaKernels(KernelSet):
@@ -1107,7 +1119,7 @@ class CudaKernels(KernelSet):
                                  seg_min_tokens=tc_from, seg_max_tokens=0x7fffffff)
                 lib, st, cut = self._lib("attention_tc"), -2, False
                 if attention_cut_pays(tuple([(s.start_pos, s.n_tokens) for s in batch.segments if s.n_tokens >= tc_from]), window, 2 * tpb_tc,
-                                      c.num_kv_heads, self.sm_count):
+                                      c.num_kv_heads, self.sm_count, cache.kv.shape[0] * c.head_dim * cache.kv.element_size()):
                     n_floats = self.sm_count * (4 * (c.head_dim + 2) * 128 + 4)
                     part = torch.empty(n_floats, dtype=torch.float32, device=q.device)
                     st = lib.spite_paged_attention_tc_cut(
