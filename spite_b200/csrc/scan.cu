@@ -815,9 +815,16 @@ int launch_state_space_chunks(const ScanParams& p, const float* a, long long a_s
     if (cudaGetLastError() != cudaSuccess) return SPITE_LAUNCH_FAILED;
     chunk::Walk w = scan_walk(p, out);
     w.skip = p.skip;
-    // 32 columns a block: two blocks of four warps on a multiprocessor wait for each other's barriers less than one of eight with 64
-    // columns does.  us, 64 / 32 columns, the same bits: 128 heads of 128 x 64, one request of 2,048 tokens 199 / 175, five of 410
-    // 224 / 195; 64 heads, five of 410 134 / 117; 64 x 64, 64 heads, three of 666 79 / 61; 16 columns 253 in the first
+    // 32 columns a block: two blocks of four warps on a multiprocessor (three up to 64 keys) wait for each other's barriers less than one of
+    // eight with 64 columns does.  us, 64 / 32 columns, the same bits: 128 heads of 128 x 64, one request of 2,048 tokens 199 / 175, five of 410
+    // 224 / 195; 64 heads, five of 410 134 / 117; 64 x 64, 64 heads, three of 666 79 / 61; 16 columns 253 in the first.
+    // 64 where all blocks are resident at once that way and not with 32: of blocks for up to 64 keys a multiprocessor holds three with 32
+    // columns, two with 64.  With the first kernel, 64 / 32: 64 heads of 64 x 64, four of 2,048 288 / 325, 16 heads of 64 x 128, eight of 2,048
+    // 366 / 403, eight of 256 69 / 75; with half or twice the blocks 187 / 177 and 538 / 521, 228 / 218; of 128 x 128, as many blocks 579 / 532.
+    if constexpr (DP == 64) {
+        const long long groups = (long long)p.heads * out.numbering.segments;
+        if ((p.vdim + 63) / 64 * groups <= 2 * 148 && (p.vdim + 31) / 32 * groups > 3 * 148) return launch_walk<DP / 2, 2, 4, HEAD_DECAY>(w, s_waits, st);
+    }
     return launch_walk<DP / 2, 2, 2, HEAD_DECAY>(w, s_waits, st);
 }
 template <int DP, bool BONUS>
