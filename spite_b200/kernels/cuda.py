@@ -179,7 +179,8 @@ def _check(status, what):
 
 @functools.lru_cache(maxsize=4096)
 def stream_cut(N: int, K: int, groups: float, most_groups: int, swiglu: bool, slots: int, smem: int, nt: int, max_slices: int, cluster_max_splits: int, *,
-               item_cost: float, split_item_cost: float, split_cost: float, slice_each: float, lone_rate: float, cluster_cost: float):
+               slice_each: float, split_item_cost: float, split_cost: float, cluster_cost: float, lone_rate: float, lone_rate_slices: float,
+               token_cost: float):
     """(k slices inside a block, k splits across blocks) of the weight-streaming kernel for a product of N output columns
     (per group) and depth K on `slots` resident blocks of `smem` bytes, `nt` token columns.
 
@@ -190,11 +191,12 @@ def stream_cut(N: int, K: int, groups: float, most_groups: int, swiglu: bool, sl
     splits across blocks (partial sums through global memory, a ticket, a second pass over as many partial
     tiles as there are splits).  The cost of a choice, in stages of 16 KiB on all blocks: the stages of its full rounds of
     items; those of its last round, which cost as much less as there are fewer items, since a block that shares the memory with fewer
-    others pulls up to `lone_rate` times as much; and for every round what an item costs besides its stages: `item_cost` for any,
-    `split_item_cost` + `split_cost` a split if its sums cross blocks through global memory, `cluster_cost` if the splits, no more than
-    `cluster_max_splits`, can be one thread-block cluster with all clusters resident at once (of `most_groups` groups, where `groups`
-    is how many are expected to have tokens), `slice_each` a slice if slices meet in shared memory.  (The kernel set's costs are
-    `CudaKernels.stream_costs`.)"""
+    others pulls up to `lone_rate` times as much (`lone_rate_slices` with slices); a stage brings the tokens of its slices too
+    (`token_cost` of their bytes, which come from L2); and for every round what an item costs besides its stages: `split_item_cost` +
+    `split_cost` a split if its sums cross blocks through global memory (a split's sums are fewer with lower tiles and
+    more with more tokens), `cluster_cost` if the splits, no more than `cluster_max_splits`, can be one thread-block cluster with all
+    clusters resident at once (of `most_groups` groups, where `groups` is how many are expected to have tokens), `slice_each` a slice if
+    slices meet in shared memory.  (The kernel set's costs are `CudaKernels.stream_costs`.)"""
     best, best_cost = (1, 1), None
     for slices in (1, 2, 4, 8):
         if K % (64 * slices) or (swiglu and slices == 8):
@@ -208,15 +210,17 @@ def stream_cut(N: int, K: int, groups: float, most_groups: int, swiglu: bool, sl
         row_tiles = -(-N // (rows // 2 if swiglu else rows))
         tiles = row_tiles * groups
         stages = K // (64 * slices)
-        for s in range(1, min(32, stages) + 1):
+        lone = 1.0 / (lone_rate_slices if slices > 1 else lone_rate)
+        stage_cost = 1.0 + token_cost * slices * nt / 128
+        for s in range(1, min(16, stages) + 1):
             full = tiles * s // slots
             rest = tiles * s - full * slots
-            fixed = item_cost + (slice_each * slices if slices > 1 else 0.0)
+            fixed = slice_each * slices if slices > 1 else 0.0
             if s > 1 and slices == 1 and s <= cluster_max_splits and row_tiles * most_groups * s <= slots:
                 fixed += cluster_cost                         # the splits as one cluster: their sums meet in shared memory
             elif s > 1:
-                fixed += split_item_cost + split_cost * s
-            cost = (full + (max(rest / slots, 1.0 / lone_rate) if rest else 0.0)) * -(-stages // s) + (full + (rest > 0)) * fixed
+                fixed += split_item_cost + split_cost * s * math.sqrt(nt / 8) / slices
+            cost = (full + (max(rest / slots, lone) if rest else 0.0)) * -(-stages // s) * stage_cost + (full + (rest > 0)) * fixed
             if best_cost is None or cost < best_cost:
                 best, best_cost = (slices, s), cost
             if tiles * s >= 4 * slots:
@@ -277,17 +281,20 @@ def attention_cut_pays(segments: tuple, window, pair_tokens: int, kv_heads: int,
 
 
 class CudaKernels(KernelSet):
-    #: What a work item costs besides its stages, and what is left of them where blocks are alone (see stream_cut), in stages of 16 KiB.
-    #: Found by search over 240 one-group products (1024 x 1024 to 5120 x 16384, with and without SwiGLU, 1 to 32 rows, each after a
-    #: norm in a graph, against every cut): the choice is 1.3 % slower than the best cut on average; the costs before, with slices
-    #: from six rows and clusters to three only, 7.4 %.  us, before / now: 2048 x 2048 at 1 / 4 / 8 rows 7.5 / 6.2, 8.9 / 6.4, 6.4 /
-    #: 6.4; 4096 x 2048 7.8 / 6.6, 9.0 / 6.8, 6.9 / 6.9; 1024 x 4096 9.8 / 7.1, 9.9 / 7.1, 9.2 / 7.1; 5120 x 16384 at 24 rows 58.5 / 50.3.
-    #: The same costs over 45 products of grouped rows (16 or 32 experts, 1 to 16 rows): 1.0 % from the best, before 7.1 %.
-    stream_costs = dict(item_cost=4.0, split_item_cost=1.5, split_cost=0.5, slice_each=0.25, lone_rate=1.25, cluster_cost=8.0)
-    #: Up to this many rows two to four k splits of a tile are a thread-block cluster (0: never), if all are resident at once:
-    #: 8192 x 2048 in four splits at 4 rows 10.1 us, through global memory 11.5; six and more splits gain nothing over slices.
+    #: What a work item costs besides its stages, and what is left of them where blocks are alone (see stream_cut), in stages of 16 KiB.  Found
+    #: by search over half of 3,209 products drawn at random (256 to 32,768 columns, depths of 256 to 16,384, with and without SwiGLU,
+    #: 1 to 32 rows, three of ten of 8 to 128 experts, each after a norm in a graph, against every cut); on the other half the choice is
+    #: 1.6 % slower than the best cut on average, and more than 10 % for 3.6 % of them; with the costs before, found over 285
+    #: products of rounder sizes, 2.9 % and 10 %.  us, before / now: SwiGLU 3584 x 14336 at 16 rows 60 / 54, 1536 x 2880 at 16 12.6 / 10.8;
+    #: 6144 x 5120 at 32 rows 29.4 / 24.4; 2048 x 2048 at 8 rows 6.4 / 6.4.
+    stream_costs = dict(slice_each=0.37, split_item_cost=2.1, split_cost=0.65, cluster_cost=4.0, token_cost=0.21)
+    #: (one slice, several) in the deeper ring, in the other
+    stream_lone_rates = ((1.42, 1.22), (1.78, 1.53))
+    #: Up to this many rows two to four k splits of a tile are a thread-block cluster (0: never), if all are resident at once; in the other ring
+    #: two.  Over 2,632 products, cluster / through global memory, mean: deeper ring, two to four splits 0.94 to 0.97, six and more 0.95 to
+    #: 1.06; the other ring, two 0.98, three 1.00, four 1.03, six 1.1.
     stream_cluster_max_rows = 16
-    stream_cluster_max_splits = 4
+    stream_cluster_max_splits = (4, 2)
 
     #: One-group products and grouped ones of up to 3 rows, or of up to 8 whose weights are few (this many bytes), run in the deeper ring.  us, deeper /
     #: other, 8 rows: 8192 x 2048 7.7 / 9.1, 7168 x 5120 14.5 / 17.8; 16 rows 8.6 / 10.8, 16.2 / 20.6; one block per multiprocessor with 110
@@ -782,13 +789,13 @@ class CudaKernels(KernelSet):
         and the k splits across blocks so that the work items are many enough to spread evenly, and lends the
         scratch for the partial sums of the splits."""
         swiglu = p.epilogue == EPI_SWIGLU
-        groups, rows = min(p.n_groups, p.M) if grouped else 1, max_rows_per_group if even_groups else p.M
-        smem, blocks, nt, slices, splits = self._stream_plan(p.M, p.N, p.K, p.n_groups, swiglu, max_rows_per_group, grouped, even_groups)
+        groups = min(p.n_groups, p.M) if grouped else 1
+        smem, blocks, nt, slices, splits, cluster = self._stream_plan(p.M, p.N, p.K, p.n_groups, swiglu, max_rows_per_group, grouped, even_groups)
         tile_rows = 128 // slices
         tiles = -(-p.N // (tile_rows // 2 if swiglu else tile_rows)) * groups
         lib = self._lib("gemm_stream")
         stream = self._raw_stream()
-        if slices == 1 and 2 <= splits <= self.stream_cluster_max_splits and rows <= self.stream_cluster_max_rows:
+        if cluster:
             # the k splits of a tile as one thread-block cluster: their sums meet in shared memory
             st = lib.spite_gemm_stream(C.byref(p), max_rows_per_group, 1, 1, blocks, smem, splits, None, C.c_longlong(0),
                                        None, 0, C.c_void_p(stream))
@@ -806,17 +813,20 @@ class CudaKernels(KernelSet):
             C.c_longlong(n_floats), C.c_void_p(_ptr(tickets)), self._tickets_n, C.c_void_p(stream))
 
     def _stream_plan(self, M: int, N: int, K: int, n_groups: int, swiglu: bool, max_rows_per_group: int, grouped: bool, even_groups: bool):
-        """(shared memory per block, resident blocks, token columns, k slices, k splits) for a product of M rows (in `n_groups` groups if `grouped`)."""
+        """(shared memory per block, resident blocks, token columns, k slices, k splits, whether the splits may be one cluster) for a product of M
+        rows (in `n_groups` groups if `grouped`)."""
         groups, rows = min(n_groups, M) if grouped else 1, max_rows_per_group if even_groups else M
         # how many groups have tokens: all of them, or as many as rows that fall on them at random reach
         likely = groups if even_groups or groups == 1 else n_groups * (1.0 - (1.0 - 1.0 / n_groups) ** M)
         deep = not grouped or rows <= 3 or (rows <= 8 and likely * N * K * (4 if swiglu else 2) < self.stream_deep_bytes)
-        smem, blocks = self.stream_shape[0 if deep else 1]
+        ring = 0 if deep else 1
+        smem, blocks = self.stream_shape[ring]
         nt = 8 if max_rows_per_group <= 8 else 16 if max_rows_per_group <= 16 else 32
-        slices, splits = self.stream_force or stream_cut(
-            N, K, likely, groups, swiglu, blocks, smem, nt, 4 if nt > 16 else 8,
-            self.stream_cluster_max_splits if rows <= self.stream_cluster_max_rows else 0, **self.stream_costs)
-        return smem, blocks, nt, slices, splits
+        most = self.stream_cluster_max_splits[0 if self.stream_force else ring] if rows <= self.stream_cluster_max_rows else 0
+        lone, lone_slices = self.stream_lone_rates[ring]
+        slices, splits = self.stream_force or stream_cut(N, K, likely, groups, swiglu, blocks, smem, nt, 4 if nt > 16 else 8, most, lone_rate=lone,
+                                                         lone_rate_slices=lone_slices, **self.stream_costs)
+        return smem, blocks, nt, slices, splits, slices == 1 and 2 <= splits <= most
 
     def attention_tc_error(self) -> int:
         """Error code left by a tcgen05 attention block that gave up waiting (0: none); clears it. Synchronises."""
