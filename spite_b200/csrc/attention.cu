@@ -86,8 +86,8 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(const QkPrepareParams p
         }
     }
 
-    // (Measured and not kept: a warp loading four heads before working on the first, 61 against 33 us for 2,048
-    // tokens of 56 heads; one head a warp with more blocks, 51 us.)
+    // (Measured and not kept in this kernel, which moves pairs: a warp loading four heads before working on the first, 61 against 33 us for
+    // 2,048 tokens of 56 heads; one head a warp with more blocks, 51 us.  With 16-byte words it pays: qk_prepare_vec_kernel below.)
     const bool norm = p.qk_norm_eps > 0.f;
     const bool norm_first = norm && p.norm_before_rotation;
     const float norm_n = (float)(p.norm_dim > 0 ? p.norm_dim : hd);

@@ -603,8 +603,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                     // Three of sixteen pairs go through the multiply-add units instead (not on a window's edge or the diagonal, where a
                     // masked key must get 0), and the turn is passed on a quarter before the end, so that the other row tile's first
-                    // exponentials follow the last ones here.  us, 2,048 tokens behind 6,144, 40 heads: 343; turn passed early 336;
-                    // one pair in 4 317; both 310; 3 in 16 307; one pair in 2, 3 328, 327; without turns 324.
+                    // exponentials follow the last ones here.  us, the kernel alone in a loop, cut, 2,048 tokens behind 6,144, 40 heads: 343; turn
+                    // passed early 336; one pair in 4 317; both 310; 3 in 16 307; one pair in 2, 3 328, 327; without turns 324.  (A polynomial that
+                    // passed over NaN; with the one above 1.3 % more.  With L2 flushed between the calls 320 and 325.)
                     unsigned packed[BN / 2];
                     f2 sum2[4] = {0ull, 0ull, 0ull, 0ull};
                     const f2 scale2 = pack2(scale, scale), neg_m2 = pack2(neg_m, neg_m);
